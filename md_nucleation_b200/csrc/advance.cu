@@ -49,6 +49,17 @@ using namespace mdn;
 
 namespace {
 
+/* taper weight, and the atom's kind in one word: type (bits 0-6), the
+ * Born-Mayer-Huggins row of an ion atom (bit 7), vapor slot + 1 (bits 8-31, 0
+ * for ion atoms), so that a pair reads both with one 8-byte access */
+struct AtomTag {
+  float w;
+  unsigned k;
+};
+__device__ __forceinline__ int tag_type(unsigned k) { return (int)(k & 127u); }
+__device__ __forceinline__ int tag_bmh(unsigned k) { return (int)((k >> 7) & 1u); }
+__device__ __forceinline__ int tag_slot(unsigned k) { return (int)(k >> 8) - 1; }
+
 /* pointers into the dynamic shared memory of a CTA */
 struct Core {
   double* x;        /* [3*nc] positions                        */
@@ -57,12 +68,9 @@ struct Core {
   long long* acc;   /* [3*nc] this CTA's fixed-point force sums */
   unsigned* chunk;  /* [9*nc] the same sums in 32-bit chunks (acc_add) */
   float4* pos;      /* [nc] (x - ion centre, charge), FP32     */
-  float* w;         /* [nc] taper weight                       */
-  int* type;        /* [nc] atom type                          */
-  int* mol;         /* [nc] -1 for ion atoms, else vapor slot  */
+  AtomTag* tag;     /* [nc] taper weight and kind              */
   unsigned* excl;   /* AMBER exclusions, n_ion rows            */
-  float* ljA;       /* [nt*nt] 48 eps s^12                     */
-  float* ljB;       /* [nt*nt] 24 eps s^6                      */
+  float2* lj;       /* [nt*nt] 48 eps s^12, 24 eps s^6         */
   double* c2;       /* [nt] 0.5*dt*4.184e-4 / mass             */
   int* vcolor;      /* scratch                                 */
 };
@@ -125,9 +133,8 @@ __device__ __forceinline__ void load_ion(Ctx& x) {
       x.c.v[3 * i + k] = a->ion_v[3 * g + k];
       x.c.f[3 * i + k] = a->ion_f[3 * g + k];
     }
-    x.c.type[i] = x.ib[P->o_ion_type + i];
-    x.c.mol[i] = -1;
-    x.c.w[i] = 1.0f;
+    x.c.tag[i].w = 1.0f;
+    x.c.tag[i].k = (unsigned)x.ib[P->o_ion_type + i] | (x.ib[P->o_ion_bmh + i] ? 128u : 0u);
   }
 }
 
@@ -146,9 +153,8 @@ __device__ __forceinline__ void load_vapor(Ctx& x) {
       x.c.v[3 * i + k] = a->vslab_v[3 * g + k];
       x.c.f[3 * i + k] = a->vslab_f[3 * g + k];
     }
-    x.c.type[i] = x.ib[P->o_vap_type + at];
-    x.c.mol[i] = s;
-    x.c.w[i] = a->vslab_w[g];
+    x.c.tag[i].w = a->vslab_w[g];
+    x.c.tag[i].k = (unsigned)x.ib[P->o_vap_type + at] | ((unsigned)(s + 1) << 8);
   }
 }
 
@@ -174,7 +180,7 @@ __device__ __forceinline__ void store_core(Ctx& x) {
       a->vslab_v[3 * g + k] = x.c.v[3 * i + k];
       a->vslab_f[3 * g + k] = x.c.f[3 * i + k];
     }
-    a->vslab_w[g] = x.c.w[i];
+    a->vslab_w[g] = x.c.tag[i].w;
   }
 }
 
@@ -183,7 +189,7 @@ __device__ __forceinline__ void store_core(Ctx& x) {
 /* ------------------------------------------------------------------------- */
 __device__ __forceinline__ void core_kick(Ctx& x) {
   for (int i = threadIdx.x; i < x.n_core; i += blockDim.x) {
-    double c2 = x.c.c2[x.c.type[i]];
+    double c2 = x.c.c2[tag_type(x.c.tag[i].k)];
     for (int k = 0; k < 3; k++) x.c.v[3 * i + k] += x.c.f[3 * i + k] * c2;
   }
 }
@@ -195,7 +201,7 @@ __device__ __forceinline__ double ion_temperature(Ctx& x) {
   if (threadIdx.x < 32) {
     double K = 0;
     for (int i = threadIdx.x; i < P->n_ion; i += 32) {
-      double m = x.db[P->d_mass + x.c.type[i]];
+      double m = x.db[P->d_mass + tag_type(x.c.tag[i].k)];
       K += x.c.v[3 * i] * x.c.v[3 * i] * m;
       K += x.c.v[3 * i + 1] * x.c.v[3 * i + 1] * m;
       K += x.c.v[3 * i + 2] * x.c.v[3 * i + 2] * m;
@@ -444,7 +450,7 @@ __device__ __forceinline__ void ion_centre(Ctx& x) {
   if (threadIdx.x < 32) {
     double s[6] = {0, 0, 0, 0, 0, 0};
     for (int i = threadIdx.x; i < P->n_ion; i += 32) {
-      double m = x.db[P->d_mass + x.c.type[i]];
+      double m = x.db[P->d_mass + tag_type(x.c.tag[i].k)];
       for (int k = 0; k < 3; k++) {
         s[k] += x.c.x[3 * i + k] * m;
         s[3 + k] += x.c.v[3 * i + k] * m;
@@ -466,7 +472,7 @@ __device__ __forceinline__ void ion_centre_exact(Ctx& x) {
   if (threadIdx.x == 0) {
     double s[6] = {0, 0, 0, 0, 0, 0};
     for (int i = 0; i < P->n_ion; i++) {
-      double m = x.db[P->d_mass + x.c.type[i]];
+      double m = x.db[P->d_mass + tag_type(x.c.tag[i].k)];
       for (int k = 0; k < 3; k++) {
         s[k] += x.c.x[3 * i + k] * m;
         s[3 + k] += x.c.v[3 * i + k] * m;
@@ -500,8 +506,8 @@ __device__ __forceinline__ void core_weights_pos(Ctx& x, bool weights) {
   const double* com = x.D->ion_com;
   for (int i = threadIdx.x; i < x.n_core; i += blockDim.x) {
     if (i >= P->n_ion) {
-      if (x.c.w[i] < 0.0f) x.c.w[i] = 0.0f;
-      else if (weights) x.c.w[i] = (float)taper(P, com, x.c.x + 3 * i);
+      if (x.c.tag[i].w < 0.0f) x.c.tag[i].w = 0.0f;
+      else if (weights) x.c.tag[i].w = (float)taper(P, com, x.c.x + 3 * i);
     }
     double q = i < P->n_ion ? x.db[P->d_ion_q + i] : x.db[P->d_vap_q + (i - P->n_ion) % P->a_v];
     x.c.pos[i] = make_float4((float)(x.c.x[3 * i] - com[0]), (float)(x.c.x[3 * i + 1] - com[1]),
@@ -719,7 +725,7 @@ __device__ __forceinline__ double born_d(double r2, int ti, int tj, double qq) {
 
 /* taper weight of core atom i in FP64: the float copy is exact at 0 and 1 */
 __device__ __forceinline__ double weight_d(const Ctx& x, int i) {
-  const float w = x.c.w[i];
+  const float w = x.c.tag[i].w;
   if (w == 0.0f || w == 1.0f) return (double)w;
   return taper(x.P, x.D->ion_com, x.c.x + 3 * i);
 }
@@ -766,161 +772,173 @@ __device__ __forceinline__ bool term_on(const Ctx& x, unsigned bit) {
  * distinct j (no bank conflicts), and it keeps the reaction on that j in a
  * register that moves one lane down after every step: after 32 steps lane l
  * holds the whole reaction on j = 32 jb + l.  Diagonal tiles take steps
- * 1..15 and half of step 16.  Each side is summed over the tile's steps in
- * the pair precision, in that fixed order, and reaches the core sums once
- * per tile as a 64-bit integer (one conversion per atom and tile instead of
- * one per pair, 32-bit shuffles for the reactions), so the result does not
- * depend on the launch shape. */
-template <bool FP64>
-__device__ __forceinline__ void core_pairs_t(Ctx& x, bool eflag) {
+ * 1..15 and half of step 16, then the reactions move the rest of the way in
+ * one shuffle.  Each side is summed over the tile's steps in the pair
+ * precision, in that fixed order, and reaches the core sums once per tile as
+ * a 64-bit integer, so the result does not depend on the launch shape.
+ *
+ * What bounds it: the dependent chain of one pair (a warp runs one tile, and
+ * a small core has fewer tiles than the SM has warps).  So which pairs count
+ * (the exclusions, the ion-vapor and vapor-vapor switches, the atoms of one
+ * molecule, the diagonal's half) is worked out once per tile as one bit per
+ * step, the LJ + Coulomb form is the same for all three kinds (an ion atom's
+ * weight is 1), and the steps carry no branch on the kind, so that the
+ * compiler interleaves several of them.  Against a branch on the kind per
+ * pair: 36.0 -> 32.2 ms per 100 steps of 256 mixed replicas (tuned launch),
+ * 2.23 -> 1.85 ms on one 13-atom core, bit-identical results. */
+template <bool FP64, bool E>
+__device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk, long long& e_ion, long long& e_vi,
+                                          long long& e_vv) {
   const RepParams* P = x.P;
-  const int ni = P->n_ion, nc = x.n_core, nt = P->n_types;
+  const int ni = P->n_ion, nc = x.n_core, nt = P->n_types, av = P->a_v;
   const bool amber = term_on(x, MDN_I_AMBER), bmh = term_on(x, MDN_I_BMH);
   const bool vi = term_on(x, MDN_I_VI), vv = term_on(x, MDN_I_VV);
-  if (!(amber || bmh || vi || vv)) return;
-  const float qqf = (float)P->qqrd2e;
-  const int nblk = (nc + 31) >> 5;
-  const int tiles = nblk * (nblk + 1) / 2;
+  const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int nwb = blockDim.x >> 5;
-  const int* bmht = x.ib + P->o_ion_bmh;
-  long long e_ion = 0, e_vi = 0, e_vv = 0;
-  for (int t = x.rank * nwb + (threadIdx.x >> 5); t < tiles; t += x.C * nwb) {
-    int ib = 0, rem = t;
-    while (rem >= nblk - ib) {
-      rem -= nblk - ib;
-      ib++;
-    }
-    const int jb = ib + rem;
-    const bool diag = ib == jb;
-    const int i = ib * 32 + lane;
-    const bool act = i < nc;
-    const int ii = act ? i : 0;
-    const float4 pi = x.c.pos[ii];
-    const int ti = x.c.type[ii], mi = x.c.mol[ii];
-    const float wi = x.c.w[ii];
-    const bool iion = ii < ni;
-    const int bi = (bmh && iion) ? bmht[ii] : 0;
-    double xd[3] = {0, 0, 0}, wid = 1.0, qid = 0.0;
-    if constexpr (FP64) {
-      for (int k = 0; k < 3; k++) xd[k] = x.c.x[3 * ii + k];
-      wid = weight_d(x, ii);
-      qid = charge_d(x, ii);
-    }
-    /* the tile's sums in the pair arithmetic's own precision, in a fixed
-     * order (the tile's steps), turned into fixed point once per atom */
-    using Acc = typename std::conditional<FP64, double, float>::type;
-    Acc F0 = 0, F1 = 0, F2 = 0, R0 = 0, R1 = 0, R2 = 0;
-    for (int s = 0; s < 32; s++) {
-      const int j = jb * 32 + ((lane + s) & 31);
-      bool take = act && j < nc;
-      if (diag) take = take && s != 0 && (s < 16 || (s == 16 && lane < 16));
-      if (take) {
-        const float4 pj = x.c.pos[j];
-        const int tj = x.c.type[j], mj = x.c.mol[j];
-        const float wj = x.c.w[j];
-        const bool jion = j < ni;
-        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        float fp = 0.0f;
-        bool any = false;
-        int bucket = 0;
-        if (iion && jion) {
-          const bool ex = amber && ((x.c.excl[i * P->excl_words + (j >> 5)] >> (j & 31)) & 1u);
-          if (amber && !ex) {
-            float ee;
-            fp += lj_coul(r2, x.c.ljA[ti * nt + tj], x.c.ljB[ti * nt + tj], qqf * pi.w * pj.w, true, &ee);
-            any = true;
-          }
-          if (bmh) {
-            float ee;
-            fp += born(r2, bi, bmht[j], qqf * pi.w * pj.w, &ee);
-            any = true;
-          }
-          bucket = 1;
-        } else if (iion != jion) {
-          if (vi) {
-            float ee;
-            fp = lj_coul(r2, x.c.ljA[ti * nt + tj], x.c.ljB[ti * nt + tj], qqf * pi.w * pj.w, true, &ee) * (wi * wj);
-            any = true;
-            bucket = 2;
-          }
-        } else if (mi != mj) {
-          if (vv) {
-            float ee;
-            fp = lj_coul(r2, x.c.ljA[ti * nt + tj], x.c.ljB[ti * nt + tj], qqf * pi.w * pj.w, true, &ee) * (wi * wj);
-            any = true;
-            bucket = 3;
-          }
-        }
-        if (any) {
-          Acc fx, fy, fz;
-          if constexpr (FP64) {
-            /* the same terms in FP64 from the FP64 positions and tables */
-            const double ex = xd[0] - x.c.x[3 * j], ey = xd[1] - x.c.x[3 * j + 1], ez = xd[2] - x.c.x[3 * j + 2];
-            const double R2d = ex * ex + ey * ey + ez * ez;
-            const double qq = P->qqrd2e * qid * charge_d(x, j);
-            const double Ad = x.db[P->d_ljA + ti * nt + tj], Bd = x.db[P->d_ljB + ti * nt + tj];
-            double fd = 0.0;
-            if (bucket == 1) {
-              if (amber && !((x.c.excl[i * P->excl_words + (j >> 5)] >> (j & 31)) & 1u))
-                fd += lj_coul_d(R2d, Ad, Bd, qq, true);
-              if (bmh) fd += born_d(R2d, bi, bmht[j], qq);
-            } else {
-              fd = lj_coul_d(R2d, Ad, Bd, qq, true) * (wid * weight_d(x, j));
-            }
-            fx = fd * ex;
-            fy = fd * ey;
-            fz = fd * ez;
-          } else {
-            fx = fp * dx;
-            fy = fp * dy;
-            fz = fp * dz;
-          }
-          F0 += fx; F1 += fy; F2 += fz;
-          R0 -= fx; R1 -= fy; R2 -= fz;
-          if (eflag) {
-            const double R2e = r2d(x.c.x + 3 * i, x.c.x + 3 * j);
-            const double qi = i < ni ? x.db[P->d_ion_q + i] : x.db[P->d_vap_q + (i - ni) % P->a_v];
-            const double qj = j < ni ? x.db[P->d_ion_q + j] : x.db[P->d_vap_q + (j - ni) % P->a_v];
-            const double qq = P->qqrd2e * qi * qj;
-            double ed = 0;
-            if (bucket == 1) {
-              if (amber && !((x.c.excl[i * P->excl_words + (j >> 5)] >> (j & 31)) & 1u))
-                ed += lj_coul_energy(R2e, x.db[P->d_ljA + ti * nt + tj], x.db[P->d_ljB + ti * nt + tj], qq);
-              if (bmh) ed += born_energy(R2e, bi, bmht[j], qq);
-              e_ion += efixd(ed);
-            } else {
-              ed = lj_coul_energy(R2e, x.db[P->d_ljA + ti * nt + tj], x.db[P->d_ljB + ti * nt + tj], qq);
-              if (bucket == 2) e_vi += efixd(ed);
-              else e_vv += efixd(ed);
-            }
-          }
-        }
+  int ib = 0, rem = t;
+  while (rem >= nblk - ib) {
+    rem -= nblk - ib;
+    ib++;
+  }
+  const int jb = ib + rem, j0 = jb * 32;
+  const bool diag = ib == jb;
+  const int i = ib * 32 + lane;
+  const bool act = i < nc;
+  const int ii = act ? i : 0;
+  const AtomTag gi = x.c.tag[ii];
+  const int rowi = tag_type(gi.k) * nt;
+  /* the lowest n bits */
+  auto low = [](int n) -> unsigned { return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : (1u << n) - 1u; };
+  /* bit jl of on: the pair (i, j0 + jl) has the LJ + Coulomb form; of born:
+   * the Born-Mayer-Huggins form */
+  unsigned on = 0, born_on = 0;
+  if (act) {
+    const unsigned live = low(nc - j0), ionj = low(ni - j0);
+    if (ii < ni) {
+      if (amber) on |= ionj & ~(j0 < ni ? x.c.excl[ii * P->excl_words + jb] : 0u);
+      if (vi) on |= live & ~ionj;
+      if (bmh) born_on = ionj;
+    } else {
+      if (vi) on |= ionj;
+      if (vv) {
+        const int m0 = ni + tag_slot(gi.k) * av - j0; /* the molecule's own atoms */
+        on |= live & ~ionj & ~(low(m0 + av) & ~low(m0));
       }
-      R0 = __shfl_sync(0xffffffffu, R0, (lane + 1) & 31);
-      R1 = __shfl_sync(0xffffffffu, R1, (lane + 1) & 31);
-      R2 = __shfl_sync(0xffffffffu, R2, (lane + 1) & 31);
     }
-    auto fix = [](Acc v) -> long long {
-      if constexpr (FP64) return fixd(v);
-      else return fixf(v);
-    };
-    if (act && (F0 != 0 || F1 != 0 || F2 != 0)) {
-      const long long F[3] = {fix(F0), fix(F1), fix(F2)};
-      acc_add(x, i, F);
-    }
-    const int jj = jb * 32 + lane;
-    if (jj < nc && (R0 != 0 || R1 != 0 || R2 != 0)) {
-      const long long Rv[3] = {fix(R0), fix(R1), fix(R2)};
-      acc_add(x, jj, Rv);
+    /* rotated so that bit s is step s */
+    on = __funnelshift_r(on, on, lane);
+    born_on = __funnelshift_r(born_on, born_on, lane);
+    if (diag) {
+      const unsigned half = lane < 16 ? 0x1fffeu : 0xfffeu;
+      on &= half;
+      born_on &= half;
     }
   }
-  if (eflag) {
+  const unsigned any_on = __reduce_or_sync(FULL, on | born_on);
+  if (any_on == 0) return;
+  using Acc = typename std::conditional<FP64, double, float>::type;
+  Acc F0 = 0, F1 = 0, F2 = 0, R0 = 0, R1 = 0, R2 = 0;
+  float4 pi = make_float4(0, 0, 0, 0);
+  float qi = 0;
+  double xd[3] = {0, 0, 0}, wid = 1.0, qid = 0.0;
+  if constexpr (FP64 || E) {
+    for (int k = 0; k < 3; k++) xd[k] = x.c.x[3 * ii + k];
+    wid = FP64 ? weight_d(x, ii) : 1.0;
+    qid = P->qqrd2e * charge_d(x, ii);
+  }
+  if constexpr (!FP64) {
+    pi = x.c.pos[ii];
+    qi = (float)P->qqrd2e * pi.w;
+  }
+  auto step = [&](int s) {
+    const int jl = (lane + s) & 31;
+    const int j = j0 + jl < nc ? j0 + jl : 0;
+    const AtomTag gj = x.c.tag[j];
+    const int tt = rowi + tag_type(gj.k);
+    if constexpr (FP64) {
+      if (((on | born_on) >> s) & 1u) {
+        const double ex = xd[0] - x.c.x[3 * j], ey = xd[1] - x.c.x[3 * j + 1], ez = xd[2] - x.c.x[3 * j + 2];
+        const double R2d = ex * ex + ey * ey + ez * ez;
+        const double qq = qid * charge_d(x, j);
+        double fd = 0.0;
+        if ((on >> s) & 1u)
+          fd = lj_coul_d(R2d, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qq, true) * (wid * weight_d(x, j));
+        if ((born_on >> s) & 1u) fd += born_d(R2d, tag_bmh(gi.k), tag_bmh(gj.k), qq);
+        const double fx = fd * ex, fy = fd * ey, fz = fd * ez;
+        F0 += fx; F1 += fy; F2 += fz;
+        R0 -= fx; R1 -= fy; R2 -= fz;
+      }
+    } else {
+      const float4 pj = x.c.pos[j];
+      const float2 AB = x.c.lj[tt];
+      const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      const float qq = qi * pj.w;
+      float ee;
+      float fp = lj_coul(r2, AB.x, AB.y, qq, true, &ee) * (gi.w * gj.w);
+      fp = ((on >> s) & 1u) ? fp : 0.0f;
+      if ((born_on >> s) & 1u) fp += born(r2, tag_bmh(gi.k), tag_bmh(gj.k), qq, &ee);
+      if (((on | born_on) >> s) & 1u) {
+        const float fx = fp * dx, fy = fp * dy, fz = fp * dz;
+        F0 += fx; F1 += fy; F2 += fz;
+        R0 -= fx; R1 -= fy; R2 -= fz;
+      }
+    }
+    if constexpr (E) {
+      if (((on | born_on) >> s) & 1u) {
+        const double R2e = r2d(xd, x.c.x + 3 * j);
+        const double qq = qid * charge_d(x, j);
+        double ed = 0;
+        if ((on >> s) & 1u) ed += lj_coul_energy(R2e, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qq);
+        if ((born_on >> s) & 1u) ed += born_energy(R2e, tag_bmh(gi.k), tag_bmh(gj.k), qq);
+        const bool iion = ii < ni, jion = j < ni;
+        if (iion && jion) e_ion += efixd(ed);
+        else if (iion != jion) e_vi += efixd(ed);
+        else e_vv += efixd(ed);
+      }
+    }
+  };
+  const int s1 = diag ? 17 : 32;
+#pragma unroll 4
+  for (int s = 0; s < s1; s++) {
+    if ((any_on >> s) & 1u) step(s);
+    R0 = __shfl_sync(FULL, R0, (lane + 1) & 31);
+    R1 = __shfl_sync(FULL, R1, (lane + 1) & 31);
+    R2 = __shfl_sync(FULL, R2, (lane + 1) & 31);
+  }
+  if (diag) {
+    R0 = __shfl_sync(FULL, R0, (lane + 15) & 31);
+    R1 = __shfl_sync(FULL, R1, (lane + 15) & 31);
+    R2 = __shfl_sync(FULL, R2, (lane + 15) & 31);
+  }
+  auto fix = [](Acc v) -> long long {
+    if constexpr (FP64) return fixd(v);
+    else return fixf(v);
+  };
+  if (act && (F0 != 0 || F1 != 0 || F2 != 0)) {
+    const long long F[3] = {fix(F0), fix(F1), fix(F2)};
+    acc_add(x, i, F);
+  }
+  const int jj = j0 + lane;
+  if (jj < nc && (R0 != 0 || R1 != 0 || R2 != 0)) {
+    const long long Rv[3] = {fix(R0), fix(R1), fix(R2)};
+    acc_add(x, jj, Rv);
+  }
+}
+
+template <bool FP64, bool E>
+__device__ __forceinline__ void core_pairs_t(Ctx& x) {
+  const int nblk = (x.n_core + 31) >> 5;
+  const int tiles = nblk * (nblk + 1) / 2;
+  const int nwb = blockDim.x >> 5;
+  long long e_ion = 0, e_vi = 0, e_vv = 0;
+  for (int t = x.rank * nwb + (threadIdx.x >> 5); t < tiles; t += x.C * nwb)
+    core_tile<FP64, E>(x, t, nblk, e_ion, e_vi, e_vv);
+  if constexpr (E) {
     e_ion = warp_sum_ll(e_ion);
     e_vi = warp_sum_ll(e_vi);
     e_vv = warp_sum_ll(e_vv);
-    if (lane == 0) {
+    if ((threadIdx.x & 31) == 0) {
       energy_add(x, MDN_U_ION, e_ion);
       energy_add(x, MDN_U_VI, e_vi);
       energy_add(x, MDN_U_VV, e_vv);
@@ -938,7 +956,11 @@ constexpr bool kFP64Pairs = true;
 constexpr bool kFP64Pairs = false;
 #endif
 
-__device__ __forceinline__ void core_pairs(Ctx& x, bool eflag) { core_pairs_t<kFP64Pairs>(x, eflag); }
+__device__ __forceinline__ void core_pairs(Ctx& x, bool eflag) {
+  if (!(term_on(x, MDN_I_AMBER) || term_on(x, MDN_I_BMH) || term_on(x, MDN_I_VI) || term_on(x, MDN_I_VV))) return;
+  if (eflag) core_pairs_t<kFP64Pairs, true>(x);
+  else core_pairs_t<kFP64Pairs, false>(x);
+}
 
 /* MDN_GG_TERMS selects the gas-gas term: compiled into its own kernels
  * (advance_gg.cu, advance_gg_fp64.cu), absent from the others */
@@ -1281,7 +1303,7 @@ __device__ __forceinline__ void gas_gg_pass_t(Ctx& x, bool eflag, bool fresh) {
                         dz = (float)(X[3 * at + 2] - Y[2]);
             const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             float ee;
-            const float fp = lj_coul(r2, x.c.ljA[ta * nt + tb], x.c.ljB[ta * nt + tb], 0.0f, false, &ee) *
+            const float fp = lj_coul(r2, x.c.lj[ta * nt + tb].x, x.c.lj[ta * nt + tb].y, 0.0f, false, &ee) *
                              (float)(w[at] * wb);
             fx = fixf(fp * dx); fy = fixf(fp * dy); fz = fixf(fp * dz);
           }
@@ -1329,7 +1351,7 @@ template <bool FP64>
 __device__ __forceinline__ void gas_core_pair(const Ctx& x, const double* Xa, float3 ga, int ta, int j,
                                               long long* f) {
   const RepParams* P = x.P;
-  const int nt = P->n_types, tj = x.c.type[j];
+  const int nt = P->n_types, tj = tag_type(x.c.tag[j].k);
   if constexpr (FP64) {
     const double ex = Xa[0] - x.c.x[3 * j], ey = Xa[1] - x.c.x[3 * j + 1], ez = Xa[2] - x.c.x[3 * j + 2];
     const double fd = lj_coul_d(ex * ex + ey * ey + ez * ez, x.db[P->d_ljA + ta * nt + tj],
@@ -1340,7 +1362,8 @@ __device__ __forceinline__ void gas_core_pair(const Ctx& x, const double* Xa, fl
     const float dx = ga.x - pj.x, dy = ga.y - pj.y, dz = ga.z - pj.z;
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     float ee;
-    const float fp = lj_coul(r2, x.c.ljA[ta * nt + tj], x.c.ljB[ta * nt + tj], 0.0f, false, &ee);
+    const float2 AB = x.c.lj[ta * nt + tj];
+    const float fp = lj_coul(r2, AB.x, AB.y, 0.0f, false, &ee);
     f[0] = fixf(fp * dx); f[1] = fixf(fp * dy); f[2] = fixf(fp * dz);
   }
 }
@@ -1355,7 +1378,7 @@ template <int AG, bool FP64>
 __device__ __forceinline__ void near_partner(Ctx& x, const double* X, const float3* gp, const int* gtype, int j,
                                              bool eflag, long long (*F)[3], long long& e) {
   const RepParams* P = x.P;
-  const int nt = P->n_types, tj = x.c.type[j];
+  const int nt = P->n_types, tj = tag_type(x.c.tag[j].k);
   long long R[3] = {0, 0, 0};
 #pragma unroll
   for (int at = 0; at < AG; at++) {
@@ -2073,7 +2096,7 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
         double sx[3] = {0, 0, 0}, sv[3] = {0, 0, 0};
         for (int at = 0; at < av; at++) {
           int i = P->n_ion + s * av + at;
-          double mm = x.db[P->d_mass + x.c.type[i]];
+          double mm = x.db[P->d_mass + tag_type(x.c.tag[i].k)];
           for (int k = 0; k < 3; k++) {
             sx[k] += x.c.x[3 * i + k] * mm;
             sv[k] += x.c.v[3 * i + k] * mm;
@@ -2389,12 +2412,9 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     x.c.v = (double*)take(sizeof(double) * 3 * nc);
     x.c.f = (double*)take(sizeof(double) * 3 * nc);
     x.c.pos = (float4*)take(sizeof(float4) * nc);
-    x.c.w = (float*)take(sizeof(float) * nc);
-    x.c.type = (int*)take(sizeof(int) * nc);
-    x.c.mol = (int*)take(sizeof(int) * nc);
+    x.c.tag = (AtomTag*)take(sizeof(AtomTag) * nc);
     x.c.excl = (unsigned*)take(sizeof(unsigned) * a.excl_cap);
-    x.c.ljA = (float*)take(sizeof(float) * a.nt_cap * a.nt_cap);
-    x.c.ljB = (float*)take(sizeof(float) * a.nt_cap * a.nt_cap);
+    x.c.lj = (float2*)take(sizeof(float2) * a.nt_cap * a.nt_cap);
     x.c.c2 = (double*)take(sizeof(double) * a.nt_cap);
   }
   /* the chunk sums start at zero and every core_reduce leaves them so */
@@ -2427,10 +2447,8 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     }
     /* tables */
     const int nt = sP.n_types;
-    for (int q = threadIdx.x; q < nt * nt; q += blockDim.x) {
-      x.c.ljA[q] = (float)x.db[sP.d_ljA + q];
-      x.c.ljB[q] = (float)x.db[sP.d_ljB + q];
-    }
+    for (int q = threadIdx.x; q < nt * nt; q += blockDim.x)
+      x.c.lj[q] = make_float2((float)x.db[sP.d_ljA + q], (float)x.db[sP.d_ljB + q]);
     for (int q = threadIdx.x; q < nt; q += blockDim.x) x.c.c2[q] = x.db[sP.d_c2 + q];
     for (int q = threadIdx.x; q < sP.n_ion * sP.excl_words; q += blockDim.x) x.c.excl[q] = (unsigned)x.ib[sP.o_excl + q];
     load_ion(x);

@@ -227,9 +227,9 @@ size_t smem_bytes(int nc, int nt, int excl) {
   s += align16(sizeof(unsigned) * 9 * nc);
   s += 3 * align16(sizeof(double) * 3 * nc);
   s += align16(sizeof(float4) * nc);
-  s += 3 * align16(sizeof(int) * nc);
+  s += align16(8 * (size_t)nc); /* AtomTag */
   s += align16(sizeof(unsigned) * excl);
-  s += 2 * align16(sizeof(float) * nt * nt);
+  s += align16(sizeof(float2) * nt * nt);
   s += align16(sizeof(double) * nt);
   return s;
 }
