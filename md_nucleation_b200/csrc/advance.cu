@@ -17,9 +17,9 @@
  *     a gas molecule interacts only with the core: molecules whose gas-ion /
  *     gas-vapor lists are empty ("far") are advanced by one thread in a single
  *     pass (kick, drift, intramolecular force, kick); "near" molecules are
- *     handled by one thread each too, walking the molecule's lists (about one
- *     entry per molecule), with shared-memory fixed-point atomics for the
- *     reaction on the core.
+ *     sorted by their number of partners and taken 32 to a warp (build_near,
+ *     near_group), with shared-memory fixed-point atomics for the reaction on
+ *     the core.
  *
  * Each step follows MD::verlet (src/verlet.cpp:20-39) exactly:
  *   kick (MD::velocity_calculation), [MD::velocity_scaling], drift with
@@ -1393,176 +1393,271 @@ __device__ __forceinline__ void near_partner(Ctx& x, const double* X, const floa
   acc_add(x, j, R);
 }
 
-/* A near molecule with more partners than this has them spread over a warp. */
-constexpr int kNearHeavy = 16;
+/* exchange one int per CTA across the cluster: returns the prefix before this
+ * rank and the total */
+__device__ __forceinline__ void cluster_prefix(Ctx& x, cg::cluster_group& cl, int* slot_in_smem, int mine, int* before,
+                               int* total) {
+  if (threadIdx.x == 0) *slot_in_smem = mine;
+  cl.sync();
+  int b = 0, t = 0;
+  for (int k = 0; k < x.C; k++) {
+    int v = *cl.map_shared_rank(slot_in_smem, k);
+    if (k < x.rank) b += v;
+    t += v;
+  }
+  *before = b;
+  *total = t;
+  cl.sync();
+}
 
-/* near molecules (those with a gas-ion or gas-vapor list entry).  Partner
- * counts (gas-ion entries, plus gas-vapor entries times the vapor atoms each
- * reaches) are uneven: the few dozen to few hundred molecules next to a
- * large ion have 30-100 gas-ion entries, the thousands near vapor 1-13
- * gas-vapor partners.  So, first, each warp takes 32 of the CTA's near
- * molecules at a time and spreads the partners of those with more than
- * kNearHeavy over its lanes, one molecule after another, their force summed
- * by shuffles and parked, as 64-bit integers, in the molecule's slab force
- * rows.  Then one thread per near molecule walks the other molecules'
- * lists (the lanes of a warp run through their molecules independently, so
- * uneven light walks even out over a lane's several molecules), takes the
- * parked force of the heavy ones, and finishes each molecule: its force,
- * the gas-gas and intramolecular terms and the second kick.  Each reaction
- * goes to the core sums by shared 32-bit integer atomics on exact chunks
- * (acc_add); all sums are integers, so neither the split nor the order
- * changes the result. */
-template <int AG, bool FP64>
-__device__ __forceinline__ void gas_near_pass_t(Ctx& x, bool eflag, bool kick) {
+/* A near molecule with more partners than this has them spread over 8 lanes. */
+constexpr int kNearHeavy = 16;
+constexpr int kNearBins = kNearHeavy + 1; /* bin 0: heavy; bin b: 17 - b partners */
+
+/* core atoms a gas-vapor entry reaches in its vapor molecule */
+__device__ __forceinline__ int gv_reach(const RepParams* P) {
+  return (P->quirks & MDN_Q_GV_GAS_COUNT) ? min(P->a_g, P->a_v) : P->a_v;
+}
+
+/* The near molecules (those with a gas-ion or gas-vapor entry) of this CTA's
+ * slab partition as records {slab slot, first item, items, 0}, most partners
+ * first, and their partners as core atom indices: `near_item` holds a heavy
+ * molecule's partners one after another, and those of a group of 32 light
+ * records interleaved (entry e of the group's lane l at 32 e + l), so that a
+ * warp reads one line per step and its lanes have (nearly) the same number
+ * of steps.  The records of a CTA start at its partition's first slot, its
+ * items where the lower ranks' end; they depend on the cluster size, which
+ * RepDyn::near_C remembers, and are built again when a launch uses another.
+ * Built at a rebuild (every few hundred steps); all threads of the cluster. */
+__device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   const RepParams* P = x.P;
   const KArgs* a = x.a;
-  constexpr int ag = AG;
-  const int av = P->a_v, par = x.D->parity, ni = P->n_ion;
-  const bool gi = term_on(x, MDN_I_GI), gv = term_on(x, MDN_I_GV);
-  const bool intra = term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
-  const bool gg = kGG && term_on(x, MDN_I_GG) && P->ggl_cap > 0;
-  const int nj = (P->quirks & MDN_Q_GV_GAS_COUNT) ? min(ag, av) : av;
+  const int par = x.D->parity, ni = P->n_ion, av = P->a_v, nj = gv_reach(P);
   int lo, hi;
   partition(x, x.D->n_gas_in, &lo, &hi);
-  /* this CTA's range of the (ascending) near list */
-  const int* nl = a->near_list + P->near_off;
-  const int nn = x.D->n_near;
-  int b0 = 0, b1 = nn;
-  {
-    int L = 0, H = nn;
-    while (L < H) { int M = (L + H) >> 1; if (nl[M] < lo) L = M + 1; else H = M; }
-    b0 = L;
-    L = b0; H = nn;
-    while (L < H) { int M = (L + H) >> 1; if (nl[M] < hi) L = M + 1; else H = M; }
-    b1 = L;
-  }
-  int gtype[AG];
-  double c2[AG];
-#pragma unroll
-  for (int at = 0; at < ag; at++) {
-    gtype[at] = x.ib[P->o_gas_type + at];
-    c2[at] = x.c.c2[gtype[at]];
-  }
-  const double* com = x.D->ion_com;
-  long long egi = 0, egv = 0, eintra = 0;
-  /* heavy molecules, spread over a warp */
-  {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    for (int c0 = b0 + (int)(threadIdx.x & ~31u); c0 < b1; c0 += blockDim.x) {
-      const int e = c0 + lane;
-      int items = 0;
-      if (e < b1) {
-        const size_t ms = gmol(P, par, nl[e]);
-        items = (gi ? (int)a->gil_n[ms] : 0) + (gv ? (int)a->gvl_n[ms] * nj : 0);
-      }
-      for (unsigned heavy = __ballot_sync(FULL, items > kNearHeavy); heavy; heavy &= heavy - 1) {
-        const int so = nl[c0 + __ffs(heavy) - 1];
-        const size_t ms = gmol(P, par, so);
-        const int ngo = gi ? a->gil_n[ms] : 0, nvo = gv ? a->gvl_n[ms] : 0;
-        const int sgo = a->near_gi[ms], svo = a->near_gv[ms];
-        float3 gpo[AG];
-        double Xo[3 * AG];
-#pragma unroll
-        for (int at = 0; at < AG; at++) {
-          const size_t g = gatom(P, par, so, at);
-#pragma unroll
-          for (int k = 0; k < 3; k++) Xo[3 * at + k] = a->slab_x[3 * g + k];
-          gpo[at] = make_float3((float)(Xo[3 * at] - com[0]), (float)(Xo[3 * at + 1] - com[1]),
-                                (float)(Xo[3 * at + 2] - com[2]));
-        }
-        long long Fo[AG][3];
-#pragma unroll
-        for (int at = 0; at < AG; at++) Fo[at][0] = Fo[at][1] = Fo[at][2] = 0;
-        const int n_it = ngo + nvo * nj;
-        for (int it = lane; it < n_it; it += 32) {
-          if (it < ngo) {
-            near_partner<AG, FP64>(x, Xo, gpo, gtype, (int)a->gil[P->gil_off + sgo + it], eflag, Fo, egi);
-          } else {
-            const int t = it - ngo, ent = t / nj, b = t - ent * nj;
-            near_partner<AG, FP64>(x, Xo, gpo, gtype, ni + (int)a->gvl[P->gvl_off + svo + ent] * av + b, eflag,
-                                   Fo, egv);
-          }
-        }
-#pragma unroll
-        for (int at = 0; at < AG; at++) {
-          const size_t g = gatom(P, par, so, at);
-#pragma unroll
-          for (int k = 0; k < 3; k++) {
-            const long long v = warp_sum_ll(Fo[at][k]);
-            if (lane == 0) a->slab_f[3 * g + k] = __longlong_as_double(v);
-          }
-        }
-      }
-    }
+  int* const hist = x.cand;        /* [kNearBins] molecules per bin, then first record  */
+  int* const cur = x.cand + 32;    /* [kNearBins] next record                           */
+  int* const heavy = x.cand + 64;  /* partners of all heavy molecules, and the next one */
+  __syncthreads();
+  if (threadIdx.x < kNearBins) hist[threadIdx.x] = 0;
+  if (threadIdx.x < 2) heavy[threadIdx.x] = 0;
+  __syncthreads();
+  auto items_of = [&](size_t ms) {
+    return a->near_gi[ms] < 0 ? 0 : (int)a->gil_n[ms] + (int)a->gvl_n[ms] * nj;
+  };
+  for (int s = lo + (int)threadIdx.x; s < hi; s += blockDim.x) {
+    const int c = items_of(gmol(P, par, s));
+    if (c == 0) continue;
+    atomicAdd(&hist[c > kNearHeavy ? 0 : kNearHeavy + 1 - c], 1);
+    if (c > kNearHeavy) atomicAdd(&heavy[0], c);
   }
   __syncthreads();
-  for (int e = b0 + (int)threadIdx.x; e < b1; e += blockDim.x) {
-    const int s = nl[e];
+  if (threadIdx.x == 0) {
+    int run = 0, items = heavy[0];
+    const int nh = hist[0];
+    for (int b = 0; b < kNearBins; b++) {
+      const int n = hist[b];
+      hist[b] = cur[b] = run;
+      /* 32-record groups that start in this bin take its count of entries */
+      if (b > 0) items += 32 * (kNearHeavy + 1 - b) * (((run + n - nh + 31) >> 5) - ((run - nh + 31) >> 5));
+      run += n;
+    }
+    hist[kNearBins] = run;
+    x.iscr[56] = nh;
+    x.iscr[57] = run;
+    heavy[2] = items;
+    x.D->near_C = x.C;
+  }
+  __syncthreads();
+  int base, tot;
+  cluster_prefix(x, cl, &x.iscr[47], heavy[2], &base, &tot);
+  const int nh = x.iscr[56], light0 = base + heavy[0];
+  int4* const rec = a->near_rec + P->near_off + lo;
+  unsigned short* const item = a->near_item + P->nit_off;
+  for (int s = lo + (int)threadIdx.x; s < hi; s += blockDim.x) {
     const size_t ms = gmol(P, par, s);
-    float3 gp[AG];
-    double X[3 * AG];
-#pragma unroll
-    for (int at = 0; at < ag; at++) {
-      size_t g = gatom(P, par, s, at);
-      for (int k = 0; k < 3; k++) X[3 * at + k] = a->slab_x[3 * g + k];
-      gp[at] = make_float3((float)(X[3 * at] - com[0]), (float)(X[3 * at + 1] - com[1]),
-                           (float)(X[3 * at + 2] - com[2]));
-    }
-    long long F[AG][3];
-#pragma unroll
-    for (int at = 0; at < AG; at++) F[at][0] = F[at][1] = F[at][2] = 0;
-    /* a heavy molecule's force was parked by its warp */
-    const int ngi = gi ? a->gil_n[ms] : 0, ngv = gv ? a->gvl_n[ms] : 0;
-    const bool heavy = ngi + ngv * nj > kNearHeavy;
-    {
-      const int sgi = a->near_gi[ms], sgv = a->near_gv[ms];
-      const int cgi = heavy ? 0 : ngi, cgv = heavy ? 0 : ngv;
-      for (int q = 0; q < cgi; q++)
-        near_partner<AG, FP64>(x, X, gp, gtype, (int)a->gil[P->gil_off + sgi + q], eflag, F, egi);
-      for (int ent = 0; ent < cgv; ent++) {
-        const int vs = a->gvl[P->gvl_off + sgv + ent];
-        for (int b = 0; b < nj; b++) near_partner<AG, FP64>(x, X, gp, gtype, ni + vs * av + b, eflag, F, egv);
+    const int c = items_of(ms);
+    if (c == 0) continue;
+    int off, stride;
+    if (c > kNearHeavy) {
+      rec[atomicAdd(&cur[0], 1)] = make_int4(s, off = base + atomicAdd(&heavy[1], c), c, 0);
+      stride = 1;
+    } else {
+      const int r = atomicAdd(&cur[kNearHeavy + 1 - c], 1), k = r - nh, g0 = k & ~31;
+      off = light0 + (k & 31);
+      for (int b = 1; b < kNearBins; b++) { /* the groups before this one */
+        const int s0 = min(hist[b] - nh, g0), s1 = min(hist[b + 1] - nh, g0);
+        off += 32 * (kNearHeavy + 1 - b) * (((s1 + 31) >> 5) - ((s0 + 31) >> 5));
       }
+      rec[r] = make_int4(s, off, c, 0);
+      stride = 32;
     }
-    double Fd[3 * AG];
+    const unsigned short* g = a->gil + P->gil_off + a->near_gi[ms];
+    for (int q = 0; q < (int)a->gil_n[ms]; q++, off += stride) item[off] = g[q];
+    const unsigned short* v = a->gvl + P->gvl_off + a->near_gv[ms];
+    for (int q = 0; q < (int)a->gvl_n[ms]; q++)
+      for (int b = 0; b < nj; b++, off += stride) item[off] = (unsigned short)(ni + (int)v[q] * av + b);
+  }
+  __syncthreads();
+}
+
+/* what a warp's groups of near molecules share */
+template <int AG>
+struct NearSums {
+  int gtype[AG];
+  double c2[AG];
+  bool gi, gv, intra, gg;
+  long long egi = 0, egv = 0, eintra = 0;
+};
+
+/* One group of near molecules, one lane each: records first .. first + n.
+ * Light molecules' lanes walk their own partners (lg = 0).  Heavy ones
+ * (30-100 partners next to a large ion) are walked by 2^lg lanes each, the
+ * lanes' sums added by shuffles and handed to the molecule's own lane, which
+ * then finishes it like a light one: force, gas-gas and intramolecular terms,
+ * second kick.  The reactions go to the core sums by
+ * shared 32-bit integer atomics on exact chunks (acc_add); all sums are
+ * integers, so neither the split nor the order changes the result. */
+template <int AG, bool FP64, bool E>
+__device__ __forceinline__ void near_group(Ctx& x, NearSums<AG>& N, int first, int n, int lg, bool kick) {
+  const RepParams* P = x.P;
+  const KArgs* a = x.a;
+  const int par = x.D->parity, ni = P->n_ion;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const double* com = x.D->ion_com;
+  const unsigned short* const item = a->near_item + P->nit_off;
+  const bool own = lane < n;
+  const int4 rc = own ? a->near_rec[P->near_off + first + lane] : make_int4(0, 0, 0, 0);
+  const size_t g0 = gatom(P, par, rc.x, 0);
+  double X[3 * AG];
+  float3 gp[AG];
 #pragma unroll
-    for (int at = 0; at < ag; at++)
-      for (int k = 0; k < 3; k++) {
-        const long long v = heavy ? __double_as_longlong(a->slab_f[3 * gatom(P, par, s, at) + k]) : F[at][k];
-        Fd[3 * at + k] = (double)v * MDN_FIX_INV;
-        if (!(fabs(Fd[3 * at + k]) < MDN_FIX_LIMIT)) set_status(x, MDN_ST_FIXED_OVERFLOW);
+  for (int q = 0; q < 3 * AG; q++) X[q] = own ? a->slab_x[3 * g0 + q] : 0.0;
+#pragma unroll
+  for (int at = 0; at < AG; at++)
+    gp[at] = make_float3((float)(X[3 * at] - com[0]), (float)(X[3 * at + 1] - com[1]),
+                         (float)(X[3 * at + 2] - com[2]));
+  long long F[AG][3];
+#pragma unroll
+  for (int at = 0; at < AG; at++) F[at][0] = F[at][1] = F[at][2] = 0;
+  if (lg > 0) {
+    const int per = 32 >> lg, sub = (1 << lg) - 1; /* molecules a round, lane's place in its molecule */
+    for (int r = 0; r < n; r += per) {
+      const int src = r + (lane >> lg);
+      const int cnt = __shfl_sync(FULL, rc.z, src), off = __shfl_sync(FULL, rc.y, src);
+      float3 gpo[AG];
+      double Xo[3 * AG];
+      long long Fo[AG][3];
+#pragma unroll
+      for (int at = 0; at < AG; at++) {
+        gpo[at] = make_float3(__shfl_sync(FULL, gp[at].x, src), __shfl_sync(FULL, gp[at].y, src),
+                              __shfl_sync(FULL, gp[at].z, src));
+        Fo[at][0] = Fo[at][1] = Fo[at][2] = 0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) Xo[3 * at + k] = FP64 || E ? __shfl_sync(FULL, X[3 * at + k], src) : 0.0;
       }
-    if (gg)
-      for (int at = 0; at < ag; at++)
-        for (int k = 0; k < 3; k++) Fd[3 * at + k] += a->slab_fgg[3 * gatom(P, par, s, at) + k];
-    if (intra) {
-      double ei = gas_intra<AG>(x, X, Fd);
-      if (eflag) eintra += efixd(ei);
+      for (int q = lane & sub; q < cnt; q += sub + 1) {
+        const int j = item[off + q];
+        const bool ion = j < ni;
+        if (ion ? N.gi : N.gv) near_partner<AG, FP64>(x, Xo, gpo, N.gtype, j, E, Fo, ion ? N.egi : N.egv);
+      }
+#pragma unroll
+      for (int at = 0; at < AG; at++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          long long v = Fo[at][k];
+          for (int m = (sub + 1) >> 1; m; m >>= 1) v += shfl_xor_ll(v, m);
+          v = __shfl_sync(FULL, v, (lane & (per - 1)) << lg);
+          if (lane >= r && lane < r + per) F[at][k] = v;
+        }
     }
-    for (int at = 0; at < ag; at++) {
-      size_t g = gatom(P, par, s, at);
-      for (int k = 0; k < 3; k++) {
-        if (kick) a->slab_v[3 * g + k] += Fd[3 * at + k] * c2[at];
-        a->slab_f[3 * g + k] = Fd[3 * at + k];
-      }
+  } else {
+    for (int q = 0; q < rc.z; q++) {
+      const int j = item[rc.y + 32 * q];
+      const bool ion = j < ni;
+      if (ion ? N.gi : N.gv) near_partner<AG, FP64>(x, X, gp, N.gtype, j, E, F, ion ? N.egi : N.egv);
     }
   }
-  if (eflag) {
-    egi = warp_sum_ll(egi);
-    egv = warp_sum_ll(egv);
-    eintra = warp_sum_ll(eintra);
+  if (!own) return;
+  double Fd[3 * AG];
+#pragma unroll
+  for (int q = 0; q < 3 * AG; q++) {
+    Fd[q] = (double)F[q / 3][q % 3] * MDN_FIX_INV;
+    if (!(fabs(Fd[q]) < MDN_FIX_LIMIT)) set_status(x, MDN_ST_FIXED_OVERFLOW);
+  }
+  if (N.gg)
+#pragma unroll
+    for (int q = 0; q < 3 * AG; q++) Fd[q] += a->slab_fgg[3 * g0 + q];
+  if (N.intra) {
+    const double ei = gas_intra<AG>(x, X, Fd);
+    if (E) N.eintra += efixd(ei);
+  }
+#pragma unroll
+  for (int q = 0; q < 3 * AG; q++) {
+    if (kick) a->slab_v[3 * g0 + q] += Fd[q] * N.c2[q / 3];
+    a->slab_f[3 * g0 + q] = Fd[q];
+  }
+}
+
+constexpr int kHeavyGroup = 16; /* heavy molecules a warp takes at a time, at most */
+
+/* How a CTA's nh heavy molecules are cut into groups: few enough per group
+ * that every warp gets one (a lone molecule is walked by the whole warp), at
+ * most kHeavyGroup; at 8 lanes each the walk of 30-100 partners keeps its
+ * lanes busy and costs three rounds of shuffles for four molecules. */
+__device__ __forceinline__ void heavy_cut(int nh, int* size, int* lg) {
+  const int nw = blockDim.x >> 5;
+  const int h = min(kHeavyGroup, max(1, (nh + nw - 1) / nw));
+  *size = h;
+  *lg = h == 1 ? 5 : h == 2 ? 4 : 3;
+}
+
+template <int AG, bool FP64, bool E>
+__device__ __forceinline__ void gas_near_pass_t(Ctx& x, bool kick) {
+  const RepParams* P = x.P;
+  NearSums<AG> N;
+  N.gi = term_on(x, MDN_I_GI);
+  N.gv = term_on(x, MDN_I_GV);
+  N.intra = term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
+  N.gg = kGG && term_on(x, MDN_I_GG) && P->ggl_cap > 0;
+#pragma unroll
+  for (int at = 0; at < AG; at++) {
+    N.gtype[at] = x.ib[P->o_gas_type + at];
+    N.c2[at] = x.c.c2[N.gtype[at]];
+  }
+  int lo, hi;
+  partition(x, x.D->n_gas_in, &lo, &hi);
+  const int nh = x.iscr[56], nn = x.iscr[57];
+  int hs, lg;
+  heavy_cut(nh, &hs, &lg);
+  const int gh = (nh + hs - 1) / hs, total = gh + ((nn - nh + 31) >> 5);
+  for (int it = threadIdx.x >> 5; it < total; it += blockDim.x >> 5) {
+    const bool heavy = it < gh;
+    const int f = heavy ? it * hs : nh + 32 * (it - gh);
+    near_group<AG, FP64, E>(x, N, lo + f, heavy ? min(hs, nh - f) : min(32, nn - f), heavy ? lg : 0, kick);
+  }
+  if (E) {
+    N.egi = warp_sum_ll(N.egi);
+    N.egv = warp_sum_ll(N.egv);
+    N.eintra = warp_sum_ll(N.eintra);
     if ((threadIdx.x & 31) == 0) {
-      energy_add(x, MDN_U_GI, egi);
-      energy_add(x, MDN_U_VG, egv);
-      energy_add(x, MDN_U_GAS, eintra);
+      energy_add(x, MDN_U_GI, N.egi);
+      energy_add(x, MDN_U_VG, N.egv);
+      energy_add(x, MDN_U_GAS, N.eintra);
     }
   }
 }
 
+template <int AG>
+__device__ __forceinline__ void gas_near_pass_e(Ctx& x, bool eflag, bool kick) {
+  if (eflag) gas_near_pass_t<AG, kFP64Pairs, true>(x, kick);
+  else gas_near_pass_t<AG, kFP64Pairs, false>(x, kick);
+}
+
 __device__ __forceinline__ void gas_near_pass(Ctx& x, bool eflag, bool kick) {
-  if (x.P->a_g == 1) gas_near_pass_t<1, kFP64Pairs>(x, eflag, kick);
-  else gas_near_pass_t<2, kFP64Pairs>(x, eflag, kick);
+  if (x.P->a_g == 1) gas_near_pass_e<1>(x, eflag, kick);
+  else gas_near_pass_e<2>(x, eflag, kick);
 }
 
 /* sum of the core partials over the cluster -> f (double), identical in every CTA */
@@ -1801,23 +1896,6 @@ __device__ __forceinline__ int classify_one(const Ctx& x, int mi, double sigma, 
   return (draw_ok << 2) | (was << 1) | in;
 }
 
-/* exchange one int per CTA across the cluster: returns the prefix before this
- * rank and the total */
-__device__ __forceinline__ void cluster_prefix(Ctx& x, cg::cluster_group& cl, int* slot_in_smem, int mine, int* before,
-                               int* total) {
-  if (threadIdx.x == 0) *slot_in_smem = mine;
-  cl.sync();
-  int b = 0, t = 0;
-  for (int k = 0; k < x.C; k++) {
-    int v = *cl.map_shared_rank(slot_in_smem, k);
-    if (k < x.rank) b += v;
-    t += v;
-  }
-  *before = b;
-  *total = t;
-  cl.sync();
-}
-
 /* gas-gas pair list of the slab (PotentialGasGas::makePair,
  * src/potential/GasGas.cpp:41-62, on the in-domain molecules it was meant
  * for): every other slab molecule whose centre lies within the list radius,
@@ -1890,7 +1968,7 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
   /* bounding sphere of the ion, exact test below */
   int* sc = x.iscr;
   int gi_tot = 0, gv_tot = 0, nn_tot = 0;
-  int gi_base = 0, gv_base = 0, nn_base = 0;
+  int gi_base = 0, gv_base = 0, nn_before = 0;
   /* pass 1: counts */
   int my_gi = 0, my_gv = 0, my_nn = 0;
   for (int s0 = lo; s0 < hi; s0 += blockDim.x) {
@@ -1923,11 +2001,11 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
   my_nn = block_sum_i(my_nn, sc);
   cluster_prefix(x, cl, &sc[40], my_gi, &gi_base, &gi_tot);
   cluster_prefix(x, cl, &sc[41], my_gv, &gv_base, &gv_tot);
-  cluster_prefix(x, cl, &sc[42], my_nn, &nn_base, &nn_tot);
+  cluster_prefix(x, cl, &sc[42], my_nn, &nn_before, &nn_tot);
   bool over = gi_tot > P->gil_cap || gv_tot > P->gvl_cap || nn_tot > P->near_cap;
   if (over && threadIdx.x == 0 && x.rank == 0) set_status(x, MDN_ST_LIST_OVERFLOW);
   /* pass 2: fill, ascending slab slot */
-  int run_gi = gi_base, run_gv = gv_base, run_nn = nn_base;
+  int run_gi = gi_base, run_gv = gv_base;
   for (int s0 = lo; s0 < hi; s0 += blockDim.x) {
     int s = s0 + threadIdx.x;
     int cgi = 0, cgv = 0;
@@ -1952,16 +2030,14 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
           if ((dx * dx + dy * dy + dz * dz) < P->ml2) cgv++;
         }
     }
-    int t_gi, t_gv, t_nn;
+    int t_gi, t_gv;
     int o_gi = block_exscan(cgi, sc, &t_gi);
     int o_gv = block_exscan(cgv, sc, &t_gv);
-    int isn = (cgi + cgv) > 0 ? 1 : 0;
-    int o_nn = block_exscan(isn, sc, &t_nn);
+    const bool isn = (cgi + cgv) > 0;
     if (s < hi) {
       size_t ms = gmol(P, par, s);
       if (isn && !over) {
         int bgi = run_gi + o_gi, bgv = run_gv + o_gv;
-        a->near_list[P->near_off + run_nn + o_nn] = s;
         a->near_gi[ms] = bgi;
         a->near_gv[ms] = bgv;
         a->gil_n[ms] = (unsigned short)cgi;
@@ -1989,7 +2065,6 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
     }
     run_gi += t_gi;
     run_gv += t_gv;
-    run_nn += t_nn;
   }
   if (threadIdx.x == 0) {
     x.D->gi_count = over ? 0 : gi_tot;
@@ -1998,6 +2073,7 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
   }
   __threadfence();
   cl.sync();
+  build_near(x, cl);
   if (kGG && P->ggl_cap > 0 && (P->interactions & MDN_I_GG)) relist_gg(x, cl);
 }
 
@@ -2456,6 +2532,9 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     if (threadIdx.x < MDN_PROF_N) s_prof[threadIdx.x] = 0;
     __syncthreads();
     const long long job_t0 = clock64();
+    if ((a.mode == MDN_MODE_STEP || a.mode == MDN_MODE_FORCES) && sD.near_C != x.C) build_near(x, cl);
+    else if (threadIdx.x < 2) iscr[56 + threadIdx.x] = a.near_cnt[2 * ((size_t)r * 8 + x.rank) + threadIdx.x];
+    __syncthreads();
     if (a.mode == MDN_MODE_STEP) {
       for (long long s = 0; s < a.n_steps; s++) {
         bool eflag = a.energy_mode == 2 || (a.energy_mode == 1 && s == a.n_steps - 1);
@@ -2488,6 +2567,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
         atomicAdd((unsigned long long*)&a.prof[(size_t)r * MDN_PROF_N + k], (unsigned long long)s_prof[k]);
     }
     store_core(x);
+    if (threadIdx.x < 2) a.near_cnt[2 * ((size_t)r * 8 + x.rank) + threadIdx.x] = iscr[56 + threadIdx.x];
     __syncthreads();
     if (x.rank == 0 && threadIdx.x == 0) {
       a.D[r] = sD;

@@ -14,13 +14,16 @@
  *   vapor slab  the atoms of the in-domain vapor molecules (the "core"
  *               together with the ion), two buffers
  *   lists       gas-ion and gas-vapor pair lists of the "near" gas molecules
- *               (those with a non-empty list), CSR by slab slot
+ *               (those with a non-empty list), CSR by slab slot, and the
+ *               records and items the near pass reads, made from them
  *   blobs       per-replica topology (int) and coefficient (double) tables
  */
 #ifndef MDN_TYPES_H
 #define MDN_TYPES_H
 
 #include <stdint.h>
+
+#include <vector_types.h>
 
 #include "mdn.h"
 
@@ -87,7 +90,7 @@ typedef struct RepParams {
   double efield[3];
   unsigned key0, key1;
   /* pool offsets (elements) */
-  long long ion_off, mol_off, slab_off, vslab_off, near_off, gil_off, gvl_off, ggl_off;
+  long long ion_off, mol_off, slab_off, vslab_off, near_off, nit_off, gil_off, gvl_off, ggl_off;
   long long slab_moff, vslab_moff; /* molecule offsets of the two slabs */
   long long iblob_off, dblob_off;
   double work;                   /* cost estimate for the job order */
@@ -98,7 +101,8 @@ typedef struct RepDyn {
   int n_vap_in, parity, status, n_near;
   int gi_count, gv_count, nvt_mode, gg_count; /* gg_count: unordered gas-gas pairs */
   long long step;
-  double zeta, margin_length, nvt_T, pad2;
+  double zeta, margin_length, nvt_T;
+  int near_C, pad2;              /* cluster size the near records were built for, 0 = none */
   double ion_com[6];
 } RepDyn;
 
@@ -123,7 +127,10 @@ typedef struct KArgs {
   double *vslab_x, *vslab_v, *vslab_f;
   float* vslab_w;
   int* vslab_mol;
-  int* near_list;          /* slab slots of near molecules, ascending          */
+  int4* near_rec;          /* near molecules of each CTA's slab partition, from its first slot:
+                              {slab slot, first item, items, 0}, most items first */
+  unsigned short* near_item; /* their partners, core atom indices (build_near) */
+  int* near_cnt;           /* [replica][8 ranks][2] heavy / all near records of the rank */
   int* near_gi;            /* [slab slot] start of its gi entries (-1 = none)  */
   int* near_gv;            /* [slab slot] start of its gv entries              */
   unsigned short *gil_n, *gvl_n; /* [slab slot] entry counts                   */

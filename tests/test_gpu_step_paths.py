@@ -39,3 +39,27 @@ def test_core_tile_edges(eng, oracle_libs, chain, n_vap, force_mode):
         assert np.abs(e.energies()[0] - Uo).max() <= 1e-4 * max(np.abs(Uo).max(), 1e-6)
     if force_mode:
         assert rel_rms(a, b) <= 1e-9
+
+
+def _run(eng, spec, shapes, steps=12, **kw):
+    """steps per launch shape (cluster, threads), from the spec's start."""
+    e = eng.Engine([spec], quirks=CHECKED, **kw)
+    for c, t in shapes:
+        e.set_launch(c, t)
+        e.step(steps, 1)
+    s = e.state(0)
+    return np.concatenate([a.ravel() for a in (s.ion_x, s.ion_v, s.ion_f, s.gas_ax, s.gas_av, s.gas_af, s.vap_ax,
+                                               s.vap_av, s.vap_af, s.mol_x, e.energies())])
+
+
+# near molecules: records built for one cluster size and used at another,
+# none / one / many heavy molecules (more than 16 partners) for a warp, one
+# and two gas atoms, a last group of a few lanes
+@pytest.mark.parametrize("gas,chain,n_gas", [("He", 0, 60), ("Ar", 20, 3000), ("N2", 90, 5000), ("N2", 200, 2500)])
+@pytest.mark.parametrize("force_mode", [0, 1])
+def test_near_records_do_not_depend_on_the_launch(eng, gas, chain, n_gas, force_mode):
+    spec = g.small_system(seed=5 + chain, gas=gas, vapor="methanol", ion="chain" if chain else "nacl",
+                          chain_atoms=chain, n_gas=n_gas, n_vap=12, box=245.0, shake_h=True)
+    a = _run(eng, spec, [(1, 512)] * 4, force_mode=force_mode)
+    b = _run(eng, spec, [(8, 512), (1, 64), (3, 96), (2, 256)], force_mode=force_mode)
+    assert np.array_equal(a, b)
