@@ -504,6 +504,7 @@ __device__ __forceinline__ double taper(const RepParams* P, const double* com, c
 __device__ __forceinline__ void core_weights_pos(Ctx& x, bool weights) {
   const RepParams* P = x.P;
   const double* com = x.D->ion_com;
+  if (threadIdx.x == 0) x.iscr[60] = blockDim.x >> 5; /* the force queue: every warp's first item is taken */
   for (int i = threadIdx.x; i < x.n_core; i += blockDim.x) {
     if (i >= P->n_ion) {
       if (x.c.tag[i].w < 0.0f) x.c.tag[i].w = 0.0f;
@@ -787,8 +788,7 @@ __device__ __forceinline__ bool term_on(const Ctx& x, unsigned bit) {
  * pair: 36.0 -> 32.2 ms per 100 steps of 256 mixed replicas (tuned launch),
  * 2.23 -> 1.85 ms on one 13-atom core, bit-identical results. */
 template <bool FP64, bool E>
-__device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk, long long& e_ion, long long& e_vi,
-                                          long long& e_vv) {
+__device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
   const RepParams* P = x.P;
   const int ni = P->n_ion, nc = x.n_core, nt = P->n_types, av = P->a_v;
   const bool amber = term_on(x, MDN_I_AMBER), bmh = term_on(x, MDN_I_BMH);
@@ -836,6 +836,7 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk, long long& e_
   }
   const unsigned any_on = __reduce_or_sync(FULL, on | born_on);
   if (any_on == 0) return;
+  long long e_ion = 0, e_vi = 0, e_vv = 0;
   using Acc = typename std::conditional<FP64, double, float>::type;
   Acc F0 = 0, F1 = 0, F2 = 0, R0 = 0, R1 = 0, R2 = 0;
   float4 pi = make_float4(0, 0, 0, 0);
@@ -924,21 +925,11 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk, long long& e_
     const long long Rv[3] = {fix(R0), fix(R1), fix(R2)};
     acc_add(x, jj, Rv);
   }
-}
-
-template <bool FP64, bool E>
-__device__ __forceinline__ void core_pairs_t(Ctx& x) {
-  const int nblk = (x.n_core + 31) >> 5;
-  const int tiles = nblk * (nblk + 1) / 2;
-  const int nwb = blockDim.x >> 5;
-  long long e_ion = 0, e_vi = 0, e_vv = 0;
-  for (int t = x.rank * nwb + (threadIdx.x >> 5); t < tiles; t += x.C * nwb)
-    core_tile<FP64, E>(x, t, nblk, e_ion, e_vi, e_vv);
   if constexpr (E) {
     e_ion = warp_sum_ll(e_ion);
     e_vi = warp_sum_ll(e_vi);
     e_vv = warp_sum_ll(e_vv);
-    if ((threadIdx.x & 31) == 0) {
+    if (lane == 0) {
       energy_add(x, MDN_U_ION, e_ion);
       energy_add(x, MDN_U_VI, e_vi);
       energy_add(x, MDN_U_VV, e_vv);
@@ -956,12 +947,6 @@ constexpr bool kFP64Pairs = true;
 constexpr bool kFP64Pairs = false;
 #endif
 
-__device__ __forceinline__ void core_pairs(Ctx& x, bool eflag) {
-  if (!(term_on(x, MDN_I_AMBER) || term_on(x, MDN_I_BMH) || term_on(x, MDN_I_VI) || term_on(x, MDN_I_VV))) return;
-  if (eflag) core_pairs_t<kFP64Pairs, true>(x);
-  else core_pairs_t<kFP64Pairs, false>(x);
-}
-
 /* MDN_GG_TERMS selects the gas-gas term: compiled into its own kernels
  * (advance_gg.cu, advance_gg_fp64.cu), absent from the others */
 #ifdef MDN_GG_TERMS
@@ -970,66 +955,98 @@ constexpr bool kGG = true;
 constexpr bool kGG = false;
 #endif
 
-__device__ __forceinline__ void core_bonded(Ctx& x, bool eflag) {
+/* The bonded terms of the core: every dihedral (the ion's, then the vapor
+ * molecules'), then every angle, then every bond, so that a warp's 32 terms
+ * are of one kind but at the two seams. */
+struct BondedCount {
+  int nd, na, nb, vd, va, vb, nv; /* ion terms, terms per vapor molecule, vapor molecules */
+  __device__ __forceinline__ int total() const { return nd + na + nb + (vd + va + vb) * nv; }
+};
+__device__ __forceinline__ BondedCount bonded_count(const Ctx& x) {
   const RepParams* P = x.P;
-  const bool amber = term_on(x, MDN_I_AMBER);
-  const bool vin = term_on(x, MDN_I_VAPOR_INTRA);
+  const bool amber = term_on(x, MDN_I_AMBER), vin = term_on(x, MDN_I_VAPOR_INTRA);
+  BondedCount c;
+  c.nd = amber ? P->n_ion_dih : 0;
+  c.na = amber ? P->n_ion_angles : 0;
+  c.nb = amber ? P->n_ion_bonds : 0;
+  c.vd = vin ? P->n_vap_dih : 0;
+  c.va = vin ? P->n_vap_angles : 0;
+  c.vb = vin ? P->n_vap_bonds : 0;
+  c.nv = x.D->n_vap_in;
+  return c;
+}
+
+/* terms 32 k .. 32 k + 31, one per lane */
+template <bool E>
+__device__ __forceinline__ void bonded_terms(Ctx& x, const BondedCount& bc, int k) {
+  const RepParams* P = x.P;
   const bool qb = (P->quirks & MDN_Q_ENERGY_BUCKETS) != 0;
-  const int nb = amber ? P->n_ion_bonds : 0, na = amber ? P->n_ion_angles : 0, nd = amber ? P->n_ion_dih : 0;
-  const int vterms = vin ? (P->n_vap_bonds + P->n_vap_angles + P->n_vap_dih) : 0;
-  const long long total = (long long)nb + na + nd + (long long)vterms * x.D->n_vap_in;
-  long long eU[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (long long t = (long long)x.rank * blockDim.x + threadIdx.x; t < total; t += (long long)x.C * blockDim.x) {
-    BondOut o;
-    int idx[4];
-    int n = 0, bucket = MDN_U_ION;
-    const double* X = x.c.x;
-    int base = 0;
-    long long u = t;
-    int kind;  /* 0 bond, 1 angle, 2 dihedral */
-    const int* row;
-    if (u < nb) { kind = 0; row = x.ib + P->o_ion_bonds + 3 * u; }
-    else if ((u -= nb) < na) { kind = 1; row = x.ib + P->o_ion_angles + 4 * u; }
-    else if ((u -= na) < nd) { kind = 2; row = x.ib + P->o_ion_dih + 5 * u; }
-    else {
-      u -= nd;
-      int s = (int)(u / vterms), q = (int)(u - (long long)s * vterms);
-      base = P->n_ion + s * P->a_v;
-      if (q < P->n_vap_bonds) { kind = 0; row = x.ib + P->o_vap_bonds + 3 * q; bucket = qb ? MDN_U_GAS : MDN_U_VAP; }
-      else if ((q -= P->n_vap_bonds) < P->n_vap_angles) { kind = 1; row = x.ib + P->o_vap_angles + 4 * q; bucket = qb ? MDN_U_GAS : MDN_U_VAP; }
-      else { q -= P->n_vap_angles; kind = 2; row = x.ib + P->o_vap_dih + 5 * q; bucket = qb ? MDN_U_ION : MDN_U_VAP; }
+  const int lane = threadIdx.x & 31;
+  int u = 32 * k + lane;
+  const bool on = u < bc.total();
+  long long e = 0;
+  int bucket = MDN_U_ION;
+  if (on) {
+    /* kind: 2 dihedral, 1 angle, 0 bond; the row's place among the ion's
+     * (base 0) or in vapor molecule s */
+    int kind = 2, n_ion = bc.nd, per = bc.vd;
+    if (u >= bc.nd + bc.vd * bc.nv) {
+      u -= bc.nd + bc.vd * bc.nv;
+      kind = 1, n_ion = bc.na, per = bc.va;
+      if (u >= bc.na + bc.va * bc.nv) {
+        u -= bc.na + bc.va * bc.nv;
+        kind = 0, n_ion = bc.nb, per = bc.vb;
+      }
     }
-    if (kind == 0) {
-      idx[0] = base + row[0]; idx[1] = base + row[1];
-      bond_fd(X, x.db + P->d_bond + 2 * row[2], idx[0], idx[1], o);
-      n = 2;
+    const bool vap = u >= n_ion;
+    int base = 0;
+    if (vap) {
+      const int s = (u - n_ion) / per;
+      u = u - n_ion - s * per;
+      base = P->n_ion + s * P->a_v;
+      bucket = qb ? (kind == 2 ? MDN_U_ION : MDN_U_GAS) : MDN_U_VAP;
+    }
+    const double* X = x.c.x + 3 * base;
+    BondOut o;
+    int n;
+    const int* row;
+    if (kind == 2) {
+      row = x.ib + (vap ? P->o_vap_dih : P->o_ion_dih) + 5 * u;
+      dihedral_fd(X, x.db + P->d_dih + 15 * row[4], x.ib[P->o_dih_multi + row[4]], row[0], row[1], row[2], row[3], o);
+      n = 4;
     } else if (kind == 1) {
-      idx[0] = base + row[0]; idx[1] = base + row[1]; idx[2] = base + row[2];
-      angle_fd(X, x.db + P->d_angle + 2 * row[3], idx[0], idx[1], idx[2], o);
+      row = x.ib + (vap ? P->o_vap_angles : P->o_ion_angles) + 4 * u;
+      angle_fd(X, x.db + P->d_angle + 2 * row[3], row[0], row[1], row[2], o);
       n = 3;
     } else {
-      idx[0] = base + row[0]; idx[1] = base + row[1]; idx[2] = base + row[2]; idx[3] = base + row[3];
-      dihedral_fd(X, x.db + P->d_dih + 15 * row[4], x.ib[P->o_dih_multi + row[4]], idx[0], idx[1], idx[2],
-                  idx[3], o);
-      n = 4;
+      row = x.ib + (vap ? P->o_vap_bonds : P->o_ion_bonds) + 3 * u;
+      bond_fd(X, x.db + P->d_bond + 2 * row[2], row[0], row[1], o);
+      n = 2;
     }
-    for (int q = 0; q < n; q++) {
-      long long F[3] = {fixd(o.f[q][0]), fixd(o.f[q][1]), fixd(o.f[q][2])};
-      acc_add(x, idx[q], F);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (q >= n) break;
+      const long long F[3] = {fixd(o.f[q][0]), fixd(o.f[q][1]), fixd(o.f[q][2])};
+      acc_add(x, base + row[q], F);
     }
-    if (eflag) eU[bucket] += efixd(o.e);
+    if (E) e = efixd(o.e);
   }
-  if (eflag)
-    for (int b = 0; b < 8; b++) {
-      long long s = warp_sum_ll(eU[b]);
-      if ((threadIdx.x & 31) == 0) energy_add(x, b, s);
+  if (E) {
+    for (int b = MDN_U_ION; b <= MDN_U_VAP; b++) {
+      const long long s = warp_sum_ll(bucket == b ? e : 0);
+      if (lane == 0) energy_add(x, b, s);
     }
-  if (term_on(x, MDN_I_EFIELD) && x.rank == 0)
-    for (int i = threadIdx.x; i < P->n_ion; i += blockDim.x) {
-      double coeff = 5.55e-5 * x.db[P->d_ion_q + i];
-      long long F[3] = {fixd(coeff * P->efield[0]), fixd(coeff * P->efield[1]), fixd(coeff * P->efield[2])};
-      acc_add(x, i, F);
-    }
+  }
+}
+
+/* the uniform field on the ion's charges, one warp */
+__device__ __forceinline__ void field_terms(Ctx& x) {
+  const RepParams* P = x.P;
+  for (int i = threadIdx.x & 31; i < P->n_ion; i += 32) {
+    const double coeff = 5.55e-5 * x.db[P->d_ion_q + i];
+    const long long F[3] = {fixd(coeff * P->efield[0]), fixd(coeff * P->efield[1]), fixd(coeff * P->efield[2])};
+    acc_add(x, i, F);
+  }
 }
 
 /* ------------------------------------------------------------------------- */
@@ -1501,15 +1518,6 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   __syncthreads();
 }
 
-/* what a warp's groups of near molecules share */
-template <int AG>
-struct NearSums {
-  int gtype[AG];
-  double c2[AG];
-  bool gi, gv, intra, gg;
-  long long egi = 0, egv = 0, eintra = 0;
-};
-
 /* One group of near molecules, one lane each: records first .. first + n.
  * Light molecules' lanes walk their own partners (lg = 0).  Heavy ones
  * (30-100 partners next to a large ion) are walked by 2^lg lanes each, the
@@ -1519,9 +1527,14 @@ struct NearSums {
  * shared 32-bit integer atomics on exact chunks (acc_add); all sums are
  * integers, so neither the split nor the order changes the result. */
 template <int AG, bool FP64, bool E>
-__device__ __forceinline__ void near_group(Ctx& x, NearSums<AG>& N, int first, int n, int lg, bool kick) {
+__device__ __forceinline__ void near_group(Ctx& x, int first, int n, int lg, bool kick) {
   const RepParams* P = x.P;
   const KArgs* a = x.a;
+  const bool gi = term_on(x, MDN_I_GI), gv = term_on(x, MDN_I_GV);
+  int gtype[AG];
+#pragma unroll
+  for (int at = 0; at < AG; at++) gtype[at] = x.iscr[58 + at];
+  long long egi = 0, egv = 0, eintra = 0;
   const int par = x.D->parity, ni = P->n_ion;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -1560,7 +1573,7 @@ __device__ __forceinline__ void near_group(Ctx& x, NearSums<AG>& N, int first, i
       for (int q = lane & sub; q < cnt; q += sub + 1) {
         const int j = item[off + q];
         const bool ion = j < ni;
-        if (ion ? N.gi : N.gv) near_partner<AG, FP64>(x, Xo, gpo, N.gtype, j, E, Fo, ion ? N.egi : N.egv);
+        if (ion ? gi : gv) near_partner<AG, FP64>(x, Xo, gpo, gtype, j, E, Fo, ion ? egi : egv);
       }
 #pragma unroll
       for (int at = 0; at < AG; at++)
@@ -1576,27 +1589,38 @@ __device__ __forceinline__ void near_group(Ctx& x, NearSums<AG>& N, int first, i
     for (int q = 0; q < rc.z; q++) {
       const int j = item[rc.y + 32 * q];
       const bool ion = j < ni;
-      if (ion ? N.gi : N.gv) near_partner<AG, FP64>(x, X, gp, N.gtype, j, E, F, ion ? N.egi : N.egv);
+      if (ion ? gi : gv) near_partner<AG, FP64>(x, X, gp, gtype, j, E, F, ion ? egi : egv);
     }
   }
-  if (!own) return;
-  double Fd[3 * AG];
+  if (own) {
+    double Fd[3 * AG];
 #pragma unroll
-  for (int q = 0; q < 3 * AG; q++) {
-    Fd[q] = (double)F[q / 3][q % 3] * MDN_FIX_INV;
-    if (!(fabs(Fd[q]) < MDN_FIX_LIMIT)) set_status(x, MDN_ST_FIXED_OVERFLOW);
+    for (int q = 0; q < 3 * AG; q++) {
+      Fd[q] = (double)F[q / 3][q % 3] * MDN_FIX_INV;
+      if (!(fabs(Fd[q]) < MDN_FIX_LIMIT)) set_status(x, MDN_ST_FIXED_OVERFLOW);
+    }
+    if (kGG && term_on(x, MDN_I_GG) && P->ggl_cap > 0)
+#pragma unroll
+      for (int q = 0; q < 3 * AG; q++) Fd[q] += a->slab_fgg[3 * g0 + q];
+    if (term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0) {
+      const double ei = gas_intra<AG>(x, X, Fd);
+      if (E) eintra = efixd(ei);
+    }
+#pragma unroll
+    for (int q = 0; q < 3 * AG; q++) {
+      if (kick) a->slab_v[3 * g0 + q] += Fd[q] * x.c.c2[gtype[q / 3]];
+      a->slab_f[3 * g0 + q] = Fd[q];
+    }
   }
-  if (N.gg)
-#pragma unroll
-    for (int q = 0; q < 3 * AG; q++) Fd[q] += a->slab_fgg[3 * g0 + q];
-  if (N.intra) {
-    const double ei = gas_intra<AG>(x, X, Fd);
-    if (E) N.eintra += efixd(ei);
-  }
-#pragma unroll
-  for (int q = 0; q < 3 * AG; q++) {
-    if (kick) a->slab_v[3 * g0 + q] += Fd[q] * N.c2[q / 3];
-    a->slab_f[3 * g0 + q] = Fd[q];
+  if (E) {
+    egi = warp_sum_ll(egi);
+    egv = warp_sum_ll(egv);
+    eintra = warp_sum_ll(eintra);
+    if (lane == 0) {
+      energy_add(x, MDN_U_GI, egi);
+      energy_add(x, MDN_U_VG, egv);
+      energy_add(x, MDN_U_GAS, eintra);
+    }
   }
 }
 
@@ -1611,53 +1635,6 @@ __device__ __forceinline__ void heavy_cut(int nh, int* size, int* lg) {
   const int h = min(kHeavyGroup, max(1, (nh + nw - 1) / nw));
   *size = h;
   *lg = h == 1 ? 5 : h == 2 ? 4 : 3;
-}
-
-template <int AG, bool FP64, bool E>
-__device__ __forceinline__ void gas_near_pass_t(Ctx& x, bool kick) {
-  const RepParams* P = x.P;
-  NearSums<AG> N;
-  N.gi = term_on(x, MDN_I_GI);
-  N.gv = term_on(x, MDN_I_GV);
-  N.intra = term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
-  N.gg = kGG && term_on(x, MDN_I_GG) && P->ggl_cap > 0;
-#pragma unroll
-  for (int at = 0; at < AG; at++) {
-    N.gtype[at] = x.ib[P->o_gas_type + at];
-    N.c2[at] = x.c.c2[N.gtype[at]];
-  }
-  int lo, hi;
-  partition(x, x.D->n_gas_in, &lo, &hi);
-  const int nh = x.iscr[56], nn = x.iscr[57];
-  int hs, lg;
-  heavy_cut(nh, &hs, &lg);
-  const int gh = (nh + hs - 1) / hs, total = gh + ((nn - nh + 31) >> 5);
-  for (int it = threadIdx.x >> 5; it < total; it += blockDim.x >> 5) {
-    const bool heavy = it < gh;
-    const int f = heavy ? it * hs : nh + 32 * (it - gh);
-    near_group<AG, FP64, E>(x, N, lo + f, heavy ? min(hs, nh - f) : min(32, nn - f), heavy ? lg : 0, kick);
-  }
-  if (E) {
-    N.egi = warp_sum_ll(N.egi);
-    N.egv = warp_sum_ll(N.egv);
-    N.eintra = warp_sum_ll(N.eintra);
-    if ((threadIdx.x & 31) == 0) {
-      energy_add(x, MDN_U_GI, N.egi);
-      energy_add(x, MDN_U_VG, N.egv);
-      energy_add(x, MDN_U_GAS, N.eintra);
-    }
-  }
-}
-
-template <int AG>
-__device__ __forceinline__ void gas_near_pass_e(Ctx& x, bool eflag, bool kick) {
-  if (eflag) gas_near_pass_t<AG, kFP64Pairs, true>(x, kick);
-  else gas_near_pass_t<AG, kFP64Pairs, false>(x, kick);
-}
-
-__device__ __forceinline__ void gas_near_pass(Ctx& x, bool eflag, bool kick) {
-  if (x.P->a_g == 1) gas_near_pass_e<1>(x, eflag, kick);
-  else gas_near_pass_e<2>(x, eflag, kick);
 }
 
 /* sum of the core partials over the cluster -> f (double), identical in every CTA */
@@ -1698,20 +1675,75 @@ __device__ __forceinline__ void core_reduce(Ctx& x, cg::cluster_group& cl) {
     }
 }
 
-/* all forces of the step (after positions and lists are final) and the second kick */
+/* All forces of the step (after positions and lists are final) as one queue
+ * of warp-sized items: 32 bonded terms, a core pair tile, a group of near
+ * molecules.  They all add integers to the core sums, so they need no order
+ * and no barrier among them; a warp takes its next item from a shared
+ * counter, so that the CTA waits for its slowest warp once per step and not
+ * once per kind.  The long items come first (the FP64 bonded terms, the
+ * tiles, the heavy and then ever lighter near groups).  Bonded terms and
+ * tiles are dealt to the cluster's CTAs in turn; near groups belong to the
+ * CTA of their slab partition.  With the cycle accounting on, the kinds run
+ * one after another, each with its own barrier. */
+template <bool E>
+__device__ __forceinline__ void force_items(Ctx& x, bool kick) {
+  const RepParams* P = x.P;
+  const int nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+  const bool pairs = term_on(x, MDN_I_AMBER) || term_on(x, MDN_I_BMH) || term_on(x, MDN_I_VI) || term_on(x, MDN_I_VV);
+  const BondedCount bc = bonded_count(x);
+  const int nblk = pairs ? (x.n_core + 31) >> 5 : 0;
+  const int field = term_on(x, MDN_I_EFIELD) ? 1 : 0;
+  const int n_bond = field + ((bc.total() + 31) >> 5), n_tile = nblk * (nblk + 1) / 2;
+  int lo, hi;
+  partition(x, x.D->n_gas_in, &lo, &hi);
+  const int nh = x.iscr[56], nn = x.iscr[57];
+  int hs, lg;
+  heavy_cut(nh, &hs, &lg);
+  const int gh = (nh + hs - 1) / hs;
+  /* this CTA's items: bonded and tiles g = rank, rank + C, ..., then near */
+  const int mb = (n_bond - x.rank + x.C - 1) / x.C, mc = (n_bond + n_tile - x.rank + x.C - 1) / x.C;
+  const int total = mc + gh + ((nn - nh + 31) >> 5);
+  const bool prof = x.a->prof != nullptr;
+  for (int ph = 0; ph < (prof ? 3 : 1); ph++) {
+    int first = 0, last = total;
+    if (prof) {
+      first = ph == 0 ? mc : ph == 1 ? 0 : mb;
+      last = ph == 0 ? total : ph == 1 ? mb : mc;
+      __syncthreads();
+      prof_start(x);
+      if (threadIdx.x == 0) x.iscr[60] = nw;
+      __syncthreads();
+    }
+    for (int it = first + (int)(threadIdx.x >> 5); it < last;) {
+      if (it < mb) {
+        const int g = x.rank + it * x.C;
+        if (g < field) field_terms(x);
+        else bonded_terms<E>(x, bc, g - field);
+      } else if (it < mc) {
+        core_tile<kFP64Pairs, E>(x, x.rank + it * x.C - n_bond, nblk);
+      } else {
+        const int k = it - mc;
+        const bool heavy = k < gh;
+        const int f = heavy ? k * hs : nh + 32 * (k - gh), n = heavy ? min(hs, nh - f) : min(32, nn - f);
+        if (P->a_g == 1) near_group<1, kFP64Pairs, E>(x, lo + f, n, heavy ? lg : 0, kick);
+        else near_group<2, kFP64Pairs, E>(x, lo + f, n, heavy ? lg : 0, kick);
+      }
+      int next = 0;
+      if (lane == 0) next = atomicAdd(&x.iscr[60], 1);
+      it = first + __shfl_sync(0xffffffffu, next, 0);
+    }
+    if (prof) {
+      __syncthreads();
+      prof_end(x, ph == 0 ? MDN_PROF_NEAR : ph == 1 ? MDN_PROF_BONDED : MDN_PROF_PAIRS);
+    }
+  }
+}
+
+/* the forces, and the second kick */
 __device__ __forceinline__ void forces_and_kick(Ctx& x, cg::cluster_group& cl, bool eflag, bool kick) {
-  prof_start(x);
-  gas_near_pass(x, eflag, kick);
+  if (eflag) force_items<true>(x, kick);
+  else force_items<false>(x, kick);
   __syncthreads();
-  prof_end(x, MDN_PROF_NEAR);
-  prof_start(x);
-  core_bonded(x, eflag);
-  __syncthreads();
-  prof_end(x, MDN_PROF_BONDED);
-  prof_start(x);
-  core_pairs(x, eflag);
-  __syncthreads();
-  prof_end(x, MDN_PROF_PAIRS);
   prof_start(x);
   core_reduce(x, cl);
   if (kick) {
@@ -2531,9 +2563,11 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     load_vapor(x);
     if (threadIdx.x < MDN_PROF_N) s_prof[threadIdx.x] = 0;
     __syncthreads();
+    if (threadIdx.x < sP.a_g) iscr[58 + threadIdx.x] = x.ib[sP.o_gas_type + threadIdx.x];
     const long long job_t0 = clock64();
     if ((a.mode == MDN_MODE_STEP || a.mode == MDN_MODE_FORCES) && sD.near_C != x.C) build_near(x, cl);
-    else if (threadIdx.x < 2) iscr[56 + threadIdx.x] = a.near_cnt[2 * ((size_t)r * 8 + x.rank) + threadIdx.x];
+    else if (threadIdx.x < 2)
+      iscr[56 + threadIdx.x] = a.near_cnt[2 * ((size_t)r * 8 + x.rank) + threadIdx.x];
     __syncthreads();
     if (a.mode == MDN_MODE_STEP) {
       for (long long s = 0; s < a.n_steps; s++) {
