@@ -15,8 +15,8 @@
  *     split evenly over the cluster's CTAs;
  *   - gas-gas interactions are absent from the reference's configurations, so
  *     a gas molecule interacts only with the core: molecules whose gas-ion /
- *     gas-vapor lists are empty ("far") are advanced by one thread in a single
- *     pass (kick, drift, intramolecular force, kick); "near" molecules are
+ *     gas-vapor lists are empty ("far") are advanced by one thread each, where
+ *     they are many through all steps to the next rebuild at once; "near" ones are
  *     sorted by their number of partners and taken 32 to a warp (build_near,
  *     near_group), with shared-memory fixed-point atomics for the reaction on
  *     the core.
@@ -320,17 +320,33 @@ __device__ bool shake_group(double* X, const double* R, const int* rig, const do
   return false;
 }
 
-template <int AG>
-__device__ __forceinline__ void gas_integrate_t(Ctx& x, bool fused, bool eflag, int tid, int nthr);
+__device__ __forceinline__ bool gas_rigid(const RepParams* P) {
+  return (P->interactions & MDN_I_SHAKE) && P->n_gas_rigid > 0 && P->a_g == 2;
+}
 
-__device__ __forceinline__ void gas_integrate(Ctx& x, bool fused, bool eflag, int tid, int nthr);
+/* Which gas molecules a step integrates beside the core's constraints:
+ * all of this CTA's, first kick and drift only, on the steps that rebuild the
+ * domain (the lists follow the drift) or need the gas-gas forces (every
+ * position first); on others the far ones, complete with their own bond and
+ * second kick, unless gas_far_steps has already made their steps, and the
+ * near ones, unless they are drifted where their forces are taken
+ * (near_group).  That saves a pass over their slab rows, but it lengthens the
+ * force items, while here the warps are idle: so it is done for more near
+ * molecules than threads (dense domains: 4.96 -> 4.69 ms per 50 steps; the
+ * 150-atom chain in thin gas would go from 1.89 to 1.93 ms per 100 steps),
+ * and not for a rigid gas, whose constraint is longer still. */
+struct GasWork {
+  bool all, far, near;
+};
 
-/* Drift of the core, its constraints, and the gas integration of the step.
+__device__ __forceinline__ void gas_integrate(Ctx& x, GasWork w, bool eflag, int tid, int nthr);
+
+/* Drift of the core, its constraints, and the step's gas integration.
  * The constraints and the gas are independent (the gas pass touches only
  * the gas slab), so they run side by side: warp 0 sweeps the ion's
  * constraints, the next warps take one vapor molecule per thread, and the
  * remaining warps integrate the gas molecules. */
-__device__ __forceinline__ void core_drift_shake(Ctx& x, bool fused, bool eflag) {
+__device__ __forceinline__ void core_drift_shake(Ctx& x, GasWork gas, bool eflag) {
   const RepParams* P = x.P;
   /* positions before the drift (the SHAKE reference vectors) live in the
    * 64-bit sum buffer: core_reduce overwrites it only after this step's
@@ -439,7 +455,7 @@ __device__ __forceinline__ void core_drift_shake(Ctx& x, bool fused, bool eflag)
         }
     }
   } else if (warp >= w_gas0) {
-    gas_integrate(x, fused, eflag, threadIdx.x - 32 * w_gas0, blockDim.x - 32 * w_gas0);
+    gas_integrate(x, gas, eflag, threadIdx.x - 32 * w_gas0, blockDim.x - 32 * w_gas0);
   }
   __syncthreads();
 }
@@ -1119,88 +1135,164 @@ __device__ __forceinline__ int shake_gas2(const Ctx& x, double* X, const double*
   return converge ? 0 : MDN_ST_SHAKE_NOCONV;
 }
 
-/* kick + drift (+SHAKE) of the gas molecules of this CTA; far molecules also
- * get their intramolecular force and the second kick when `fused`. */
-/* kick, drift, gas SHAKE and (fused, for molecules without list entries)
- * the intramolecular force and second kick of the gas molecules; thread tid
- * of the nthr (whole warps) that take part */
+/* first kick, drift and constraint of one gas molecule in registers: X, V
+ * and F of its atoms (F the force of the last evaluation) */
 template <int AG>
-__device__ __forceinline__ void gas_integrate_t(Ctx& x, bool fused, bool eflag, int tid, int nthr) {
+__device__ __forceinline__ void gas_drift(Ctx& x, double* X, double* V, const double* F, const double* c2, bool sh,
+                                          bool vcorr, double dt) {
+  double R[3 * AG];
+#pragma unroll
+  for (int q = 0; q < 3 * AG; q++) {
+    V[q] += F[q] * c2[q / 3];
+    R[q] = X[q];
+    X[q] = X[q] + V[q] * dt;
+  }
+  if constexpr (AG == 2) {
+    if (sh) {
+      double Xd[3 * AG];
+#pragma unroll
+      for (int q = 0; q < 3 * AG; q++) Xd[q] = X[q];
+      const int st = shake_gas2(x, X, R);
+      if (st) set_status(x, st);
+      if (vcorr)
+#pragma unroll
+        for (int q = 0; q < 3 * AG; q++) V[q] += (X[q] - Xd[q]) / dt;
+    }
+  }
+}
+
+template <int AG>
+__device__ __forceinline__ void gas_finite(const Ctx& x, const double* X, const double* V) {
+  if (!isfinite(X[0] + X[1] + X[2] + V[0] + V[1] + V[2])) set_status(x, MDN_ST_NONFINITE);
+}
+
+/* thread tid of the nthr (whole warps) that take part */
+template <int AG>
+__device__ __forceinline__ void gas_integrate_t(Ctx& x, GasWork w, bool eflag, int tid, int nthr) {
   const RepParams* P = x.P;
   const KArgs* a = x.a;
-  constexpr int ag = AG;
   const int par = x.D->parity;
-  const bool sh = (P->interactions & MDN_I_SHAKE) && P->n_gas_rigid > 0;
   const bool vcorr = !(P->quirks & MDN_Q_SHAKE_NO_VCORR);
-  const bool intra = term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
-  const double dt = P->dt;
+  const bool intra = AG == 2 && term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
   int lo, hi;
   partition(x, x.D->n_gas_in, &lo, &hi);
-  double m[AG], c2[AG];
+  double c2[AG];
 #pragma unroll
-  for (int at = 0; at < ag; at++) {
-    int t = x.ib[P->o_gas_type + at];
-    m[at] = x.db[P->d_mass + t];
-    c2[at] = x.c.c2[t];
-  }
+  for (int at = 0; at < AG; at++) c2[at] = x.c.c2[x.iscr[58 + at]];
+  const int nf = w.far ? x.iscr[61] : 0, n = w.all ? hi - lo : nf + (w.near ? x.iscr[57] : 0);
   long long eg = 0;
-  for (int s = lo + tid; s < hi; s += nthr) {
-    double X[3 * AG], V[3 * AG], F[3 * AG], R[3 * AG];
-    for (int at = 0; at < ag; at++) {
-      size_t g = gatom(P, par, s, at);
-      for (int k = 0; k < 3; k++) {
-        X[3 * at + k] = a->slab_x[3 * g + k];
-        V[3 * at + k] = a->slab_v[3 * g + k];
-        F[3 * at + k] = a->slab_f[3 * g + k];
-      }
-    }
-    for (int at = 0; at < ag; at++)
-      for (int k = 0; k < 3; k++) {
-        V[3 * at + k] += F[3 * at + k] * c2[at];
-        R[3 * at + k] = X[3 * at + k];
-        X[3 * at + k] = X[3 * at + k] + V[3 * at + k] * dt;
-        F[3 * at + k] = 0.0;
-      }
-    if constexpr (AG == 2) {
-      if (sh) {
-        double Xd[3 * AG];
+  for (int e = tid; e < n; e += nthr) {
+    const int s = w.all ? lo + e
+                        : e < nf ? a->far_list[P->near_off + lo + e] : a->near_rec[P->near_off + lo + e - nf].x;
+    const size_t g0 = 3 * gatom(P, par, s, 0);
+    double X[3 * AG], V[3 * AG], F[3 * AG];
 #pragma unroll
-        for (int q = 0; q < 3 * ag; q++) Xd[q] = X[q];
-        int st = shake_gas2(x, X, R);
-        if (st) set_status(x, st);
-        if (vcorr)
-#pragma unroll
-          for (int q = 0; q < 3 * ag; q++) V[q] += (X[q] - Xd[q]) / dt;
-      }
+    for (int q = 0; q < 3 * AG; q++) {
+      X[q] = a->slab_x[g0 + q];
+      V[q] = a->slab_v[g0 + q];
+      F[q] = a->slab_f[g0 + q];
     }
-    if (!isfinite(X[0] + X[1] + X[2] + V[0] + V[1] + V[2])) set_status(x, MDN_ST_NONFINITE);
-    bool near = fused ? (a->near_gi[gmol(P, par, s)] >= 0) : true;
-    if (!near) {
+    gas_drift<AG>(x, X, V, F, c2, gas_rigid(P), vcorr, P->dt);
+    gas_finite<AG>(x, X, V);
+#pragma unroll
+    for (int q = 0; q < 3 * AG; q++) F[q] = 0.0;
+    if (!w.all && e < nf) {
       if (intra) {
-        double e = gas_intra<AG>(x, X, F);
-        if (eflag) eg += efixd(e);
+        const double ei = gas_intra<AG>(x, X, F);
+        if (eflag) eg += efixd(ei);
       }
-      for (int at = 0; at < ag; at++)
-        for (int k = 0; k < 3; k++) V[3 * at + k] += F[3 * at + k] * c2[at];
+#pragma unroll
+      for (int q = 0; q < 3 * AG; q++) V[q] += F[q] * c2[q / 3];
     }
-    for (int at = 0; at < ag; at++) {
-      size_t g = gatom(P, par, s, at);
-      for (int k = 0; k < 3; k++) {
-        a->slab_x[3 * g + k] = X[3 * at + k];
-        a->slab_v[3 * g + k] = V[3 * at + k];
-        a->slab_f[3 * g + k] = F[3 * at + k];
-      }
+#pragma unroll
+    for (int q = 0; q < 3 * AG; q++) {
+      a->slab_x[g0 + q] = X[q];
+      a->slab_v[g0 + q] = V[q];
+      a->slab_f[g0 + q] = F[q];
     }
   }
-  if (eflag && intra) {
+  if (eflag && intra && w.far) {
     eg = warp_sum_ll(eg);
     if ((threadIdx.x & 31) == 0) energy_add(x, MDN_U_GAS, eg);
   }
 }
 
-__device__ __forceinline__ void gas_integrate(Ctx& x, bool fused, bool eflag, int tid, int nthr) {
-  if (x.P->a_g == 1) gas_integrate_t<1>(x, fused, eflag, tid, nthr);
-  else gas_integrate_t<2>(x, fused, eflag, tid, nthr);
+__device__ __forceinline__ void gas_integrate(Ctx& x, GasWork w, bool eflag, int tid, int nthr) {
+  if (x.P->a_g == 1) gas_integrate_t<1>(x, w, eflag, tid, nthr);
+  else gas_integrate_t<2>(x, w, eflag, tid, nthr);
+}
+
+/* The far molecules (no list entry) over the next k steps at once, for a
+ * CTA with more of them than threads.  Until the next rebuild nothing but
+ * their own bond acts on them, so the k steps of a molecule run in one
+ * thread's registers: the slab is read and written once per k steps (k: to
+ * the rebuild or the end of the launch) instead of once per step, 144 B per
+ * atom each time.  With fewer molecules the k dependent steps of a thread
+ * would be waited for (134 rigid N2 over 8 CTAs: 2.06 ms per 100 steps
+ * against 1.89 ms beside the core's constraints, GasWork).  The operations of each step are those of gas_drift
+ * and the second kick, in their order.  energy_mode, last: as one_step's
+ * eflag, energies of every step or of the last of these k. */
+template <int AG>
+__device__ __forceinline__ void gas_far_steps_t(Ctx& x, long long k, int energy_mode, bool last) {
+  const RepParams* P = x.P;
+  const KArgs* a = x.a;
+  const int par = x.D->parity;
+  const bool sh = gas_rigid(P);
+  const bool vcorr = !(P->quirks & MDN_Q_SHAKE_NO_VCORR);
+  const bool intra = AG == 2 && term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
+  const double dt = P->dt;
+  int lo, hi;
+  partition(x, x.D->n_gas_in, &lo, &hi);
+  const int* far = a->far_list + P->near_off + lo;
+  const int n_far = x.iscr[61];
+  double c2[AG];
+#pragma unroll
+  for (int at = 0; at < AG; at++) c2[at] = x.c.c2[x.iscr[58 + at]];
+  long long eg = 0;
+  for (int e = threadIdx.x; e < n_far; e += blockDim.x) {
+    const size_t g0 = 3 * gatom(P, par, far[e], 0);
+    double X[3 * AG], V[3 * AG], F[3 * AG];
+#pragma unroll
+    for (int q = 0; q < 3 * AG; q++) {
+      X[q] = a->slab_x[g0 + q];
+      V[q] = a->slab_v[g0 + q];
+      F[q] = a->slab_f[g0 + q];
+    }
+    for (long long t = 0; t < k; t++) {
+      gas_drift<AG>(x, X, V, F, c2, sh, vcorr, dt);
+#pragma unroll
+      for (int q = 0; q < 3 * AG; q++) F[q] = 0.0;
+      if (intra) {
+        const double ei = gas_intra<AG>(x, X, F);
+        if (energy_mode == 2 || (energy_mode == 1 && last && t == k - 1)) eg += efixd(ei);
+      }
+#pragma unroll
+      for (int q = 0; q < 3 * AG; q++) V[q] += F[q] * c2[q / 3];
+      if (AG == 1 && t == 0) {
+        /* no force from here on: V stays as it is */
+        for (t = 1; t < k; t++)
+#pragma unroll
+          for (int q = 0; q < 3 * AG; q++) X[q] = X[q] + V[q] * dt;
+        break;
+      }
+    }
+    gas_finite<AG>(x, X, V);
+#pragma unroll
+    for (int q = 0; q < 3 * AG; q++) {
+      a->slab_x[g0 + q] = X[q];
+      a->slab_v[g0 + q] = V[q];
+      a->slab_f[g0 + q] = F[q];
+    }
+  }
+  if (intra && (energy_mode == 2 || (energy_mode == 1 && last))) {
+    eg = warp_sum_ll(eg);
+    if ((threadIdx.x & 31) == 0) energy_add(x, MDN_U_GAS, eg);
+  }
+}
+
+__device__ __forceinline__ void gas_far_steps(Ctx& x, long long k, int energy_mode, bool last) {
+  if (x.P->a_g == 1) gas_far_steps_t<1>(x, k, energy_mode, last);
+  else gas_far_steps_t<2>(x, k, energy_mode, last);
 }
 
 /* after a rebuild: intramolecular force and second kick of the far molecules */
@@ -1445,7 +1537,8 @@ __device__ __forceinline__ int gv_reach(const RepParams* P) {
  * of steps.  The records of a CTA start at its partition's first slot, its
  * items where the lower ranks' end; they depend on the cluster size, which
  * RepDyn::near_C remembers, and are built again when a launch uses another.
- * Built at a rebuild (every few hundred steps); all threads of the cluster. */
+ * The other molecules' slots follow in far_list, ascending.  Built at a
+ * rebuild (every few hundred steps); all threads of the cluster. */
 __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   const RepParams* P = x.P;
   const KArgs* a = x.a;
@@ -1491,6 +1584,16 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   const int nh = x.iscr[56], light0 = base + heavy[0];
   int4* const rec = a->near_rec + P->near_off + lo;
   unsigned short* const item = a->near_item + P->nit_off;
+  int n_far = 0;
+  for (int s0 = lo; s0 < hi; s0 += blockDim.x) {
+    const int s = s0 + (int)threadIdx.x;
+    const int f = s < hi && items_of(gmol(P, par, s)) == 0 ? 1 : 0;
+    int t;
+    const int o = block_exscan(f, x.iscr, &t);
+    if (f) a->far_list[P->near_off + lo + n_far + o] = s;
+    n_far += t;
+  }
+  if (threadIdx.x == 0) x.iscr[61] = n_far;
   for (int s = lo + (int)threadIdx.x; s < hi; s += blockDim.x) {
     const size_t ms = gmol(P, par, s);
     const int c = items_of(ms);
@@ -1523,11 +1626,12 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
  * (30-100 partners next to a large ion) are walked by 2^lg lanes each, the
  * lanes' sums added by shuffles and handed to the molecule's own lane, which
  * then finishes it like a light one: force, gas-gas and intramolecular terms,
- * second kick.  The reactions go to the core sums by
+ * second kick.  With `drift` the molecule's first kick and drift come first,
+ * in the same registers: its slab rows are read and written once per step.  The reactions go to the core sums by
  * shared 32-bit integer atomics on exact chunks (acc_add); all sums are
  * integers, so neither the split nor the order changes the result. */
 template <int AG, bool FP64, bool E>
-__device__ __forceinline__ void near_group(Ctx& x, int first, int n, int lg, bool kick) {
+__device__ __forceinline__ void near_group(Ctx& x, int first, int n, int lg, bool kick, bool drift) {
   const RepParams* P = x.P;
   const KArgs* a = x.a;
   const bool gi = term_on(x, MDN_I_GI), gv = term_on(x, MDN_I_GV);
@@ -1543,10 +1647,21 @@ __device__ __forceinline__ void near_group(Ctx& x, int first, int n, int lg, boo
   const bool own = lane < n;
   const int4 rc = own ? a->near_rec[P->near_off + first + lane] : make_int4(0, 0, 0, 0);
   const size_t g0 = gatom(P, par, rc.x, 0);
-  double X[3 * AG];
+  double X[3 * AG], V[3 * AG];
   float3 gp[AG];
 #pragma unroll
-  for (int q = 0; q < 3 * AG; q++) X[q] = own ? a->slab_x[3 * g0 + q] : 0.0;
+  for (int q = 0; q < 3 * AG; q++) {
+    X[q] = own ? a->slab_x[3 * g0 + q] : 0.0;
+    V[q] = own && kick ? a->slab_v[3 * g0 + q] : 0.0;
+  }
+  if (drift && own) { /* a rigid gas was drifted before */
+#pragma unroll
+    for (int q = 0; q < 3 * AG; q++) {
+      V[q] += a->slab_f[3 * g0 + q] * x.c.c2[gtype[q / 3]];
+      X[q] = X[q] + V[q] * P->dt;
+    }
+    gas_finite<AG>(x, X, V);
+  }
 #pragma unroll
   for (int at = 0; at < AG; at++)
     gp[at] = make_float3((float)(X[3 * at] - com[0]), (float)(X[3 * at + 1] - com[1]),
@@ -1608,7 +1723,8 @@ __device__ __forceinline__ void near_group(Ctx& x, int first, int n, int lg, boo
     }
 #pragma unroll
     for (int q = 0; q < 3 * AG; q++) {
-      if (kick) a->slab_v[3 * g0 + q] += Fd[q] * x.c.c2[gtype[q / 3]];
+      if (drift) a->slab_x[3 * g0 + q] = X[q];
+      if (kick) a->slab_v[3 * g0 + q] = V[q] + Fd[q] * x.c.c2[gtype[q / 3]];
       a->slab_f[3 * g0 + q] = Fd[q];
     }
   }
@@ -1686,7 +1802,7 @@ __device__ __forceinline__ void core_reduce(Ctx& x, cg::cluster_group& cl) {
  * CTA of their slab partition.  With the cycle accounting on, the kinds run
  * one after another, each with its own barrier. */
 template <bool E>
-__device__ __forceinline__ void force_items(Ctx& x, bool kick) {
+__device__ __forceinline__ void force_items(Ctx& x, bool kick, bool drift) {
   const RepParams* P = x.P;
   const int nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   const bool pairs = term_on(x, MDN_I_AMBER) || term_on(x, MDN_I_BMH) || term_on(x, MDN_I_VI) || term_on(x, MDN_I_VV);
@@ -1725,8 +1841,8 @@ __device__ __forceinline__ void force_items(Ctx& x, bool kick) {
         const int k = it - mc;
         const bool heavy = k < gh;
         const int f = heavy ? k * hs : nh + 32 * (k - gh), n = heavy ? min(hs, nh - f) : min(32, nn - f);
-        if (P->a_g == 1) near_group<1, kFP64Pairs, E>(x, lo + f, n, heavy ? lg : 0, kick);
-        else near_group<2, kFP64Pairs, E>(x, lo + f, n, heavy ? lg : 0, kick);
+        if (P->a_g == 1) near_group<1, kFP64Pairs, E>(x, lo + f, n, heavy ? lg : 0, kick, drift);
+        else near_group<2, kFP64Pairs, E>(x, lo + f, n, heavy ? lg : 0, kick, drift);
       }
       int next = 0;
       if (lane == 0) next = atomicAdd(&x.iscr[60], 1);
@@ -1740,9 +1856,9 @@ __device__ __forceinline__ void force_items(Ctx& x, bool kick) {
 }
 
 /* the forces, and the second kick */
-__device__ __forceinline__ void forces_and_kick(Ctx& x, cg::cluster_group& cl, bool eflag, bool kick) {
-  if (eflag) force_items<true>(x, kick);
-  else force_items<false>(x, kick);
+__device__ __forceinline__ void forces_and_kick(Ctx& x, cg::cluster_group& cl, bool eflag, bool kick, bool drift) {
+  if (eflag) force_items<true>(x, kick, drift);
+  else force_items<false>(x, kick, drift);
   __syncthreads();
   prof_start(x);
   core_reduce(x, cl);
@@ -2422,7 +2538,8 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
 }
 
 /* ------------------------------------------------------------------------- */
-__device__ __forceinline__ void one_step(Ctx& x, cg::cluster_group& cl, bool eflag) {
+__device__ __forceinline__ void one_step(Ctx& x, cg::cluster_group& cl, bool eflag, bool rebuild, bool gg,
+                                         bool far_done) {
   const RepParams* P = x.P;
   prof_start(x);
   core_kick(x);
@@ -2434,11 +2551,8 @@ __device__ __forceinline__ void one_step(Ctx& x, cg::cluster_group& cl, bool efl
       for (int k = 0; k < 3; k++) x.c.v[3 * i + k] *= ratio;
     __syncthreads();
   }
-  const bool rebuild = x.D->loop_pair + 1 > x.D->loop_update;
-  /* with gas-gas forces no gas molecule can take its force during its own
-   * drift: they need every molecule's new position */
-  const bool gg = kGG && (P->interactions & MDN_I_GG) && P->ggl_cap > 0;
-  core_drift_shake(x, !rebuild && !gg, eflag);
+  const bool apart = rebuild || gg, fused = !apart && !gas_rigid(P) && x.iscr[57] > (int)blockDim.x;
+  core_drift_shake(x, GasWork{apart, !apart && !far_done, !apart && !fused}, eflag);
   ion_centre(x);
   if (x.D->nvt_mode == MDN_NVT_NH) {
     double T = ion_temperature(x);
@@ -2460,13 +2574,13 @@ __device__ __forceinline__ void one_step(Ctx& x, cg::cluster_group& cl, bool efl
     prof_end(x, MDN_PROF_REBUILD);
   }
   if (gg) gas_gg_pass(x, cl, eflag, rebuild);
-  if (rebuild || gg) {
+  if (apart) {
     prof_start(x);
     gas_far_pass(x, eflag, true);
     __syncthreads();
     prof_end(x, MDN_PROF_REBUILD);
   }
-  forces_and_kick(x, cl, eflag, true);
+  forces_and_kick(x, cl, eflag, true, fused);
   if (x.D->nvt_mode == MDN_NVT_NH) {
     double Coeff = exp(-x.D->zeta * 0.5 * P->dt);
     for (int i = threadIdx.x; i < P->n_ion; i += blockDim.x)
@@ -2566,13 +2680,28 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     if (threadIdx.x < sP.a_g) iscr[58 + threadIdx.x] = x.ib[sP.o_gas_type + threadIdx.x];
     const long long job_t0 = clock64();
     if ((a.mode == MDN_MODE_STEP || a.mode == MDN_MODE_FORCES) && sD.near_C != x.C) build_near(x, cl);
-    else if (threadIdx.x < 2)
-      iscr[56 + threadIdx.x] = a.near_cnt[2 * ((size_t)r * 8 + x.rank) + threadIdx.x];
+    else if (threadIdx.x < 3)
+      iscr[threadIdx.x < 2 ? 56 + threadIdx.x : 61] = a.near_cnt[3 * ((size_t)r * 8 + x.rank) + threadIdx.x];
     __syncthreads();
     if (a.mode == MDN_MODE_STEP) {
+      const bool gg = kGG && (sP.interactions & MDN_I_GG) && sP.ggl_cap > 0;
+      long long ahead = 0; /* steps the far molecules have already made */
+      bool far_done = false;
       for (long long s = 0; s < a.n_steps; s++) {
-        bool eflag = a.energy_mode == 2 || (a.energy_mode == 1 && s == a.n_steps - 1);
-        one_step(x, cl, eflag);
+        const bool eflag = a.energy_mode == 2 || (a.energy_mode == 1 && s == a.n_steps - 1);
+        const bool rebuild = sD.loop_pair + 1 > sD.loop_update;
+        if (rebuild || gg) {
+          far_done = false;
+        } else {
+          if (ahead == 0 && (far_done = iscr[61] > (int)blockDim.x)) {
+            ahead = min(a.n_steps - s, (long long)sD.loop_update - sD.loop_pair);
+            prof_start(x);
+            gas_far_steps(x, ahead, a.energy_mode, s + ahead == a.n_steps);
+            prof_end(x, MDN_PROF_GAS_INT);
+          }
+          if (far_done) ahead--;
+        }
+        one_step(x, cl, eflag, rebuild, gg, far_done);
       }
     } else if (a.mode == MDN_MODE_FORCES) {
       /* the ion centre serves only as the origin of the FP32 coordinates here */
@@ -2584,7 +2713,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
       gas_gg_pass(x, cl, true, false);
       gas_far_pass(x, true, false);
       __syncthreads();
-      forces_and_kick(x, cl, true, false);
+      forces_and_kick(x, cl, true, false, false);
       if (threadIdx.x == 0)
         for (int k = 0; k < 6; k++) sD.ion_com[k] = keep[k];
       __syncthreads();
@@ -2601,7 +2730,8 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
         atomicAdd((unsigned long long*)&a.prof[(size_t)r * MDN_PROF_N + k], (unsigned long long)s_prof[k]);
     }
     store_core(x);
-    if (threadIdx.x < 2) a.near_cnt[2 * ((size_t)r * 8 + x.rank) + threadIdx.x] = iscr[56 + threadIdx.x];
+    if (threadIdx.x < 3)
+      a.near_cnt[3 * ((size_t)r * 8 + x.rank) + threadIdx.x] = iscr[threadIdx.x < 2 ? 56 + threadIdx.x : 61];
     __syncthreads();
     if (x.rank == 0 && threadIdx.x == 0) {
       a.D[r] = sD;

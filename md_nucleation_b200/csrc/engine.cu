@@ -159,7 +159,7 @@ struct mdn_handle {
   int* vslab_mol = nullptr;
   int4* near_rec = nullptr;
   unsigned short* near_item = nullptr;
-  int* near_cnt = nullptr;
+  int *near_cnt = nullptr, *far_list = nullptr;
   int *near_gi = nullptr, *near_gv = nullptr;
   unsigned short *gil_n = nullptr, *gvl_n = nullptr, *gil = nullptr, *gvl = nullptr;
   int *ggl_start = nullptr, *ggl_n = nullptr, *ggl = nullptr, *slab_ins = nullptr;
@@ -205,7 +205,7 @@ namespace {
 void free_all(mdn_handle* h) {
   void* ptrs[] = {h->dP, h->dD, h->d_iblob, h->d_dblob, h->ion_x, h->ion_v, h->ion_f, h->mol_x, h->mol_v,
                   h->region, h->slot, h->slab_x, h->slab_v, h->slab_f, h->slab_mol, h->vslab_x, h->vslab_v,
-                  h->vslab_f, h->vslab_w, h->vslab_mol, h->near_rec, h->near_item, h->near_cnt, h->near_gi, h->near_gv, h->gil_n,
+                  h->vslab_f, h->vslab_w, h->vslab_mol, h->near_rec, h->near_item, h->near_cnt, h->far_list, h->near_gi, h->near_gv, h->gil_n,
                   h->gvl_n, h->gil, h->gvl, h->energy, h->events, h->n_events, h->status, h->job_order,
                   h->job_counter, h->snap_off, h->snap_type, h->snap_x, h->snap_v, h->d_ctl_mode,
                   h->d_ctl_T, h->d_prof, h->job_order2, h->job_counter2, h->ggl_start, h->ggl_n, h->ggl,
@@ -306,7 +306,7 @@ long long launch(mdn_handle* h, int mode, long long n_steps, int energy_mode, un
   a.slab_x = h->slab_x; a.slab_v = h->slab_v; a.slab_f = h->slab_f; a.slab_mol = h->slab_mol;
   a.vslab_x = h->vslab_x; a.vslab_v = h->vslab_v; a.vslab_f = h->vslab_f; a.vslab_w = h->vslab_w;
   a.vslab_mol = h->vslab_mol;
-  a.near_rec = h->near_rec; a.near_item = h->near_item; a.near_cnt = h->near_cnt;
+  a.near_rec = h->near_rec; a.near_item = h->near_item; a.near_cnt = h->near_cnt; a.far_list = h->far_list;
   a.near_gi = h->near_gi; a.near_gv = h->near_gv;
   a.gil_n = h->gil_n; a.gvl_n = h->gvl_n; a.gil = h->gil; a.gvl = h->gvl;
   a.ggl_start = h->ggl_start; a.ggl_n = h->ggl_n; a.ggl = h->ggl;
@@ -779,7 +779,8 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
   ALLOC(h->vslab_mol, vslab_mols);
   ALLOC(h->near_rec, near_tot);
   ALLOC(h->near_item, nit_tot);
-  ALLOC(h->near_cnt, 16 * (size_t)R);
+  ALLOC(h->near_cnt, 24 * (size_t)R);
+  ALLOC(h->far_list, near_tot);
   ALLOC(h->near_gi, slab_mols);
   ALLOC(h->near_gv, slab_mols);
   ALLOC(h->gil_n, slab_mols);
@@ -832,7 +833,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
   ck(cudaMemset(h->energy, 0, sizeof(long long) * 8 * R), "energy");
   ck(cudaMemset(h->n_events, 0, sizeof(int)), "events");
   ck(cudaMemset(h->status, 0, sizeof(int) * R), "status");
-  ck(cudaMemset(h->near_cnt, 0, sizeof(int) * 16 * R), "near_cnt");
+  ck(cudaMemset(h->near_cnt, 0, sizeof(int) * 24 * R), "near_cnt");
   ck(cudaMemset(h->near_gi, 0xff, sizeof(int) * slab_mols), "near_gi");
   if (h->slab_ins) ck(cudaMemset(h->slab_ins, 0xff, sizeof(int) * slab_mols), "slab_ins");
   if (h->ggl_n) ck(cudaMemset(h->ggl_n, 0, sizeof(int) * slab_mols), "ggl_n");

@@ -130,7 +130,8 @@ typedef struct KArgs {
   int4* near_rec;          /* near molecules of each CTA's slab partition, from its first slot:
                               {slab slot, first item, items, 0}, most items first */
   unsigned short* near_item; /* their partners, core atom indices (build_near) */
-  int* near_cnt;           /* [replica][8 ranks][2] heavy / all near records of the rank */
+  int* far_list;           /* slab slots of the other molecules, from the partition's first slot */
+  int* near_cnt;           /* [replica][8 ranks][3] heavy / all near records, far molecules */
   int* near_gi;            /* [slab slot] start of its gi entries (-1 = none)  */
   int* near_gv;            /* [slab slot] start of its gv entries              */
   unsigned short *gil_n, *gvl_n; /* [slab slot] entry counts                   */
