@@ -64,7 +64,9 @@ __device__ __forceinline__ int tag_slot(unsigned k) { return (int)(k >> 8) - 1; 
 struct Core {
   double* x;        /* [3*nc] positions                        */
   double* v;        /* [3*nc] velocities                       */
-  double* f;        /* [3*nc] force of the last evaluation     */
+  double* f;        /* [3*nc] force of the last evaluation; from the drift to the
+                     * next evaluation, the positions before the drift (the SHAKE
+                     * reference vectors) */
   long long* acc;   /* [3*nc] this CTA's fixed-point force sums */
   unsigned* chunk;  /* [9*nc] the same sums in 32-bit chunks (acc_add) */
   float4* pos;      /* [nc] (x - ion centre, charge), FP32     */
@@ -72,7 +74,7 @@ struct Core {
   unsigned* excl;   /* AMBER exclusions, n_ion rows            */
   float2* lj;       /* [nt*nt] 48 eps s^12, 24 eps s^6         */
   double* c2;       /* [nt] 0.5*dt*4.184e-4 / mass             */
-  int* vcolor;      /* scratch                                 */
+  double* mass;     /* [nt]                                    */
 };
 
 struct Ctx {
@@ -83,6 +85,7 @@ struct Ctx {
   int r;            /* replica                          */
   int rank, C;      /* cluster rank and size            */
   int n_core;       /* atoms in the core                */
+  bool settled;     /* every CTA of the cluster has read this one's sums (settle) */
   int* iscr;        /* >= 64 ints of scratch            */
   int* cand;        /* [MDN_INSERT_MAX_VAPOR + 1] entering vapor molecules, count last */
   double* trial;    /* [3*MDN_MAX_VAP_ATOMS] trial atoms */
@@ -133,6 +136,7 @@ __device__ __forceinline__ void load_ion(Ctx& x) {
       x.c.v[3 * i + k] = a->ion_v[3 * g + k];
       x.c.f[3 * i + k] = a->ion_f[3 * g + k];
     }
+    x.c.pos[i].w = (float)x.db[P->d_ion_q + i];
     x.c.tag[i].w = 1.0f;
     x.c.tag[i].k = (unsigned)x.ib[P->o_ion_type + i] | (x.ib[P->o_ion_bmh + i] ? 128u : 0u);
   }
@@ -153,6 +157,7 @@ __device__ __forceinline__ void load_vapor(Ctx& x) {
       x.c.v[3 * i + k] = a->vslab_v[3 * g + k];
       x.c.f[3 * i + k] = a->vslab_f[3 * g + k];
     }
+    x.c.pos[i].w = (float)x.db[P->d_vap_q + at];
     x.c.tag[i].w = a->vslab_w[g];
     x.c.tag[i].k = (unsigned)x.ib[P->o_vap_type + at] | ((unsigned)(s + 1) << 8);
   }
@@ -187,10 +192,25 @@ __device__ __forceinline__ void store_core(Ctx& x) {
 /* ------------------------------------------------------------------------- */
 /* integration of the core                                                    */
 /* ------------------------------------------------------------------------- */
-__device__ __forceinline__ void core_kick(Ctx& x) {
-  for (int i = threadIdx.x; i < x.n_core; i += blockDim.x) {
-    double c2 = x.c.c2[tag_type(x.c.tag[i].k)];
-    for (int k = 0; k < 3; k++) x.c.v[3 * i + k] += x.c.f[3 * i + k] * c2;
+/* First kick (unless it was made) and drift of the core, each thread its own
+ * components (thread t: t, t + blockDim.x, ... of the 3 n_core), those whose
+ * force it summed and whose second kick it made (core_reduce_kick): no
+ * barrier in between.  The positions before the drift stay in c.f for the
+ * constraints. */
+__device__ __forceinline__ double core_c2(const Ctx& x, int q) { return x.c.c2[tag_type(x.c.tag[q / 3].k)]; }
+
+__device__ __forceinline__ void core_drift(Ctx& x, bool kick) {
+  const double dt = x.P->dt;
+  const int n3 = 3 * x.n_core;
+  for (int q = threadIdx.x; q < n3; q += blockDim.x) {
+    double v = x.c.v[q];
+    if (kick) {
+      v += x.c.f[q] * core_c2(x, q);
+      x.c.v[q] = v;
+    }
+    const double xo = x.c.x[q];
+    x.c.f[q] = xo;
+    x.c.x[q] = xo + v * dt;
   }
 }
 
@@ -201,7 +221,7 @@ __device__ __forceinline__ double ion_temperature(Ctx& x) {
   if (threadIdx.x < 32) {
     double K = 0;
     for (int i = threadIdx.x; i < P->n_ion; i += 32) {
-      double m = x.db[P->d_mass + tag_type(x.c.tag[i].k)];
+      double m = x.c.mass[tag_type(x.c.tag[i].k)];
       K += x.c.v[3 * i] * x.c.v[3 * i] * m;
       K += x.c.v[3 * i + 1] * x.c.v[3 * i + 1] * m;
       K += x.c.v[3 * i + 2] * x.c.v[3 * i + 2] * m;
@@ -253,12 +273,14 @@ __device__ __forceinline__ double shake_res_c(const double* Xi, const double* Xj
  * constraint table (d^2, 1/m_i, 1/m_j).  Returns true once every
  * (|s_k|^2 - d_k^2)^2 <= 1e-20 A^4, the sweeps' criterion; false after 50
  * steps or a singular system, and the caller sweeps from there. */
-__device__ bool shake_group(double* X, const double* R, const int* rig, const double* ct, const int* ks, int n) {
-  int I[3], J[3];
-  double r[3][3], d2[3], ci[3], cj[3], w[3][3];
+template <int N>
+__device__ __forceinline__ bool shake_group_n(double* X, const double* R, const int* rig, const double* ct,
+                                              const int* ks) {
+  int I[N], J[N];
+  double r[N][3], d2[N], ci[N], cj[N], w[N][N];
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const int c = ks[k < n ? k : 0];
+  for (int k = 0; k < N; k++) {
+    const int c = ks[k];
     I[k] = rig[3 * c];
     J[k] = rig[3 * c + 1];
     d2[k] = ct[3 * c];
@@ -267,57 +289,73 @@ __device__ bool shake_group(double* X, const double* R, const int* rig, const do
 #pragma unroll
     for (int q = 0; q < 3; q++) r[k][q] = R[3 * I[k] + q] - R[3 * J[k] + q];
   }
-  /* d s_k / d l_l = w_kl r_l; rows and columns past n: the identity */
+  /* d s_k / d l_l = w_kl r_l */
 #pragma unroll
-  for (int k = 0; k < 3; k++)
+  for (int k = 0; k < N; k++)
 #pragma unroll
-    for (int l = 0; l < 3; l++) {
+    for (int l = 0; l < N; l++) {
       const double ai = I[k] == I[l] ? ci[l] : (I[k] == J[l] ? -cj[l] : 0.0);
       const double aj = J[k] == I[l] ? ci[l] : (J[k] == J[l] ? -cj[l] : 0.0);
-      w[k][l] = (k < n && l < n) ? ai - aj : 0.0;
+      w[k][l] = ai - aj;
     }
   for (int it = 0; it < 50; it++) {
-    double s[3][3], f[3];
+    double s[N][3], f[N];
     bool ok = true;
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
+    for (int k = 0; k < N; k++) {
 #pragma unroll
       for (int q = 0; q < 3; q++) s[k][q] = X[3 * I[k] + q] - X[3 * J[k] + q];
-      const double dr = s[k][0] * s[k][0] + s[k][1] * s[k][1] + s[k][2] * s[k][2] - d2[k];
-      f[k] = k < n ? dr : 0.0;
-      if (k < n && !(dr * dr <= 1e-20)) ok = false;
+      f[k] = s[k][0] * s[k][0] + s[k][1] * s[k][1] + s[k][2] * s[k][2] - d2[k];
+      if (!(f[k] * f[k] <= 1e-20)) ok = false;
     }
     if (ok) return true;
-    double A[3][3];
+    double A[N][N];
 #pragma unroll
-    for (int k = 0; k < 3; k++)
+    for (int k = 0; k < N; k++)
 #pragma unroll
-      for (int l = 0; l < 3; l++)
-        A[k][l] = (k < n && l < n) ? 2.0 * (s[k][0] * r[l][0] + s[k][1] * r[l][1] + s[k][2] * r[l][2]) * w[k][l]
-                                   : (k == l ? 1.0 : 0.0);
-    /* A d = -f by Cramer's rule */
-    const double c00 = A[1][1] * A[2][2] - A[1][2] * A[2][1];
-    const double c01 = A[1][0] * A[2][2] - A[1][2] * A[2][0];
-    const double c02 = A[1][0] * A[2][1] - A[1][1] * A[2][0];
-    const double det = A[0][0] * c00 - A[0][1] * c01 + A[0][2] * c02;
-    if (!(fabs(det) > 1e-300)) return false;
-    const double inv = 1.0 / det;
-    const double b0 = -f[0], b1 = -f[1], b2 = -f[2];
-    const double D0 = (b0 * c00 - A[0][1] * (b1 * A[2][2] - A[1][2] * b2) + A[0][2] * (b1 * A[2][1] - A[1][1] * b2)) * inv;
-    const double D1 = (A[0][0] * (b1 * A[2][2] - A[1][2] * b2) - b0 * c01 + A[0][2] * (A[1][0] * b2 - b1 * A[2][0])) * inv;
-    const double D2 = (A[0][0] * (A[1][1] * b2 - b1 * A[2][1]) - A[0][1] * (A[1][0] * b2 - b1 * A[2][0]) + b0 * c02) * inv;
-    const double Dl[3] = {D0, D1, D2};
+      for (int l = 0; l < N; l++)
+        A[k][l] = 2.0 * (s[k][0] * r[l][0] + s[k][1] * r[l][1] + s[k][2] * r[l][2]) * w[k][l];
+    /* A d = -f by Cramer's rule; for one and two constraints what the rule
+     * for three gives with identity rows, without its products by 0 and 1 */
+    double Dl[N];
+    if constexpr (N == 1) {
+      if (!(fabs(A[0][0]) > 1e-300)) return false;
+      Dl[0] = -f[0] * (1.0 / A[0][0]);
+    } else if constexpr (N == 2) {
+      const double det = A[0][0] * A[1][1] - A[0][1] * A[1][0];
+      if (!(fabs(det) > 1e-300)) return false;
+      const double inv = 1.0 / det;
+      const double b0 = -f[0], b1 = -f[1];
+      Dl[0] = (b0 * A[1][1] - A[0][1] * b1) * inv;
+      Dl[1] = (A[0][0] * b1 - b0 * A[1][0]) * inv;
+    } else {
+      const double c00 = A[1][1] * A[2][2] - A[1][2] * A[2][1];
+      const double c01 = A[1][0] * A[2][2] - A[1][2] * A[2][0];
+      const double c02 = A[1][0] * A[2][1] - A[1][1] * A[2][0];
+      const double det = A[0][0] * c00 - A[0][1] * c01 + A[0][2] * c02;
+      if (!(fabs(det) > 1e-300)) return false;
+      const double inv = 1.0 / det;
+      const double b0 = -f[0], b1 = -f[1], b2 = -f[2];
+      Dl[0] = (b0 * c00 - A[0][1] * (b1 * A[2][2] - A[1][2] * b2) + A[0][2] * (b1 * A[2][1] - A[1][1] * b2)) * inv;
+      Dl[1] = (A[0][0] * (b1 * A[2][2] - A[1][2] * b2) - b0 * c01 + A[0][2] * (A[1][0] * b2 - b1 * A[2][0])) * inv;
+      Dl[2] = (A[0][0] * (A[1][1] * b2 - b1 * A[2][1]) - A[0][1] * (A[1][0] * b2 - b1 * A[2][0]) + b0 * c02) * inv;
+    }
 #pragma unroll
-    for (int l = 0; l < 3; l++) {
-      if (l >= n) break;
+    for (int l = 0; l < N; l++)
 #pragma unroll
       for (int q = 0; q < 3; q++) {
         X[3 * I[l] + q] += Dl[l] * ci[l] * r[l][q];
         X[3 * J[l] + q] -= Dl[l] * cj[l] * r[l][q];
       }
-    }
   }
   return false;
+}
+
+__device__ __forceinline__ bool shake_group(double* X, const double* R, const int* rig, const double* ct,
+                                            const int* ks, int n) {
+  if (n == 1) return shake_group_n<1>(X, R, rig, ct, ks);
+  if (n == 2) return shake_group_n<2>(X, R, rig, ct, ks);
+  return shake_group_n<3>(X, R, rig, ct, ks);
 }
 
 __device__ __forceinline__ bool gas_rigid(const RepParams* P) {
@@ -341,56 +379,32 @@ struct GasWork {
 
 __device__ __forceinline__ void gas_integrate(Ctx& x, GasWork w, bool eflag, int tid, int nthr);
 
-/* Drift of the core, its constraints, and the step's gas integration.
- * The constraints and the gas are independent (the gas pass touches only
- * the gas slab), so they run side by side: warp 0 sweeps the ion's
- * constraints, the next warps take one vapor molecule per thread, and the
- * remaining warps integrate the gas molecules. */
-__device__ __forceinline__ void core_drift_shake(Ctx& x, GasWork gas, bool eflag) {
+/* which of the core's molecules have constraints */
+struct CoreCons {
+  bool ion;  /* the ion's constraints are on */
+  int nv;    /* vapor molecules whose constraints are on */
+};
+__device__ __forceinline__ CoreCons core_cons(const Ctx& x) {
   const RepParams* P = x.P;
-  /* positions before the drift (the SHAKE reference vectors) live in the
-   * 64-bit sum buffer: core_reduce overwrites it only after this step's
-   * forces, and no CTA of the cluster reads it any more (core_reduce ends
-   * with a cluster barrier) */
-  double* const xold = (double*)x.c.acc;
   const bool sh = (P->interactions & MDN_I_SHAKE) != 0;
-  const bool vcorr = !(P->quirks & MDN_Q_SHAKE_NO_VCORR);
-  const double dt = P->dt;
-  for (int i = threadIdx.x; i < x.n_core; i += blockDim.x) {
-    for (int k = 0; k < 3; k++) {
-      double xo = x.c.x[3 * i + k];
-      xold[3 * i + k] = xo;
-      x.c.x[3 * i + k] = xo + x.c.v[3 * i + k] * dt;
-    }
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  const bool ion_sh = sh && P->n_ion_rigid > 0;
-  const int nv = (sh && P->n_vap_rigid > 0) ? x.D->n_vap_in : 0;
-  /* warps of the ion constraints, of the vapor molecules, then of the gas */
-  const int w_ion = ion_sh ? 1 : 0;
-  const int w_vap = nv > 0 ? min((nv + 31) >> 5, max(1, (nwarps - w_ion) / 2)) : 0;
-  const int w_gas0 = min(w_ion + w_vap, nwarps - 1);
-  if (ion_sh && warp == 0) {
-    /* sweeps in colour order (a colour's constraints share no atom, so
-     * the lanes may take them in any order) until every constraint holds
-     * after a sweep */
+  return CoreCons{sh && P->n_ion_rigid > 0, sh && P->n_vap_rigid > 0 ? x.D->n_vap_in : 0};
+}
+
+/* The sweeps in colour order (a colour's constraints share no atom, so the
+ * lanes may take them in any order) until every constraint holds after a
+ * sweep: for the ion by warp 0, for a vapor molecule by one thread.  Taken
+ * when a molecule has no groups (more than three constraints share atoms)
+ * or Newton's method gave one up; marked vapor molecules have a nonzero word
+ * at their first chunk sum, which is cleared. */
+__device__ __forceinline__ void core_sweeps(Ctx& x, const CoreCons& cc, bool ion, bool vapor) {
+  const RepParams* P = x.P;
+  const double* const xold = x.c.f;
+  const int lane = threadIdx.x & 31;
+  if (ion && threadIdx.x < 32) {
     const int* rig = x.ib + P->o_ion_rigid;
     const int* col = x.ib + P->o_ion_color;
-    /* the ion's groups (an atom and its constrained hydrogens) share no
-     * atom: the lanes solve them independently */
-    bool done = false;
-    if (P->n_ion_groups > 0) {
-      const int* grp = x.ib + P->o_ion_grp;
-      const int* gst = x.ib + P->o_ion_gstart;
-      bool ok = true;
-      for (int g = lane; g < P->n_ion_groups; g += 32)
-        ok = shake_group(x.c.x, xold, rig, x.db + P->d_ion_cons, grp + gst[g], gst[g + 1] - gst[g]) && ok;
-      done = __all_sync(0xffffffffu, ok);
-      __syncwarp();
-    }
     int sweeps = 0;
-    for (; !done;) {
+    for (;;) {
       for (int c = 0; c < P->n_ion_colors; c++) {
         for (int k = lane; k < P->n_ion_rigid; k += 32) {
           if (col[k] != c) continue;
@@ -409,32 +423,19 @@ __device__ __forceinline__ void core_drift_shake(Ctx& x, GasWork gas, bool eflag
         break;
       }
     }
-    if (vcorr)
-      for (int i = lane; i < P->n_ion; i += 32)
-        for (int k = 0; k < 3; k++) {
-          /* displacement by the constraints = x - (xold + v*dt) */
-          double xd = xold[3 * i + k] + x.c.v[3 * i + k] * dt;
-          x.c.v[3 * i + k] += (x.c.x[3 * i + k] - xd) / dt;
-        }
-  } else if (nv > 0 && warp >= w_ion && warp < w_ion + w_vap) {
-    /* vapor molecules: one thread each, in place in shared memory, sweeps
-     * in colour order until every constraint holds after a sweep */
+  }
+  if (vapor) {
     const int av = P->a_v, nr = P->n_vap_rigid, nco = P->n_vap_colors;
     const int* rig = x.ib + P->o_vap_rigid;
     const int* col = x.ib + P->o_vap_color;
     const double* ct = x.db + P->d_vap_cons;
-    for (int s = threadIdx.x - 32 * w_ion; s < nv; s += 32 * w_vap) {
+    for (int s = threadIdx.x; s < cc.nv; s += blockDim.x) {
       const int base = P->n_ion + s * av;
+      if (P->n_vap_groups > 0 && x.c.chunk[9 * base] == 0) continue;
+      x.c.chunk[9 * base] = 0;
       double* X = x.c.x + 3 * base;
       const double* R = xold + 3 * base;
       bool conv = false;
-      if (P->n_vap_groups > 0) {
-        const int* grp = x.ib + P->o_vap_grp;
-        const int* gst = x.ib + P->o_vap_gstart;
-        conv = true;
-        for (int g = 0; g < P->n_vap_groups; g++)
-          conv = shake_group(X, R, rig, ct, grp + gst[g], gst[g + 1] - gst[g]) && conv;
-      }
       for (int sweep = 0; sweep < MDN_SHAKE_MAX_SWEEPS && !conv; sweep++) {
         for (int c = 0; c < nco; c++)
           for (int k = 0; k < nr; k++) {
@@ -447,38 +448,75 @@ __device__ __forceinline__ void core_drift_shake(Ctx& x, GasWork gas, bool eflag
           if (!(shake_res_c(X + 3 * rig[3 * k], X + 3 * rig[3 * k + 1], ct + 3 * k) <= 1e-20)) conv = false;
       }
       if (!conv && x.rank == 0) set_status(x, MDN_ST_SHAKE_NOCONV);
-      if (vcorr)
-        for (int q = 0; q < 3 * av; q++) {
-          /* displacement by the constraints = x - (xold + v*dt) */
-          const double xd = R[q] + x.c.v[3 * base + q] * dt;
-          x.c.v[3 * base + q] += (X[q] - xd) / dt;
-        }
     }
-  } else if (warp >= w_gas0) {
-    gas_integrate(x, gas, eflag, threadIdx.x - 32 * w_gas0, blockDim.x - 32 * w_gas0);
   }
   __syncthreads();
 }
 
-/* ion centre: warp 0, lane-strided partial sums, butterfly, fixed order */
-__device__ __forceinline__ void ion_centre(Ctx& x) {
+/* The core's constraints, one group (constraints that share atoms) per
+ * thread, in units of a warp whose groups have the same number of
+ * constraints: the ion's groups of three, two and one (an atom and its
+ * hydrogens), then the same group of every vapor molecule.  The step's gas
+ * integration runs beside them (the gas pass touches only the gas slab), on
+ * the warps that have no unit.  (One thread per vapor molecule, and the
+ * ion's groups on one warp, made the serial solution of several groups the
+ * longest chain of the step; groups of different sizes in one warp would be
+ * solved one size after another.)  The velocities take the constraints'
+ * displacement in core_place. */
+__device__ __forceinline__ void core_shake(Ctx& x, const CoreCons& cc, GasWork gas, bool eflag) {
   const RepParams* P = x.P;
-  if (threadIdx.x < 32) {
-    double s[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < P->n_ion; i += 32) {
-      double m = x.db[P->d_mass + tag_type(x.c.tag[i].k)];
-      for (int k = 0; k < 3; k++) {
-        s[k] += x.c.x[3 * i + k] * m;
-        s[3 + k] += x.c.v[3 * i + k] * m;
+  const double* const xold = x.c.f;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int n3 = cc.ion ? P->ion_groups_n[2] : 0, n2 = cc.ion ? P->ion_groups_n[1] : 0,
+            n1 = cc.ion ? P->ion_groups_n[0] : 0;
+  const int u3 = (n3 + 31) >> 5, u2 = u3 + ((n2 + 31) >> 5), u1 = u2 + ((n1 + 31) >> 5);
+  const int per = (cc.nv + 31) >> 5, units = u1 + P->n_vap_groups * per;
+  const bool any_gas = gas.all || gas.far || gas.near;
+  const int w_sh = min(units, any_gas ? max(1, (3 * nwarps) >> 2) : nwarps);
+  if (warp < w_sh)
+    for (int u = warp; u < units; u += w_sh) {
+      if (u < u1) {
+        /* the ion's groups are stored by size, largest first */
+        const int in = u < u3 ? 32 * u + lane : u < u2 ? 32 * (u - u3) + lane : 32 * (u - u2) + lane;
+        const int n = u < u3 ? 3 : u < u2 ? 2 : 1;
+        const int g = in + (n < 3 ? n3 : 0) + (n < 2 ? n2 : 0);
+        if (in < (n == 3 ? n3 : n == 2 ? n2 : n1) &&
+            !shake_group(x.c.x, xold, x.ib + P->o_ion_rigid, x.db + P->d_ion_cons,
+                         x.ib + P->o_ion_grp + x.ib[P->o_ion_gstart + g], n))
+          atomicOr(&x.iscr[62], 1);
+      } else {
+        const int g = (u - u1) / per, m = 32 * (u - u1 - g * per) + lane, base = P->n_ion + m * P->a_v;
+        const int g0 = x.ib[P->o_vap_gstart + g];
+        if (m < cc.nv && !shake_group(x.c.x + 3 * base, xold + 3 * base, x.ib + P->o_vap_rigid, x.db + P->d_vap_cons,
+                                      x.ib + P->o_vap_grp + g0, x.ib[P->o_vap_gstart + g + 1] - g0)) {
+          x.c.chunk[9 * base] = 1;
+          atomicOr(&x.iscr[62], 2);
+        }
       }
     }
-    for (int k = 0; k < 6; k++) s[k] = warp_sum_d(s[k]);
-    if (threadIdx.x == 0) {
-      double mInv = 1 / P->ion_msum;
-      for (int k = 0; k < 6; k++) x.D->ion_com[k] = s[k] * mInv;
-    }
-  }
+  const int w_gas0 = min(w_sh, nwarps - 1);
+  if (any_gas && warp >= w_gas0)
+    gas_integrate(x, gas, eflag, threadIdx.x - 32 * w_gas0, blockDim.x - 32 * w_gas0);
   __syncthreads();
+  const int fail = x.iscr[62];
+  const bool ion = cc.ion && (u1 == 0 || (fail & 1)), vapor = cc.nv > 0 && (P->n_vap_groups == 0 || (fail & 2));
+  if (ion || vapor) core_sweeps(x, cc, ion, vapor);
+}
+
+/* Centre of the ion atoms' `src` (positions or velocities): every warp for
+ * itself, lane-strided partial sums then a butterfly, so the result depends
+ * on the atom order only, and no warp waits for another's */
+__device__ __forceinline__ void ion_centre(const Ctx& x, const double* src, double* com) {
+  const RepParams* P = x.P;
+  double s[3] = {0, 0, 0};
+  for (int i = threadIdx.x & 31; i < P->n_ion; i += 32) {
+    const double m = x.c.mass[tag_type(x.c.tag[i].k)];
+#pragma unroll
+    for (int k = 0; k < 3; k++) s[k] += src[3 * i + k] * m;
+  }
+  const double mInv = 1 / P->ion_msum;
+#pragma unroll
+  for (int k = 0; k < 3; k++) com[k] = warp_sum_d(s[k]) * mInv;
 }
 
 /* the ion centre in the reference's own order (sequential sum), used where a
@@ -488,7 +526,7 @@ __device__ __forceinline__ void ion_centre_exact(Ctx& x) {
   if (threadIdx.x == 0) {
     double s[6] = {0, 0, 0, 0, 0, 0};
     for (int i = 0; i < P->n_ion; i++) {
-      double m = x.db[P->d_mass + tag_type(x.c.tag[i].k)];
+      double m = x.c.mass[tag_type(x.c.tag[i].k)];
       for (int k = 0; k < 3; k++) {
         s[k] += x.c.x[3 * i + k] * m;
         s[3 + k] += x.c.v[3 * i + k] * m;
@@ -512,23 +550,31 @@ __device__ __forceinline__ double taper(const RepParams* P, const double* com, c
   return C * C;
 }
 
-/* taper weights of the vapor atoms (when `weights`) and the FP32 coordinates
- * of the core relative to the ion centre.  A molecule inserted by the rebuild
- * of this step carries w < 0 and gets 0 for this step: MD::update_position
- * ran before the rebuild, while the molecule was still outside
- * (src/verlet.cpp:109-134), so the reference leaves its weights unset. */
-__device__ __forceinline__ void core_weights_pos(Ctx& x, bool weights) {
+/* The core's place relative to the ion centre `com`: the FP32 coordinates,
+ * the vapor atoms' taper weights (when `weights`) and, with `cc`, what the
+ * constraints' displacement adds to the velocities.  A molecule inserted by
+ * the rebuild of this step carries w < 0 and gets 0 for this step:
+ * MD::update_position ran before the rebuild, while the molecule was still
+ * outside (src/verlet.cpp:109-134), so the reference leaves its weights
+ * unset. */
+__device__ __forceinline__ void core_place(Ctx& x, const double* com, bool weights, const CoreCons& cc) {
   const RepParams* P = x.P;
-  const double* com = x.D->ion_com;
+  const double dt = P->dt;
   if (threadIdx.x == 0) x.iscr[60] = blockDim.x >> 5; /* the force queue: every warp's first item is taken */
   for (int i = threadIdx.x; i < x.n_core; i += blockDim.x) {
+    double* const X = x.c.x + 3 * i;
     if (i >= P->n_ion) {
       if (x.c.tag[i].w < 0.0f) x.c.tag[i].w = 0.0f;
-      else if (weights) x.c.tag[i].w = (float)taper(P, com, x.c.x + 3 * i);
+      else if (weights) x.c.tag[i].w = (float)taper(P, com, X);
     }
-    double q = i < P->n_ion ? x.db[P->d_ion_q + i] : x.db[P->d_vap_q + (i - P->n_ion) % P->a_v];
-    x.c.pos[i] = make_float4((float)(x.c.x[3 * i] - com[0]), (float)(x.c.x[3 * i + 1] - com[1]),
-                             (float)(x.c.x[3 * i + 2] - com[2]), (float)q);
+    if (i < P->n_ion ? cc.ion : cc.nv > 0)
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        /* displacement by the constraints = x - (xold + v*dt) */
+        const double v = x.c.v[3 * i + k], xd = x.c.f[3 * i + k] + v * dt;
+        x.c.v[3 * i + k] = v + (X[k] - xd) / dt;
+      }
+    x.c.pos[i] = make_float4((float)(X[0] - com[0]), (float)(X[1] - com[1]), (float)(X[2] - com[2]), x.c.pos[i].w);
   }
   __syncthreads();
 }
@@ -762,7 +808,7 @@ __device__ __forceinline__ double charge_d(const Ctx& x, int i) {
  * sums are exact for up to 65,536 terms per atom and evaluation (one per
  * near gas molecule, whose list holds at most 64,511, plus at most one per
  * pair tile and per bonded term); the high sum only matters modulo 2^32.
- * core_reduce folds the three into the 64-bit sum exactly, so the result
+ * core_reduce_kick folds the three into the 64-bit sum exactly, so the result
  * does not depend on the order of the adds. */
 __device__ __forceinline__ void acc_add(Ctx& x, int i, const long long* f3) {
   unsigned* A = x.c.chunk + 9 * i;
@@ -1753,12 +1799,30 @@ __device__ __forceinline__ void heavy_cut(int nh, int* size, int* lg) {
   *lg = h == 1 ? 5 : h == 2 ? 4 : 3;
 }
 
-/* sum of the core partials over the cluster -> f (double), identical in every CTA */
-__device__ __forceinline__ void core_reduce(Ctx& x, cg::cluster_group& cl) {
+/* Waits until every CTA of the cluster has read this one's sums, if that
+ * has not been waited for: before they are written again, and before any
+ * other barrier of the cluster. */
+__device__ __forceinline__ void settle(Ctx& x) {
+  if (!x.settled) {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    x.settled = true;
+  }
+}
+
+/* The sums of the core over the cluster as forces, identical in every CTA,
+ * and the second kick (with `cool`, the thermostat's factor on the ion
+ * too).  Each thread keeps to its own components, so what follows up to the next
+ * drift needs no barrier; and the wait for the other CTAs to have read this
+ * one's sums is left to the next evaluation (settle), by when they have. */
+__device__ __forceinline__ void core_reduce_kick(Ctx& x, bool kick, bool cool) {
+  const RepParams* P = x.P;
+  long long* const mine = x.c.acc;
+  const bool one = x.C == 1;
+  settle(x);
+  /* fold the chunk sums into 64-bit sums and clear them for the next
+   * evaluation */
   const int n3 = 3 * x.n_core;
-  long long* mine = x.c.acc;
-  /* fold the chunk sums into this CTA's 64-bit sums (each thread its own
-   * elements) and clear them for the next evaluation */
   for (int q = threadIdx.x; q < n3; q += blockDim.x) {
     unsigned* c = x.c.chunk + 3 * q;
     const unsigned long long s =
@@ -1766,29 +1830,47 @@ __device__ __forceinline__ void core_reduce(Ctx& x, cg::cluster_group& cl) {
     c[0] = c[1] = c[2] = 0;
     mine[q] = (long long)s;
   }
-  if (x.C > 1) {
-    cl.sync();
-    for (int q = threadIdx.x; q < n3; q += blockDim.x) {
-      long long s = 0;
-      for (int k = 0; k < x.C; k++) {
-        const long long* other = cl.map_shared_rank(mine, k);
-        s += other[q];
-      }
-      x.c.f[q] = (double)s * MDN_FIX_INV;
-    }
-    /* every CTA has read this one's sums: the buffer is free again (the
-     * next step's SHAKE keeps its reference positions there) */
-    cl.sync();
-  } else {
-    for (int q = threadIdx.x; q < n3; q += blockDim.x) x.c.f[q] = (double)mine[q] * MDN_FIX_INV;
+  if (!one) {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
-  __syncthreads();
-  /* flag saturated forces, and positions that are no longer finite */
-  if (x.rank == 0)
-    for (int q = threadIdx.x; q < n3; q += blockDim.x) {
-      if (!(fabs(x.c.f[q]) < MDN_FIX_LIMIT)) set_status(x, MDN_ST_FIXED_OVERFLOW);
-      if (!isfinite(x.c.x[q]) || !isfinite(x.c.v[q])) set_status(x, MDN_ST_NONFINITE);
+  if (threadIdx.x == 0) x.iscr[62] = 0; /* the constraints' failure marks */
+  const double coeff = cool ? exp(-x.D->zeta * 0.5 * P->dt) : 1.0;
+  const unsigned at = (unsigned)__cvta_generic_to_shared(mine);
+  for (int q = threadIdx.x; q < n3; q += blockDim.x) {
+    long long s = 0;
+    if (one) {
+      s = mine[q];
+    } else {
+#pragma unroll 8
+      for (int r = 0; r < x.C; r++) {
+        unsigned far;
+        long long v;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(far) : "r"(at + 8 * q), "r"(r));
+        asm volatile("ld.shared::cluster.s64 %0, [%1];" : "=l"(v) : "r"(far));
+        s += v;
+      }
     }
+    const double f = (double)s * MDN_FIX_INV;
+    double v = x.c.v[q];
+    x.c.f[q] = f;
+    /* flag saturated forces, and positions that are no longer finite */
+    if (x.rank == 0) {
+      if (!(fabs(f) < MDN_FIX_LIMIT)) set_status(x, MDN_ST_FIXED_OVERFLOW);
+      if (!isfinite(x.c.x[q] + v)) set_status(x, MDN_ST_NONFINITE);
+    }
+    if (kick) {
+      v += f * core_c2(x, q);
+      if (cool && q < 3 * P->n_ion) v *= coeff;
+      x.c.v[q] = v;
+    }
+  }
+  if (!one) {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    x.settled = false;
+  }
 }
 
 /* All forces of the step (after positions and lists are final) as one queue
@@ -1853,20 +1935,6 @@ __device__ __forceinline__ void force_items(Ctx& x, bool kick, bool drift) {
       prof_end(x, ph == 0 ? MDN_PROF_NEAR : ph == 1 ? MDN_PROF_BONDED : MDN_PROF_PAIRS);
     }
   }
-}
-
-/* the forces, and the second kick */
-__device__ __forceinline__ void forces_and_kick(Ctx& x, cg::cluster_group& cl, bool eflag, bool kick, bool drift) {
-  if (eflag) force_items<true>(x, kick, drift);
-  else force_items<false>(x, kick, drift);
-  __syncthreads();
-  prof_start(x);
-  core_reduce(x, cl);
-  if (kick) {
-    core_kick(x);
-    __syncthreads();
-  }
-  prof_end(x, MDN_PROF_REDUCE);
 }
 
 /* ------------------------------------------------------------------------- */
@@ -2320,7 +2388,7 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
         double sx[3] = {0, 0, 0}, sv[3] = {0, 0, 0};
         for (int at = 0; at < av; at++) {
           int i = P->n_ion + s * av + at;
-          double mm = x.db[P->d_mass + tag_type(x.c.tag[i].k)];
+          double mm = x.c.mass[tag_type(x.c.tag[i].k)];
           for (int k = 0; k < 3; k++) {
             sx[k] += x.c.x[3 * i + k] * mm;
             sv[k] += x.c.v[3 * i + k] * mm;
@@ -2533,62 +2601,98 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
   /* reload the vapor part of the core from the new vapor slab */
   load_vapor(x);
   __syncthreads();
-  core_weights_pos(x, true);
-  relist(x, cl);
+  core_place(x, x.D->ion_com, true, CoreCons{false, 0});
 }
 
 /* ------------------------------------------------------------------------- */
-__device__ __forceinline__ void one_step(Ctx& x, cg::cluster_group& cl, bool eflag, bool rebuild, bool gg,
-                                         bool far_done) {
+/* what the launch is asked to do with a replica */
+struct Turn {
+  bool step, forces;  /* an MD step / the forces alone (else the rebuild or the lists alone) */
+  bool rebuild, eflag, gg, last;
+  bool far_done;      /* the far molecules have made this step (gas_far_steps) */
+};
+
+/* One step, or the part of it that the launch's mode asks for.  Between the
+ * second kick of a step and the drift of the next each thread keeps to its
+ * own components of the core, so a step has four block barriers: after the drift, the
+ * constraints, the coordinates and the force items.  loop_pair is the
+ * caller's copy of MD::loopPair. */
+__device__ __forceinline__ void one_turn(Ctx& x, cg::cluster_group& cl, const Turn& t, int& loop_pair) {
   const RepParams* P = x.P;
+  const int nvt = x.D->nvt_mode;
   prof_start(x);
-  core_kick(x);
-  __syncthreads();
-  if (x.D->nvt_mode == MDN_NVT_SCALE) {
-    double T = ion_temperature(x);
-    double ratio = sqrt(300.0 / T);
-    for (int i = threadIdx.x; i < P->n_ion; i += blockDim.x)
-      for (int k = 0; k < 3; k++) x.c.v[3 * i + k] *= ratio;
+  /* with gas-gas forces, and before a rebuild, every gas molecule is drifted
+   * first; otherwise GasWork says where */
+  const bool apart = t.rebuild || t.gg, fused = !apart && !gas_rigid(P) && x.iscr[57] > (int)blockDim.x;
+  CoreCons cc = {false, 0};
+  if (t.step) {
+    loop_pair++;
+    if (nvt == MDN_NVT_SCALE) {
+      for (int q = threadIdx.x; q < 3 * x.n_core; q += blockDim.x) x.c.v[q] += x.c.f[q] * core_c2(x, q);
+      __syncthreads();
+      const double ratio = sqrt(300.0 / ion_temperature(x));
+      for (int q = threadIdx.x; q < 3 * P->n_ion; q += blockDim.x) x.c.v[q] *= ratio;
+    }
+    core_drift(x, nvt != MDN_NVT_SCALE);
     __syncthreads();
+    cc = core_cons(x);
+    core_shake(x, cc, GasWork{apart, !apart && !t.far_done, !apart && !fused}, t.eflag);
   }
-  const bool apart = rebuild || gg, fused = !apart && !gas_rigid(P) && x.iscr[57] > (int)blockDim.x;
-  core_drift_shake(x, GasWork{apart, !apart && !far_done, !apart && !fused}, eflag);
-  ion_centre(x);
-  if (x.D->nvt_mode == MDN_NVT_NH) {
-    double T = ion_temperature(x);
+  if (t.step || t.forces) {
+    double com[3];
+    ion_centre(x, x.c.x, com);
+    if (threadIdx.x == 0)
+      for (int k = 0; k < 3; k++) x.D->ion_com[k] = com[k];
+    if (P->quirks & MDN_Q_SHAKE_NO_VCORR) cc = CoreCons{false, 0};
+    core_place(x, com, t.step, cc);
+  }
+  if (t.step && nvt == MDN_NVT_NH) {
+    const double T = ion_temperature(x);
     if (threadIdx.x == 0) {
       int g = P->n_ion * 3;
       x.D->zeta += (T - x.D->nvt_T) * g * P->kb_real * 0.0001 * P->dt;
     }
     __syncthreads();
   }
-  core_weights_pos(x, true);
+  if (t.step && t.last && threadIdx.x < 32) {
+    /* the ion centre's velocity, as MD::update_position leaves it */
+    double vel[3];
+    ion_centre(x, x.c.v, vel);
+    if (threadIdx.x == 0)
+      for (int k = 0; k < 3; k++) x.D->ion_com[3 + k] = vel[k];
+  }
   prof_end(x, MDN_PROF_CORE_INT);
-  prof_start(x);
-  if (threadIdx.x == 0) x.D->loop_pair += 1;
-  __syncthreads();
-  prof_end(x, MDN_PROF_GAS_INT);
-  if (rebuild) {
+  if (t.rebuild) {
     prof_start(x);
+    settle(x);
+    if (threadIdx.x == 0 && t.step) x.D->loop_pair = loop_pair;
+    __syncthreads();
     make_pair(x, cl);
+    loop_pair = 0;
     prof_end(x, MDN_PROF_REBUILD);
   }
-  if (gg) gas_gg_pass(x, cl, eflag, rebuild);
-  if (apart) {
+  if (t.rebuild || !(t.step || t.forces)) {
+    settle(x);
+    relist(x, cl);
+  }
+  if (!(t.step || t.forces)) return;
+  if (t.gg) {
+    settle(x);
+    gas_gg_pass(x, cl, t.eflag, t.rebuild);
+  }
+  if (apart || t.forces) {
     prof_start(x);
-    gas_far_pass(x, eflag, true);
+    gas_far_pass(x, t.eflag, t.step);
     __syncthreads();
     prof_end(x, MDN_PROF_REBUILD);
   }
-  forces_and_kick(x, cl, eflag, true, fused);
-  if (x.D->nvt_mode == MDN_NVT_NH) {
-    double Coeff = exp(-x.D->zeta * 0.5 * P->dt);
-    for (int i = threadIdx.x; i < P->n_ion; i += blockDim.x)
-      for (int k = 0; k < 3; k++) x.c.v[3 * i + k] *= Coeff;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) x.D->step += 1;
+  if (t.eflag) force_items<true>(x, t.step, fused && t.step);
+  else force_items<false>(x, t.step, fused && t.step);
   __syncthreads();
+  prof_start(x);
+  core_reduce_kick(x, t.step, t.step && nvt == MDN_NVT_NH);
+  prof_end(x, MDN_PROF_REDUCE);
+  if (t.step && threadIdx.x == 0) x.D->step += 1;
 }
 
 }  // namespace
@@ -2623,6 +2727,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
   x.dscr = dscr;
   x.cand = cand;
   x.trial = trial;
+  x.settled = true;
   /* carve the dynamic shared memory */
   {
     unsigned char* p = dsm;
@@ -2638,9 +2743,11 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     x.c.excl = (unsigned*)take(sizeof(unsigned) * a.excl_cap);
     x.c.lj = (float2*)take(sizeof(float2) * a.nt_cap * a.nt_cap);
     x.c.c2 = (double*)take(sizeof(double) * a.nt_cap);
+    x.c.mass = (double*)take(sizeof(double) * a.nt_cap);
   }
-  /* the chunk sums start at zero and every core_reduce leaves them so */
+  /* the chunk sums start at zero and every core_reduce_kick leaves them so */
   for (int q = threadIdx.x; q < 9 * a.nc_cap; q += blockDim.x) x.c.chunk[q] = 0;
+  if (threadIdx.x == 0) iscr[62] = 0;
   __syncthreads();
   for (;;) {
     if (x.rank == 0 && threadIdx.x == 0) s_job = atomicAdd(a.job_counter, 1);
@@ -2671,7 +2778,10 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     const int nt = sP.n_types;
     for (int q = threadIdx.x; q < nt * nt; q += blockDim.x)
       x.c.lj[q] = make_float2((float)x.db[sP.d_ljA + q], (float)x.db[sP.d_ljB + q]);
-    for (int q = threadIdx.x; q < nt; q += blockDim.x) x.c.c2[q] = x.db[sP.d_c2 + q];
+    for (int q = threadIdx.x; q < nt; q += blockDim.x) {
+      x.c.c2[q] = x.db[sP.d_c2 + q];
+      x.c.mass[q] = x.db[sP.d_mass + q];
+    }
     for (int q = threadIdx.x; q < sP.n_ion * sP.excl_words; q += blockDim.x) x.c.excl[q] = (unsigned)x.ib[sP.o_excl + q];
     load_ion(x);
     load_vapor(x);
@@ -2683,45 +2793,49 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     else if (threadIdx.x < 3)
       iscr[threadIdx.x < 2 ? 56 + threadIdx.x : 61] = a.near_cnt[3 * ((size_t)r * 8 + x.rank) + threadIdx.x];
     __syncthreads();
-    if (a.mode == MDN_MODE_STEP) {
-      const bool gg = kGG && (sP.interactions & MDN_I_GG) && sP.ggl_cap > 0;
+    {
+      Turn t;
+      t.step = a.mode == MDN_MODE_STEP;
+      t.forces = a.mode == MDN_MODE_FORCES;
+      t.gg = kGG && (sP.interactions & MDN_I_GG) && sP.ggl_cap > 0;
+      t.rebuild = a.mode == MDN_MODE_MAKE_PAIR;
+      t.eflag = t.forces;
+      t.far_done = t.last = false;
+      int loop_pair = sD.loop_pair, loop_update = sD.loop_update;
       long long ahead = 0; /* steps the far molecules have already made */
-      bool far_done = false;
-      for (long long s = 0; s < a.n_steps; s++) {
-        const bool eflag = a.energy_mode == 2 || (a.energy_mode == 1 && s == a.n_steps - 1);
-        const bool rebuild = sD.loop_pair + 1 > sD.loop_update;
-        if (rebuild || gg) {
-          far_done = false;
-        } else {
-          if (ahead == 0 && (far_done = iscr[61] > (int)blockDim.x)) {
-            ahead = min(a.n_steps - s, (long long)sD.loop_update - sD.loop_pair);
-            prof_start(x);
-            gas_far_steps(x, ahead, a.energy_mode, s + ahead == a.n_steps);
-            prof_end(x, MDN_PROF_GAS_INT);
+      /* FORCES: the ion centre serves only as the origin of the FP32
+       * coordinates, and the stored one is kept */
+      double keep[3];
+      for (int k = 0; k < 3; k++) keep[k] = sD.ion_com[k];
+      __syncthreads();
+      const long long n = t.step ? a.n_steps : 1;
+      for (long long s = 0; s < n; s++) {
+        if (t.step) {
+          t.last = s == n - 1;
+          t.eflag = a.energy_mode == 2 || (a.energy_mode == 1 && t.last);
+          t.rebuild = loop_pair + 1 > loop_update;
+          if (t.rebuild || t.gg) {
+            t.far_done = false;
+          } else {
+            if (ahead == 0 && (t.far_done = iscr[61] > (int)blockDim.x)) {
+              ahead = min(n - s, (long long)loop_update - loop_pair);
+              prof_start(x);
+              gas_far_steps(x, ahead, a.energy_mode, s + ahead == n);
+              prof_end(x, MDN_PROF_GAS_INT);
+            }
+            if (t.far_done) ahead--;
           }
-          if (far_done) ahead--;
         }
-        one_step(x, cl, eflag, rebuild, gg, far_done);
+        one_turn(x, cl, t, loop_pair);
+        if (t.rebuild) loop_update = sD.loop_update;
       }
-    } else if (a.mode == MDN_MODE_FORCES) {
-      /* the ion centre serves only as the origin of the FP32 coordinates here */
-      double keep[6];
-      for (int k = 0; k < 6; k++) keep[k] = sD.ion_com[k];
+      settle(x);
       __syncthreads();
-      ion_centre(x);
-      core_weights_pos(x, false);
-      gas_gg_pass(x, cl, true, false);
-      gas_far_pass(x, true, false);
-      __syncthreads();
-      forces_and_kick(x, cl, true, false, false);
-      if (threadIdx.x == 0)
-        for (int k = 0; k < 6; k++) sD.ion_com[k] = keep[k];
-      __syncthreads();
-    } else if (a.mode == MDN_MODE_MAKE_PAIR) {
-      core_weights_pos(x, false);
-      make_pair(x, cl);
-    } else if (a.mode == MDN_MODE_RELIST) {
-      relist(x, cl);
+      if (threadIdx.x == 0) {
+        if (t.step) sD.loop_pair = loop_pair;
+        if (t.forces)
+          for (int k = 0; k < 3; k++) sD.ion_com[k] = keep[k];
+      }
     }
     __syncthreads();
     if (a.prof && threadIdx.x == 0) {

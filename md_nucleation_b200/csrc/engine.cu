@@ -97,9 +97,9 @@ int color_rigid(const int* rig, int n, std::vector<int>& color) {
 }
 
 /* the constraints' connected groups (constraints sharing an atom, joined
- * transitively): order = constraint indices group by group, start = group
- * starts (n_groups + 1).  Returns the number of groups, or 0 when a group
- * holds more than 3 constraints (the kernel then sweeps). */
+ * transitively), largest first: order = constraint indices group by group,
+ * start = group starts (n_groups + 1).  Returns the number of groups, or 0
+ * when a group holds more than 3 constraints (the kernel then sweeps). */
 int group_rigid(const int* rig, int n, std::vector<int>& order, std::vector<int>& start) {
   order.clear();
   start.clear();
@@ -126,6 +126,16 @@ int group_rigid(const int* rig, int n, std::vector<int>& order, std::vector<int>
       return 0;
     }
   }
+  start.push_back((int)order.size());
+  const std::vector<int> o = order, s = start;
+  order.clear();
+  start.clear();
+  for (int size = 3; size >= 1; size--)
+    for (size_t g = 0; g + 1 < s.size(); g++)
+      if (s[g + 1] - s[g] == size) {
+        start.push_back((int)order.size());
+        order.insert(order.end(), o.begin() + s[g], o.begin() + s[g + 1]);
+      }
   start.push_back((int)order.size());
   return (int)start.size() - 1;
 }
@@ -232,7 +242,7 @@ size_t smem_bytes(int nc, int nt, int excl) {
   s += align16(8 * (size_t)nc); /* AtomTag */
   s += align16(sizeof(unsigned) * excl);
   s += align16(sizeof(float2) * nt * nt);
-  s += align16(sizeof(double) * nt);
+  s += 2 * align16(sizeof(double) * nt);
   return s;
 }
 
@@ -519,6 +529,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
       P.n_ion_groups = group_rigid(d.ion.rigid, d.ion.n_rigid, go, gs);
       P.o_ion_grp = ipush(go.data(), (int)go.size());
       P.o_ion_gstart = ipush(gs.data(), (int)gs.size());
+      for (int g = 0; g < P.n_ion_groups; g++) P.ion_groups_n[gs[g + 1] - gs[g] - 1]++;
     }
     /* AMBER exclusions: 1-2 (bonds and rigid pairs), 1-3, 1-4 (compute_AMBER.cpp:256-278) */
     P.excl_words = (d.ion.n_atoms + 31) / 32;

@@ -76,6 +76,7 @@ typedef struct RepParams {
   /* SHAKE constraints in groups of coupled ones (sharing atoms), at most 3
    * per group, solved together (shake_group); 0 groups = colour sweeps */
   int n_ion_groups, o_ion_grp, o_ion_gstart;
+  int ion_groups_n[3];           /* ion groups of 1, 2 and 3 constraints; stored largest first */
   int n_vap_groups, o_vap_grp, o_vap_gstart;
   /* offsets inside the double blob */
   int d_bond, d_angle, d_dih, d_ljA, d_ljB, d_mass, d_c2;
