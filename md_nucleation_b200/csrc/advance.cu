@@ -49,6 +49,14 @@ using namespace mdn;
 
 namespace {
 
+/* MDN_GG_TERMS selects the gas-gas term: compiled into its own kernels
+ * (advance_gg.cu, advance_gg_fp64.cu), absent from the others */
+#ifdef MDN_GG_TERMS
+constexpr bool kGG = true;
+#else
+constexpr bool kGG = false;
+#endif
+
 /* taper weight, and the atom's kind in one word: type (bits 0-6), the
  * Born-Mayer-Huggins row of an ion atom (bit 7), vapor slot + 1 (bits 8-31, 0
  * for ion atoms), so that a pair reads both with one 8-byte access */
@@ -1009,13 +1017,6 @@ constexpr bool kFP64Pairs = true;
 constexpr bool kFP64Pairs = false;
 #endif
 
-/* MDN_GG_TERMS selects the gas-gas term: compiled into its own kernels
- * (advance_gg.cu, advance_gg_fp64.cu), absent from the others */
-#ifdef MDN_GG_TERMS
-constexpr bool kGG = true;
-#else
-constexpr bool kGG = false;
-#endif
 
 /* The bonded terms of the core: every dihedral (the ion's, then the vapor
  * molecules'), then every angle, then every bond, so that a warp's 32 terms
@@ -1117,6 +1118,60 @@ __device__ __forceinline__ void field_terms(Ctx& x) {
 __device__ __forceinline__ void partition(const Ctx& x, int n, int* lo, int* hi) {
   *lo = (int)(((long long)n * x.rank) / x.C);
   *hi = (int)(((long long)n * (x.rank + 1)) / x.C);
+}
+
+/* This CTA's part of the slab.  Kept in shared memory (set_slab_part, where
+ * n_gas_in is set): two 64-bit divisions would stand at the start of every
+ * item that works on gas molecules. */
+__device__ __forceinline__ void slab_part(const Ctx& x, int* lo, int* hi) {
+  *lo = x.iscr[53];
+  *hi = x.iscr[54];
+}
+__device__ __forceinline__ void set_slab_part(const Ctx& x) { /* one thread; a barrier follows */
+  partition(x, x.D->n_gas_in, &x.iscr[53], &x.iscr[54]);
+}
+
+/* The near molecules' x, v and f between rebuilds: rows of 32 molecules by
+ * component, in record order (heavy ones first, the light ones from the next
+ * multiple of 32), so that a warp's group reads and writes whole lines.  In
+ * the slab the records of a group, sorted by partners, lie apart: each of its
+ * 18 loads and 18 stores touched 32 lines, 220 of the 494 thousand cycles
+ * that the near pass of a 20,000-atom domain took on one CTA.  near_copy
+ * brings them from the slab and back: at the start and the end of a launch
+ * and around a rebuild. */
+__device__ __forceinline__ int near_row(const Ctx& x, int k) { /* row of record k of this CTA */
+  const int nh = x.iscr[56];
+  return k < nh ? k : ((nh + 31) & ~31) + k - nh;
+}
+__device__ __forceinline__ double* near_base(const Ctx& x) {
+  const RepParams* P = x.P;
+  int lo, hi;
+  slab_part(x, &lo, &hi);
+  return x.a->near_s + P->ns_off + (size_t)9 * P->a_g * (((lo + 31) & ~31) + 64 * x.rank);
+}
+/* component q (x, then v, then f; 3 a_g of each) of a row */
+template <int AG>
+__device__ __forceinline__ double* near_at(double* base, int row) {
+  return base + (size_t)(row >> 5) * (32 * 9 * AG) + (row & 31);
+}
+
+/* the row of record k, slab slot s; in the kernels with gas-gas terms the
+ * slab's own, which those terms read on every step */
+struct NearRow {
+  double *px, *pv, *pf;
+  __device__ __forceinline__ double& x(int q) const { return px[kGG ? q : 32 * q]; }
+  __device__ __forceinline__ double& v(int q) const { return pv[kGG ? q : 32 * q]; }
+  __device__ __forceinline__ double& f(int q) const { return pf[kGG ? q : 32 * q]; }
+};
+template <int AG>
+__device__ __forceinline__ NearRow near_ref(const Ctx& x, int k, int s) {
+  if constexpr (kGG) {
+    const size_t g0 = 3 * gatom(x.P, x.D->parity, s, 0);
+    return NearRow{x.a->slab_x + g0, x.a->slab_v + g0, x.a->slab_f + g0};
+  } else {
+    double* const S = near_at<AG>(near_base(x), near_row(x, k));
+    return NearRow{S, S + 32 * 3 * AG, S + 32 * 6 * AG};
+  }
 }
 
 /* intramolecular bond force of one gas molecule (PotentialGasIntra), FP64 */
@@ -1221,28 +1276,34 @@ __device__ __forceinline__ void gas_integrate_t(Ctx& x, GasWork w, bool eflag, i
   const bool vcorr = !(P->quirks & MDN_Q_SHAKE_NO_VCORR);
   const bool intra = AG == 2 && term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
   int lo, hi;
-  partition(x, x.D->n_gas_in, &lo, &hi);
+  slab_part(x, &lo, &hi);
   double c2[AG];
 #pragma unroll
   for (int at = 0; at < AG; at++) c2[at] = x.c.c2[x.iscr[58 + at]];
   const int nf = w.far ? x.iscr[61] : 0, n = w.all ? hi - lo : nf + (w.near ? x.iscr[57] : 0);
   long long eg = 0;
   for (int e = tid; e < n; e += nthr) {
-    const int s = w.all ? lo + e
-                        : e < nf ? a->far_list[P->near_off + lo + e] : a->near_rec[P->near_off + lo + e - nf].x;
-    const size_t g0 = 3 * gatom(P, par, s, 0);
+    /* the slab's rows, or a near molecule's */
+    const bool slab = w.all || e < nf;
+    const size_t g0 = slab ? 3 * gatom(P, par, w.all ? lo + e : a->far_list[P->near_off + lo + e], 0) : 0;
+    const NearRow S =
+        near_ref<AG>(x, slab ? 0 : e - nf, kGG && !slab ? a->near_rec[P->near_off + lo + e - nf].x : 0);
+    double* const rx = slab ? a->slab_x + g0 : S.px;
+    double* const rv = slab ? a->slab_v + g0 : S.pv;
+    double* const rf = slab ? a->slab_f + g0 : S.pf;
+    const int st = slab || kGG ? 1 : 32;
     double X[3 * AG], V[3 * AG], F[3 * AG];
 #pragma unroll
     for (int q = 0; q < 3 * AG; q++) {
-      X[q] = a->slab_x[g0 + q];
-      V[q] = a->slab_v[g0 + q];
-      F[q] = a->slab_f[g0 + q];
+      X[q] = rx[st * q];
+      V[q] = rv[st * q];
+      F[q] = rf[st * q];
     }
     gas_drift<AG>(x, X, V, F, c2, gas_rigid(P), vcorr, P->dt);
     gas_finite<AG>(x, X, V);
 #pragma unroll
     for (int q = 0; q < 3 * AG; q++) F[q] = 0.0;
-    if (!w.all && e < nf) {
+    if (!w.all && slab) {
       if (intra) {
         const double ei = gas_intra<AG>(x, X, F);
         if (eflag) eg += efixd(ei);
@@ -1252,9 +1313,9 @@ __device__ __forceinline__ void gas_integrate_t(Ctx& x, GasWork w, bool eflag, i
     }
 #pragma unroll
     for (int q = 0; q < 3 * AG; q++) {
-      a->slab_x[g0 + q] = X[q];
-      a->slab_v[g0 + q] = V[q];
-      a->slab_f[g0 + q] = F[q];
+      rx[st * q] = X[q];
+      rv[st * q] = V[q];
+      rf[st * q] = F[q];
     }
   }
   if (eflag && intra && w.far) {
@@ -1288,7 +1349,7 @@ __device__ __forceinline__ void gas_far_steps_t(Ctx& x, long long k, int energy_
   const bool intra = AG == 2 && term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
   const double dt = P->dt;
   int lo, hi;
-  partition(x, x.D->n_gas_in, &lo, &hi);
+  slab_part(x, &lo, &hi);
   const int* far = a->far_list + P->near_off + lo;
   const int n_far = x.iscr[61];
   double c2[AG];
@@ -1351,7 +1412,7 @@ __device__ __forceinline__ void gas_far_pass_t(Ctx& x, bool eflag, bool kick) {
   const bool intra = term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0;
   const bool gg = kGG && term_on(x, MDN_I_GG) && P->ggl_cap > 0;
   int lo, hi;
-  partition(x, x.D->n_gas_in, &lo, &hi);
+  slab_part(x, &lo, &hi);
   double c2[AG];
 #pragma unroll
   for (int at = 0; at < ag; at++) c2[at] = x.c.c2[x.ib[P->o_gas_type + at]];
@@ -1410,7 +1471,7 @@ __device__ __forceinline__ void gas_gg_pass_t(Ctx& x, bool eflag, bool fresh) {
   const KArgs* a = x.a;
   const int par = x.D->parity, nt = P->n_types, nreb = x.D->n_rebuilds;
   int lo, hi;
-  partition(x, x.D->n_gas_in, &lo, &hi);
+  slab_part(x, &lo, &hi);
   int gtype[AG];
 #pragma unroll
   for (int at = 0; at < AG; at++) gtype[at] = x.ib[P->o_gas_type + at];
@@ -1590,7 +1651,7 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   const KArgs* a = x.a;
   const int par = x.D->parity, ni = P->n_ion, av = P->a_v, nj = gv_reach(P);
   int lo, hi;
-  partition(x, x.D->n_gas_in, &lo, &hi);
+  slab_part(x, &lo, &hi);
   int* const hist = x.cand;        /* [kNearBins] molecules per bin, then first record  */
   int* const cur = x.cand + 32;    /* [kNearBins] next record                           */
   int* const heavy = x.cand + 64;  /* partners of all heavy molecules, and the next one */
@@ -1667,6 +1728,38 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   __syncthreads();
 }
 
+template <int AG, bool OUT>
+__device__ __forceinline__ void near_copy_t(Ctx& x) {
+  const RepParams* P = x.P;
+  const KArgs* a = x.a;
+  const int par = x.D->parity, nn = x.iscr[57];
+  int lo, hi;
+  slab_part(x, &lo, &hi);
+  double* const base = near_base(x);
+  for (int k = threadIdx.x; k < nn; k += blockDim.x) {
+    const size_t g0 = 3 * gatom(P, par, a->near_rec[P->near_off + lo + k].x, 0);
+    double* const S = near_at<AG>(base, near_row(x, k));
+#pragma unroll
+    for (int q = 0; q < 3 * AG; q++) {
+      if (OUT) {
+        a->slab_x[g0 + q] = S[32 * q];
+        a->slab_v[g0 + q] = S[32 * (q + 3 * AG)];
+        a->slab_f[g0 + q] = S[32 * (q + 6 * AG)];
+      } else {
+        S[32 * q] = a->slab_x[g0 + q];
+        S[32 * (q + 3 * AG)] = a->slab_v[g0 + q];
+        S[32 * (q + 6 * AG)] = a->slab_f[g0 + q];
+      }
+    }
+  }
+}
+template <bool OUT>
+__device__ __forceinline__ void near_copy(Ctx& x) {
+  if constexpr (kGG) return;
+  if (x.P->a_g == 1) near_copy_t<1, OUT>(x);
+  else near_copy_t<2, OUT>(x);
+}
+
 /* One group of near molecules, one lane each: records first .. first + n.
  * Light molecules' lanes walk their own partners (lg = 0).  Heavy ones
  * (30-100 partners next to a large ion) are walked by 2^lg lanes each, the
@@ -1691,19 +1784,21 @@ __device__ __forceinline__ void near_group(Ctx& x, int first, int n, int lg, boo
   const double* com = x.D->ion_com;
   const unsigned short* const item = a->near_item + P->nit_off;
   const bool own = lane < n;
-  const int4 rc = own ? a->near_rec[P->near_off + first + lane] : make_int4(0, 0, 0, 0);
-  const size_t g0 = gatom(P, par, rc.x, 0);
+  int lo, hi;
+  slab_part(x, &lo, &hi);
+  const int4 rc = own ? a->near_rec[P->near_off + lo + first + lane] : make_int4(0, 0, 0, 0);
+  const NearRow S = near_ref<AG>(x, first + (own ? lane : 0), rc.x);
   double X[3 * AG], V[3 * AG];
   float3 gp[AG];
 #pragma unroll
   for (int q = 0; q < 3 * AG; q++) {
-    X[q] = own ? a->slab_x[3 * g0 + q] : 0.0;
-    V[q] = own && kick ? a->slab_v[3 * g0 + q] : 0.0;
+    X[q] = S.x(q);
+    V[q] = S.v(q);
   }
-  if (drift && own) { /* a rigid gas was drifted before */
+  if (drift) { /* a rigid gas was drifted before */
 #pragma unroll
     for (int q = 0; q < 3 * AG; q++) {
-      V[q] += a->slab_f[3 * g0 + q] * x.c.c2[gtype[q / 3]];
+      V[q] += S.f(q) * x.c.c2[gtype[q / 3]];
       X[q] = X[q] + V[q] * P->dt;
     }
     gas_finite<AG>(x, X, V);
@@ -1762,16 +1857,16 @@ __device__ __forceinline__ void near_group(Ctx& x, int first, int n, int lg, boo
     }
     if (kGG && term_on(x, MDN_I_GG) && P->ggl_cap > 0)
 #pragma unroll
-      for (int q = 0; q < 3 * AG; q++) Fd[q] += a->slab_fgg[3 * g0 + q];
+      for (int q = 0; q < 3 * AG; q++) Fd[q] += a->slab_fgg[3 * gatom(P, par, rc.x, 0) + q];
     if (term_on(x, MDN_I_GAS_INTRA) && P->n_gas_bonds > 0) {
       const double ei = gas_intra<AG>(x, X, Fd);
       if (E) eintra = efixd(ei);
     }
 #pragma unroll
     for (int q = 0; q < 3 * AG; q++) {
-      if (drift) a->slab_x[3 * g0 + q] = X[q];
-      if (kick) a->slab_v[3 * g0 + q] = V[q] + Fd[q] * x.c.c2[gtype[q / 3]];
-      a->slab_f[3 * g0 + q] = Fd[q];
+      if (drift) S.x(q) = X[q];
+      if (kick) S.v(q) = V[q] + Fd[q] * x.c.c2[gtype[q / 3]];
+      S.f(q) = Fd[q];
     }
   }
   if (E) {
@@ -1892,8 +1987,6 @@ __device__ __forceinline__ void force_items(Ctx& x, bool kick, bool drift) {
   const int nblk = pairs ? (x.n_core + 31) >> 5 : 0;
   const int field = term_on(x, MDN_I_EFIELD) ? 1 : 0;
   const int n_bond = field + ((bc.total() + 31) >> 5), n_tile = nblk * (nblk + 1) / 2;
-  int lo, hi;
-  partition(x, x.D->n_gas_in, &lo, &hi);
   const int nh = x.iscr[56], nn = x.iscr[57];
   int hs, lg;
   heavy_cut(nh, &hs, &lg);
@@ -1923,8 +2016,8 @@ __device__ __forceinline__ void force_items(Ctx& x, bool kick, bool drift) {
         const int k = it - mc;
         const bool heavy = k < gh;
         const int f = heavy ? k * hs : nh + 32 * (k - gh), n = heavy ? min(hs, nh - f) : min(32, nn - f);
-        if (P->a_g == 1) near_group<1, kFP64Pairs, E>(x, lo + f, n, heavy ? lg : 0, kick, drift);
-        else near_group<2, kFP64Pairs, E>(x, lo + f, n, heavy ? lg : 0, kick, drift);
+        if (P->a_g == 1) near_group<1, kFP64Pairs, E>(x, f, n, heavy ? lg : 0, kick, drift);
+        else near_group<2, kFP64Pairs, E>(x, f, n, heavy ? lg : 0, kick, drift);
       }
       int next = 0;
       if (lane == 0) next = atomicAdd(&x.iscr[60], 1);
@@ -2180,7 +2273,7 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
   const int par = x.D->parity, ni = P->n_ion, nv = x.D->n_vap_in;
   const bool gi = (P->interactions & MDN_I_GI) != 0, gv = (P->interactions & MDN_I_GV) != 0;
   int lo, hi;
-  partition(x, x.D->n_gas_in, &lo, &hi);
+  slab_part(x, &lo, &hi);
   /* bounding sphere of the ion, exact test below */
   int* sc = x.iscr;
   int gi_tot = 0, gv_tot = 0, nn_tot = 0;
@@ -2363,7 +2456,7 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
   /* updateInCenters: gas slab partition of this CTA, vapor core by rank 0 */
   {
     int lo, hi;
-    partition(x, x.D->n_gas_in, &lo, &hi);
+    slab_part(x, &lo, &hi);
     for (int s = lo + threadIdx.x; s < hi; s += blockDim.x) {
       int m = a->slab_mol[gmol(P, par, s)];
       double sx[3] = {0, 0, 0}, sv[3] = {0, 0, 0};
@@ -2590,6 +2683,7 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
     if (core_over && x.rank == 0) set_status(x, MDN_ST_CORE_OVERFLOW);
     x.D->parity = npar;
     x.D->n_gas_in = slab_over ? 0 : gin_tot;
+    set_slab_part(x);
     x.D->n_vap_in = core_over ? 0 : vin_tot;
     double vmax = sqrt(vm2);
     double lu = x.D->margin_length / (vmax * P->dt);
@@ -2626,6 +2720,7 @@ __device__ __forceinline__ void one_turn(Ctx& x, cg::cluster_group& cl, const Tu
   const bool apart = t.rebuild || t.gg, fused = !apart && !gas_rigid(P) && x.iscr[57] > (int)blockDim.x;
   CoreCons cc = {false, 0};
   if (t.step) {
+    if (t.rebuild) near_copy<true>(x); /* the rebuild reads the slab */
     loop_pair++;
     if (nvt == MDN_NVT_SCALE) {
       for (int q = threadIdx.x; q < 3 * x.n_core; q += blockDim.x) x.c.v[q] += x.c.f[q] * core_c2(x, q);
@@ -2683,12 +2778,14 @@ __device__ __forceinline__ void one_turn(Ctx& x, cg::cluster_group& cl, const Tu
   if (apart || t.forces) {
     prof_start(x);
     gas_far_pass(x, t.eflag, t.step);
+    near_copy<false>(x);
     __syncthreads();
     prof_end(x, MDN_PROF_REBUILD);
   }
   if (t.eflag) force_items<true>(x, t.step, fused && t.step);
   else force_items<false>(x, t.step, fused && t.step);
   __syncthreads();
+  if (t.forces) near_copy<true>(x);
   prof_start(x);
   core_reduce_kick(x, t.step, t.step && nvt == MDN_NVT_NH);
   prof_end(x, MDN_PROF_REDUCE);
@@ -2762,6 +2859,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
       sD = a.D[r];
       sD.nvt_mode = a.ctl_mode[r];
       sD.nvt_T = a.ctl_T[r];
+      set_slab_part(x);
     }
     __syncthreads();
     x.ib = a.iblob + sP.iblob_off;
@@ -2785,14 +2883,13 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     for (int q = threadIdx.x; q < sP.n_ion * sP.excl_words; q += blockDim.x) x.c.excl[q] = (unsigned)x.ib[sP.o_excl + q];
     load_ion(x);
     load_vapor(x);
+    if (threadIdx.x < sP.a_g) iscr[58 + threadIdx.x] = x.ib[sP.o_gas_type + threadIdx.x];
+    if (threadIdx.x < 3) /* build_near's counts; it makes them anew for another cluster size */
+      iscr[threadIdx.x < 2 ? 56 + threadIdx.x : 61] = a.near_cnt[3 * ((size_t)r * 8 + x.rank) + threadIdx.x];
     if (threadIdx.x < MDN_PROF_N) s_prof[threadIdx.x] = 0;
     __syncthreads();
-    if (threadIdx.x < sP.a_g) iscr[58 + threadIdx.x] = x.ib[sP.o_gas_type + threadIdx.x];
     const long long job_t0 = clock64();
     if ((a.mode == MDN_MODE_STEP || a.mode == MDN_MODE_FORCES) && sD.near_C != x.C) build_near(x, cl);
-    else if (threadIdx.x < 3)
-      iscr[threadIdx.x < 2 ? 56 + threadIdx.x : 61] = a.near_cnt[3 * ((size_t)r * 8 + x.rank) + threadIdx.x];
-    __syncthreads();
     {
       Turn t;
       t.step = a.mode == MDN_MODE_STEP;
@@ -2809,6 +2906,10 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
       for (int k = 0; k < 3; k++) keep[k] = sD.ion_com[k];
       __syncthreads();
       const long long n = t.step ? a.n_steps : 1;
+      if (t.step) {
+        near_copy<false>(x);
+        __syncthreads();
+      }
       for (long long s = 0; s < n; s++) {
         if (t.step) {
           t.last = s == n - 1;
@@ -2830,6 +2931,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
         if (t.rebuild) loop_update = sD.loop_update;
       }
       settle(x);
+      if (t.step) near_copy<true>(x);
       __syncthreads();
       if (threadIdx.x == 0) {
         if (t.step) sD.loop_pair = loop_pair;

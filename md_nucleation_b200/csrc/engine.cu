@@ -169,6 +169,7 @@ struct mdn_handle {
   int* vslab_mol = nullptr;
   int4* near_rec = nullptr;
   unsigned short* near_item = nullptr;
+  double* near_s = nullptr;
   int *near_cnt = nullptr, *far_list = nullptr;
   int *near_gi = nullptr, *near_gv = nullptr;
   unsigned short *gil_n = nullptr, *gvl_n = nullptr, *gil = nullptr, *gvl = nullptr;
@@ -215,7 +216,7 @@ namespace {
 void free_all(mdn_handle* h) {
   void* ptrs[] = {h->dP, h->dD, h->d_iblob, h->d_dblob, h->ion_x, h->ion_v, h->ion_f, h->mol_x, h->mol_v,
                   h->region, h->slot, h->slab_x, h->slab_v, h->slab_f, h->slab_mol, h->vslab_x, h->vslab_v,
-                  h->vslab_f, h->vslab_w, h->vslab_mol, h->near_rec, h->near_item, h->near_cnt, h->far_list, h->near_gi, h->near_gv, h->gil_n,
+                  h->vslab_f, h->vslab_w, h->vslab_mol, h->near_rec, h->near_item, h->near_cnt, h->near_s, h->far_list, h->near_gi, h->near_gv, h->gil_n,
                   h->gvl_n, h->gil, h->gvl, h->energy, h->events, h->n_events, h->status, h->job_order,
                   h->job_counter, h->snap_off, h->snap_type, h->snap_x, h->snap_v, h->d_ctl_mode,
                   h->d_ctl_T, h->d_prof, h->job_order2, h->job_counter2, h->ggl_start, h->ggl_n, h->ggl,
@@ -316,7 +317,7 @@ long long launch(mdn_handle* h, int mode, long long n_steps, int energy_mode, un
   a.slab_x = h->slab_x; a.slab_v = h->slab_v; a.slab_f = h->slab_f; a.slab_mol = h->slab_mol;
   a.vslab_x = h->vslab_x; a.vslab_v = h->vslab_v; a.vslab_f = h->vslab_f; a.vslab_w = h->vslab_w;
   a.vslab_mol = h->vslab_mol;
-  a.near_rec = h->near_rec; a.near_item = h->near_item; a.near_cnt = h->near_cnt; a.far_list = h->far_list;
+  a.near_rec = h->near_rec; a.near_item = h->near_item; a.near_cnt = h->near_cnt; a.near_s = h->near_s; a.far_list = h->far_list;
   a.near_gi = h->near_gi; a.near_gv = h->near_gv;
   a.gil_n = h->gil_n; a.gvl_n = h->gvl_n; a.gil = h->gil; a.gvl = h->gvl;
   a.ggl_start = h->ggl_start; a.ggl_n = h->ggl_n; a.ggl = h->ggl;
@@ -446,7 +447,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
   std::vector<double> dblob;
   h->P.resize(R);
   h->D0.resize(R);
-  size_t ion_tot = 0, mol_tot = 0, slab_atoms = 0, slab_mols = 0, vslab_atoms = 0, vslab_mols = 0, near_tot = 0, nit_tot = 0,
+  size_t ion_tot = 0, mol_tot = 0, slab_atoms = 0, slab_mols = 0, vslab_atoms = 0, vslab_mols = 0, near_tot = 0, nit_tot = 0, ns_tot = 0,
          gil_tot = 0, gvl_tot = 0, ggl_tot = 0;
   for (int r = 0; r < R; r++) {
     const mdn_replica_desc& d = descs[r];
@@ -693,6 +694,10 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
     vslab_mols += (size_t)2 * P.vcap;
     P.near_off = (long long)near_tot;
     near_tot += P.slab_cap;
+    /* rows of whole 32s, and per CTA the ends of the heavy and the light
+     * molecules' rows */
+    P.ns_off = (long long)ns_tot;
+    ns_tot += (size_t)9 * P.a_g * (((P.slab_cap + 31) & ~31) + 64 * 8 + 32);
     /* every entry once, a gas-vapor one once per vapor atom it reaches, and
      * per CTA (at most 8) the last group's padding: 32 lanes x 16 entries */
     P.nit_off = (long long)nit_tot;
@@ -792,6 +797,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
   ALLOC(h->near_item, nit_tot);
   ALLOC(h->near_cnt, 24 * (size_t)R);
   ALLOC(h->far_list, near_tot);
+  ALLOC(h->near_s, ns_tot);
   ALLOC(h->near_gi, slab_mols);
   ALLOC(h->near_gv, slab_mols);
   ALLOC(h->gil_n, slab_mols);

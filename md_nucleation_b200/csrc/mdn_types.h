@@ -91,7 +91,7 @@ typedef struct RepParams {
   double efield[3];
   unsigned key0, key1;
   /* pool offsets (elements) */
-  long long ion_off, mol_off, slab_off, vslab_off, near_off, nit_off, gil_off, gvl_off, ggl_off;
+  long long ion_off, mol_off, slab_off, vslab_off, near_off, nit_off, ns_off, gil_off, gvl_off, ggl_off;
   long long slab_moff, vslab_moff; /* molecule offsets of the two slabs */
   long long iblob_off, dblob_off;
   double work;                   /* cost estimate for the job order */
@@ -131,6 +131,7 @@ typedef struct KArgs {
   int4* near_rec;          /* near molecules of each CTA's slab partition, from its first slot:
                               {slab slot, first item, items, 0}, most items first */
   unsigned short* near_item; /* their partners, core atom indices (build_near) */
+  double* near_s;          /* x, v, f of the near molecules between rebuilds (near_row) */
   int* far_list;           /* slab slots of the other molecules, from the partition's first slot */
   int* near_cnt;           /* [replica][8 ranks][3] heavy / all near records, far molecules */
   int* near_gi;            /* [slab slot] start of its gi entries (-1 = none)  */
