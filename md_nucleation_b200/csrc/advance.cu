@@ -853,8 +853,11 @@ __device__ __forceinline__ bool term_on(const Ctx& x, unsigned bit) {
  * (the exclusions, the ion-vapor and vapor-vapor switches, the atoms of one
  * molecule, the diagonal's half) is worked out once per tile as one bit per
  * step, the LJ + Coulomb form is the same for all three kinds (an ion atom's
- * weight is 1), and the steps carry no branch on the kind, so that the
- * compiler interleaves several of them.  Against a branch on the kind per
+ * weight is 1), and the steps carry no branch, so that the compiler
+ * interleaves several of them; only a tile with few steps or with
+ * Born-Mayer-Huggins pairs (the ion's own, a small cluster) tests each step
+ * (with the test in every tile the pairs of 786 atoms took 331 thousand
+ * cycles on one CTA, without 244).  Against a branch on the kind per
  * pair: 36.0 -> 32.2 ms per 100 steps of 256 mixed replicas (tuned launch),
  * 2.23 -> 1.85 ms on one 13-atom core, bit-identical results. */
 template <bool FP64, bool E>
@@ -921,9 +924,9 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
     pi = x.c.pos[ii];
     qi = (float)P->qqrd2e * pi.w;
   }
-  auto step = [&](int s) {
-    const int jl = (lane + s) & 31;
-    const int j = j0 + jl < nc ? j0 + jl : 0;
+  auto step = [&](int s, auto with_born) {
+    constexpr bool kBorn = decltype(with_born)::value;
+    const int j = min(j0 + ((lane + s) & 31), nc - 1);
     const AtomTag gj = x.c.tag[j];
     const int tt = rowi + tag_type(gj.k);
     if constexpr (FP64) {
@@ -934,7 +937,7 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
         double fd = 0.0;
         if ((on >> s) & 1u)
           fd = lj_coul_d(R2d, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qq, true) * (wid * weight_d(x, j));
-        if ((born_on >> s) & 1u) fd += born_d(R2d, tag_bmh(gi.k), tag_bmh(gj.k), qq);
+        if (kBorn && ((born_on >> s) & 1u)) fd += born_d(R2d, tag_bmh(gi.k), tag_bmh(gj.k), qq);
         const double fx = fd * ex, fy = fd * ey, fz = fd * ez;
         F0 += fx; F1 += fy; F2 += fz;
         R0 -= fx; R1 -= fy; R2 -= fz;
@@ -948,7 +951,7 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
       float ee;
       float fp = lj_coul(r2, AB.x, AB.y, qq, true, &ee) * (gi.w * gj.w);
       fp = ((on >> s) & 1u) ? fp : 0.0f;
-      if ((born_on >> s) & 1u) fp += born(r2, tag_bmh(gi.k), tag_bmh(gj.k), qq, &ee);
+      if (kBorn && ((born_on >> s) & 1u)) fp += born(r2, tag_bmh(gi.k), tag_bmh(gj.k), qq, &ee);
       if (((on | born_on) >> s) & 1u) {
         const float fx = fp * dx, fy = fp * dy, fz = fp * dz;
         F0 += fx; F1 += fy; F2 += fz;
@@ -961,7 +964,7 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
         const double qq = qid * charge_d(x, j);
         double ed = 0;
         if ((on >> s) & 1u) ed += lj_coul_energy(R2e, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qq);
-        if ((born_on >> s) & 1u) ed += born_energy(R2e, tag_bmh(gi.k), tag_bmh(gj.k), qq);
+        if (kBorn && ((born_on >> s) & 1u)) ed += born_energy(R2e, tag_bmh(gi.k), tag_bmh(gj.k), qq);
         const bool iion = ii < ni, jion = j < ni;
         if (iion && jion) e_ion += efixd(ed);
         else if (iion != jion) e_vi += efixd(ed);
@@ -970,12 +973,22 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
     }
   };
   const int s1 = diag ? 17 : 32;
-#pragma unroll 4
-  for (int s = 0; s < s1; s++) {
-    if ((any_on >> s) & 1u) step(s);
+  auto pass_on = [&]() {
     R0 = __shfl_sync(FULL, R0, (lane + 1) & 31);
     R1 = __shfl_sync(FULL, R1, (lane + 1) & 31);
     R2 = __shfl_sync(FULL, R2, (lane + 1) & 31);
+  };
+  if (__any_sync(FULL, born_on != 0) || __popc(any_on) < 12) {
+    for (int s = 0; s < s1; s++) {
+      if ((any_on >> s) & 1u) step(s, std::true_type());
+      pass_on();
+    }
+  } else {
+#pragma unroll 4
+    for (int s = 0; s < s1; s++) {
+      step(s, std::false_type());
+      pass_on();
+    }
   }
   if (diag) {
     R0 = __shfl_sync(FULL, R0, (lane + 15) & 31);
