@@ -1639,9 +1639,15 @@ __device__ __forceinline__ void cluster_prefix(Ctx& x, cg::cluster_group& cl, in
   cl.sync();
 }
 
-/* A near molecule with more partners than this has them spread over 8 lanes. */
+/* A near molecule with more partners than this has them spread over several lanes. */
 constexpr int kNearHeavy = 16;
-constexpr int kNearBins = kNearHeavy + 1; /* bin 0: heavy; bin b: 17 - b partners */
+/* bins of the near molecules by partners, most first: the heavy ones by
+ * eights, then one bin per number */
+constexpr int kHeavyBins = 32;
+constexpr int kNearBins = kHeavyBins + kNearHeavy;
+__device__ __forceinline__ int near_bin(int c) {
+  return c > kNearHeavy ? max(0, kHeavyBins - 1 - (c - kNearHeavy - 1) / 8) : kHeavyBins + kNearHeavy - c;
+}
 
 /* core atoms a gas-vapor entry reaches in its vapor molecule */
 __device__ __forceinline__ int gv_reach(const RepParams* P) {
@@ -1665,9 +1671,9 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   const int par = x.D->parity, ni = P->n_ion, av = P->a_v, nj = gv_reach(P);
   int lo, hi;
   slab_part(x, &lo, &hi);
-  int* const hist = x.cand;        /* [kNearBins] molecules per bin, then first record  */
-  int* const cur = x.cand + 32;    /* [kNearBins] next record                           */
-  int* const heavy = x.cand + 64;  /* partners of all heavy molecules, and the next one */
+  int* const hist = x.cand;        /* [kNearBins + 1] molecules per bin, then first record */
+  int* const cur = x.cand + 64;    /* [kNearBins] next record                              */
+  int* const heavy = x.cand + 128; /* partners of all heavy molecules, and the next one    */
   __syncthreads();
   if (threadIdx.x < kNearBins) hist[threadIdx.x] = 0;
   if (threadIdx.x < 2) heavy[threadIdx.x] = 0;
@@ -1678,18 +1684,19 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   for (int s = lo + (int)threadIdx.x; s < hi; s += blockDim.x) {
     const int c = items_of(gmol(P, par, s));
     if (c == 0) continue;
-    atomicAdd(&hist[c > kNearHeavy ? 0 : kNearHeavy + 1 - c], 1);
+    atomicAdd(&hist[near_bin(c)], 1);
     if (c > kNearHeavy) atomicAdd(&heavy[0], c);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    int run = 0, items = heavy[0];
-    const int nh = hist[0];
+    int run = 0, items = heavy[0], nh = 0;
     for (int b = 0; b < kNearBins; b++) {
       const int n = hist[b];
       hist[b] = cur[b] = run;
+      if (b == kHeavyBins) nh = run;
       /* 32-record groups that start in this bin take its count of entries */
-      if (b > 0) items += 32 * (kNearHeavy + 1 - b) * (((run + n - nh + 31) >> 5) - ((run - nh + 31) >> 5));
+      if (b >= kHeavyBins)
+        items += 32 * (kNearBins - b) * (((run + n - nh + 31) >> 5) - ((run - nh + 31) >> 5));
       run += n;
     }
     hist[kNearBins] = run;
@@ -1720,14 +1727,14 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
     if (c == 0) continue;
     int off, stride;
     if (c > kNearHeavy) {
-      rec[atomicAdd(&cur[0], 1)] = make_int4(s, off = base + atomicAdd(&heavy[1], c), c, 0);
+      rec[atomicAdd(&cur[near_bin(c)], 1)] = make_int4(s, off = base + atomicAdd(&heavy[1], c), c, 0);
       stride = 1;
     } else {
-      const int r = atomicAdd(&cur[kNearHeavy + 1 - c], 1), k = r - nh, g0 = k & ~31;
+      const int r = atomicAdd(&cur[near_bin(c)], 1), k = r - nh, g0 = k & ~31;
       off = light0 + (k & 31);
-      for (int b = 1; b < kNearBins; b++) { /* the groups before this one */
+      for (int b = kHeavyBins; b < kNearBins; b++) { /* the groups before this one */
         const int s0 = min(hist[b] - nh, g0), s1 = min(hist[b + 1] - nh, g0);
-        off += 32 * (kNearHeavy + 1 - b) * (((s1 + 31) >> 5) - ((s0 + 31) >> 5));
+        off += 32 * (kNearBins - b) * (((s1 + 31) >> 5) - ((s0 + 31) >> 5));
       }
       rec[r] = make_int4(s, off, c, 0);
       stride = 32;
@@ -1894,15 +1901,15 @@ __device__ __forceinline__ void near_group(Ctx& x, int first, int n, int lg, boo
   }
 }
 
-constexpr int kHeavyGroup = 16; /* heavy molecules a warp takes at a time, at most */
-
-/* How a CTA's nh heavy molecules are cut into groups: few enough per group
- * that every warp gets one (a lone molecule is walked by the whole warp), at
- * most kHeavyGroup; at 8 lanes each the walk of 30-100 partners keeps its
- * lanes busy and costs three rounds of shuffles for four molecules. */
+/* How a CTA's nh heavy molecules are cut into groups: one at a time walked by
+ * the whole warp while there are up to four per warp, then two, and at most
+ * four, by 8 lanes each.  A group is one item of the queue, and the longest
+ * lists have several hundred partners: with up to 16 molecules to a group,
+ * in no order, the pass waited for the longest groups (641 heavy molecules
+ * with 65 partners on average, one CTA: 269 of 396 thousand cycles). */
 __device__ __forceinline__ void heavy_cut(int nh, int* size, int* lg) {
   const int nw = blockDim.x >> 5;
-  const int h = min(kHeavyGroup, max(1, (nh + nw - 1) / nw));
+  const int h = min(4, max(1, (nh + 4 * nw - 1) / (4 * nw)));
   *size = h;
   *lg = h == 1 ? 5 : h == 2 ? 4 : 3;
 }
