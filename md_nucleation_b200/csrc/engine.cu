@@ -1534,18 +1534,30 @@ static int order_by_measured(mdn_handle* h, long long n_steps, int* status) {
   return MDN_OK;
 }
 
+/* One block of the tuner: n_steps, timed without the first of them, in which
+ * the replicas make their near records for the block's cluster size. */
+static int tune_block(mdn_handle* h, long long n_steps, float* ms, int* status) {
+  for (int part = n_steps > 1 ? 0 : 1; part < 2; part++) {
+    const int rc = mdn_step(h, part == 0 ? 1 : n_steps > 1 ? n_steps - 1 : 1, 0);
+    if (rc == MDN_ERR_REPLICA) *status = rc;
+    else if (rc != MDN_OK) return rc;
+  }
+  *ms = (float)h->last_ms;
+  return MDN_OK;
+}
+
 int mdn_tune_launch(mdn_handle* h, long long n_steps, int* best) {
   if (!h || n_steps <= 0) return fail(MDN_ERR_ARG, "bad arguments");
   int best_c = 0, status = MDN_OK;
   float best_ms = 0;
   for (int c = 1; c <= 8; c *= 2) {
     h->opt.cluster_size = c;
-    int rc = mdn_step(h, n_steps, 0);
-    if (rc == MDN_ERR_REPLICA) status = rc;
-    else if (rc != MDN_OK) return rc;
-    if (best_c == 0 || h->last_ms < best_ms) {
+    float ms;
+    const int rc = tune_block(h, n_steps, &ms, &status);
+    if (rc) return rc;
+    if (best_c == 0 || ms < best_ms) {
       best_c = c;
-      best_ms = h->last_ms;
+      best_ms = ms;
     }
   }
   h->opt.cluster_size = best_c;
@@ -1556,10 +1568,7 @@ int mdn_tune_launch(mdn_handle* h, long long n_steps, int* best) {
      * order */
     int rc = order_by_measured(h, n_steps, &status);
     if (rc) return rc;
-    rc = mdn_step(h, n_steps, 0);
-    if (rc == MDN_ERR_REPLICA) status = rc;
-    else if (rc != MDN_OK) return rc;
-    best_ms = h->last_ms;
+    if ((rc = tune_block(h, n_steps, &best_ms, &status))) return rc;
   }
   /* then the k slowest replicas on larger clusters (2 or 4 times, at most 8
    * CTAs), one each, in a concurrent launch beside the rest */
@@ -1570,17 +1579,17 @@ int mdn_tune_launch(mdn_handle* h, long long n_steps, int* best) {
         if (k * sc + best_c > h->num_sms) break;
         h->split_n = k;
         h->split_cluster = sc;
-        int rc = mdn_step(h, n_steps, 0);
-        if (rc == MDN_ERR_REPLICA) status = rc;
-        else if (rc != MDN_OK) {
+        float ms;
+        const int rc = tune_block(h, n_steps, &ms, &status);
+        if (rc) {
           h->split_n = save_n;
           h->split_cluster = save_c;
           return rc;
         }
-        if (h->last_ms < best_ms) {
+        if (ms < best_ms) {
           best_n = k;
           best_sc = sc;
-          best_ms = h->last_ms;
+          best_ms = ms;
         }
       }
   if (save_n == 0) {
