@@ -915,10 +915,19 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
   float4 pi = make_float4(0, 0, 0, 0);
   float qi = 0;
   double xd[3] = {0, 0, 0}, wid = 1.0, qid = 0.0;
+  /* charge and taper weight of j0 + lane in FP64: once per tile, handed round
+   * by shuffles (a division, loads and for a vapor atom in the shell a cosine
+   * per pair otherwise) */
+  double q_own = 0.0, w_own = 1.0;
   if constexpr (FP64 || E) {
     for (int k = 0; k < 3; k++) xd[k] = x.c.x[3 * ii + k];
-    wid = FP64 ? weight_d(x, ii) : 1.0;
     qid = P->qqrd2e * charge_d(x, ii);
+    const int jo = min(j0 + lane, nc - 1);
+    q_own = charge_d(x, jo);
+    if (FP64) {
+      wid = weight_d(x, ii);
+      w_own = weight_d(x, jo);
+    }
   }
   if constexpr (!FP64) {
     pi = x.c.pos[ii];
@@ -928,15 +937,18 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
     constexpr bool kBorn = decltype(with_born)::value;
     const int j = min(j0 + ((lane + s) & 31), nc - 1);
     const AtomTag gj = x.c.tag[j];
+    double qj = 0.0, wj = 1.0;
+    if constexpr (FP64 || E) qj = __shfl_sync(FULL, q_own, (lane + s) & 31);
+    if constexpr (FP64) wj = __shfl_sync(FULL, w_own, (lane + s) & 31);
     const int tt = rowi + tag_type(gj.k);
     if constexpr (FP64) {
       if (((on | born_on) >> s) & 1u) {
         const double ex = xd[0] - x.c.x[3 * j], ey = xd[1] - x.c.x[3 * j + 1], ez = xd[2] - x.c.x[3 * j + 2];
         const double R2d = ex * ex + ey * ey + ez * ez;
-        const double qq = qid * charge_d(x, j);
+        const double qq = qid * qj;
         double fd = 0.0;
         if ((on >> s) & 1u)
-          fd = lj_coul_d(R2d, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qq, true) * (wid * weight_d(x, j));
+          fd = lj_coul_d(R2d, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qq, true) * (wid * wj);
         if (kBorn && ((born_on >> s) & 1u)) fd += born_d(R2d, tag_bmh(gi.k), tag_bmh(gj.k), qq);
         const double fx = fd * ex, fy = fd * ey, fz = fd * ez;
         F0 += fx; F1 += fy; F2 += fz;
@@ -961,7 +973,7 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
     if constexpr (E) {
       if (((on | born_on) >> s) & 1u) {
         const double R2e = r2d(xd, x.c.x + 3 * j);
-        const double qq = qid * charge_d(x, j);
+        const double qq = qid * qj;
         double ed = 0;
         if ((on >> s) & 1u) ed += lj_coul_energy(R2e, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qq);
         if (kBorn && ((born_on >> s) & 1u)) ed += born_energy(R2e, tag_bmh(gi.k), tag_bmh(gj.k), qq);
