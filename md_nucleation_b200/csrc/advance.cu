@@ -732,10 +732,17 @@ __device__ __forceinline__ double r2d(const double* a, const double* b) {
   double dx = a[0] - b[0], dy = a[1] - b[1], dz = a[2] - b[2];
   return dx * dx + dy * dy + dz * dz;
 }
-__device__ __forceinline__ double lj_coul_energy(double r2, double A, double B, double qq) {
+/* the pair's A / 12 and B / 6 come from tables (d_ljA12, d_ljB6): one
+ * division per pair instead of three, and no square root without charges */
+__device__ __forceinline__ double lj_energy(double r2, double A12, double B6) {
   double r2inv = 1 / r2;
   double r6inv = r2inv * r2inv * r2inv;
-  return r6inv * (A / 12.0 * r6inv - B / 6.0) + qq * sqrt(r2inv);
+  return r6inv * (A12 * r6inv - B6);
+}
+__device__ __forceinline__ double lj_coul_energy(double r2, double A12, double B6, double qq) {
+  double r2inv = 1 / r2;
+  double r6inv = r2inv * r2inv * r2inv;
+  return r6inv * (A12 * r6inv - B6) + qq * sqrt(r2inv);
 }
 
 /* Born-Mayer-Huggins (Tosi-Fumi NaCl, src/potential/BMHFT/potentialBMHFT.hpp:21-39) */
@@ -975,7 +982,7 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
         const double R2e = r2d(xd, x.c.x + 3 * j);
         const double qq = qid * qj;
         double ed = 0;
-        if ((on >> s) & 1u) ed += lj_coul_energy(R2e, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qq);
+        if ((on >> s) & 1u) ed += lj_coul_energy(R2e, x.db[P->d_ljA12 + tt], x.db[P->d_ljB6 + tt], qq);
         if (kBorn && ((born_on >> s) & 1u)) ed += born_energy(R2e, tag_bmh(gi.k), tag_bmh(gj.k), qq);
         const bool iion = ii < ni, jion = j < ni;
         if (iion && jion) e_ion += efixd(ed);
@@ -1550,8 +1557,8 @@ __device__ __forceinline__ void gas_gg_pass_t(Ctx& x, bool eflag, bool fresh) {
           }
           F[at][0] += fx; F[at][1] += fy; F[at][2] += fz;
           if (eflag && t > s)
-            egg += efixd(lj_coul_energy(r2d(X + 3 * at, Y), x.db[P->d_ljA + ta * nt + tb],
-                                        x.db[P->d_ljB + ta * nt + tb], 0.0));
+            egg += efixd(lj_energy(r2d(X + 3 * at, Y), x.db[P->d_ljA12 + ta * nt + tb],
+                                   x.db[P->d_ljB6 + ta * nt + tb]));
         }
       }
     }
@@ -1628,8 +1635,8 @@ __device__ __forceinline__ void near_partner(Ctx& x, const double* X, const floa
     F[at][0] += f[0]; F[at][1] += f[1]; F[at][2] += f[2];
     R[0] -= f[0]; R[1] -= f[1]; R[2] -= f[2];
     if (eflag)
-      e += efixd(lj_coul_energy(r2d(X + 3 * at, x.c.x + 3 * j), x.db[P->d_ljA + gtype[at] * nt + tj],
-                                x.db[P->d_ljB + gtype[at] * nt + tj], 0.0));
+      e += efixd(lj_energy(r2d(X + 3 * at, x.c.x + 3 * j), x.db[P->d_ljA12 + gtype[at] * nt + tj],
+                           x.db[P->d_ljB6 + gtype[at] * nt + tj]));
   }
   acc_add(x, j, R);
 }

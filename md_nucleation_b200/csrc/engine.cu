@@ -612,6 +612,10 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
         }
       P.d_ljA = dpush(A.data(), nt * nt);
       P.d_ljB = dpush(B.data(), nt * nt);
+      for (double& v : A) v /= 12.0; /* the pair energies' coefficients */
+      for (double& v : B) v /= 6.0;
+      P.d_ljA12 = dpush(A.data(), nt * nt);
+      P.d_ljB6 = dpush(B.data(), nt * nt);
       P.d_mass = dpush(d.atom_mass, nt);
       std::vector<double> c2(nt);
       for (int t = 0; t < nt; t++) c2[t] = P.coeff / d.atom_mass[t];

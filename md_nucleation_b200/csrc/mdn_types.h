@@ -79,7 +79,7 @@ typedef struct RepParams {
   int ion_groups_n[3];           /* ion groups of 1, 2 and 3 constraints; stored largest first */
   int n_vap_groups, o_vap_grp, o_vap_gstart;
   /* offsets inside the double blob */
-  int d_bond, d_angle, d_dih, d_ljA, d_ljB, d_mass, d_c2;
+  int d_bond, d_angle, d_dih, d_ljA, d_ljB, d_ljA12, d_ljB6, d_mass, d_c2;
   int d_ion_q, d_gas_x, d_gas_q, d_vap_x, d_vap_q;
   int d_ion_cons, d_gas_cons, d_vap_cons; /* per SHAKE constraint: d^2, 1/m_i, 1/m_j */
   int ggl_cap;                   /* gas-gas list entries (both directions), 0 without gg */
