@@ -5,9 +5,10 @@
  *
  * Forward: the engine advances the window (FP32 pair terms, FP64
  * integration) and the replica's in-domain atoms are gathered every K steps
- * (checkpoints).  Backward: one CTA per segment, last segment first,
- * recomputes the segment in FP64 from its checkpoint, keeping x_t, v_t, F_t
- * and the SHAKE multipliers of each step, then runs the adjoint of
+ * (checkpoints).  Backward: every segment is recomputed in FP64 from its
+ * checkpoint at once, one cluster each, keeping x_t, v_t, F_t, the taper
+ * weights and the SHAKE multipliers of each step; then one cluster runs, last
+ * segment first, the adjoint of
  *   (1) v_a = v + c F          (2) y = x + dt v_a          (3) x' = SHAKE(y; x)
  *   (4) v_b = v_a + (x' - y)/dt (5) F' = F(x'; theta)      (6) v' = v_b + c F'
  * (MD::verlet, src/verlet.cpp:20-39, with the SHAKE step of src/shake.cpp:6-92
@@ -18,11 +19,20 @@
  *     dependence on the ion centre; forward-mode (dual number) products for
  *     the bonded terms, whose force Jacobians are symmetric (F = -grad U);
  *   - (3): the adjoint of the converged projection x' = y + sum_k g_k D_k r_k
- *     (r_k the constraint vector at the step's start): G^T mu = rho solved by
- *     colour-ordered Gauss-Seidel sweeps, lambda_y = lambda - sum_k mu_k B_k^T,
- *     plus the g_k D_k dr_k terms into the previous positions.
- * Parameter derivatives accumulate in FP64 in shared memory; atomics make
- * sums independent of the launch shape up to FP64 rounding order.
+ *     (r_k the constraint vector at the step's start): G^T mu = rho solved per
+ *     group of constraints that share atoms, lambda_y = lambda - sum_k mu_k
+ *     B_k^T, plus the g_k D_k dr_k terms into the previous positions.
+ *
+ * What bounds it: a step is a few ten thousand FP64 pair products between two
+ * points where all CTAs meet.  So nothing is scattered: a warp takes an atom
+ * and sums over its row of partners (each pair evaluated from both sides), a
+ * bonded term's forces go to rows of their own that the atoms' owners read,
+ * and a warp takes a constraint group with everything that happens to its
+ * atoms between two force products.  A step has two cluster barriers.  (With
+ * FP64 atomics per pair, 150 thousand on 1,476 addresses, a reverse step of
+ * 492 atoms took 164 us, of which the atomics 130; a recomputed one 127 us.)
+ * Parameter derivatives are summed per warp and row of parameters, then in
+ * shared memory; the sums agree between runs up to FP64 rounding order.
  */
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -34,6 +44,7 @@
 #include <algorithm>
 #include <map>
 #include <set>
+#include <type_traits>
 #include <vector>
 
 #include "mdn.h"
@@ -193,6 +204,14 @@ __constant__ double kBornD[2][2][5] = {
 /* ------------------------------------------------------------------------- */
 /* the dense system of the window                                              */
 /* ------------------------------------------------------------------------- */
+struct Unit {
+  int na, nc;     /* atoms (<= 8), constraints (<= 3) */
+  int atom[8];
+  int cons[3];
+  int ci[3], cj[3]; /* the constraints' atoms as places in atom[] */
+};
+constexpr int kPrimary = 8; /* this side of the pair counts its parameter derivatives */
+
 struct Sys {
   int N, n_ion, nt;
   const int* type;       /* [N] */
@@ -201,9 +220,6 @@ struct Sys {
   const double* c;       /* [N] kick coefficient 0.5 dt 4.184e-4 / m */
   const unsigned char* vapor; /* [N] 1 for vapor atoms (taper weights) */
   int n_pairs;
-  const int* pi;
-  const int* pj;
-  const unsigned char* pk;
   const double* A;       /* [nt*nt] */
   const double* B;
   const double* eps;     /* [nt*nt] pair eps / sigma (for the derivatives) */
@@ -224,6 +240,20 @@ struct Sys {
   const int* cons_nb_off; /* CSR: constraints sharing an atom with constraint k */
   const int* cons_nb;
   int n_cons_nb;          /* entries of cons_nb */
+  /* pairs by atom, from both sides: the partners of atom i are row[row_off[i]
+   * .. row_off[i + 1]), x the partner, y its kind and kPrimary */
+  const int* row_off;
+  const int2* row;
+  const int* row_order;   /* [N] atoms, longest rows first */
+  /* bonded terms by atom: tb_at[tb_off[i] .. tb_off[i + 1]) are the rows of
+   * Buf::tb (4 per term) that act on atom i */
+  const int* tb_off;
+  const int* tb_at;
+  /* what one warp carries from one force product to the next: a group of
+   * constraints that share atoms, or up to 8 unconstrained atoms; n_units = 0
+   * when a group has more than three constraints (shake / shake_adjoint) */
+  int n_units;
+  const Unit* units;
   double ri2, RI2, rcenter, overlap;
   double ion_msum, qqrd2e, dt;
   double efield[3];
@@ -242,14 +272,14 @@ struct Buf {
   double* lx;    /* [3N] adjoint of x, carried across segments */
   double* lv;    /* [3N] adjoint of v */
   double* lf;    /* [3N] adjoint of F */
-  double* tmp;   /* [3N] */
   double* xb;    /* [3N] accumulates the adjoint of the previous positions */
-  double* w;     /* [N] taper weights at the current positions */
-  double* dw;    /* [3N] their gradients */
-  double* om;    /* [N] weight adjoints of the current pass */
+  double* w;     /* [(K+1)*N] taper weights of each step of the segment */
+  double* dw;    /* [(K+1)*3N] their gradients */
+  double* mg;    /* [(K+1)*3*(n_vmol+1)] count term: d/d(centre of vapor molecule m), then minus their sum */
+  double* tb;    /* [4*terms*3] bonded terms' forces (or products) */
+  double* part;  /* [8*3] the CTAs' shares of the weights' pull on the ion centre */
   double* mu;    /* [n_cons] */
   double* grad;  /* [n_params] */
-  double* J;     /* [1] */
   int* flag;     /* [2] SHAKE convergence scratch, status */
 };
 
@@ -289,8 +319,6 @@ __device__ __forceinline__ void csync() {
   }
 }
 
-/* three sums over the cluster at once, the same in every CTA (the CTAs'
- * sums added in rank order; two cluster barriers) */
 /* three sums over the block, the same in every thread; red >= 67 doubles */
 __device__ void block_sum3(double* v, double* red) {
 #pragma unroll
@@ -311,384 +339,353 @@ __device__ void block_sum3(double* v, double* red) {
   __syncthreads();
 }
 
-__device__ void cluster_sum3(double* v, double* red) {
-  cg::cluster_group cl = cg::this_cluster();
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  __syncthreads();
-  if (l == 0)
-    for (int k = 0; k < 3; k++) red[4 * w + k] = v[k]; /* red holds >= 4 * 16 + 3 doubles */
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    double t = 0;
-    for (int q = 0; q < nw; q++) t += red[4 * q + threadIdx.x];
-    red[64 + threadIdx.x] = t;
-  }
-  if (cl.num_blocks() > 1) {
-    cl.sync();
-    for (int k = 0; k < 3; k++) {
-      double t = 0;
-      for (unsigned r = 0; r < cl.num_blocks(); r++) t += *cl.map_shared_rank(&red[64 + k], r);
-      v[k] = t;
-    }
-    cl.sync();
-  } else {
-    __syncthreads();
-    for (int k = 0; k < 3; k++) v[k] = red[64 + k];
-    __syncthreads();
-  }
-}
+/* x, v, f, ... that other CTAs write are read from L2 */
+__device__ __forceinline__ int cwarp() { return ctid() >> 5; }
+__device__ __forceinline__ int cnwarps() { return cnthr() >> 5; }
 
-/* ion centre of x (mass-weighted) into cent[0..2] */
+/* ion centre of x (mass-weighted) into cent[0..2]; x was written by the whole
+ * cluster */
 __device__ void ion_centre(const Sys& S, const double* x, double* cent, double* red) {
-  double sx = 0, sy = 0, sz = 0;
-  for (int i = threadIdx.x; i < S.n_ion; i += blockDim.x) {
-    sx += x[3 * i] * S.mass[i];
-    sy += x[3 * i + 1] * S.mass[i];
-    sz += x[3 * i + 2] * S.mass[i];
-  }
-  sx = block_sum(sx, red);
-  sy = block_sum(sy, red);
-  sz = block_sum(sz, red);
-  if (threadIdx.x == 0) {
-    cent[0] = sx / S.ion_msum;
-    cent[1] = sy / S.ion_msum;
-    cent[2] = sz / S.ion_msum;
-  }
+  double v[3] = {0, 0, 0};
+  for (int i = threadIdx.x; i < S.n_ion; i += blockDim.x)
+    for (int k = 0; k < 3; k++) v[k] += __ldcg(x + 3 * i + k) * S.mass[i];
+  block_sum3(v, red);
+  if (threadIdx.x < 3) cent[threadIdx.x] = v[threadIdx.x] / S.ion_msum;
   __syncthreads();
 }
 
-/* taper weights and their gradients (src/verlet.cpp:109-134) */
-__device__ void weights(const Sys& S, const Buf& B, const double* x, const double* cent) {
+/* taper weight of atom i and its gradient (src/verlet.cpp:109-134) */
+__device__ __forceinline__ double weight_of(const Sys& S, const double* x, const double* cent, int i, double* g) {
+  g[0] = g[1] = g[2] = 0;
+  if (!S.vapor[i]) return 1;
   const double a = 3.141592653589793 / S.overlap * 0.5;
-  for (int i = ctid(); i < S.N; i += cnthr()) {
-    double w = 1, g0 = 0, g1 = 0, g2 = 0;
-    if (S.vapor[i]) {
-      double dx = x[3 * i] - cent[0], dy = x[3 * i + 1] - cent[1], dz = x[3 * i + 2] - cent[2];
-      double r2 = dx * dx + dy * dy + dz * dz;
-      if (r2 < S.ri2) w = 1;
-      else if (r2 > S.RI2) w = 0;
-      else {
-        double r = sqrt(r2);
-        double C = cos(a * (r - S.rcenter));
-        w = C * C;
-        double dwdr = -2.0 * C * sin(a * (r - S.rcenter)) * a;
-        g0 = dwdr * dx / r;
-        g1 = dwdr * dy / r;
-        g2 = dwdr * dz / r;
+  double dx = __ldcg(x + 3 * i) - cent[0], dy = __ldcg(x + 3 * i + 1) - cent[1], dz = __ldcg(x + 3 * i + 2) - cent[2];
+  double r2 = dx * dx + dy * dy + dz * dz;
+  if (r2 < S.ri2) return 1;
+  if (r2 > S.RI2) return 0;
+  double r = sqrt(r2);
+  double C = cos(a * (r - S.rcenter));
+  double dwdr = -2.0 * C * sin(a * (r - S.rcenter)) * a;
+  g[0] = dwdr * dx / r;
+  g[1] = dwdr * dy / r;
+  g[2] = dwdr * dz / r;
+  return C * C;
+}
+
+/* What the reverse sweep needs of the positions x of step t besides x: the
+ * weights and the count term's derivatives.  Every CTA of the cluster makes
+ * all of it for itself in its own shared memory (sw: the weights) and the
+ * first one keeps it; returns this thread's share of the count term. */
+__device__ double place_terms(const Sys& S, const Buf& B, const double* x, int t, double* cent, double* sw,
+                              double* red) {
+  const bool lead = cg::this_cluster().block_rank() == 0;
+  ion_centre(S, x, cent, red);
+  for (int i = threadIdx.x; i < S.N; i += blockDim.x) {
+    double g[3];
+    const double w = weight_of(S, x, cent, i, g);
+    sw[i] = w;
+    if (lead) {
+      B.w[(size_t)t * S.N + i] = w;
+      for (int k = 0; k < 3; k++) B.dw[(size_t)t * 3 * S.N + 3 * i + k] = g[k];
+    }
+  }
+  double jp = 0;
+  if (lead && S.w_count != 0) {
+    double C[3] = {0, 0, 0};
+    double* const mg = B.mg + (size_t)t * 3 * (S.n_vmol + 1);
+    for (int m = threadIdx.x; m < S.n_vmol; m += blockDim.x) {
+      const int a0 = S.vmol_first + m * S.a_v;
+      double cm[3] = {0, 0, 0};
+      for (int a = 0; a < S.a_v; a++)
+        for (int q = 0; q < 3; q++) cm[q] += __ldcg(x + 3 * (a0 + a) + q) * S.mass[a0 + a];
+      for (int q = 0; q < 3; q++) cm[q] /= S.vmol_mass;
+      double dv[3] = {cm[0] - cent[0], cm[1] - cent[1], cm[2] - cent[2]};
+      double rho = sqrt(dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2]);
+      double sgm = 1.0 / (1.0 + exp((rho - S.R0) / S.W));
+      jp += S.w_count * sgm;
+      double dSdrho = -sgm * (1.0 - sgm) / S.W * S.w_count * S.inv_n;
+      for (int q = 0; q < 3; q++) {
+        const double c = dSdrho * dv[q] / rho;
+        mg[3 * m + q] = c;
+        C[q] += c;
       }
     }
-    B.w[i] = w;
-    B.dw[3 * i] = g0;
-    B.dw[3 * i + 1] = g1;
-    B.dw[3 * i + 2] = g2;
+    block_sum3(C, red);
+    if (threadIdx.x < 3) mg[3 * S.n_vmol + threadIdx.x] = -C[threadIdx.x];
   }
-  /* no barrier: the callers' next barrier comes before any read */
+  __syncthreads();
+  return jp;
 }
 
 /* force factor f(u) and df/du of one pair (u = r^2), parameter derivatives
- * of f (d eps, d sigma, d s at s = 1), and the pair's weight */
+ * of f (d eps, d sigma, d s at s = 1) */
 struct PairEval {
-  double f, fp, fe, fs_sig, fq, W;
+  double f, fp, fe, fs_sig, fq;
   int p;  /* parameter base, -1 */
-  bool ljp;
 };
 
-__device__ __forceinline__ PairEval eval_pair(const Sys& S, const Buf& B, int i, int j, int kind, double u) {
+__device__ __forceinline__ PairEval eval_pair(const Sys& S, int i, int j, int kind, double u) {
   PairEval o;
   o.p = -1;
-  o.ljp = false;
   o.fe = o.fs_sig = o.fq = 0;
-  o.W = 1;
-  const int ti = S.type[i], tj = S.type[j];
-  const int tt = ti * S.nt + tj;
+  const int tt = S.type[i] * S.nt + S.type[j];
+  const double ui = 1.0 / u;
   double f = 0, fp = 0;
   if (kind == PK_ION_BMH) {
     const double* cB = kBornD[S.bmh[i]][S.bmh[j]];
     double r = sqrt(u);
     double e = exp(cB[4] * (cB[3] - r));
     double qq = S.qqrd2e * S.q[i] * S.q[j];
-    double g = cB[4] * cB[0] * r * e - cB[1] * pow(r, -6.0) - cB[2] * pow(r, -8.0) + qq / r;
-    double gp = cB[4] * cB[0] * e * (1.0 - cB[4] * r) + 6.0 * cB[1] * pow(r, -7.0) + 8.0 * cB[2] * pow(r, -9.0) - qq / u;
-    f = g / u;
-    double dfdr = gp / u - 2.0 * g / (u * r);
+    const double u3 = ui * ui * ui, u4 = u3 * ui;
+    double g = cB[4] * cB[0] * r * e - cB[1] * u3 - cB[2] * u4 + qq / r;
+    double gp = cB[4] * cB[0] * e * (1.0 - cB[4] * r) + (6.0 * cB[1] * u3 + 8.0 * cB[2] * u4 ) / r - qq * ui;
+    f = g * ui;
+    double dfdr = gp * ui - 2.0 * g * ui / r;
     fp = dfdr / (2.0 * r);
-    o.fq = 2.0 * qq / (r * u); /* Coulomb scales as s^2 */
+    o.fq = 2.0 * qq * ui / r; /* Coulomb scales as s^2 */
   } else {
-    const double Aij = S.A[tt], Bij = S.B[tt];
-    const double u2 = u * u, u4 = u2 * u2, u3 = u2 * u, u7 = u4 * u3, u8 = u4 * u4;
-    f = Aij / u7 - Bij / u4;
-    fp = -7.0 * Aij / u8 + 4.0 * Bij / (u4 * u);
+    const double u2 = ui * ui, u4 = u2 * u2, u7 = u4 * u2 * ui;
+    const double a7 = S.A[tt] * u7, b4 = S.B[tt] * u4;
+    f = a7 - b4;
+    fp = (4.0 * b4 - 7.0 * a7) * ui;
     if (kind == PK_GI || kind == PK_VI) {
       o.p = S.pidx[tt];
       if (o.p >= 0) {
-        o.ljp = true;
         o.fe = f / S.eps[tt];
-        o.fs_sig = (12.0 * Aij / u7 - 6.0 * Bij / u4) / S.sig[tt];
+        o.fs_sig = (12.0 * a7 - 6.0 * b4) / S.sig[tt];
       }
     }
     if (kind == PK_VI || kind == PK_VV || kind == PK_ION_LJC) {
-      double qq = S.qqrd2e * S.q[i] * S.q[j];
-      double r = sqrt(u);
-      double fc = qq / (u * r);
+      const double fc = S.qqrd2e * S.q[i] * S.q[j] * ui * sqrt(ui);
       f += fc;
-      fp += -1.5 * fc / u;
+      fp += -1.5 * fc * ui;
       if (kind == PK_VI) o.fq = fc;
       else if (kind == PK_ION_LJC) o.fq = 2.0 * fc;
     }
-    if (kind == PK_VI || kind == PK_VV) o.W = __ldcg(B.w + i) * __ldcg(B.w + j);
   }
   o.f = f;
   o.fp = fp;
   return o;
 }
 
-/* F(x): all terms, FP64 */
-__device__ void forces(const Sys& S, const Buf& B, const double* x, double* F) {
-  for (int q = threadIdx.x; q < 3 * S.N; q += blockDim.x) F[q] = 0;
-  __syncthreads();
-  for (int p = threadIdx.x; p < S.n_pairs; p += blockDim.x) {
-    const int i = S.pi[p], j = S.pj[p], k = S.pk[p];
-    double d0 = x[3 * i] - x[3 * j], d1 = x[3 * i + 1] - x[3 * j + 1], d2 = x[3 * i + 2] - x[3 * j + 2];
-    double u = d0 * d0 + d1 * d1 + d2 * d2;
-    PairEval e = eval_pair(S, B, i, j, k, u);
-    double g = e.W * e.f;
-    atomicAdd(&F[3 * i], g * d0);
-    atomicAdd(&F[3 * i + 1], g * d1);
-    atomicAdd(&F[3 * i + 2], g * d2);
-    atomicAdd(&F[3 * j], -g * d0);
-    atomicAdd(&F[3 * j + 1], -g * d1);
-    atomicAdd(&F[3 * j + 2], -g * d2);
-  }
-  const int nb = S.n_bonds, na = S.n_angles, nd = S.n_dih;
-  for (int t = threadIdx.x; t < nb + na + nd; t += blockDim.x) {
-    int at[4], n;
-    double X[4][3], f[4][3];
-    if (t < nb) {
-      const int* r = S.bonds + 3 * t;
-      at[0] = r[0]; at[1] = r[1]; n = 2;
-      for (int a = 0; a < n; a++)
-        for (int k = 0; k < 3; k++) X[a][k] = x[3 * at[a] + k];
-      bond_t<double>(X, S.bond_c + 2 * r[2], f);
-    } else if (t < nb + na) {
-      const int* r = S.angles + 4 * (t - nb);
-      at[0] = r[0]; at[1] = r[1]; at[2] = r[2]; n = 3;
-      for (int a = 0; a < n; a++)
-        for (int k = 0; k < 3; k++) X[a][k] = x[3 * at[a] + k];
-      angle_t<double>(X, S.angle_c + 2 * r[3], f);
-    } else {
-      const int* r = S.dih + 5 * (t - nb - na);
-      at[0] = r[0]; at[1] = r[1]; at[2] = r[2]; at[3] = r[3]; n = 4;
-      for (int a = 0; a < n; a++)
-        for (int k = 0; k < 3; k++) X[a][k] = x[3 * at[a] + k];
-      dihedral_t<double>(X, S.dih_c + 15 * r[4], S.dih_multi[r[4]], f);
-    }
-    for (int a = 0; a < n; a++)
-      for (int k = 0; k < 3; k++) atomicAdd(&F[3 * at[a] + k], f[a][k]);
-  }
-  if (S.efield_on)
-    for (int i = threadIdx.x; i < S.n_ion; i += blockDim.x) {
-      double co = 5.55e-5 * S.q[i];
-      for (int k = 0; k < 3; k++) atomicAdd(&F[3 * i + k], co * S.efield[k]);
-    }
-  __syncthreads();
-}
-
-/* The parameter derivatives of the pair loops, summed in registers: the
- * pairs are sorted by kind and type pair, so a thread's run of pairs keeps
- * one (eps, sigma) row for many pairs and adds its sums to the shared
- * gradient when the row changes; the charge scale, which every charged pair
- * touches, is summed over the warp first.  (Adding every pair's terms to the
- * few shared rows directly serialised the pair loops on those addresses.) */
 __device__ __forceinline__ double warp_sum_dd(double v) {
 #pragma unroll
   for (int m = 16; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
   return v;
 }
 
-struct ParamSums {
-  int p = -1;
-  double e = 0, s = 0, q = 0;
-  __device__ __forceinline__ void add_lj(double* sgrad, int row, double de, double ds) {
-    if (row != p) {
-      flush_lj(sgrad);
-      p = row;
-    }
-    e += de;
-    s += ds;
-  }
-  __device__ __forceinline__ void flush_lj(double* sgrad) {
-    if (p >= 0) {
-      atomicAdd(&sgrad[p], e);
-      atomicAdd(&sgrad[p + 1], s);
-    }
-    p = -1;
-    e = s = 0;
-  }
-  /* all threads of the block */
-  __device__ __forceinline__ void finish(double* sgrad, int n_params) {
-    flush_lj(sgrad);
-    const double t = warp_sum_dd(q);
-    if ((threadIdx.x & 31) == 0 && t != 0) atomicAdd(&sgrad[n_params - 1], t);
-    q = 0;
-  }
-};
-
-/* out += J_F(x)^T lam; grad += (dF/dtheta)^T lam.  Weights must be current. */
-__device__ void force_vjp(const Sys& S, const Buf& B, const double* x, const double* lam, double* out,
-                          double* sgrad, const double* cent, double* red) {
-  /* B.om was zeroed before the caller's last cluster barrier */
-  ParamSums ps;
-  for (int p = ctid(); p < S.n_pairs; p += cnthr()) {
-    const int i = S.pi[p], j = S.pj[p], k = S.pk[p];
-    double d[3] = {x[3 * i] - x[3 * j], x[3 * i + 1] - x[3 * j + 1], x[3 * i + 2] - x[3 * j + 2]};
-    double u = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-    PairEval e = eval_pair(S, B, i, j, k, u);
-    double m[3] = {__ldcg(lam + 3 * i) - __ldcg(lam + 3 * j), __ldcg(lam + 3 * i + 1) - __ldcg(lam + 3 * j + 1),
-                   __ldcg(lam + 3 * i + 2) - __ldcg(lam + 3 * j + 2)};
-    double dm = d[0] * m[0] + d[1] * m[1] + d[2] * m[2];
-    for (int q = 0; q < 3; q++) {
-      double g = e.W * (e.f * m[q] + 2.0 * e.fp * dm * d[q]);
-      atomicAdd(&out[3 * i + q], g);
-      atomicAdd(&out[3 * j + q], -g);
-    }
-    if (k == PK_VI || k == PK_VV) {
-      double t = e.f * dm;
-      if (S.vapor[i]) atomicAdd(&B.om[i], __ldcg(B.w + j) * t);
-      if (S.vapor[j]) atomicAdd(&B.om[j], __ldcg(B.w + i) * t);
-    }
-    if (e.ljp) ps.add_lj(sgrad, e.p, e.W * e.fe * dm, e.W * e.fs_sig * dm);
-    if (e.fq != 0) ps.q += e.W * e.fq * dm;
-  }
-  ps.finish(sgrad, S.n_params);
-  csync();
-  /* weights: x_i directly, and the ion centre c they are measured from */
-  double s0 = 0, s1 = 0, s2 = 0;
-  for (int i = ctid(); i < S.N; i += cnthr()) {
-    if (!S.vapor[i]) continue;
-    double o = __ldcg(B.om + i);
-    double g0 = o * __ldcg(B.dw + 3 * i), g1 = o * __ldcg(B.dw + 3 * i + 1), g2 = o * __ldcg(B.dw + 3 * i + 2);
-    atomicAdd(out + 3 * i, g0);
-    atomicAdd(out + 3 * i + 1, g1);
-    atomicAdd(out + 3 * i + 2, g2);
-    s0 += g0;
-    s1 += g1;
-    s2 += g2;
-  }
-  {
-    double sv[3] = {s0, s1, s2};
-    cluster_sum3(sv, red);
-    s0 = sv[0];
-    s1 = sv[1];
-    s2 = sv[2];
-  }
-  for (int a = ctid(); a < S.n_ion; a += cnthr()) {
-    double fr = S.mass[a] / S.ion_msum;
-    atomicAdd(out + 3 * a, -fr * s0);
-    atomicAdd(out + 3 * a + 1, -fr * s1);
-    atomicAdd(out + 3 * a + 2, -fr * s2);
-  }
-  /* bonded terms: J lam by forward-mode products (symmetric Jacobians) */
+/* 32 bonded terms 32 k .. of x into their rows of B.tb: their forces, or with
+ * lam the products of their Jacobians (symmetric: F = -grad U) with lam by
+ * forward mode */
+template <class T>
+__device__ __forceinline__ void bonded_rows(const Sys& S, const Buf& B, const double* x, const double* lam, int k) {
+  constexpr bool dual = !std::is_same<T, double>::value;
   const int nb = S.n_bonds, na = S.n_angles, nd = S.n_dih;
-  for (int t = ctid(); t < nb + na + nd; t += cnthr()) {
-    int at[4], n;
-    Dual X[4][3], f[4][3];
-    const int* r;
-    if (t < nb) { r = S.bonds + 3 * t; n = 2; }
-    else if (t < nb + na) { r = S.angles + 4 * (t - nb); n = 3; }
-    else { r = S.dih + 5 * (t - nb - na); n = 4; }
-    for (int a = 0; a < n; a++) {
-      at[a] = r[a];
-      for (int k = 0; k < 3; k++) X[a][k] = mk(x[3 * at[a] + k], __ldcg(lam + 3 * at[a] + k));
+  /* the long terms first; the rows are numbered bonds, angles, dihedrals */
+  int t = 32 * k + (int)(threadIdx.x & 31);
+  if (t >= nb + na + nd) return;
+  t = t < nd ? nb + na + t : t < nd + na ? nb + t - nd : t - nd - na;
+  int n;
+  T X[4][3], f[4][3];
+  const int* r;
+  if (t < nb) { r = S.bonds + 3 * t; n = 2; }
+  else if (t < nb + na) { r = S.angles + 4 * (t - nb); n = 3; }
+  else { r = S.dih + 5 * (t - nb - na); n = 4; }
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    if (a >= n) break;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      if constexpr (dual) X[a][q] = mk(__ldcg(x + 3 * r[a] + q), __ldcg(lam + 3 * r[a] + q));
+      else X[a][q] = __ldcg(x + 3 * r[a] + q);
     }
-    if (n == 2) bond_t<Dual>(X, S.bond_c + 2 * r[2], f);
-    else if (n == 3) angle_t<Dual>(X, S.angle_c + 2 * r[3], f);
-    else dihedral_t<Dual>(X, S.dih_c + 15 * r[4], S.dih_multi[r[4]], f);
-    for (int a = 0; a < n; a++)
-      for (int k = 0; k < 3; k++) atomicAdd(&out[3 * at[a] + k], f[a][k].d);
   }
-  if (S.efield_on) {
-    double sq = 0;
-    for (int i = ctid(); i < S.n_ion; i += cnthr())
-      sq += 5.55e-5 * S.q[i] *
-            (S.efield[0] * __ldcg(lam + 3 * i) + S.efield[1] * __ldcg(lam + 3 * i + 1) +
-             S.efield[2] * __ldcg(lam + 3 * i + 2));
-    /* this CTA's share; the CTAs' gradients are summed at the end */
-    sq = block_sum(sq, red);
-    if (threadIdx.x == 0) sgrad[S.n_params - 1] += sq;
+  if (n == 2) bond_t<T>(X, S.bond_c + 2 * r[2], f);
+  else if (n == 3) angle_t<T>(X, S.angle_c + 2 * r[3], f);
+  else dihedral_t<T>(X, S.dih_c + 15 * r[4], S.dih_multi[r[4]], f);
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    if (a >= n) break;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      if constexpr (dual) B.tb[12 * (size_t)t + 3 * a + q] = f[a][q].d;
+      else B.tb[12 * (size_t)t + 3 * a + q] = f[a][q];
+    }
   }
-  csync();
 }
 
-/* objective at x: value (returned by thread partial), gradient into out
- * (scaled by inv_n) and parameter derivatives into sgrad */
-__device__ double objective(const Sys& S, const double* x, double* out, double* sgrad, const double* cent,
-                            bool grad, double* red) {
-  double jp = 0;
-  ParamSums ps;
-  if (S.w_energy != 0)
-    for (int p = ctid(); p < S.n_pairs; p += cnthr()) {
-      if (S.pk[p] != PK_VI) continue;
-      const int i = S.pi[p], j = S.pj[p];
-      const int tt = S.type[i] * S.nt + S.type[j];
-      double d[3] = {x[3 * i] - x[3 * j], x[3 * i + 1] - x[3 * j + 1], x[3 * i + 2] - x[3 * j + 2]};
-      double u = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-      double r = sqrt(u), u3 = u * u * u;
-      double qq = S.qqrd2e * S.q[i] * S.q[j];
-      double Ulj = S.A[tt] / 12.0 / (u3 * u3) - S.B[tt] / 6.0 / u3;
-      jp += S.w_energy * (Ulj + qq / r);
-      if (!grad) continue;
-      double dUdu = -S.A[tt] / 2.0 / (u3 * u3 * u) + S.B[tt] / 2.0 / (u3 * u) - 0.5 * qq / (u * r);
-      double c = 2.0 * dUdu * S.w_energy * S.inv_n;
-      for (int q = 0; q < 3; q++) {
-        atomicAdd(&out[3 * i + q], c * d[q]);
-        atomicAdd(&out[3 * j + q], -c * d[q]);
-      }
-      const int pb = S.pidx[tt];
-      if (pb >= 0)
-        ps.add_lj(sgrad, pb, S.w_energy * S.inv_n * Ulj / S.eps[tt],
-                  S.w_energy * S.inv_n * (S.A[tt] / (u3 * u3) - S.B[tt] / u3) / S.sig[tt]);
-      ps.q += S.w_energy * S.inv_n * qq / r;
-    }
-  if (grad) ps.finish(sgrad, S.n_params);
-  if (S.w_count != 0) {
-    /* every CTA takes every molecule (a handful); the first CTA adds the
-     * value and the vapor atoms' terms, and the ion atoms' shares of the
-     * centre's derivative are summed over the molecules first and then added
-     * once per ion atom, split over the cluster */
-    const bool lead = cg::this_cluster().block_rank() == 0;
-    double C[3] = {0, 0, 0};
-    for (int m = threadIdx.x; m < S.n_vmol; m += blockDim.x) {
-      const int a0 = S.vmol_first + m * S.a_v;
-      double cm[3] = {0, 0, 0};
-      for (int a = 0; a < S.a_v; a++)
-        for (int q = 0; q < 3; q++) cm[q] += x[3 * (a0 + a) + q] * S.mass[a0 + a];
-      for (int q = 0; q < 3; q++) cm[q] /= S.vmol_mass;
-      double dv[3] = {cm[0] - cent[0], cm[1] - cent[1], cm[2] - cent[2]};
-      double rho = sqrt(dv[0] * dv[0] + dv[1] * dv[1] + dv[2] * dv[2]);
-      double sgm = 1.0 / (1.0 + exp((rho - S.R0) / S.W));
-      if (lead) jp += S.w_count * sgm;
-      if (!grad) continue;
-      double dSdrho = -sgm * (1.0 - sgm) / S.W * S.w_count * S.inv_n;
-      if (lead)
-        for (int a = 0; a < S.a_v; a++) {
-          double fr = S.mass[a0 + a] / S.vmol_mass;
-          for (int q = 0; q < 3; q++) atomicAdd(&out[3 * (a0 + a) + q], dSdrho * fr * dv[q] / rho);
-        }
-      for (int q = 0; q < 3; q++) C[q] += dSdrho * dv[q] / rho;
-    }
-    if (grad) {
-      block_sum3(C, red);
-      for (int b = ctid(); b < S.n_ion; b += cnthr()) {
-        double fr = S.mass[b] / S.ion_msum;
-        for (int q = 0; q < 3; q++) atomicAdd(&out[3 * b + q], -fr * C[q]);
-      }
-    }
+/* the bonded terms' rows of component q of atom i, summed */
+__device__ __forceinline__ double bonded_sum(const Sys& S, const Buf& B, int i, int q) {
+  double t = 0;
+  for (int e = S.tb_off[i]; e < S.tb_off[i + 1]; e++) t += __ldcg(B.tb + 3 * (size_t)S.tb_at[e] + q);
+  return t;
+}
+
+/* The warp items of a force evaluation (or product), the CTA's own: bonded
+ * terms by 32 (dual, and longest), then atoms, longest rows first.  Items are
+ * dealt to the CTAs in turn and taken by the warps from a counter. */
+template <class Bonded, class Row>
+__device__ __forceinline__ void force_queue(const Sys& S, int* next, Bonded&& bonded, Row&& row) {
+  const int nbk = (S.n_bonds + S.n_angles + S.n_dih + 31) >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cg::this_cluster().block_rank(), C = (int)cg::this_cluster().num_blocks();
+  for (;;) {
+    int it = 0;
+    if (lane == 0) it = atomicAdd(next, 1);
+    it = rank + __shfl_sync(0xffffffffu, it, 0) * C;
+    if (it >= nbk + S.N) break;
+    if (it < nbk) bonded(it);
+    else row(S.row_order[it - nbk]);
+    __syncwarp();
   }
-  /* no barrier: out is read only after the callers' next one */
+}
+
+/* pair forces on every atom into F (the bonded terms into B.tb); returns the
+ * thread's share of the window's ion-vapor energy */
+__device__ double force_rows(const Sys& S, const Buf& B, const double* x, const double* sw, double* F, int* next) {
+  const int lane = threadIdx.x & 31;
+  double jp = 0;
+  force_queue(S, next, [&](int k) { bonded_rows<double>(S, B, x, nullptr, k); },
+              [&](int i) {
+                const double xi[3] = {__ldcg(x + 3 * i), __ldcg(x + 3 * i + 1), __ldcg(x + 3 * i + 2)};
+                double a[3] = {0, 0, 0};
+                for (int e = S.row_off[i] + lane; e < S.row_off[i + 1]; e += 32) {
+                  const int2 pr = S.row[e];
+                  const int j = pr.x, kind = pr.y & 7;
+                  const double d0 = xi[0] - __ldcg(x + 3 * j), d1 = xi[1] - __ldcg(x + 3 * j + 1),
+                               d2 = xi[2] - __ldcg(x + 3 * j + 2);
+                  const double u = d0 * d0 + d1 * d1 + d2 * d2;
+                  const PairEval ev = eval_pair(S, i, j, kind, u);
+                  double g = ev.f;
+                  if (kind == PK_VI || kind == PK_VV) g *= sw[i] * sw[j];
+                  a[0] += g * d0;
+                  a[1] += g * d1;
+                  a[2] += g * d2;
+                  if (kind == PK_VI && (pr.y & kPrimary)) {
+                    const int tt = S.type[i] * S.nt + S.type[j];
+                    const double u3 = u * u * u;
+                    jp += S.w_energy * (S.A[tt] / 12.0 / (u3 * u3) - S.B[tt] / 6.0 / u3 +
+                                        S.qqrd2e * S.q[i] * S.q[j] / sqrt(u));
+                  }
+                }
+                for (int k = 0; k < 3; k++) a[k] = warp_sum_dd(a[k]);
+                if (lane < 3) {
+                  double t = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];
+                  if (S.efield_on && i < S.n_ion) t += 5.55e-5 * S.q[i] * S.efield[lane];
+                  F[3 * i + lane] = t;
+                }
+              });
   return jp;
+}
+
+/* lx += J_F(x)^T lam (+ the objective's gradient when obj), the bonded terms'
+ * products into B.tb, grad += (dF/dtheta)^T lam (+ the objective's); the
+ * CTA's share of the weights' pull on the ion centre into B.part.  xs, ls: x
+ * and lam in shared memory, or x and lam themselves where they do not fit.
+ * qsum: the lane's share of the charge scale's derivative. */
+template <bool STAGED>
+__device__ __forceinline__ double at_of(const double* p, int q) {
+  if (STAGED) return p[q];
+  return __ldcg(p + q);
+}
+template <bool STAGED>
+__device__ void vjp_rows(const Sys& S, const Buf& B, const double* x, int t, const double* xs, const double* ls,
+                         bool obj, double* sgrad, double* spart, double& qsum, int* next) {
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xffffffffu;
+  const double* const w = B.w + (size_t)t * S.N;
+  const double* const dw = B.dw + (size_t)t * 3 * S.N;
+  const double* const mg = B.mg + (size_t)t * 3 * (S.n_vmol + 1);
+  double pull = 0; /* lanes 0..2: component of the share */
+  force_queue(
+      S, next, [&](int k) { bonded_rows<Dual>(S, B, x, B.lf, k); },
+      [&](int i) {
+        double xi[3], li[3], a[3] = {0, 0, 0}, om = 0;
+        for (int q = 0; q < 3; q++) {
+          xi[q] = at_of<STAGED>(xs, 3 * i + q);
+          li[q] = at_of<STAGED>(ls, 3 * i + q);
+        }
+        const int e1 = S.row_off[i + 1];
+        const double wi = w[i];
+        const bool vap = S.vapor[i] != 0;
+        for (int e0 = S.row_off[i]; e0 < e1; e0 += 32) {
+          int p = -1;
+          double pe = 0, ps = 0;
+          if (e0 + lane < e1) {
+            const int2 pr = S.row[e0 + lane];
+            const int j = pr.x, kind = pr.y & 7;
+            const bool primary = (pr.y & kPrimary) != 0;
+            double d[3], m[3];
+            for (int q = 0; q < 3; q++) {
+              d[q] = xi[q] - at_of<STAGED>(xs, 3 * j + q);
+              m[q] = li[q] - at_of<STAGED>(ls, 3 * j + q);
+            }
+            const double u = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+            const PairEval ev = eval_pair(S, i, j, kind, u);
+            const double dm = d[0] * m[0] + d[1] * m[1] + d[2] * m[2];
+            double W = 1;
+            if (kind == PK_VI || kind == PK_VV) {
+              const double wj = w[j];
+              W = wi * wj;
+              if (vap) om += wj * (ev.f * dm);
+            }
+            const double cm = W * ev.f;
+            double cd = W * (2.0 * ev.fp * dm);
+            if (primary) {
+              if (ev.p >= 0) {
+                p = ev.p;
+                pe = W * ev.fe * dm;
+                ps = W * ev.fs_sig * dm;
+              }
+              qsum += W * ev.fq * dm;
+            }
+            if (obj && kind == PK_VI && S.w_energy != 0) {
+              const int tt = S.type[i] * S.nt + S.type[j];
+              const double ui = 1.0 / u, u3 = ui * ui * ui, a6 = S.A[tt] * (u3 * u3), b3 = S.B[tt] * u3;
+              const double qr = S.qqrd2e * S.q[i] * S.q[j] * sqrt(ui), sc = S.w_energy * S.inv_n;
+              cd += sc * ui * (b3 - a6 - qr);
+              if (primary) {
+                if (p >= 0) {
+                  pe += sc * (a6 / 12.0 - b3 / 6.0) / S.eps[tt];
+                  ps += sc * (a6 - b3) / S.sig[tt];
+                }
+                qsum += sc * qr;
+              }
+            }
+            for (int q = 0; q < 3; q++) a[q] += cm * m[q] + cd * d[q];
+          }
+          /* parameter rows present in the warp, one after another */
+          for (unsigned todo = __ballot_sync(FULL, p >= 0); todo;) {
+            const int r = __shfl_sync(FULL, p, __ffs(todo) - 1);
+            const double se = warp_sum_dd(p == r ? pe : 0.0), ss = warp_sum_dd(p == r ? ps : 0.0);
+            if (lane == 0) {
+              atomicAdd(&sgrad[r], se);
+              atomicAdd(&sgrad[r + 1], ss);
+            }
+            todo &= ~__ballot_sync(FULL, p == r);
+          }
+        }
+        for (int q = 0; q < 3; q++) a[q] = warp_sum_dd(a[q]);
+        if (vap) om = warp_sum_dd(om);
+        if (lane < 3) {
+          double v = lane == 0 ? a[0] : lane == 1 ? a[1] : a[2];
+          if (vap) {
+            const double g = om * dw[3 * i + lane];
+            v += g;
+            pull += g;
+            if (obj && S.w_count != 0)
+              v += S.mass[i] / S.vmol_mass * mg[3 * ((i - S.vmol_first) / S.a_v) + lane];
+          }
+          if (S.efield_on && i < S.n_ion) qsum += 5.55e-5 * S.q[i] * S.efield[lane] * li[lane];
+          B.lx[3 * i + lane] = __ldcg(B.lx + 3 * i + lane) + v;
+        }
+      });
+  if (lane < 3) spart[3 * (threadIdx.x >> 5) + lane] = pull;
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double v = 0;
+    for (int k = 0; k < (int)(blockDim.x >> 5); k++) v += spart[3 * k + threadIdx.x];
+    B.part[3 * cg::this_cluster().block_rank() + threadIdx.x] = v;
+  }
 }
 
 /* SHAKE of every constraint of y against the reference positions xr,
@@ -828,145 +825,311 @@ __device__ void shake_adjoint(const Sys& S, const Buf& B, const double* x, const
   csync();
 }
 
-/* The FP64 recompute of one segment: K steps from (X[0], V[0]), keeping x,
- * v, F and the converged SHAKE multipliers of every step; returns the
- * segment's sum of the objective.  first = 1 for the window's first segment,
- * whose start forces are the ones the state holds (f0; zero on a replica
- * that was never stepped, since the reference evaluates no force before the
- * first kick); other segments evaluate F(x_0). */
-__device__ double recompute(const Sys& S, const Buf& B, int K, int first, const double* f0, double* red,
-                            double* cent) {
-  const int n3 = 3 * S.N;
-  if (first) {
-    for (int q = threadIdx.x; q < n3; q += blockDim.x) B.F[q] = f0[q];
-    __syncthreads();
-  } else {
-    ion_centre(S, B.X, cent, red);
-    weights(S, B, B.X, cent);
-    forces(S, B, B.X, B.F);
-  }
-  double jacc = 0;
-  for (int t = 1; t <= K; t++) {
-    const double* x0 = B.X + (size_t)(t - 1) * n3;
-    const double* v0 = B.V + (size_t)(t - 1) * n3;
-    const double* f0t = B.F + (size_t)(t - 1) * n3;
-    double* x1 = B.X + (size_t)t * n3;
-    double* v1 = B.V + (size_t)t * n3;
-    double* f1 = B.F + (size_t)t * n3;
-    for (int q = threadIdx.x; q < n3; q += blockDim.x) {
-      const int i = q / 3;
-      double va = v0[q] + S.c[i] * f0t[q];
-      v1[q] = va;
-      x1[q] = x0[q] + S.dt * va;
-    }
-    __syncthreads();
-    if (S.n_cons > 0) {
-      shake(S, B, x1, x0, B.gam + (size_t)(t - 1) * S.n_cons);
-      if (S.vcorr)
-        for (int q = threadIdx.x; q < n3; q += blockDim.x) {
-          double y = x0[q] + S.dt * v1[q];
-          v1[q] += (x1[q] - y) / S.dt;
-        }
-      __syncthreads();
-    }
-    ion_centre(S, x1, cent, red);
-    weights(S, B, x1, cent);
-    forces(S, B, x1, f1);
-    for (int q = threadIdx.x; q < n3; q += blockDim.x) v1[q] += S.c[q / 3] * f1[q];
-    __syncthreads();
-    jacc += objective(S, x1, nullptr, nullptr, cent, false, red);
-  }
-  return block_sum(jacc, red);
+/* The values of one component of a unit's constraints in every lane of its
+ * warp: lane 3 a + q holds component q of the unit's atom a */
+__device__ __forceinline__ double comp(double v, int a, int q) { return __shfl_sync(0xffffffffu, v, 3 * a + q); }
+
+/* A d = b for up to three unknowns (identity rows past n), Cramer's rule */
+__device__ __forceinline__ void solve3(const double (*A)[3], const double* b, double* d) {
+  const double c00 = A[1][1] * A[2][2] - A[1][2] * A[2][1];
+  const double c01 = A[1][0] * A[2][2] - A[1][2] * A[2][0];
+  const double c02 = A[1][0] * A[2][1] - A[1][1] * A[2][0];
+  const double inv = 1.0 / (A[0][0] * c00 - A[0][1] * c01 + A[0][2] * c02);
+  const double e12 = b[1] * A[2][2] - A[1][2] * b[2], e11 = b[1] * A[2][1] - A[1][1] * b[2],
+               e10 = A[1][0] * b[2] - b[1] * A[2][0];
+  d[0] = (b[0] * c00 - A[0][1] * e12 + A[0][2] * e11) * inv;
+  d[1] = (A[0][0] * e12 - b[0] * c01 + A[0][2] * e10) * inv;
+  d[2] = (-A[0][0] * e11 - A[0][1] * e10 + b[0] * c02) * inv;
 }
 
-/* Every segment's recompute at once, one CTA each: CTA s starts from
- * checkpoint s (cpx, cpv) and writes its segment's trajectory at
- * B.X/V/F/gam + s * stride; its scratch (weights, SHAKE flags) at its own
- * offsets; Jseg[s] = the segment's objective sum, flags[2 s + 1] its
- * SHAKE status. */
+/* d s_k / d l_l = coef(k, l) r_l for constraints k, l of a unit */
+__device__ __forceinline__ double cons_coef(const Sys& S, const Unit& U, int k, int l) {
+  const double mi = 1.0 / S.mass[U.atom[U.ci[l]]], mj = 1.0 / S.mass[U.atom[U.cj[l]]];
+  double c = 0;
+  if (U.ci[l] == U.ci[k]) c += mi;
+  if (U.cj[l] == U.ci[k]) c -= mj;
+  if (U.ci[l] == U.cj[k]) c -= mi;
+  if (U.cj[l] == U.cj[k]) c += mj;
+  return c;
+}
+
+/* Newton's method on a unit's constraints: y (this lane's component) moves
+ * along the reference bond vectors of xr; gam: the multipliers.  One step
+ * past the sweeps' criterion, (|s|^2 - d^2)^2 <= 1e-20 A^4, which brings the
+ * residuals to rounding; false after 50 steps. */
+__device__ bool unit_shake(const Sys& S, const Unit& U, double& y, double xr, double* gam) {
+  const int lane = threadIdx.x & 31, a = lane / 3, q = lane - 3 * a;
+  double r[3][3], cf[3][3], d2[3];
+  for (int k = 0; k < 3; k++) {
+    gam[k] = 0;
+    if (k >= U.nc) continue;
+    const double dk = S.bond_c[2 * S.cons[3 * U.cons[k] + 2] + 1];
+    d2[k] = dk * dk;
+    for (int c = 0; c < 3; c++) r[k][c] = comp(xr, U.ci[k], c) - comp(xr, U.cj[k], c);
+    for (int l = 0; l < U.nc; l++) cf[k][l] = cons_coef(S, U, k, l);
+  }
+  bool done = false;
+  for (int it = 0; it < 50; it++) {
+    double A[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, b[3] = {0, 0, 0}, d[3];
+    bool ok = true;
+    for (int k = 0; k < 3; k++) {
+      if (k >= U.nc) continue;
+      double sk[3];
+      for (int c = 0; c < 3; c++) sk[c] = comp(y, U.ci[k], c) - comp(y, U.cj[k], c);
+      b[k] = d2[k] - (sk[0] * sk[0] + sk[1] * sk[1] + sk[2] * sk[2]);
+      if (!(b[k] * b[k] <= 1e-20)) ok = false;
+      for (int l = 0; l < 3; l++)
+        if (l < U.nc) A[k][l] = 2.0 * (sk[0] * r[l][0] + sk[1] * r[l][1] + sk[2] * r[l][2]) * cf[k][l];
+    }
+    if (ok && done) return true;
+    done = ok;
+    solve3(A, b, d);
+    for (int k = 0; k < 3; k++) {
+      if (k >= U.nc) continue;
+      gam[k] += d[k];
+      const double rq = q == 0 ? r[k][0] : q == 1 ? r[k][1] : r[k][2];
+      if (a == U.ci[k]) y += d[k] * rq / S.mass[U.atom[a]];
+      if (a == U.cj[k]) y -= d[k] * rq / S.mass[U.atom[a]];
+    }
+  }
+  return false;
+}
+
+/* Adjoint of a unit's converged projection x = y + sum_k g_k D_k r_k: lam
+ * (this lane's component of the adjoint of x) becomes that of y; returns what
+ * goes into the adjoint of the reference positions xr */
+__device__ double unit_shake_adjoint(const Sys& S, const Unit& U, double x, double xr, const double* gam, double& lam) {
+  const int lane = threadIdx.x & 31, a = lane / 3, q = lane - 3 * a;
+  double sk[3][3], A[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, rho[3] = {0, 0, 0}, mu[3];
+  const double lm = lam / (a < U.na ? S.mass[U.atom[a]] : 1.0);
+  for (int k = 0; k < 3; k++) {
+    if (k >= U.nc) continue;
+    for (int c = 0; c < 3; c++) sk[k][c] = comp(x, U.ci[k], c) - comp(x, U.cj[k], c);
+  }
+  for (int l = 0; l < 3; l++) {
+    if (l >= U.nc) continue;
+    double r[3];
+    for (int c = 0; c < 3; c++) {
+      r[c] = comp(xr, U.ci[l], c) - comp(xr, U.cj[l], c);
+      rho[l] += r[c] * (comp(lm, U.ci[l], c) - comp(lm, U.cj[l], c));
+    }
+    for (int k = 0; k < 3; k++)
+      if (k < U.nc) A[l][k] = (sk[k][0] * r[0] + sk[k][1] * r[1] + sk[k][2] * r[2]) * cons_coef(S, U, k, l);
+  }
+  solve3(A, rho, mu);
+  for (int k = 0; k < 3; k++) {
+    if (k >= U.nc) continue;
+    const double s = q == 0 ? sk[k][0] : q == 1 ? sk[k][1] : sk[k][2];
+    if (a == U.ci[k]) lam -= mu[k] * s;
+    if (a == U.cj[k]) lam += mu[k] * s;
+  }
+  const double ly = lam / (a < U.na ? S.mass[U.atom[a]] : 1.0);
+  double xb = 0;
+  for (int l = 0; l < 3; l++) {
+    if (l >= U.nc) continue;
+    double t = 0;
+    for (int c = 0; c < 3; c++) {
+      const double d = comp(ly, U.ci[l], c) - comp(ly, U.cj[l], c);
+      if (c == q) t = gam[l] * d;
+    }
+    if (a == U.ci[l]) xb += t;
+    if (a == U.cj[l]) xb -= t;
+  }
+  return xb;
+}
+
+/* Every segment's recompute at once, one cluster each: cluster s starts from
+ * checkpoint s (cpx, cpv) and writes its segment's positions, multipliers,
+ * weights and count-term derivatives.  first: the window's first segment
+ * takes the start forces that the state holds (f0; zero on a replica that was
+ * never stepped, since the reference evaluates no force before the first
+ * kick), the others evaluate F(x_0).  A step is: kick, kick, drift and
+ * constraints by units | everything that depends on the new positions.
+ * Jseg[CTA] = its share of the segment's objective sum, flags[2 s + 1] the
+ * SHAKE status.  sw_smem = 0: the weights do not fit shared memory (one CTA
+ * per segment then). */
 __global__ void __launch_bounds__(ADJ_THREADS, 1) adjoint_recompute(Sys S, Buf B, int K, long long n_steps,
                                                                     const double* cpx, const double* cpv,
-                                                                    const double* f0, double* Jseg) {
-  __shared__ double red[40];
+                                                                    const double* f0, double* Jseg, int sw_smem) {
+  __shared__ double red[72];
   __shared__ double cent[3];
-  const int s = blockIdx.x;
-  const int n3 = 3 * S.N;
+  __shared__ int next;
+  extern __shared__ double csh[];
+  const int s = (int)(blockIdx.x / cg::this_cluster().num_blocks());
+  const int n3 = 3 * S.N, lane = threadIdx.x & 31;
   const int Ks = (int)min((long long)K, n_steps - (long long)s * K);
   Buf b = B;
-  const size_t xs = (size_t)(K + 1) * n3;
-  b.X += s * xs;
-  b.V += s * xs;
-  b.F += s * xs;
+  b.X += (size_t)s * (K + 1) * n3;
+  b.V += (size_t)s * n3;
+  b.F += (size_t)s * n3;
   b.gam += (size_t)s * K * max(S.n_cons, 1);
-  b.w += (size_t)s * S.N;
-  b.dw += (size_t)s * n3;
+  b.w += (size_t)s * (K + 1) * S.N;
+  b.dw += (size_t)s * (K + 1) * n3;
+  b.mg += (size_t)s * (K + 1) * 3 * (S.n_vmol + 1);
+  b.tb += (size_t)s * 12 * max(1, S.n_bonds + S.n_angles + S.n_dih);
   b.flag += 2 * s;
-  for (int q = threadIdx.x; q < n3; q += blockDim.x) {
+  for (int q = ctid(); q < n3; q += cnthr()) {
     b.X[q] = cpx[(size_t)s * n3 + q];
     b.V[q] = cpv[(size_t)s * n3 + q];
+    if (s == 0) b.F[q] = f0[q];
   }
-  if (threadIdx.x == 0) b.flag[1] = 0;
-  __syncthreads();
-  const double j = recompute(S, b, Ks, s == 0 ? 1 : 0, f0, red, cent);
-  if (threadIdx.x == 0) Jseg[s] = j;
+  if (ctid() == 0) b.flag[1] = 0;
+  double jacc = 0;
+  for (int t = 0; t <= Ks; t++) {
+    double* const x1 = b.X + (size_t)t * n3;
+    if (t > 0) {
+      const double* const x0 = x1 - n3;
+      double* const gam = b.gam + (size_t)(t - 1) * S.n_cons;
+      const bool bonded = t > 1 || s > 0; /* F holds the pair forces alone */
+      for (int u = cwarp(); u < S.n_units; u += cnwarps()) {
+        const Unit& U = S.units[u];
+        const bool on = lane < 3 * U.na;
+        const int i = U.atom[on ? lane / 3 : 0], q = 3 * i + lane % 3;
+        double xo = 0, va = 0, y = 0, g[3];
+        if (on) {
+          const double c = S.c[i], f = __ldcg(b.F + q) + (bonded ? bonded_sum(S, b, i, lane % 3) : 0.0);
+          va = __ldcg(b.V + q);
+          if (t > 1) va += c * f;
+          va += c * f;
+          xo = __ldcg(x0 + q);
+          y = xo + S.dt * va;
+        }
+        const double yd = y;
+        if (U.nc > 0) {
+          if (!unit_shake(S, U, y, xo, g) && lane == 0) b.flag[1] = MDN_ST_SHAKE_NOCONV;
+          if (S.vcorr) va += (y - yd) / S.dt;
+          if (lane < U.nc) gam[U.cons[lane]] = lane == 0 ? g[0] : lane == 1 ? g[1] : g[2];
+        }
+        if (on) {
+          x1[q] = y;
+          b.V[q] = va;
+        }
+      }
+      if (S.n_units == 0) { /* one CTA */
+        for (int q = threadIdx.x; q < n3; q += blockDim.x) {
+          const int i = q / 3;
+          const double f = b.F[q] + (bonded ? bonded_sum(S, b, i, q - 3 * i) : 0.0);
+          double va = b.V[q];
+          if (t > 1) va += S.c[i] * f;
+          va += S.c[i] * f;
+          b.V[q] = va;
+          x1[q] = x0[q] + S.dt * va;
+        }
+        __syncthreads();
+        shake(S, b, x1, x0, gam);
+        if (S.vcorr)
+          for (int q = threadIdx.x; q < n3; q += blockDim.x) {
+            double y = x0[q] + S.dt * b.V[q];
+            b.V[q] += (x1[q] - y) / S.dt;
+          }
+      }
+    }
+    if (threadIdx.x == 0) next = 0;
+    csync();
+    double* const sw = sw_smem ? csh : b.w + (size_t)t * S.N;
+    const double jc = place_terms(S, b, x1, t, cent, sw, red);
+    double je = 0;
+    if (t > 0 || s > 0) je = force_rows(S, b, x1, sw, b.F, &next);
+    if (t > 0) jacc += jc + je;
+    csync();
+  }
+  jacc = block_sum(jacc, red);
+  if (threadIdx.x == 0) Jseg[blockIdx.x] = jacc;
 }
 
 /* The reverse sweep of one segment over its recomputed trajectory (B
- * pointing at it), last step first; the adjoints of x, v, F carry over from
- * the segment after it.  f0_theta = 1 on the first segment when its start
- * forces came from a force evaluation at x_0, whose parameter dependence
- * then enters the gradient. */
-__global__ void __launch_bounds__(ADJ_THREADS, 1) adjoint_segment(Sys S, Buf B, int K, int first,
-                                                                  int f0_theta) {
+ * pointing at it), last step first, on one cluster; the adjoints of x, v, F
+ * carry over from the segment after it.  A step is: the force product by
+ * atoms | by units, what remains of the product (bonded rows, the weights'
+ * pull on the ion centre), the adjoints of the constraints, the drift and
+ * the first kick, and of the second kick of the step before it.  f0_theta = 1
+ * on the first segment when its start forces came from a force evaluation at
+ * x_0, whose parameter dependence then enters the gradient.  STAGED: x and
+ * the force adjoint fit shared memory. */
+template <bool STAGED>
+__global__ void __launch_bounds__(ADJ_THREADS, 1) adjoint_segment(Sys S, Buf B, int K, int first, int f0_theta) {
   __shared__ double sgrad[MAX_PARAMS];
-  __shared__ double red[72];
-  __shared__ double cent[3];
-  extern __shared__ double csh[]; /* 2 n_cons + n_cons_nb doubles for the SHAKE adjoint */
-  const int n3 = 3 * S.N;
+  __shared__ double spart[3 * (ADJ_THREADS / 32)];
+  __shared__ double red[40];
+  __shared__ int next;
+  extern __shared__ double csh[]; /* x and lam when staged, then 2 n_cons + n_cons_nb doubles for shake_adjoint */
+  const int n3 = 3 * S.N, lane = threadIdx.x & 31;
+  double* const xs = csh;
+  double* const ls = csh + n3;
+  const bool vc = S.n_cons > 0 && S.vcorr;
+  double qsum = 0;
   for (int p = threadIdx.x; p < S.n_params; p += blockDim.x) sgrad[p] = 0;
-  for (int i = ctid(); i < S.N; i += cnthr()) B.om[i] = 0;
-  __syncthreads();
-  for (int t = K; t >= 1; t--) {
-    const double* x0 = B.X + (size_t)(t - 1) * n3;
+  /* (6) of the segment's last step: F-bar += c V-bar */
+  for (int q = ctid(); q < n3; q += cnthr()) B.lf[q] = __ldcg(B.lf + q) + S.c[q / 3] * __ldcg(B.lv + q);
+  csync();
+  for (int t = K; t >= 0; t--) {
+    if (t == 0 && !(first && f0_theta)) break;
     const double* x1 = B.X + (size_t)t * n3;
-    /* every CTA its own copy of the centre */
-    ion_centre(S, x1, cent, red);
-    weights(S, B, x1, cent);
-    /* objective at x_t */
-    objective(S, x1, B.lx, sgrad, cent, true, red);
-    /* (6): F-bar += c V-bar (each thread its own elements throughout) */
-    for (int q = ctid(); q < n3; q += cnthr()) B.lf[q] += S.c[q / 3] * B.lv[q];
+    /* objective at x_t and (5): x-bar += J^T F-bar; at t = 0 only for the
+     * parameters of F(x_0) */
+    if (threadIdx.x == 0) next = 0;
+    if (STAGED)
+      for (int q = threadIdx.x; q < n3; q += blockDim.x) {
+        xs[q] = x1[q];
+        ls[q] = __ldcg(B.lf + q);
+      }
+    __syncthreads();
+    vjp_rows<STAGED>(S, B, x1, t, STAGED ? xs : x1, STAGED ? ls : B.lf, t > 0, sgrad, spart, qsum, &next);
     csync();
-    /* (5): x-bar += J^T F-bar */
-    force_vjp(S, B, x1, B.lf, B.lx, sgrad, cent, red);
-    /* (4): v_b = v_a + (x_t - y)/dt */
-    const bool vc = S.n_cons > 0 && S.vcorr;
-    for (int q = ctid(); q < n3; q += cnthr()) {
-      if (vc) B.lx[q] = __ldcg(B.lx + q) + B.lv[q] / S.dt;
-      B.xb[q] = 0;
+    if (t == 0) break;
+    const double* x0 = x1 - n3;
+    const double* const gam = B.gam + (size_t)(t - 1) * S.n_cons;
+    const double* const mg = B.mg + (size_t)t * 3 * (S.n_vmol + 1) + 3 * S.n_vmol;
+    double pull[3] = {0, 0, 0};
+    for (int k = 0; k < 3; k++) {
+      for (unsigned r = 0; r < cg::this_cluster().num_blocks(); r++) pull[k] -= __ldcg(B.part + 3 * r + k);
+      pull[k] += mg[k];
     }
-    csync();
-    /* (3): SHAKE adjoint: lx becomes the adjoint of y; xb gets the r-terms */
-    if (S.n_cons > 0) shake_adjoint(S, B, x1, x0, B.gam + (size_t)(t - 1) * S.n_cons, B.lx, B.xb, csh);
-    /* (2) y = x + dt v_a; (1) v_a = v + c F */
-    for (int q = ctid(); q < n3; q += cnthr()) {
-      double ly = __ldcg(B.lx + q);
-      if (vc) ly -= B.lv[q] / S.dt;
-      const double lva = B.lv[q] + S.dt * ly;
-      B.lx[q] = ly + __ldcg(B.xb + q);
+    /* what the force product leaves to the owner of component q of atom i */
+    auto rest = [&](int i, int k) {
+      double v = bonded_sum(S, B, i, k);
+      if (i < S.n_ion) v += S.mass[i] / S.ion_msum * (k == 0 ? pull[0] : k == 1 ? pull[1] : pull[2]);
+      return v;
+    };
+    /* (2) y = x + dt v_a; (1) v_a = v + c F; (6) of the step before */
+    auto carry = [&](int q, double ly, double xb, double lv) {
+      const double lva = lv + S.dt * ly, cl = S.c[q / 3] * lva;
+      B.lx[q] = ly + xb;
       B.lv[q] = lva;
-      B.lf[q] = S.c[q / 3] * lva;
+      B.lf[q] = t > 1 ? cl + cl : cl;
+    };
+    for (int u = cwarp(); u < S.n_units; u += cnwarps()) {
+      const Unit& U = S.units[u];
+      const bool on = lane < 3 * U.na;
+      const int k = lane % 3, i = U.atom[on ? lane / 3 : 0], q = 3 * i + k;
+      double lam = 0, lv = 0, xb = 0, g[3] = {0, 0, 0};
+      if (on) {
+        lv = __ldcg(B.lv + q);
+        /* (4): v_b = v_a + (x_t - y)/dt */
+        lam = __ldcg(B.lx + q) + rest(i, k) + (vc ? lv / S.dt : 0.0);
+      }
+      if (U.nc > 0) {
+        for (int c = 0; c < U.nc; c++) g[c] = gam[U.cons[c]];
+        xb = unit_shake_adjoint(S, U, on ? x1[q] : 0.0, on ? x0[q] : 0.0, g, lam);
+      }
+      if (on) carry(q, vc ? lam - lv / S.dt : lam, xb, lv);
     }
-    /* the weight adjoints of the next force product start at zero */
-    for (int i = ctid(); i < S.N; i += cnthr()) B.om[i] = 0;
+    if (S.n_units == 0) {
+      for (int q = ctid(); q < n3; q += cnthr()) {
+        B.lx[q] = __ldcg(B.lx + q) + rest(q / 3, q % 3) + (vc ? B.lv[q] / S.dt : 0.0);
+        B.xb[q] = 0;
+      }
+      csync();
+      shake_adjoint(S, B, x1, x0, gam, B.lx, B.xb, STAGED ? csh + 2 * n3 : csh);
+      for (int q = ctid(); q < n3; q += cnthr()) {
+        const double lv = B.lv[q], ly = __ldcg(B.lx + q);
+        carry(q, vc ? ly - lv / S.dt : ly, __ldcg(B.xb + q), lv);
+      }
+    }
     csync();
   }
-  if (first && f0_theta) {
-    /* F(x_0): its parameter dependence */
-    ion_centre(S, B.X, cent, red);
-    weights(S, B, B.X, cent);
-    force_vjp(S, B, B.X, B.lf, B.tmp, sgrad, cent, red);
-  }
+  qsum = block_sum(qsum, red);
+  if (threadIdx.x == 0) sgrad[S.n_params - 1] += qsum;
   __syncthreads();
   /* the CTAs' shares of the gradient */
   for (int p = threadIdx.x; p < S.n_params; p += blockDim.x)
@@ -1276,9 +1439,100 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
     pk.swap(pk2);
   }
   S.n_pairs = (int)pi.size();
-  S.pi = dput(pi, owned);
-  S.pj = dput(pj, owned);
-  S.pk = dput(pk, owned);
+  /* the pairs by atom, from both sides, in the sorted order (so that a
+   * warp's lanes stay on few parameter rows).  One side is primary, the ion
+   * atom's where there is one, the lower index in an ion-ion pair. */
+  {
+    std::vector<int> off(N + 1, 0), at, order(N);
+    for (size_t k = 0; k < pi.size(); k++) {
+      off[pi[k] + 1]++;
+      off[pj[k] + 1]++;
+    }
+    for (int i = 0; i < N; i++) off[i + 1] += off[i];
+    at.assign(off.begin(), off.end() - 1);
+    std::vector<int2> row(2 * pi.size());
+    for (size_t k = 0; k < pi.size(); k++) {
+      const int a = pi[k], b = pj[k];
+      row[at[a]++] = make_int2(b, pk[k] | (a < b ? kPrimary : 0));
+      row[at[b]++] = make_int2(a, pk[k] | (b < a ? kPrimary : 0));
+    }
+    for (int i = 0; i < N; i++) order[i] = i;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int a, int b) { return off[a + 1] - off[a] > off[b + 1] - off[b]; });
+    S.row_off = dput(off, owned);
+    S.row = dput(row, owned);
+    S.row_order = dput(order, owned);
+  }
+  /* the bonded terms' rows (4 per term: bonds, angles, dihedrals) by atom */
+  {
+    std::vector<std::vector<int>> by(N);
+    int t = 0;
+    auto add = [&](const std::vector<int>& v, int w) {
+      for (size_t r = 0; r < v.size(); r += w, t++)
+        for (int k = 0; k < w - 1; k++) by[v[r + k]].push_back(4 * t + k);
+    };
+    add(bonds, 3);
+    add(angles, 4);
+    add(dih, 5);
+    std::vector<int> off(N + 1, 0), at;
+    for (int i = 0; i < N; i++) {
+      at.insert(at.end(), by[i].begin(), by[i].end());
+      off[i + 1] = (int)at.size();
+    }
+    S.tb_off = dput(off, owned);
+    S.tb_at = dput(at, owned);
+  }
+  /* the units */
+  {
+    std::vector<Unit> units;
+    std::vector<char> seen_c(ncons, 0), seen_a(N, 0);
+    bool big = false;
+    for (int k = 0; k < ncons && !big; k++) {
+      if (seen_c[k]) continue;
+      std::vector<int> cs(1, k);
+      seen_c[k] = 1;
+      for (size_t q = 0; q < cs.size(); q++)
+        for (int e = nboff[cs[q]]; e < nboff[cs[q] + 1]; e++)
+          if (!seen_c[nb[e]]) {
+            seen_c[nb[e]] = 1;
+            cs.push_back(nb[e]);
+          }
+      if (cs.size() > 3) {
+        big = true;
+        break;
+      }
+      Unit U;
+      memset(&U, 0, sizeof U);
+      auto place = [&](int atom) {
+        for (int a = 0; a < U.na; a++)
+          if (U.atom[a] == atom) return a;
+        U.atom[U.na] = atom;
+        seen_a[atom] = 1;
+        return U.na++;
+      };
+      for (int c : cs) {
+        U.cons[U.nc] = c;
+        U.ci[U.nc] = place(cons[3 * c]);
+        U.cj[U.nc] = place(cons[3 * c + 1]);
+        U.nc++;
+      }
+      units.push_back(U);
+    }
+    Unit U;
+    memset(&U, 0, sizeof U);
+    for (int i = 0; i < N && !big; i++) {
+      if (seen_a[i]) continue;
+      U.atom[U.na++] = i;
+      if (U.na == 8) {
+        units.push_back(U);
+        U.na = 0;
+      }
+    }
+    if (U.na > 0) units.push_back(U);
+    if (big) units.clear();
+    S.n_units = (int)units.size();
+    S.units = dput(units, owned);
+  }
   S.A = dput(A, owned);
   S.B = dput(Bt, owned);
   S.eps = dput(E, owned);
@@ -1330,23 +1584,24 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
   Buf Bf;
   memset(&Bf, 0, sizeof Bf);
   /* every segment's recomputed trajectory (the recomputes run at once) */
+  const size_t n_terms = std::max(1, S.n_bonds + S.n_angles + S.n_dih);
   Bf.X = dzero<double>((size_t)nseg * (K + 1) * n3, owned);
-  Bf.V = dzero<double>((size_t)nseg * (K + 1) * n3, owned);
-  Bf.F = dzero<double>((size_t)nseg * (K + 1) * n3, owned);
+  Bf.V = dzero<double>((size_t)nseg * n3, owned);
+  Bf.F = dzero<double>((size_t)nseg * n3, owned);
   Bf.gam = dzero<double>((size_t)nseg * K * std::max(ncons, 1), owned);
   Bf.lx = dzero<double>(n3, owned);
   Bf.lv = dzero<double>(n3, owned);
   Bf.lf = dzero<double>(n3, owned);
-  Bf.tmp = dzero<double>(n3, owned);
   Bf.xb = dzero<double>(n3, owned);
-  Bf.w = dzero<double>((size_t)nseg * N, owned);
-  Bf.dw = dzero<double>((size_t)nseg * n3, owned);
-  Bf.om = dzero<double>(N, owned);
+  Bf.w = dzero<double>((size_t)nseg * (K + 1) * N, owned);
+  Bf.dw = dzero<double>((size_t)nseg * (K + 1) * n3, owned);
+  Bf.mg = dzero<double>((size_t)nseg * (K + 1) * 3 * (nvin + 1), owned);
+  Bf.tb = dzero<double>((size_t)nseg * 12 * n_terms, owned);
+  Bf.part = dzero<double>(3 * ADJ_CLUSTER, owned);
   Bf.mu = dzero<double>(std::max(ncons, 1), owned);
   Bf.grad = dzero<double>(n_params, owned);
-  Bf.J = dzero<double>(1, owned);
   Bf.flag = dzero<int>(2 * (size_t)nseg, owned);
-  double* d_jseg = dzero<double>(nseg, owned);
+  double* d_jseg = dzero<double>((size_t)nseg * ADJ_CLUSTER, owned);
   /* the forces the state holds at the window start */
   std::vector<double> f0(3 * (size_t)N, 0.0);
   for (int i = 0; i < ni; i++)
@@ -1411,52 +1666,74 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
     cleanup();
     return err(MDN_ERR_CAPACITY, "mdn_adjoint: %d constraints in the domain, too many for the reverse sweep", ncons);
   }
-  if (cbytes > 48 * 1024 &&
-      cudaFuncSetAttribute(adjoint_segment, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cbytes) != cudaSuccess) {
+  /* x and the force adjoint of the reverse sweep in shared memory where they
+   * fit beside the constraints' scratch; likewise the recompute's weights */
+  const size_t fall = S.n_units == 0 ? cbytes : 0;
+  const bool staged = 2 * n3 * sizeof(double) + fall <= 200 * 1024;
+  const size_t seg_bytes = (staged ? 2 * n3 * sizeof(double) : 0) + fall;
+  const bool sw_smem = N * sizeof(double) <= 200 * 1024;
+  const size_t rec_bytes = sw_smem ? N * sizeof(double) : 0;
+  auto* const segment = staged ? adjoint_segment<true> : adjoint_segment<false>;
+  if (cudaFuncSetAttribute(segment, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+      cudaFuncSetAttribute(adjoint_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
+          cudaSuccess) {
     cleanup();
-    return err(MDN_ERR_CUDA, "mdn_adjoint: reverse sweep shared memory");
+    return err(MDN_ERR_CUDA, "mdn_adjoint: shared memory");
   }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(ADJ_THREADS);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, stream);
-  adjoint_recompute<<<(unsigned)nseg, ADJ_THREADS, 0, stream>>>(S, Bf, K, spec->n_steps, cpx, cpv, d_f0, d_jseg);
-  for (long long s = nseg - 1; s >= 0; s--) {
+  /* the recompute on clusters as large as let every segment run at once; one
+   * CTA each where the constraints go through block barriers or the weights
+   * through global memory.  Fewer CTAs if the GPU cannot place that many. */
+  int sms = 1, Cr = ADJ_CLUSTER;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sa.dev);
+  while (Cr > 1 && (nseg * Cr > sms || S.n_units == 0 || !sw_smem)) Cr /= 2;
+  cudaError_t le = cudaErrorUnknown;
+  for (; Cr >= 1; Cr /= 2) {
+    cfg.gridDim = dim3((unsigned)(nseg * Cr));
+    cfg.dynamicSmemBytes = rec_bytes;
+    attr[0].val.clusterDim.x = Cr;
+    le = cudaLaunchKernelEx(&cfg, adjoint_recompute, S, Bf, K, (long long)spec->n_steps, (const double*)cpx,
+                            (const double*)cpv, (const double*)d_f0, d_jseg, sw_smem ? 1 : 0);
+    if (le == cudaSuccess || Cr == 1) break;
+    cudaGetLastError();
+  }
+  for (long long s = nseg - 1; s >= 0 && le == cudaSuccess; s--) {
     const int n = (int)std::min<long long>(K, spec->n_steps - s * K);
     Buf b = Bf;
     b.X += s * (K + 1) * n3;
-    b.V += s * (K + 1) * n3;
-    b.F += s * (K + 1) * n3;
     b.gam += (size_t)s * K * std::max(ncons, 1);
+    b.w += (size_t)s * (K + 1) * N;
+    b.dw += (size_t)s * (K + 1) * n3;
+    b.mg += (size_t)s * (K + 1) * 3 * (nvin + 1);
     /* one cluster of ADJ_CLUSTER CTAs per segment (fewer if the GPU cannot
      * place that many) */
-    cudaError_t le = cudaErrorUnknown;
-    if (ADJ_CLUSTER > 8) {
-      cudaFuncSetAttribute(adjoint_segment, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      cudaGetLastError();
-    }
     for (int C = ADJ_CLUSTER; C >= 1; C /= 2) {
-      cudaLaunchConfig_t cfg;
-      memset(&cfg, 0, sizeof cfg);
       cfg.gridDim = dim3(C);
-      cfg.blockDim = dim3(ADJ_THREADS);
-      cfg.dynamicSmemBytes = cbytes;
-      cfg.stream = stream;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
+      cfg.dynamicSmemBytes = seg_bytes;
       attr[0].val.clusterDim.x = C;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      le = cudaLaunchKernelEx(&cfg, adjoint_segment, S, b, n, s == 0 ? 1 : 0, f0_theta);
+      le = cudaLaunchKernelEx(&cfg, segment, S, b, n, s == 0 ? 1 : 0, f0_theta);
       if (le == cudaSuccess) break;
       cudaGetLastError();
     }
-    if (le != cudaSuccess) {
-      cleanup();
-      return err(MDN_ERR_CUDA, "mdn_adjoint: reverse sweep launch: %s", cudaGetErrorString(le));
-    }
+  }
+  if (le != cudaSuccess) {
+    cudaStreamSynchronize(stream);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    cleanup();
+    return err(MDN_ERR_CUDA, "mdn_adjoint: launch: %s", cudaGetErrorString(le));
   }
   cudaEventRecord(e1, stream);
   cudaError_t ce = cudaStreamSynchronize(stream);
@@ -1474,10 +1751,10 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
   for (long long s = 0; s < nseg; s++) flags[1] |= fl[2 * s + 1];
   /* J: the segments' objective sums, last first (the order the sequential
    * form added them in) */
-  std::vector<double> js((size_t)nseg, 0.0);
-  cudaMemcpy(js.data(), d_jseg, sizeof(double) * nseg, cudaMemcpyDeviceToHost);
+  std::vector<double> js((size_t)nseg * Cr, 0.0);
+  cudaMemcpy(js.data(), d_jseg, sizeof(double) * js.size(), cudaMemcpyDeviceToHost);
   double jsum = 0.0;
-  for (long long s = nseg - 1; s >= 0; s--) jsum += js[s] * S.inv_n;
+  for (long long s = (long long)js.size() - 1; s >= 0; s--) jsum += js[s] * S.inv_n;
   *J = jsum;
   cudaMemcpy(grad, Bf.grad, sizeof(double) * n_params, cudaMemcpyDeviceToHost);
   if (ms) {
