@@ -28,9 +28,10 @@
  * and sums over its row of partners (each pair evaluated from both sides), a
  * bonded term's forces go to rows of their own that the atoms' owners read,
  * and a warp takes a constraint group with everything that happens to its
- * atoms between two force products.  A step has two cluster barriers.  (With
- * FP64 atomics per pair, 150 thousand on 1,476 addresses, a reverse step of
- * 492 atoms took 164 us, of which the atomics 130; a recomputed one 127 us.)
+ * atoms between two force products.  A step has two cluster barriers.  492
+ * atoms, 25 thousand pairs: a reverse step takes 26 us, a recomputed one 21,
+ * most of it the latency of FP64 chains.  (With FP64 atomics per pair, 150
+ * thousand on 1,476 addresses, 164 us, of which the atomics 130, and 127.)
  * Parameter derivatives are summed per warp and row of parameters, then in
  * shared memory; the sums agree between runs up to FP64 rounding order.
  */
@@ -61,7 +62,7 @@ __attribute__((visibility("hidden"))) void mdn_snapshot_args(const mdn_handle* h
 namespace {
 
 constexpr int ADJ_THREADS = 512;
-constexpr int ADJ_CLUSTER = 8; /* CTAs of a reverse sweep (16 measured no faster) */
+constexpr int ADJ_CLUSTER = 16; /* CTAs of a reverse sweep: 21.6 ms for the 400 steps above, 8 took 27.7 */
 constexpr int MAX_PARAMS = 512;
 constexpr int SHAKE_SWEEPS = 1000;
 
@@ -209,6 +210,8 @@ struct Unit {
   int atom[8];
   int cons[3];
   int ci[3], cj[3]; /* the constraints' atoms as places in atom[] */
+  double d2[3];     /* squared lengths */
+  double cf[3][3];  /* d s_k / d l_l = cf[k][l] r_l (s_k the bond vector, l_l the multiplier) */
 };
 constexpr int kPrimary = 8; /* this side of the pair counts its parameter derivatives */
 
@@ -222,8 +225,8 @@ struct Sys {
   int n_pairs;
   const double* A;       /* [nt*nt] */
   const double* B;
-  const double* eps;     /* [nt*nt] pair eps / sigma (for the derivatives) */
-  const double* sig;
+  const double* ieps;    /* [nt*nt] 1 / pair eps, 1 / pair sigma (for the derivatives) */
+  const double* isig;
   const int* pidx;       /* [nt*nt] parameter base index (eps; sigma = +1), -1 */
   const int* bmh;        /* [N] Born-Mayer-Huggins row of ion atoms */
   int n_bonds, n_angles, n_dih;
@@ -245,8 +248,8 @@ struct Sys {
   const int* row_off;
   const int2* row;
   const int* row_order;   /* [N] atoms, longest rows first */
-  /* bonded terms by atom: tb_at[tb_off[i] .. tb_off[i + 1]) are the rows of
-   * Buf::tb (4 per term) that act on atom i */
+  /* bonded terms by atom: rows tb_off[i] .. tb_off[i + 1] of Buf::tb act on
+   * atom i; tb_at[4 t + a] is the row of term t's a-th atom */
   const int* tb_off;
   const int* tb_at;
   /* what one warp carries from one force product to the next: a group of
@@ -276,8 +279,8 @@ struct Buf {
   double* w;     /* [(K+1)*N] taper weights of each step of the segment */
   double* dw;    /* [(K+1)*3N] their gradients */
   double* mg;    /* [(K+1)*3*(n_vmol+1)] count term: d/d(centre of vapor molecule m), then minus their sum */
-  double* tb;    /* [4*terms*3] bonded terms' forces (or products) */
-  double* part;  /* [8*3] the CTAs' shares of the weights' pull on the ion centre */
+  double* tb;    /* [rows*3] bonded terms' forces (or products) */
+  double* part;  /* [ADJ_CLUSTER*3] the CTAs' shares of the weights' pull on the ion centre */
   double* mu;    /* [n_cons] */
   double* grad;  /* [n_params] */
   int* flag;     /* [2] SHAKE convergence scratch, status */
@@ -340,7 +343,10 @@ __device__ void block_sum3(double* v, double* red) {
 }
 
 /* x, v, f, ... that other CTAs write are read from L2 */
-__device__ __forceinline__ int cwarp() { return ctid() >> 5; }
+/* this warp among the cluster's, the CTAs in turn */
+__device__ __forceinline__ int cwarp() {
+  return (int)((threadIdx.x >> 5) * cg::this_cluster().num_blocks() + cg::this_cluster().block_rank());
+}
 __device__ __forceinline__ int cnwarps() { return cnthr() >> 5; }
 
 /* ion centre of x (mass-weighted) into cent[0..2]; x was written by the whole
@@ -421,13 +427,14 @@ __device__ double place_terms(const Sys& S, const Buf& B, const double* x, int t
  * of f (d eps, d sigma, d s at s = 1) */
 struct PairEval {
   double f, fp, fe, fs_sig, fq;
+  double ui, a7, b4; /* 1 / u, the two LJ terms of f */
   int p;  /* parameter base, -1 */
 };
 
 __device__ __forceinline__ PairEval eval_pair(const Sys& S, int i, int j, int kind, double u) {
   PairEval o;
   o.p = -1;
-  o.fe = o.fs_sig = o.fq = 0;
+  o.fe = o.fs_sig = o.fq = o.a7 = o.b4 = 0;
   const int tt = S.type[i] * S.nt + S.type[j];
   const double ui = 1.0 / u;
   double f = 0, fp = 0;
@@ -448,11 +455,13 @@ __device__ __forceinline__ PairEval eval_pair(const Sys& S, int i, int j, int ki
     const double a7 = S.A[tt] * u7, b4 = S.B[tt] * u4;
     f = a7 - b4;
     fp = (4.0 * b4 - 7.0 * a7) * ui;
+    o.a7 = a7;
+    o.b4 = b4;
     if (kind == PK_GI || kind == PK_VI) {
       o.p = S.pidx[tt];
       if (o.p >= 0) {
-        o.fe = f / S.eps[tt];
-        o.fs_sig = (12.0 * a7 - 6.0 * b4) / S.sig[tt];
+        o.fe = f * S.ieps[tt];
+        o.fs_sig = (12.0 * a7 - 6.0 * b4) * S.isig[tt];
       }
     }
     if (kind == PK_VI || kind == PK_VV || kind == PK_ION_LJC) {
@@ -465,6 +474,7 @@ __device__ __forceinline__ PairEval eval_pair(const Sys& S, int i, int j, int ki
   }
   o.f = f;
   o.fp = fp;
+  o.ui = ui;
   return o;
 }
 
@@ -506,18 +516,21 @@ __device__ __forceinline__ void bonded_rows(const Sys& S, const Buf& B, const do
 #pragma unroll
   for (int a = 0; a < 4; a++) {
     if (a >= n) break;
+    double* const row = B.tb + 3 * (size_t)S.tb_at[4 * t + a];
 #pragma unroll
     for (int q = 0; q < 3; q++) {
-      if constexpr (dual) B.tb[12 * (size_t)t + 3 * a + q] = f[a][q].d;
-      else B.tb[12 * (size_t)t + 3 * a + q] = f[a][q];
+      if constexpr (dual) row[q] = f[a][q].d;
+      else row[q] = f[a][q];
     }
   }
 }
 
 /* the bonded terms' rows of component q of atom i, summed */
 __device__ __forceinline__ double bonded_sum(const Sys& S, const Buf& B, int i, int q) {
+  const int e1 = S.tb_off[i + 1];
   double t = 0;
-  for (int e = S.tb_off[i]; e < S.tb_off[i + 1]; e++) t += __ldcg(B.tb + 3 * (size_t)S.tb_at[e] + q);
+#pragma unroll 16
+  for (int e = S.tb_off[i]; e < e1; e++) t += __ldcg(B.tb + 3 * (size_t)e + q);
   return t;
 }
 
@@ -560,12 +573,9 @@ __device__ double force_rows(const Sys& S, const Buf& B, const double* x, const 
                   a[0] += g * d0;
                   a[1] += g * d1;
                   a[2] += g * d2;
-                  if (kind == PK_VI && (pr.y & kPrimary)) {
-                    const int tt = S.type[i] * S.nt + S.type[j];
-                    const double u3 = u * u * u;
-                    jp += S.w_energy * (S.A[tt] / 12.0 / (u3 * u3) - S.B[tt] / 6.0 / u3 +
-                                        S.qqrd2e * S.q[i] * S.q[j] / sqrt(u));
-                  }
+                  /* U = u (a7 / 12 - b4 / 6) + u fc, fq = fc */
+                  if (kind == PK_VI && (pr.y & kPrimary))
+                    jp += S.w_energy * u * (ev.a7 * (1.0 / 12.0) - ev.b4 * (1.0 / 6.0) + ev.fq);
                 }
                 for (int k = 0; k < 3; k++) a[k] = warp_sum_dd(a[k]);
                 if (lane < 3) {
@@ -639,16 +649,16 @@ __device__ void vjp_rows(const Sys& S, const Buf& B, const double* x, int t, con
               qsum += W * ev.fq * dm;
             }
             if (obj && kind == PK_VI && S.w_energy != 0) {
-              const int tt = S.type[i] * S.nt + S.type[j];
-              const double ui = 1.0 / u, u3 = ui * ui * ui, a6 = S.A[tt] * (u3 * u3), b3 = S.B[tt] * u3;
-              const double qr = S.qqrd2e * S.q[i] * S.q[j] * sqrt(ui), sc = S.w_energy * S.inv_n;
-              cd += sc * ui * (b3 - a6 - qr);
+              /* dU/du = -(a7 - b4 + fc) / 2 with fc = fq, U as in force_rows */
+              const double sc = S.w_energy * S.inv_n;
+              cd += sc * (ev.b4 - ev.a7 - ev.fq);
               if (primary) {
                 if (p >= 0) {
-                  pe += sc * (a6 / 12.0 - b3 / 6.0) / S.eps[tt];
-                  ps += sc * (a6 - b3) / S.sig[tt];
+                  const int tt = S.type[i] * S.nt + S.type[j];
+                  pe += sc * u * (ev.a7 * (1.0 / 12.0) - ev.b4 * (1.0 / 6.0)) * S.ieps[tt];
+                  ps += sc * u * (ev.a7 - ev.b4) * S.isig[tt];
                 }
-                qsum += sc * qr;
+                qsum += sc * u * ev.fq;
               }
             }
             for (int q = 0; q < 3; q++) a[q] += cm * m[q] + cd * d[q];
@@ -842,54 +852,63 @@ __device__ __forceinline__ void solve3(const double (*A)[3], const double* b, do
   d[2] = (-A[0][0] * e11 - A[0][1] * e10 + b[0] * c02) * inv;
 }
 
-/* d s_k / d l_l = coef(k, l) r_l for constraints k, l of a unit */
-__device__ __forceinline__ double cons_coef(const Sys& S, const Unit& U, int k, int l) {
-  const double mi = 1.0 / S.mass[U.atom[U.ci[l]]], mj = 1.0 / S.mass[U.atom[U.cj[l]]];
-  double c = 0;
-  if (U.ci[l] == U.ci[k]) c += mi;
-  if (U.cj[l] == U.ci[k]) c -= mj;
-  if (U.ci[l] == U.cj[k]) c -= mi;
-  if (U.cj[l] == U.cj[k]) c += mj;
-  return c;
-}
+/* a unit's constraints in registers */
+struct UnitCons {
+  int nc, ci[3], cj[3];
+  double cf[3][3];
+  __device__ __forceinline__ explicit UnitCons(const Unit& U) : nc(U.nc) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      ci[k] = U.ci[k];
+      cj[k] = U.cj[k];
+#pragma unroll
+      for (int l = 0; l < 3; l++) cf[k][l] = U.cf[k][l];
+    }
+  }
+};
+__device__ __forceinline__ double pick(const double* v, int q) { return q == 0 ? v[0] : q == 1 ? v[1] : v[2]; }
 
-/* Newton's method on a unit's constraints: y (this lane's component) moves
- * along the reference bond vectors of xr; gam: the multipliers.  One step
- * past the sweeps' criterion, (|s|^2 - d^2)^2 <= 1e-20 A^4, which brings the
- * residuals to rounding; false after 50 steps. */
-__device__ bool unit_shake(const Sys& S, const Unit& U, double& y, double xr, double* gam) {
+/* Newton's method on a unit's constraints: y (this lane's component, im its
+ * atom's inverse mass) moves along the reference bond vectors of xr; gam: the
+ * multipliers.  One step past the sweeps' criterion, (|s|^2 - d^2)^2 <= 1e-20
+ * A^4, which brings the residuals to rounding; false after 50 steps. */
+__device__ __forceinline__ bool unit_shake(const UnitCons& U, const double* d2, double im, double& y, double xr,
+                                           double* gam) {
   const int lane = threadIdx.x & 31, a = lane / 3, q = lane - 3 * a;
-  double r[3][3], cf[3][3], d2[3];
+  double r[3][3];
+#pragma unroll
   for (int k = 0; k < 3; k++) {
     gam[k] = 0;
     if (k >= U.nc) continue;
-    const double dk = S.bond_c[2 * S.cons[3 * U.cons[k] + 2] + 1];
-    d2[k] = dk * dk;
+#pragma unroll
     for (int c = 0; c < 3; c++) r[k][c] = comp(xr, U.ci[k], c) - comp(xr, U.cj[k], c);
-    for (int l = 0; l < U.nc; l++) cf[k][l] = cons_coef(S, U, k, l);
   }
   bool done = false;
   for (int it = 0; it < 50; it++) {
     double A[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, b[3] = {0, 0, 0}, d[3];
     bool ok = true;
+#pragma unroll
     for (int k = 0; k < 3; k++) {
       if (k >= U.nc) continue;
       double sk[3];
+#pragma unroll
       for (int c = 0; c < 3; c++) sk[c] = comp(y, U.ci[k], c) - comp(y, U.cj[k], c);
       b[k] = d2[k] - (sk[0] * sk[0] + sk[1] * sk[1] + sk[2] * sk[2]);
       if (!(b[k] * b[k] <= 1e-20)) ok = false;
+#pragma unroll
       for (int l = 0; l < 3; l++)
-        if (l < U.nc) A[k][l] = 2.0 * (sk[0] * r[l][0] + sk[1] * r[l][1] + sk[2] * r[l][2]) * cf[k][l];
+        if (l < U.nc) A[k][l] = 2.0 * (sk[0] * r[l][0] + sk[1] * r[l][1] + sk[2] * r[l][2]) * U.cf[k][l];
     }
     if (ok && done) return true;
     done = ok;
     solve3(A, b, d);
+#pragma unroll
     for (int k = 0; k < 3; k++) {
       if (k >= U.nc) continue;
       gam[k] += d[k];
-      const double rq = q == 0 ? r[k][0] : q == 1 ? r[k][1] : r[k][2];
-      if (a == U.ci[k]) y += d[k] * rq / S.mass[U.atom[a]];
-      if (a == U.cj[k]) y -= d[k] * rq / S.mass[U.atom[a]];
+      const double rq = d[k] * pick(r[k], q) * im;
+      if (a == U.ci[k]) y += rq;
+      if (a == U.cj[k]) y -= rq;
     }
   }
   return false;
@@ -898,40 +917,47 @@ __device__ bool unit_shake(const Sys& S, const Unit& U, double& y, double xr, do
 /* Adjoint of a unit's converged projection x = y + sum_k g_k D_k r_k: lam
  * (this lane's component of the adjoint of x) becomes that of y; returns what
  * goes into the adjoint of the reference positions xr */
-__device__ double unit_shake_adjoint(const Sys& S, const Unit& U, double x, double xr, const double* gam, double& lam) {
+__device__ __forceinline__ double unit_shake_adjoint(const UnitCons& U, double im, double x, double xr,
+                                                     const double* gam, double& lam) {
   const int lane = threadIdx.x & 31, a = lane / 3, q = lane - 3 * a;
   double sk[3][3], A[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, rho[3] = {0, 0, 0}, mu[3];
-  const double lm = lam / (a < U.na ? S.mass[U.atom[a]] : 1.0);
+  const double lm = lam * im;
+#pragma unroll
   for (int k = 0; k < 3; k++) {
     if (k >= U.nc) continue;
+#pragma unroll
     for (int c = 0; c < 3; c++) sk[k][c] = comp(x, U.ci[k], c) - comp(x, U.cj[k], c);
   }
+#pragma unroll
   for (int l = 0; l < 3; l++) {
     if (l >= U.nc) continue;
     double r[3];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
       r[c] = comp(xr, U.ci[l], c) - comp(xr, U.cj[l], c);
       rho[l] += r[c] * (comp(lm, U.ci[l], c) - comp(lm, U.cj[l], c));
     }
+#pragma unroll
     for (int k = 0; k < 3; k++)
-      if (k < U.nc) A[l][k] = (sk[k][0] * r[0] + sk[k][1] * r[1] + sk[k][2] * r[2]) * cons_coef(S, U, k, l);
+      if (k < U.nc) A[l][k] = (sk[k][0] * r[0] + sk[k][1] * r[1] + sk[k][2] * r[2]) * U.cf[k][l];
   }
   solve3(A, rho, mu);
+#pragma unroll
   for (int k = 0; k < 3; k++) {
     if (k >= U.nc) continue;
-    const double s = q == 0 ? sk[k][0] : q == 1 ? sk[k][1] : sk[k][2];
-    if (a == U.ci[k]) lam -= mu[k] * s;
-    if (a == U.cj[k]) lam += mu[k] * s;
+    const double s = mu[k] * pick(sk[k], q);
+    if (a == U.ci[k]) lam -= s;
+    if (a == U.cj[k]) lam += s;
   }
-  const double ly = lam / (a < U.na ? S.mass[U.atom[a]] : 1.0);
+  const double ly = lam * im;
   double xb = 0;
+#pragma unroll
   for (int l = 0; l < 3; l++) {
     if (l >= U.nc) continue;
-    double t = 0;
-    for (int c = 0; c < 3; c++) {
-      const double d = comp(ly, U.ci[l], c) - comp(ly, U.cj[l], c);
-      if (c == q) t = gam[l] * d;
-    }
+    double d[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) d[c] = comp(ly, U.ci[l], c) - comp(ly, U.cj[l], c);
+    const double t = gam[l] * pick(d, q);
     if (a == U.ci[l]) xb += t;
     if (a == U.cj[l]) xb -= t;
   }
@@ -985,7 +1011,9 @@ __global__ void __launch_bounds__(ADJ_THREADS, 1) adjoint_recompute(Sys S, Buf B
         const Unit& U = S.units[u];
         const bool on = lane < 3 * U.na;
         const int i = U.atom[on ? lane / 3 : 0], q = 3 * i + lane % 3;
-        double xo = 0, va = 0, y = 0, g[3];
+        double xo = 0, va = 0, y = 0, g[3], d2[3] = {U.d2[0], U.d2[1], U.d2[2]};
+        const UnitCons uc(U);
+        const double im = on ? 1.0 / S.mass[i] : 0.0;
         if (on) {
           const double c = S.c[i], f = __ldcg(b.F + q) + (bonded ? bonded_sum(S, b, i, lane % 3) : 0.0);
           va = __ldcg(b.V + q);
@@ -995,10 +1023,10 @@ __global__ void __launch_bounds__(ADJ_THREADS, 1) adjoint_recompute(Sys S, Buf B
           y = xo + S.dt * va;
         }
         const double yd = y;
-        if (U.nc > 0) {
-          if (!unit_shake(S, U, y, xo, g) && lane == 0) b.flag[1] = MDN_ST_SHAKE_NOCONV;
+        if (uc.nc > 0) {
+          if (!unit_shake(uc, d2, im, y, xo, g) && lane == 0) b.flag[1] = MDN_ST_SHAKE_NOCONV;
           if (S.vcorr) va += (y - yd) / S.dt;
-          if (lane < U.nc) gam[U.cons[lane]] = lane == 0 ? g[0] : lane == 1 ? g[1] : g[2];
+          if (lane < uc.nc) gam[U.cons[lane]] = pick(g, lane);
         }
         if (on) {
           x1[q] = y;
@@ -1080,11 +1108,10 @@ __global__ void __launch_bounds__(ADJ_THREADS, 1) adjoint_segment(Sys S, Buf B, 
     const double* x0 = x1 - n3;
     const double* const gam = B.gam + (size_t)(t - 1) * S.n_cons;
     const double* const mg = B.mg + (size_t)t * 3 * (S.n_vmol + 1) + 3 * S.n_vmol;
-    double pull[3] = {0, 0, 0};
-    for (int k = 0; k < 3; k++) {
-      for (unsigned r = 0; r < cg::this_cluster().num_blocks(); r++) pull[k] -= __ldcg(B.part + 3 * r + k);
-      pull[k] += mg[k];
-    }
+    double pull[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      pull[k] = mg[k] - warp_sum_dd(lane < (int)cg::this_cluster().num_blocks() ? __ldcg(B.part + 3 * lane + k) : 0.0);
     /* what the force product leaves to the owner of component q of atom i */
     auto rest = [&](int i, int k) {
       double v = bonded_sum(S, B, i, k);
@@ -1103,15 +1130,17 @@ __global__ void __launch_bounds__(ADJ_THREADS, 1) adjoint_segment(Sys S, Buf B, 
       const bool on = lane < 3 * U.na;
       const int k = lane % 3, i = U.atom[on ? lane / 3 : 0], q = 3 * i + k;
       double lam = 0, lv = 0, xb = 0, g[3] = {0, 0, 0};
+      const UnitCons uc(U);
+      const double im = on ? 1.0 / S.mass[i] : 0.0, xq = on ? x1[q] : 0.0, xo = on ? x0[q] : 0.0;
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+        if (c < uc.nc) g[c] = gam[U.cons[c]];
       if (on) {
         lv = __ldcg(B.lv + q);
         /* (4): v_b = v_a + (x_t - y)/dt */
         lam = __ldcg(B.lx + q) + rest(i, k) + (vc ? lv / S.dt : 0.0);
       }
-      if (U.nc > 0) {
-        for (int c = 0; c < U.nc; c++) g[c] = gam[U.cons[c]];
-        xb = unit_shake_adjoint(S, U, on ? x1[q] : 0.0, on ? x0[q] : 0.0, g, lam);
-      }
+      if (uc.nc > 0) xb = unit_shake_adjoint(uc, im, xq, xo, g, lam);
       if (on) carry(q, vc ? lam - lv / S.dt : lam, xb, lv);
     }
     if (S.n_units == 0) {
@@ -1463,7 +1492,7 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
     S.row = dput(row, owned);
     S.row_order = dput(order, owned);
   }
-  /* the bonded terms' rows (4 per term: bonds, angles, dihedrals) by atom */
+  /* the bonded terms' rows by atom (terms: bonds, angles, dihedrals) */
   {
     std::vector<std::vector<int>> by(N);
     int t = 0;
@@ -1474,10 +1503,10 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
     add(bonds, 3);
     add(angles, 4);
     add(dih, 5);
-    std::vector<int> off(N + 1, 0), at;
+    std::vector<int> off(N + 1, 0), at(4 * (size_t)t, 0);
     for (int i = 0; i < N; i++) {
-      at.insert(at.end(), by[i].begin(), by[i].end());
-      off[i + 1] = (int)at.size();
+      off[i + 1] = off[i];
+      for (int a : by[i]) at[a] = off[i + 1]++;
     }
     S.tb_off = dput(off, owned);
     S.tb_at = dput(at, owned);
@@ -1514,8 +1543,16 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
         U.cons[U.nc] = c;
         U.ci[U.nc] = place(cons[3 * c]);
         U.cj[U.nc] = place(cons[3 * c + 1]);
+        const double dk = d->bond_coeff[2 * cons[3 * c + 2] + 1];
+        U.d2[U.nc] = dk * dk;
         U.nc++;
       }
+      for (int k = 0; k < U.nc; k++)
+        for (int l = 0; l < U.nc; l++) {
+          const double mi = 1.0 / mass[U.atom[U.ci[l]]], mj = 1.0 / mass[U.atom[U.cj[l]]];
+          U.cf[k][l] = (U.ci[l] == U.ci[k] ? mi : 0.0) - (U.cj[l] == U.ci[k] ? mj : 0.0) -
+                       (U.ci[l] == U.cj[k] ? mi : 0.0) + (U.cj[l] == U.cj[k] ? mj : 0.0);
+        }
       units.push_back(U);
     }
     Unit U;
@@ -1535,8 +1572,10 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
   }
   S.A = dput(A, owned);
   S.B = dput(Bt, owned);
-  S.eps = dput(E, owned);
-  S.sig = dput(Sg, owned);
+  for (double& v : E) v = 1.0 / v;
+  for (double& v : Sg) v = 1.0 / v;
+  S.ieps = dput(E, owned);
+  S.isig = dput(Sg, owned);
   S.pidx = dput(pidx, owned);
   S.bmh = dput(bmh, owned);
   S.n_bonds = (int)bonds.size() / 3;
@@ -1676,7 +1715,9 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
   auto* const segment = staged ? adjoint_segment<true> : adjoint_segment<false>;
   if (cudaFuncSetAttribute(segment, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
       cudaFuncSetAttribute(adjoint_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
-          cudaSuccess) {
+          cudaSuccess ||
+      cudaFuncSetAttribute(segment, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaFuncSetAttribute(adjoint_recompute, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cleanup();
     return err(MDN_ERR_CUDA, "mdn_adjoint: shared memory");
   }
