@@ -1491,12 +1491,15 @@ __device__ __forceinline__ void gas_far_pass(Ctx& x, bool eflag, bool kick) {
  * unweighted into Ugg.  The reference's own routine pairs loop indices
  * instead of gas_in entries (:48-57), reads weight[0][jj] (:25), bounds the
  * partner loop by the first molecule's size (:13) and books the energy in
- * Uvg (:34); none of that is reproduced.  One thread per slab molecule of
- * this CTA walks its full (both-direction) partner list and writes its own
- * force, so no reaction is scattered and the sum does not depend on the
- * launch shape.  Weights come from the current positions and ion centre, as
+ * Uvg (:34); none of that is reproduced.  kGGLanes lanes per slab molecule
+ * of this CTA walk its full (both-direction) partner list; their integer
+ * sums are its force, so no reaction is scattered and the sum does not
+ * depend on the launch shape.  A partner is a chain of loads (list entry,
+ * position), so with one lane per molecule a CTA with 114 molecules waited
+ * for some 20 of them one after another.  Weights come from the current positions and ion centre, as
  * MD::update_position sets them (src/verlet.cpp:109-134); molecules the
  * rebuild of this step inserted have weight 0 (`fresh`: this step rebuilt). */
+constexpr int kGGLanes = 8;
 template <int AG, bool FP64>
 __device__ __forceinline__ void gas_gg_pass_t(Ctx& x, bool eflag, bool fresh) {
   const RepParams* P = x.P;
@@ -1509,7 +1512,9 @@ __device__ __forceinline__ void gas_gg_pass_t(Ctx& x, bool eflag, bool fresh) {
   for (int at = 0; at < AG; at++) gtype[at] = x.ib[P->o_gas_type + at];
   const double* com = x.D->ion_com;
   long long egg = 0;
-  for (int s = lo + (int)threadIdx.x; s < hi; s += blockDim.x) {
+  const int lane = threadIdx.x & (kGGLanes - 1);
+  for (int s0 = lo; s0 < hi; s0 += blockDim.x / kGGLanes) {
+    const int sm = s0 + (int)threadIdx.x / kGGLanes, s = min(sm, hi - 1); /* whole warps stay for the shuffles */
     const size_t ms = gmol(P, par, s);
     const bool s_new = fresh && __ldcg(a->slab_ins + ms) == nreb;
     double X[3 * AG], w[AG];
@@ -1522,8 +1527,8 @@ __device__ __forceinline__ void gas_gg_pass_t(Ctx& x, bool eflag, bool fresh) {
     long long F[AG][3];
 #pragma unroll
     for (int at = 0; at < AG; at++) F[at][0] = F[at][1] = F[at][2] = 0;
-    const int start = a->ggl_start[ms], cnt = a->ggl_n[ms];
-    for (int q = 0; q < cnt; q++) {
+    const int start = a->ggl_start[ms], cnt = sm < hi ? a->ggl_n[ms] : 0;
+    for (int q = lane; q < cnt; q += kGGLanes) {
       const int t = a->ggl[P->ggl_off + start + q];
       const bool t_new = fresh && __ldcg(a->slab_ins + gmol(P, par, t)) == nreb;
 #pragma unroll
@@ -1566,9 +1571,14 @@ __device__ __forceinline__ void gas_gg_pass_t(Ctx& x, bool eflag, bool fresh) {
     for (int at = 0; at < AG; at++) {
       const size_t g = gatom(P, par, s, at);
       for (int k = 0; k < 3; k++) {
-        const double f = (double)F[at][k] * MDN_FIX_INV;
-        if (!(fabs(f) < MDN_FIX_LIMIT)) set_status(x, MDN_ST_FIXED_OVERFLOW);
-        a->slab_fgg[3 * g + k] = f;
+        long long v = F[at][k];
+#pragma unroll
+        for (int m = kGGLanes / 2; m; m >>= 1) v += shfl_xor_ll(v, m);
+        const double f = (double)v * MDN_FIX_INV;
+        if (lane == 0 && sm < hi) {
+          if (!(fabs(f) < MDN_FIX_LIMIT)) set_status(x, MDN_ST_FIXED_OVERFLOW);
+          a->slab_fgg[3 * g + k] = f;
+        }
       }
     }
   }
