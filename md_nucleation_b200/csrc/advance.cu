@@ -531,17 +531,12 @@ __device__ __forceinline__ void ion_centre(const Ctx& x, const double* src, doub
  * threshold decision depends on it (the in/out classification) */
 __device__ __forceinline__ void ion_centre_exact(Ctx& x) {
   const RepParams* P = x.P;
-  if (threadIdx.x == 0) {
-    double s[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = 0; i < P->n_ion; i++) {
-      double m = x.c.mass[tag_type(x.c.tag[i].k)];
-      for (int k = 0; k < 3; k++) {
-        s[k] += x.c.x[3 * i + k] * m;
-        s[3 + k] += x.c.v[3 * i + k] * m;
-      }
-    }
-    double mInv = 1 / P->ion_msum;
-    for (int k = 0; k < 6; k++) x.D->ion_com[k] = s[k] * mInv;
+  if (threadIdx.x < 6) { /* one component each */
+    const double* const src = threadIdx.x < 3 ? x.c.x + threadIdx.x : x.c.v + threadIdx.x - 3;
+    double s = 0;
+    for (int i = 0; i < P->n_ion; i++) s += src[3 * i] * x.c.mass[tag_type(x.c.tag[i].k)];
+    const double mInv = 1 / P->ion_msum;
+    x.D->ion_com[threadIdx.x] = s * mInv;
   }
   __syncthreads();
 }
@@ -2091,42 +2086,37 @@ __device__ __forceinline__ void insert_vapor(const Ctx& x, int q, int n_rebuild,
  * (ion, vapor in the domain before this rebuild) or of a vapor molecule whose
  * entry this rebuild already accepted; with the gas-gas term on, nor of a gas
  * atom in the domain before this rebuild (gas molecules entering in the same
- * rebuild are not tested against each other) */
+ * rebuild are not tested against each other).  One warp, X in every lane. */
 __device__ __forceinline__ bool insert_clear(const Ctx& x, const double* X, int n, int n_rebuild) {
   const double d2min = MDN_INSERT_MIN_DIST * MDN_INSERT_MIN_DIST;
-  if (kGG && (x.P->interactions & MDN_I_GG)) {
-    const RepParams* P = x.P;
-    const int G = x.D->n_gas_in, par = x.D->parity;
-    for (int u = 0; u < G * P->a_g; u++) {
-      const double* gpos = x.a->slab_x + 3 * ((size_t)P->slab_off + (size_t)par * P->slab_cap * P->a_g + u);
-      const double g0 = __ldcg(gpos), g1 = __ldcg(gpos + 1), g2 = __ldcg(gpos + 2);
-      for (int a = 0; a < n; a++) {
-        double dx = X[3 * a] - g0, dy = X[3 * a + 1] - g1, dz = X[3 * a + 2] - g2;
-        if (dx * dx + dy * dy + dz * dz < d2min) return false;
-      }
-    }
-  }
-  for (int i = 0; i < x.n_core; i++) {
-    const double* c = x.c.x + 3 * i;
+  const int lane = threadIdx.x & 31;
+  bool clash = false;
+  auto test = [&](double c0, double c1, double c2) {
     for (int a = 0; a < n; a++) {
-      double dx = X[3 * a] - c[0], dy = X[3 * a + 1] - c[1], dz = X[3 * a + 2] - c[2];
-      if (dx * dx + dy * dy + dz * dz < d2min) return false;
+      double dx = X[3 * a] - c0, dy = X[3 * a + 1] - c1, dz = X[3 * a + 2] - c2;
+      if (dx * dx + dy * dy + dz * dz < d2min) clash = true;
     }
-  }
+  };
+  for (int i = lane; i < x.n_core; i += 32) test(x.c.x[3 * i], x.c.x[3 * i + 1], x.c.x[3 * i + 2]);
   const int nc = min(x.cand[MDN_INSERT_MAX_VAPOR], MDN_INSERT_MAX_VAPOR);
-  for (int k = 0; k < nc; k++) {
+#pragma unroll 1
+  for (int k = lane; k < nc; k += 32) {
     const int mi = x.cand[k];
     const int f = x.a->region[(size_t)x.P->mol_off + mi];
     if (!(f & 1)) continue;
     double Xv[3 * MDN_MAX_VAP_ATOMS], Vv[3 * MDN_MAX_VAP_ATOMS];
     insert_vapor(x, mi - 1 - x.P->n_gas, n_rebuild, f >> 2, Xv, Vv);
-    for (int b = 0; b < x.P->a_v; b++)
-      for (int a = 0; a < n; a++) {
-        double dx = X[3 * a] - Xv[3 * b], dy = X[3 * a + 1] - Xv[3 * b + 1], dz = X[3 * a + 2] - Xv[3 * b + 2];
-        if (dx * dx + dy * dy + dz * dz < d2min) return false;
-      }
+    for (int b = 0; b < x.P->a_v; b++) test(Xv[3 * b], Xv[3 * b + 1], Xv[3 * b + 2]);
   }
-  return true;
+  if (kGG && (x.P->interactions & MDN_I_GG)) {
+    const RepParams* P = x.P;
+    const int G = x.D->n_gas_in, par = x.D->parity;
+    for (int u = lane; u < G * P->a_g; u += 32) {
+      const double* gpos = x.a->slab_x + 3 * ((size_t)P->slab_off + (size_t)par * P->slab_cap * P->a_g + u);
+      test(__ldcg(gpos), __ldcg(gpos + 1), __ldcg(gpos + 2));
+    }
+  }
+  return !__any_sync(0xffffffffu, clash);
 }
 
 __device__ __forceinline__ void insert_gas(const Ctx& x, int q, int n_rebuild, int t, double* X, double* V) {
@@ -2188,13 +2178,13 @@ __device__ __forceinline__ void insert_vapor(const Ctx& x, int q, int n_rebuild,
 }
 
 /* free flight, in/out test, wrap and resampling of one molecule; returns
- * (draw << 2) | (was_in << 1) | now_in, draw = the insertion draw that passed
- * the overlap test (0 under MDN_Q_BLIND_INSERT).  A molecule inside the sphere
- * whose draws all overlap stays outside, unwrapped and not resampled, until
- * the next rebuild.  Entering vapor molecules become candidates that
- * vapor_entries() decides. */
+ * (was_in << 1) | now_in.  Unless MDN_Q_BLIND_INSERT is set, entering
+ * molecules become candidates: vapor ones that vapor_entries() decides,
+ * provisionally in, and gas ones (into `entries`) that gas_entries() decides,
+ * provisionally out.  A molecule inside the sphere whose draws all overlap
+ * stays outside, unwrapped and not resampled, until the next rebuild. */
 __device__ __forceinline__ int classify_one(const Ctx& x, int mi, double sigma, int n_rebuild, int loop_pair,
-                                            const double* com, int kind /* 0 gas, 1 vapor */) {
+                                            const double* com, int kind /* 0 gas, 1 vapor */, int* entries) {
   const RepParams* P = x.P;
   const size_t g = (size_t)P->mol_off + mi;
   double* X = x.a->mol_x + 3 * g;
@@ -2207,7 +2197,6 @@ __device__ __forceinline__ int classify_one(const Ctx& x, int mi, double sigma, 
   double dz = X[2] - com[2];
   double r2 = (dx * dx + dy * dy + dz * dz);
   int in = r2 < P->RI2 ? 1 : 0;
-  int draw_ok = 0;
   if (in && !was && !(P->quirks & MDN_Q_BLIND_INSERT) && kind == 1) {
     /* decided by vapor_entries(): recorded as a candidate, provisionally in;
      * beyond MDN_INSERT_MAX_VAPOR candidates in one rebuild the entry waits
@@ -2222,17 +2211,10 @@ __device__ __forceinline__ int classify_one(const Ctx& x, int mi, double sigma, 
     return 1;
   }
   if (in && !was && !(P->quirks & MDN_Q_BLIND_INSERT)) {
-    double Xt[3 * MDN_MAX_VAP_ATOMS], Vt[3 * MDN_MAX_VAP_ATOMS];
-    int t = 0;
-    for (; t < MDN_INSERT_TRIES; t++) {
-      insert_gas(x, mi - 1, n_rebuild, t, Xt, Vt);
-      if (insert_clear(x, Xt, P->a_g, n_rebuild)) break;
-    }
-    if (t == MDN_INSERT_TRIES) {
-      x.a->region[g] = 0; /* the entry waits for the next rebuild */
-      return 0;
-    }
-    draw_ok = t;
+    /* decided by gas_entries(), from this CTA's list */
+    entries[atomicAdd(&x.iscr[50], 1)] = mi;
+    x.a->region[g] = 0;
+    return 0;
   }
   if (!in) {
     double HL = P->box * 0.5;
@@ -2250,8 +2232,8 @@ __device__ __forceinline__ int classify_one(const Ctx& x, int mi, double sigma, 
     V[1] = z1 * sigma;
     V[2] = z2 * sigma;
   }
-  x.a->region[g] = (unsigned char)((draw_ok << 2) | (was << 1) | in);
-  return (draw_ok << 2) | (was << 1) | in;
+  x.a->region[g] = (unsigned char)((was << 1) | in);
+  return (was << 1) | in;
 }
 
 /* gas-gas pair list of the slab (PotentialGasGas::makePair,
@@ -2264,50 +2246,59 @@ __device__ __forceinline__ void relist_gg(Ctx& x, cg::cluster_group& cl) {
   const int par = x.D->parity, G = x.D->n_gas_in;
   int lo, hi;
   partition(x, G, &lo, &hi);
-  int* sc = x.iscr;
   const double* cen = a->mol_x + 3 * ((size_t)P->mol_off + 1);
   const int* smol = a->slab_mol + gmol(P, par, 0);
-  /* centres and slab entries of every CTA's molecules, from L2 */
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  /* a warp per molecule: its lanes test 32 others at a time (centres and slab
+   * entries of every CTA's molecules, from L2); returns the number of
+   * partners, which go to out, ascending, when it is given */
   auto partners = [&](int s, int* out) {
     const double* c = cen + 3 * (size_t)__ldcg(smol + s);
     const double c0 = __ldcg(c), c1 = __ldcg(c + 1), c2 = __ldcg(c + 2);
     int n = 0;
-    for (int t = 0; t < G; t++) {
-      if (t == s) continue;
-      const double* d = cen + 3 * (size_t)__ldcg(smol + t);
-      const double dx = c0 - __ldcg(d), dy = c1 - __ldcg(d + 1), dz = c2 - __ldcg(d + 2);
-      if ((dx * dx + dy * dy + dz * dz) < P->ml2) {
-        if (out) out[n] = t;
-        n++;
+#pragma unroll 4
+    for (int t0 = 0; t0 < G; t0 += 32) {
+      const int t = t0 + lane;
+      bool in = false;
+      if (t < G && t != s) {
+        const double* d = cen + 3 * (size_t)__ldcg(smol + t);
+        const double dx = c0 - __ldcg(d), dy = c1 - __ldcg(d + 1), dz = c2 - __ldcg(d + 2);
+        in = (dx * dx + dy * dy + dz * dz) < P->ml2;
       }
+      const unsigned m = __ballot_sync(0xffffffffu, in);
+      if (in && out) out[n + __popc(m & ((1u << lane) - 1u))] = t;
+      n += __popc(m);
     }
     return n;
   };
+  /* counts, then starts (a prefix sum over the CTA's molecules), then lists */
+  for (int s = lo + (int)(threadIdx.x >> 5); s < hi; s += nw) {
+    const int c = partners(s, nullptr);
+    if (lane == 0) a->ggl_n[gmol(P, par, s)] = c;
+  }
+  __syncthreads();
   int mine = 0;
-  for (int s = lo + (int)threadIdx.x; s < hi; s += blockDim.x) mine += partners(s, nullptr);
-  mine = block_sum_i(mine, sc);
+  for (int s0 = lo; s0 < hi; s0 += blockDim.x) {
+    const int s = s0 + (int)threadIdx.x;
+    const int c = s < hi ? a->ggl_n[gmol(P, par, s)] : 0;
+    int t;
+    const int o = block_exscan(c, x.iscr, &t);
+    if (s < hi) a->ggl_start[gmol(P, par, s)] = mine + o;
+    mine += t;
+  }
   int base, tot;
-  cluster_prefix(x, cl, &sc[46], mine, &base, &tot);
+  cluster_prefix(x, cl, &x.iscr[46], mine, &base, &tot);
   const bool over = tot > P->ggl_cap;
   if (over && threadIdx.x == 0 && x.rank == 0) set_status(x, MDN_ST_LIST_OVERFLOW);
-  int run = base;
-  for (int s0 = lo; s0 < hi; s0 += blockDim.x) {
-    const int s = s0 + threadIdx.x;
-    const int c = s < hi ? partners(s, nullptr) : 0;
-    int t_tot;
-    const int off = block_exscan(c, sc, &t_tot);
-    if (s < hi) {
-      const size_t ms = gmol(P, par, s);
-      if (!over) {
-        a->ggl_start[ms] = run + off;
-        a->ggl_n[ms] = c;
-        partners(s, a->ggl + P->ggl_off + run + off);
-      } else {
-        a->ggl_start[ms] = 0;
-        a->ggl_n[ms] = 0;
-      }
+  for (int s = lo + (int)(threadIdx.x >> 5); s < hi; s += nw) {
+    const size_t ms = gmol(P, par, s);
+    const int start = over ? 0 : base + a->ggl_start[ms];
+    if (!over) partners(s, a->ggl + P->ggl_off + start);
+    __syncwarp();
+    if (lane == 0) {
+      a->ggl_start[ms] = start;
+      if (over) a->ggl_n[ms] = 0;
     }
-    run += t_tot;
   }
   if (threadIdx.x == 0) x.D->gg_count = over ? 0 : tot / 2;
   __threadfence();
@@ -2323,8 +2314,17 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
   const bool gi = (P->interactions & MDN_I_GI) != 0, gv = (P->interactions & MDN_I_GV) != 0;
   int lo, hi;
   slab_part(x, &lo, &hi);
-  /* bounding sphere of the ion, exact test below */
   int* sc = x.iscr;
+  /* the vapor centres, from L2 (rank 0 set them), into the core's sum buffer,
+   * which no CTA reads now: from global memory each test of a gas molecule
+   * against them was two dependent loads */
+  double* const sv = (double*)x.c.acc;
+  if (gv)
+    for (int q = threadIdx.x; q < 3 * nv; q += blockDim.x) {
+      const int vm = __ldcg(a->vslab_mol + vmol(P, par, q / 3));
+      sv[q] = __ldcg(a->mol_x + 3 * ((size_t)P->mol_off + 1 + P->n_gas + vm) + q % 3);
+    }
+  __syncthreads();
   int gi_tot = 0, gv_tot = 0, nn_tot = 0;
   int gi_base = 0, gv_base = 0, nn_before = 0;
   /* pass 1: counts */
@@ -2344,9 +2344,7 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
         }
       if (gv)
         for (int q = 0; q < nv; q++) {
-          int vm = __ldcg(a->vslab_mol + vmol(P, par, q));
-          const double* vc = a->mol_x + 3 * ((size_t)P->mol_off + 1 + P->n_gas + vm);
-          double dx = cx0 - __ldcg(vc), dy = cx1 - __ldcg(vc + 1), dz = cx2 - __ldcg(vc + 2);
+          double dx = cx0 - sv[3 * q], dy = cx1 - sv[3 * q + 1], dz = cx2 - sv[3 * q + 2];
           if ((dx * dx + dy * dy + dz * dz) < P->ml2) cgv++;
         }
     }
@@ -2382,9 +2380,7 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
         }
       if (gv)
         for (int q = 0; q < nv; q++) {
-          int vm = __ldcg(a->vslab_mol + vmol(P, par, q));
-          const double* vc = a->mol_x + 3 * ((size_t)P->mol_off + 1 + P->n_gas + vm);
-          double dx = cx0 - __ldcg(vc), dy = cx1 - __ldcg(vc + 1), dz = cx2 - __ldcg(vc + 2);
+          double dx = cx0 - sv[3 * q], dy = cx1 - sv[3 * q + 1], dz = cx2 - sv[3 * q + 2];
           if ((dx * dx + dy * dy + dz * dz) < P->ml2) cgv++;
         }
     }
@@ -2409,9 +2405,7 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
         w = 0;
         if (gv)
           for (int q = 0; q < nv; q++) {
-            int vm = __ldcg(a->vslab_mol + vmol(P, par, q));
-            const double* vc = a->mol_x + 3 * ((size_t)P->mol_off + 1 + P->n_gas + vm);
-            double dx = cx0 - __ldcg(vc), dy = cx1 - __ldcg(vc + 1), dz = cx2 - __ldcg(vc + 2);
+            double dx = cx0 - sv[3 * q], dy = cx1 - sv[3 * q + 1], dz = cx2 - sv[3 * q + 2];
             if ((dx * dx + dy * dy + dz * dz) < P->ml2) a->gvl[P->gvl_off + bgv + w++] = (unsigned short)q;
           }
       } else {
@@ -2433,6 +2427,37 @@ __device__ __forceinline__ void relist(Ctx& x, cg::cluster_group& cl) {
   cl.sync();
   build_near(x, cl);
   if (kGG && P->ggl_cap > 0 && (P->interactions & MDN_I_GG)) relist_gg(x, cl);
+}
+
+/* The overlap test of the gas molecules that enter at this rebuild, the CTA's
+ * list of n: a warp each, the draws in the first lanes, each tested by the
+ * whole warp against the core (a thread that tested its own molecule against
+ * 800 core atoms held up the 31 others of its warp, one to three million
+ * cycles per rebuild).  The region flag of an accepted one is (draw << 2) | 1;
+ * returns how many this warp accepted, in its first lane. */
+__device__ __forceinline__ int gas_entries(const Ctx& x, const int* entries, int n, int nreb) {
+  const RepParams* P = x.P;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, ag = P->a_g;
+  int taken = 0;
+  for (int k = threadIdx.x >> 5; k < n; k += blockDim.x >> 5) {
+    const int mi = entries[k];
+    double Xt[3 * MDN_MAX_GAS_ATOMS], Vt[3 * MDN_MAX_GAS_ATOMS];
+    for (int q = 0; q < 3 * MDN_MAX_GAS_ATOMS; q++) Xt[q] = 0.0;
+    if (lane < MDN_INSERT_TRIES) insert_gas(x, mi - 1, nreb, lane, Xt, Vt);
+    int ok = -1;
+#pragma unroll 1
+    for (int t = 0; t < MDN_INSERT_TRIES && ok < 0; t++) {
+      double X[3 * MDN_MAX_GAS_ATOMS];
+      for (int q = 0; q < 3 * MDN_MAX_GAS_ATOMS; q++) X[q] = __shfl_sync(FULL, Xt[q], t);
+      if (insert_clear(x, X, ag, nreb)) ok = t;
+    }
+    if (lane == 0 && ok >= 0) {
+      x.a->region[(size_t)P->mol_off + mi] = (unsigned char)((ok << 2) | 1);
+      taken++;
+    }
+  }
+  return taken;
 }
 
 /* The overlap test of entering vapor molecules: against the ion, the vapor
@@ -2564,7 +2589,10 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
   double vmax2 = 0;
   /* vapor molecules (rank 0; events) */
   int my_vin = 0;
-  if (threadIdx.x == 0) x.cand[MDN_INSERT_MAX_VAPOR] = 0;
+  if (threadIdx.x == 0) {
+    x.cand[MDN_INSERT_MAX_VAPOR] = 0;
+    x.iscr[50] = 0;
+  }
   __syncthreads();
   if (x.rank == 0)
     for (int q = threadIdx.x; q < P->n_vap; q += blockDim.x) {
@@ -2591,7 +2619,7 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
           set_status(x, MDN_ST_EVENT_OVERFLOW);
         }
       }
-      int f = classify_one(x, mi, P->vap_sigma, nreb, loop_pair, com, 1);
+      int f = classify_one(x, mi, P->vap_sigma, nreb, loop_pair, com, 1, nullptr);
       my_vin += f & 1;
       const double* V = a->mol_v + 3 * g;
       double v2 = V[0] * V[0] + V[1] * V[1] + V[2] * V[2];
@@ -2608,13 +2636,16 @@ __device__ __forceinline__ void make_pair(Ctx& x, cg::cluster_group& cl) {
   }
   __syncthreads();
   /* free flight + classification of the gas molecules of this CTA's range */
+  int* const entries = a->entries + P->mol_off + 1 + mlo;
   for (int q = mlo + threadIdx.x; q < mhi; q += blockDim.x) {
-    int f = classify_one(x, 1 + q, P->gas_sigma, nreb, loop_pair, com, 0);
+    int f = classify_one(x, 1 + q, P->gas_sigma, nreb, loop_pair, com, 0, entries);
     my_in += f & 1;
     const double* V = a->mol_v + 3 * ((size_t)P->mol_off + 1 + q);
     double v2 = V[0] * V[0] + V[1] * V[1] + V[2] * V[2];
     vmax2 = fmax(vmax2, v2);
   }
+  __syncthreads();
+  my_in += gas_entries(x, entries, x.iscr[50], nreb);
   {
     const double* V = x.D->ion_com + 3;
     vmax2 = fmax(vmax2, V[0] * V[0] + V[1] * V[1] + V[2] * V[2]);

@@ -162,6 +162,7 @@ struct mdn_handle {
   double *mol_x = nullptr, *mol_v = nullptr;
   unsigned char* region = nullptr;
   int* slot = nullptr;
+  int* entries = nullptr;
   double *slab_x = nullptr, *slab_v = nullptr, *slab_f = nullptr;
   int* slab_mol = nullptr;
   double *vslab_x = nullptr, *vslab_v = nullptr, *vslab_f = nullptr;
@@ -215,7 +216,7 @@ namespace {
 
 void free_all(mdn_handle* h) {
   void* ptrs[] = {h->dP, h->dD, h->d_iblob, h->d_dblob, h->ion_x, h->ion_v, h->ion_f, h->mol_x, h->mol_v,
-                  h->region, h->slot, h->slab_x, h->slab_v, h->slab_f, h->slab_mol, h->vslab_x, h->vslab_v,
+                  h->region, h->slot, h->entries, h->slab_x, h->slab_v, h->slab_f, h->slab_mol, h->vslab_x, h->vslab_v,
                   h->vslab_f, h->vslab_w, h->vslab_mol, h->near_rec, h->near_item, h->near_cnt, h->near_s, h->far_list, h->near_gi, h->near_gv, h->gil_n,
                   h->gvl_n, h->gil, h->gvl, h->energy, h->events, h->n_events, h->status, h->job_order,
                   h->job_counter, h->snap_off, h->snap_type, h->snap_x, h->snap_v, h->d_ctl_mode,
@@ -313,7 +314,7 @@ long long launch(mdn_handle* h, int mode, long long n_steps, int energy_mode, un
   a.dblob = h->d_dblob;
   a.ion_x = h->ion_x; a.ion_v = h->ion_v; a.ion_f = h->ion_f;
   a.mol_x = h->mol_x; a.mol_v = h->mol_v;
-  a.region = h->region; a.slot = h->slot;
+  a.region = h->region; a.slot = h->slot; a.entries = h->entries;
   a.slab_x = h->slab_x; a.slab_v = h->slab_v; a.slab_f = h->slab_f; a.slab_mol = h->slab_mol;
   a.vslab_x = h->vslab_x; a.vslab_v = h->vslab_v; a.vslab_f = h->vslab_f; a.vslab_w = h->vslab_w;
   a.vslab_mol = h->vslab_mol;
@@ -788,6 +789,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
   ALLOC(h->mol_v, 3 * mol_tot);
   ALLOC(h->region, mol_tot);
   ALLOC(h->slot, mol_tot);
+  ALLOC(h->entries, mol_tot);
   ALLOC(h->slab_x, 3 * slab_atoms);
   ALLOC(h->slab_v, 3 * slab_atoms);
   ALLOC(h->slab_f, 3 * slab_atoms);

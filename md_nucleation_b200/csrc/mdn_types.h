@@ -123,6 +123,7 @@ typedef struct KArgs {
   double *mol_x, *mol_v;
   unsigned char* region;
   int* slot;
+  int* entries;            /* gas molecules that enter at a rebuild, from the CTA's first molecule */
   double *slab_x, *slab_v, *slab_f;
   int* slab_mol;
   double *vslab_x, *vslab_v, *vslab_f;
