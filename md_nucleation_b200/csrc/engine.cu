@@ -1540,15 +1540,23 @@ static int order_by_measured(mdn_handle* h, long long n_steps, int* status) {
   return MDN_OK;
 }
 
-/* One block of the tuner: n_steps, timed without the first of them, in which
- * the replicas make their near records for the block's cluster size. */
+/* One block of the tuner: n_steps as several launches, the first step (in
+ * which the replicas make their near records for the block's cluster size)
+ * and three parts of the rest.  *ms is the time of a step in the fastest
+ * part: a domain rebuild of a large replica falls into one of them. */
 static int tune_block(mdn_handle* h, long long n_steps, float* ms, int* status) {
-  for (int part = n_steps > 1 ? 0 : 1; part < 2; part++) {
-    const int rc = mdn_step(h, part == 0 ? 1 : n_steps > 1 ? n_steps - 1 : 1, 0);
+  long long done = 0;
+  *ms = 0;
+  while (done < n_steps) {
+    const bool first = done == 0 && n_steps > 1;
+    const long long n = first ? 1 : std::min(n_steps - done, std::max<long long>(2, (n_steps + 1) / 3));
+    const int rc = mdn_step(h, n, 0);
     if (rc == MDN_ERR_REPLICA) *status = rc;
     else if (rc != MDN_OK) return rc;
+    const float t = (float)(h->last_ms / (double)n);
+    if (!first && (*ms == 0 || t < *ms)) *ms = t;
+    done += n;
   }
-  *ms = (float)h->last_ms;
   return MDN_OK;
 }
 
