@@ -756,7 +756,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
   std::stable_sort(h->order.begin(), h->order.end(), [&](int a, int b) { return h->P[a].work > h->P[b].work; });
   /* automatic cluster size: the smallest power of two that lets the largest
    * replica finish within the time of an even share of the SMs
-   * (num_sms * W_max / W_total CTAs), at most 8 */
+   * (num_sms * W_max / W_total CTAs), at most 8; 1 for small replicas */
   {
     double wmax = 0, wsum = 0;
     for (int r = 0; r < R; r++) {
@@ -766,6 +766,13 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
     const double want = wsum > 0 ? h->num_sms * wmax / wsum : 1.0;
     int c = 1;
     while (c < 8 && c < want) c *= 2;
+    /* a small replica is a chain of latencies that more CTAs do not shorten,
+     * and the cluster's barriers lengthen: lone replicas of 332 and 538 units
+     * take 10.4 and 11.3 us per step on one CTA against 11.7 and 12.7 on
+     * eight.  Up to 3,000 units steps still gain (1,225: 13.4 against 15.1),
+     * but a force evaluation alone, with its FP64 energies, loses (1,019: 4 of
+     * 62 us), and both need the same near records. */
+    if (wmax < 700) c = 1;
     h->auto_cluster = c;
   }
 
