@@ -2927,7 +2927,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
   if (threadIdx.x == 0) iscr[62] = 0;
   __syncthreads();
   for (;;) {
-    if (x.rank == 0 && threadIdx.x == 0) s_job = atomicAdd(a.job_counter, 1);
+    if (x.rank == 0 && threadIdx.x == 0) s_job = (int)(atomicAdd(a.job_counter, 1u) - a.job_base);
     cl.sync();
     const int job = *cl.map_shared_rank(&s_job, 0);
     cl.sync();

@@ -155,7 +155,8 @@ typedef struct KArgs {
   const double* ctl_T;     /* [n_replicas] thermostat target (K)               */
   const int* job_order;
   int n_jobs;
-  int* job_counter;
+  unsigned* job_counter;   /* counts on from launch to launch: */
+  unsigned job_base;       /* its value at the start of this one */
   long long n_steps;
   int energy_mode, mode;
   int keep_com;            /* MAKE_PAIR: classify against the stored ion centre */
