@@ -997,11 +997,42 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
       if ((any_on >> s) & 1u) step(s, std::true_type());
       pass_on();
     }
-  } else {
+  } else if constexpr (FP64 || E) {
 #pragma unroll 4
     for (int s = 0; s < s1; s++) {
       step(s, std::false_type());
       pass_on();
+    }
+  } else {
+    /* four steps' forces at once (a step that counts no pair of the lane adds
+     * zeros), then their sums in order */
+    constexpr int kSteps = 4;
+    const int jmax = nc - 1 - j0;
+    for (int s0 = 0; s0 < s1; s0 += kSteps) {
+      float fx[kSteps], fy[kSteps], fz[kSteps];
+#pragma unroll
+      for (int u = 0; u < kSteps; u++) {
+        const int j = j0 + min((lane + s0 + u) & 31, jmax);
+        const AtomTag gj = x.c.tag[j];
+        const float4 pj = x.c.pos[j];
+        const float2 AB = x.c.lj[rowi + tag_type(gj.k)];
+        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        float ee;
+        const float f = lj_coul(r2, AB.x, AB.y, qi * pj.w, true, &ee) * (gi.w * gj.w);
+        const float fp = ((on >> u) & 1u) ? f : 0.0f;
+        fx[u] = fp * dx;
+        fy[u] = fp * dy;
+        fz[u] = fp * dz;
+      }
+      on >>= kSteps;
+#pragma unroll
+      for (int u = 0; u < kSteps; u++) {
+        if (s0 + u == s1) break; /* a diagonal tile ends within the four */
+        F0 += fx[u]; F1 += fy[u]; F2 += fz[u];
+        R0 -= fx[u]; R1 -= fy[u]; R2 -= fz[u];
+        pass_on();
+      }
     }
   }
   if (diag) {
