@@ -997,38 +997,59 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
       if ((any_on >> s) & 1u) step(s, std::true_type());
       pass_on();
     }
-  } else if constexpr (FP64 || E) {
-#pragma unroll 4
-    for (int s = 0; s < s1; s++) {
-      step(s, std::false_type());
-      pass_on();
-    }
   } else {
-    /* four steps' forces at once (a step that counts no pair of the lane adds
-     * zeros), then their sums in order */
-    constexpr int kSteps = 4;
+    /* several steps' forces (and energies) at once, a step that counts no pair
+     * of the lane adding zeros, then their sums in order */
+    constexpr int kSteps = FP64 || E ? 2 : 4;
     const int jmax = nc - 1 - j0;
     for (int s0 = 0; s0 < s1; s0 += kSteps) {
-      float fx[kSteps], fy[kSteps], fz[kSteps];
+      Acc fx[kSteps], fy[kSteps], fz[kSteps];
 #pragma unroll
       for (int u = 0; u < kSteps; u++) {
-        const int j = j0 + min((lane + s0 + u) & 31, jmax);
+        const int jl = (lane + s0 + u) & 31, j = j0 + min(jl, jmax);
         const AtomTag gj = x.c.tag[j];
-        const float4 pj = x.c.pos[j];
-        const float2 AB = x.c.lj[rowi + tag_type(gj.k)];
-        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        float ee;
-        const float f = lj_coul(r2, AB.x, AB.y, qi * pj.w, true, &ee) * (gi.w * gj.w);
-        const float fp = ((on >> u) & 1u) ? f : 0.0f;
-        fx[u] = fp * dx;
-        fy[u] = fp * dy;
-        fz[u] = fp * dz;
+        const int tt = rowi + tag_type(gj.k);
+        const bool take = (on >> u) & 1u; /* none past a diagonal tile's last step */
+        double qj = 0.0, R2d = 1.0, ex = 0.0, ey = 0.0, ez = 0.0;
+        if constexpr (FP64 || E) {
+          qj = qid * __shfl_sync(FULL, q_own, jl);
+          ex = xd[0] - x.c.x[3 * j];
+          ey = xd[1] - x.c.x[3 * j + 1];
+          ez = xd[2] - x.c.x[3 * j + 2];
+          R2d = ex * ex + ey * ey + ez * ez;
+        }
+        if constexpr (FP64) {
+          const double wj = __shfl_sync(FULL, w_own, jl);
+          const double f = lj_coul_d(R2d, x.db[P->d_ljA + tt], x.db[P->d_ljB + tt], qj, true) * (wid * wj);
+          const double fd = take ? f : 0.0;
+          fx[u] = fd * ex;
+          fy[u] = fd * ey;
+          fz[u] = fd * ez;
+        } else {
+          const float4 pj = x.c.pos[j];
+          const float2 AB = x.c.lj[tt];
+          const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+          float ee;
+          const float f = lj_coul(r2, AB.x, AB.y, qi * pj.w, true, &ee) * (gi.w * gj.w);
+          const float fp = take ? f : 0.0f;
+          fx[u] = fp * dx;
+          fy[u] = fp * dy;
+          fz[u] = fp * dz;
+        }
+        if constexpr (E) {
+          const double ed = lj_coul_energy(R2d, x.db[P->d_ljA12 + tt], x.db[P->d_ljB6 + tt], qj);
+          const long long e = take ? efixd(ed) : 0;
+          const bool iion = ii < ni, jion = j < ni;
+          e_ion += iion && jion ? e : 0;
+          e_vi += iion != jion ? e : 0;
+          e_vv += !iion && !jion ? e : 0;
+        }
       }
       on >>= kSteps;
 #pragma unroll
       for (int u = 0; u < kSteps; u++) {
-        if (s0 + u == s1) break; /* a diagonal tile ends within the four */
+        if (s0 + u == s1) break;
         F0 += fx[u]; F1 += fy[u]; F2 += fz[u];
         R0 -= fx[u]; R1 -= fy[u]; R2 -= fz[u];
         pass_on();
