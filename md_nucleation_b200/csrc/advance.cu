@@ -169,6 +169,8 @@ __device__ __forceinline__ void load_vapor(Ctx& x) {
     x.c.tag[i].w = a->vslab_w[g];
     x.c.tag[i].k = (unsigned)x.ib[P->o_vap_type + at] | ((unsigned)(s + 1) << 8);
   }
+  /* core_tile reads whole blocks of 32 */
+  for (int i = x.n_core + threadIdx.x; i < ((x.n_core + 31) & ~31); i += blockDim.x) x.c.tag[i].k = 0;
 }
 
 __device__ __forceinline__ void store_core(Ctx& x) {
@@ -710,8 +712,15 @@ __device__ __forceinline__ void dihedral_fd(const double* X, const double* co, i
 /* LJ (+ Coulomb) force factor and energy, the reference's formulas:
  *   f = r^-6 (A r^-6 - B) r^-2 [+ qqrd2e qi qj r^-1 r^-2], times w
  *   U = r^-6 (A/12 r^-6 - B/6) [+ qqrd2e qi qj / r]  (unweighted)          */
+/* rsqrtf without its scaling of subnormal arguments (three instructions per
+ * pair): the same result for every r2 of two atoms that are not in one place */
+__device__ __forceinline__ float rsqrt_ftz(float r2) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(r2));
+  return r;
+}
 __device__ __forceinline__ float lj_coul(float r2, float A, float B, float qq, bool coul, float* e) {
-  float rinv = rsqrtf(r2);
+  float rinv = rsqrt_ftz(r2);
   float r2inv = rinv * rinv;
   float r6inv = r2inv * r2inv * r2inv;
   float flj = r6inv * fmaf(A, r6inv, -B);
@@ -1001,21 +1010,22 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
     /* several steps' forces (and energies) at once, a step that counts no pair
      * of the lane adding zeros, then their sums in order */
     constexpr int kSteps = FP64 || E ? 2 : 4;
-    const int jmax = nc - 1 - j0;
+    const float2* const row = x.c.lj + rowi;
     for (int s0 = 0; s0 < s1; s0 += kSteps) {
       Acc fx[kSteps], fy[kSteps], fz[kSteps];
 #pragma unroll
       for (int u = 0; u < kSteps; u++) {
-        const int jl = (lane + s0 + u) & 31, j = j0 + min(jl, jmax);
+        const int jl = (lane + s0 + u) & 31, j = j0 + jl; /* past the core: type 0, not taken */
         const AtomTag gj = x.c.tag[j];
         const int tt = rowi + tag_type(gj.k);
         const bool take = (on >> u) & 1u; /* none past a diagonal tile's last step */
         double qj = 0.0, R2d = 1.0, ex = 0.0, ey = 0.0, ez = 0.0;
         if constexpr (FP64 || E) {
           qj = qid * __shfl_sync(FULL, q_own, jl);
-          ex = xd[0] - x.c.x[3 * j];
-          ey = xd[1] - x.c.x[3 * j + 1];
-          ez = xd[2] - x.c.x[3 * j + 2];
+          const double* const xj = x.c.x + 3 * min(j, nc - 1);
+          ex = xd[0] - xj[0];
+          ey = xd[1] - xj[1];
+          ez = xd[2] - xj[2];
           R2d = ex * ex + ey * ey + ez * ez;
         }
         if constexpr (FP64) {
@@ -1027,7 +1037,7 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
           fz[u] = fd * ez;
         } else {
           const float4 pj = x.c.pos[j];
-          const float2 AB = x.c.lj[tt];
+          const float2 AB = row[tag_type(gj.k)];
           const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
           const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
           float ee;
@@ -2960,15 +2970,15 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
   /* carve the dynamic shared memory */
   {
     unsigned char* p = dsm;
-    const int nc = a.nc_cap;
+    const int nc = a.nc_cap, nc32 = (nc + 31) & ~31;
     auto take = [&](size_t bytes) { unsigned char* q = p; p += (bytes + 15) & ~(size_t)15; return q; };
     x.c.acc = (long long*)take(sizeof(long long) * 3 * nc);
     x.c.chunk = (unsigned*)take(sizeof(unsigned) * 9 * nc);
     x.c.x = (double*)take(sizeof(double) * 3 * nc);
     x.c.v = (double*)take(sizeof(double) * 3 * nc);
     x.c.f = (double*)take(sizeof(double) * 3 * nc);
-    x.c.pos = (float4*)take(sizeof(float4) * nc);
-    x.c.tag = (AtomTag*)take(sizeof(AtomTag) * nc);
+    x.c.pos = (float4*)take(sizeof(float4) * nc32);
+    x.c.tag = (AtomTag*)take(sizeof(AtomTag) * nc32);
     x.c.excl = (unsigned*)take(sizeof(unsigned) * a.excl_cap);
     x.c.lj = (float2*)take(sizeof(float2) * a.nt_cap * a.nt_cap);
     x.c.c2 = (double*)take(sizeof(double) * a.nt_cap);
@@ -2976,6 +2986,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
   }
   /* the chunk sums start at zero and every core_reduce_kick leaves them so */
   for (int q = threadIdx.x; q < 9 * a.nc_cap; q += blockDim.x) x.c.chunk[q] = 0;
+  for (int q = threadIdx.x; q < ((a.nc_cap + 31) & ~31); q += blockDim.x) x.c.pos[q] = make_float4(0, 0, 0, 0);
   if (threadIdx.x == 0) iscr[62] = 0;
   __syncthreads();
   for (;;) {

@@ -249,8 +249,9 @@ size_t smem_bytes(int nc, int nt, int excl) {
   s += align16(sizeof(long long) * 3 * nc);
   s += align16(sizeof(unsigned) * 9 * nc);
   s += 3 * align16(sizeof(double) * 3 * nc);
-  s += align16(sizeof(float4) * nc);
-  s += align16(8 * (size_t)nc); /* AtomTag */
+  const size_t nc32 = ((size_t)nc + 31) & ~(size_t)31; /* pair tiles read whole blocks */
+  s += align16(sizeof(float4) * nc32);
+  s += align16(8 * nc32); /* AtomTag */
   s += align16(sizeof(unsigned) * excl);
   s += align16(sizeof(float2) * nt * nt);
   s += 2 * align16(sizeof(double) * nt);
