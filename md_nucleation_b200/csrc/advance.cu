@@ -279,23 +279,21 @@ __device__ __forceinline__ double shake_res_c(const double* Xi, const double* Xj
  * group at once, so the result is the sweeps' fixed point; the equations
  * are quadratic in l, and a handful of steps reach it where the sweeps of a
  * rigid water take dozens.  For one constraint a step is the sweep's own
- * update.  ks: the group's constraint indices (n of them); ct: the
- * constraint table (d^2, 1/m_i, 1/m_j).  Returns true once every
- * (|s_k|^2 - d_k^2)^2 <= 1e-20 A^4, the sweeps' criterion; false after 50
- * steps or a singular system, and the caller sweeps from there. */
+ * update.  ga, gc: the group's atoms (i, j) and coefficients (d^2, 1/m_i,
+ * 1/m_j), constraint by constraint.  Returns true once every (|s_k|^2 -
+ * d_k^2)^2 <= 1e-20 A^4, the sweeps' criterion; false after 50 steps or a
+ * singular system, and the caller sweeps from there. */
 template <int N>
-__device__ __forceinline__ bool shake_group_n(double* X, const double* R, const int* rig, const double* ct,
-                                              const int* ks) {
+__device__ __forceinline__ bool shake_group_n(double* X, const double* R, const int* ga, const double* gc) {
   int I[N], J[N];
   double r[N][3], d2[N], ci[N], cj[N], w[N][N];
 #pragma unroll
   for (int k = 0; k < N; k++) {
-    const int c = ks[k];
-    I[k] = rig[3 * c];
-    J[k] = rig[3 * c + 1];
-    d2[k] = ct[3 * c];
-    ci[k] = ct[3 * c + 1];
-    cj[k] = ct[3 * c + 2];
+    I[k] = ga[2 * k];
+    J[k] = ga[2 * k + 1];
+    d2[k] = gc[3 * k];
+    ci[k] = gc[3 * k + 1];
+    cj[k] = gc[3 * k + 2];
 #pragma unroll
     for (int q = 0; q < 3; q++) r[k][q] = R[3 * I[k] + q] - R[3 * J[k] + q];
   }
@@ -361,11 +359,10 @@ __device__ __forceinline__ bool shake_group_n(double* X, const double* R, const 
   return false;
 }
 
-__device__ __forceinline__ bool shake_group(double* X, const double* R, const int* rig, const double* ct,
-                                            const int* ks, int n) {
-  if (n == 1) return shake_group_n<1>(X, R, rig, ct, ks);
-  if (n == 2) return shake_group_n<2>(X, R, rig, ct, ks);
-  return shake_group_n<3>(X, R, rig, ct, ks);
+__device__ __forceinline__ bool shake_group(double* X, const double* R, const int* ga, const double* gc, int n) {
+  if (n == 1) return shake_group_n<1>(X, R, ga, gc);
+  if (n == 2) return shake_group_n<2>(X, R, ga, gc);
+  return shake_group_n<3>(X, R, ga, gc);
 }
 
 __device__ __forceinline__ bool gas_rigid(const RepParams* P) {
@@ -491,14 +488,12 @@ __device__ __forceinline__ void core_shake(Ctx& x, const CoreCons& cc, GasWork g
         const int n = u < u3 ? 3 : u < u2 ? 2 : 1;
         const int g = in + (n < 3 ? n3 : 0) + (n < 2 ? n2 : 0);
         if (in < (n == 3 ? n3 : n == 2 ? n2 : n1) &&
-            !shake_group(x.c.x, xold, x.ib + P->o_ion_rigid, x.db + P->d_ion_cons,
-                         x.ib + P->o_ion_grp + x.ib[P->o_ion_gstart + g], n))
+            !shake_group(x.c.x, xold, x.ib + P->o_ion_gatoms + 6 * g, x.db + P->d_ion_gcons + 9 * g, n))
           atomicOr(&x.iscr[62], 1);
       } else {
         const int g = (u - u1) / per, m = 32 * (u - u1 - g * per) + lane, base = P->n_ion + m * P->a_v;
-        const int g0 = x.ib[P->o_vap_gstart + g];
-        if (m < cc.nv && !shake_group(x.c.x + 3 * base, xold + 3 * base, x.ib + P->o_vap_rigid, x.db + P->d_vap_cons,
-                                      x.ib + P->o_vap_grp + g0, x.ib[P->o_vap_gstart + g + 1] - g0)) {
+        if (m < cc.nv && !shake_group(x.c.x + 3 * base, xold + 3 * base, x.ib + P->o_vap_gatoms + 6 * g,
+                                      x.db + P->d_vap_gcons + 9 * g, x.ib[P->o_vap_gsize + g])) {
           x.c.chunk[9 * base] = 1;
           atomicOr(&x.iscr[62], 2);
         }

@@ -545,13 +545,18 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
     std::vector<int> col;
     P.n_ion_colors = color_rigid(d.ion.rigid, d.ion.n_rigid, col);
     P.o_ion_color = ipush(col.data(), (int)col.size());
-    {
-      std::vector<int> go, gs;
-      P.n_ion_groups = group_rigid(d.ion.rigid, d.ion.n_rigid, go, gs);
-      P.o_ion_grp = ipush(go.data(), (int)go.size());
-      P.o_ion_gstart = ipush(gs.data(), (int)gs.size());
-      for (int g = 0; g < P.n_ion_groups; g++) P.ion_groups_n[gs[g + 1] - gs[g] - 1]++;
-    }
+    /* the groups' atoms, six places each */
+    auto group_atoms = [&](const mdn_topology& t, const std::vector<int>& go, const std::vector<int>& gs) {
+      std::vector<int> v(6 * std::max<size_t>(gs.size(), 1), 0);
+      for (size_t g = 0; g + 1 < gs.size(); g++)
+        for (int k = gs[g]; k < gs[g + 1]; k++)
+          for (int e = 0; e < 2; e++) v[6 * g + 2 * (k - gs[g]) + e] = t.rigid[3 * go[k] + e];
+      return ipush(v.data(), (int)v.size());
+    };
+    std::vector<int> ion_go, ion_gs, vap_go, vap_gs;
+    P.n_ion_groups = group_rigid(d.ion.rigid, d.ion.n_rigid, ion_go, ion_gs);
+    P.o_ion_gatoms = group_atoms(d.ion, ion_go, ion_gs);
+    for (int g = 0; g < P.n_ion_groups; g++) P.ion_groups_n[ion_gs[g + 1] - ion_gs[g] - 1]++;
     /* AMBER exclusions: 1-2 (bonds and rigid pairs), 1-3, 1-4 (compute_AMBER.cpp:256-278) */
     P.excl_words = (d.ion.n_atoms + 31) / 32;
     {
@@ -583,15 +588,16 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
       P.o_vap_rigid = ipush(d.vapor.rigid, 3 * d.vapor.n_rigid);
       P.n_vap_colors = color_rigid(d.vapor.rigid, d.vapor.n_rigid, col);
       P.o_vap_color = ipush(col.data(), (int)col.size());
-      std::vector<int> go, gs;
-      P.n_vap_groups = group_rigid(d.vapor.rigid, d.vapor.n_rigid, go, gs);
-      P.o_vap_grp = ipush(go.data(), (int)go.size());
-      P.o_vap_gstart = ipush(gs.data(), (int)gs.size());
+      P.n_vap_groups = group_rigid(d.vapor.rigid, d.vapor.n_rigid, vap_go, vap_gs);
+      P.o_vap_gatoms = group_atoms(d.vapor, vap_go, vap_gs);
+      std::vector<int> size;
+      for (int g = 0; g < P.n_vap_groups; g++) size.push_back(vap_gs[g + 1] - vap_gs[g]);
+      P.o_vap_gsize = ipush(size.data(), (int)size.size());
     } else {
       int zero = 0;
       P.o_vap_type = ipush(&zero, 1);
       P.o_vap_bonds = P.o_vap_angles = P.o_vap_dih = P.o_vap_rigid = P.o_vap_color = P.o_vap_type;
-      P.o_vap_grp = P.o_vap_gstart = P.o_vap_type;
+      P.o_vap_gatoms = P.o_vap_gsize = P.o_vap_type;
       P.n_vap_groups = 0;
     }
     P.o_dih_multi = ipush(d.dihedral_multi, d.n_dihedral_types);
@@ -614,6 +620,21 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
       }
       return dpush(c.data(), (int)c.size());
     };
+    auto group_cons = [&](const mdn_topology& t, const std::vector<int>& go, const std::vector<int>& gs) {
+      std::vector<double> v(9 * std::max<size_t>(gs.size(), 1), 0.0);
+      for (size_t g = 0; g + 1 < gs.size(); g++)
+        for (int k = gs[g]; k < gs[g + 1]; k++) {
+          const int* rig = t.rigid + 3 * go[k];
+          const double dk = d.bond_coeff[2 * rig[2] + 1];
+          double* const c = &v[9 * g + 3 * (k - gs[g])];
+          c[0] = dk * dk;
+          c[1] = 1.0 / d.atom_mass[t.type[rig[0]]];
+          c[2] = 1.0 / d.atom_mass[t.type[rig[1]]];
+        }
+      return dpush(v.data(), (int)v.size());
+    };
+    P.d_ion_gcons = group_cons(d.ion, ion_go, ion_gs);
+    P.d_vap_gcons = group_cons(d.vapor, vap_go, vap_gs);
     P.d_ion_cons = cons_table(d.ion);
     P.d_gas_cons = cons_table(d.gas);
     P.d_vap_cons = d.n_vapor > 0 ? cons_table(d.vapor) : P.d_ion_cons;

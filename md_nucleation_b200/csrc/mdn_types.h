@@ -75,12 +75,13 @@ typedef struct RepParams {
   int o_dih_multi;
   /* SHAKE constraints in groups of coupled ones (sharing atoms), at most 3
    * per group, solved together (shake_group); 0 groups = colour sweeps */
-  int n_ion_groups, o_ion_grp, o_ion_gstart;
+  int n_ion_groups, o_ion_gatoms; /* per group 6 atom indices: i, j of each constraint */
   int ion_groups_n[3];           /* ion groups of 1, 2 and 3 constraints; stored largest first */
-  int n_vap_groups, o_vap_grp, o_vap_gstart;
+  int n_vap_groups, o_vap_gatoms, o_vap_gsize;
   /* offsets inside the double blob */
   int d_bond, d_angle, d_dih, d_ljA, d_ljB, d_ljA12, d_ljB6, d_mass, d_c2;
   int d_ion_q, d_gas_x, d_gas_q, d_vap_x, d_vap_q;
+  int d_ion_gcons, d_vap_gcons;  /* per group 9: d^2, 1/m_i, 1/m_j of each constraint */
   int d_ion_cons, d_gas_cons, d_vap_cons; /* per SHAKE constraint: d^2, 1/m_i, 1/m_j */
   int ggl_cap;                   /* gas-gas list entries (both directions), 0 without gg */
   /* run parameters */
