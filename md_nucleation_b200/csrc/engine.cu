@@ -162,7 +162,8 @@ struct mdn_handle {
   std::vector<std::vector<int>> type_names;  /* unused placeholder */
   int nc_cap = 0, nt_cap = 0, excl_cap = 0;
   size_t smem = 0;
-  /* device pools */
+  /* device pools, all cut from one allocation */
+  char* arena = nullptr;
   RepParams* dP = nullptr;
   RepDyn* dD = nullptr;
   int* d_iblob = nullptr;
@@ -192,7 +193,8 @@ struct mdn_handle {
   int* status = nullptr;
   int auto_cluster = 1;  /* cluster size when mdn_options.cluster_size is 0 */
   JobQueue queue;
-  int* h_status = nullptr; /* page-locked copy of status (check_status) */
+  std::vector<int> h_status; /* copy of status (check_status) */
+  char* stage = nullptr;     /* kStage bytes (Fetch) */
   /* split step launch: the split_n largest replicas in a second, concurrent
    * launch with clusters of split_cluster CTAs (0: one launch) */
   int split_n = 0, split_cluster = 0;
@@ -223,16 +225,9 @@ struct mdn_handle {
 namespace {
 
 void free_all(mdn_handle* h) {
-  void* ptrs[] = {h->dP, h->dD, h->d_iblob, h->d_dblob, h->ion_x, h->ion_v, h->ion_f, h->mol_x, h->mol_v,
-                  h->region, h->slot, h->entries, h->slab_x, h->slab_v, h->slab_f, h->slab_mol, h->vslab_x, h->vslab_v,
-                  h->vslab_f, h->vslab_w, h->vslab_mol, h->near_rec, h->near_item, h->near_cnt, h->near_s, h->far_list, h->near_gi, h->near_gv, h->gil_n,
-                  h->gvl_n, h->gil, h->gvl, h->energy, h->events, h->n_events, h->status, h->queue.d_order,
-                  h->queue.d_counter, h->snap_off, h->snap_type, h->snap_x, h->snap_v, h->d_ctl_mode,
-                  h->d_ctl_T, h->d_prof, h->queue2.d_order, h->queue2.d_counter, h->ggl_start, h->ggl_n, h->ggl,
-                  h->slab_fgg, h->slab_ins};
+  void* ptrs[] = {h->arena, h->snap_off, h->snap_type, h->snap_x, h->snap_v, h->d_prof};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  if (h->h_status) cudaFreeHost(h->h_status);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -382,6 +377,41 @@ long long launch(mdn_handle* h, int mode, long long n_steps, int energy_mode, un
   }
   return 1;
 }
+
+/* Device-to-host copies that are waited for together.  A copy into the
+ * caller's memory blocks (9 us each, however small, 16 of them in a state
+ * download); these are put side by side on the device first and come over in
+ * one copy.  What does not fit the staging is copied directly. */
+constexpr size_t kStage = 1 << 20;
+struct Fetch {
+  mdn_handle* h;
+  size_t used = 0;
+  struct Item {
+    void* to;
+    size_t at, bytes;
+  };
+  std::vector<Item> items;
+  explicit Fetch(mdn_handle* h_) : h(h_) {}
+  cudaError_t add(void* to, const void* from, size_t bytes) {
+    if (bytes == 0) return cudaSuccess;
+    if (used + bytes > kStage) return cudaMemcpy(to, from, bytes, cudaMemcpyDeviceToHost);
+    items.push_back({to, used, bytes});
+    cudaError_t e = cudaMemcpyAsync(h->stage + used, from, bytes, cudaMemcpyDeviceToDevice, h->stream);
+    used = (used + bytes + 15) & ~(size_t)15;
+    return e;
+  }
+  cudaError_t wait() {
+    std::vector<char> host(used);
+    cudaError_t e = used > 0 ? cudaMemcpyAsync(host.data(), h->stage, used, cudaMemcpyDeviceToHost, h->stream)
+                             : cudaSuccess;
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess)
+      for (const Item& i : items) memcpy(i.to, host.data() + i.at, i.bytes);
+    items.clear();
+    used = 0;
+    return e;
+  }
+};
 
 int sync_check(mdn_handle* h) {
   cudaError_t e = cudaStreamSynchronize(h->stream);
@@ -816,65 +846,82 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
     h->auto_cluster = c;
   }
 
-#define ALLOC(ptr, count)                                                          \
-  do {                                                                             \
-    cudaError_t e_ = cudaMalloc((void**)&(ptr), sizeof(*(ptr)) * std::max<size_t>(1, (count))); \
-    if (e_ != cudaSuccess) {                                                       \
-      free_all(h);                                                                 \
-      delete h;                                                                    \
-      return fail(MDN_ERR_CUDA, "cudaMalloc(%s): %s", #ptr, cudaGetErrorString(e_)); \
-    }                                                                              \
-  } while (0)
-  ALLOC(h->dP, R);
-  ALLOC(h->dD, R);
-  ALLOC(h->d_iblob, iblob.size());
-  ALLOC(h->d_dblob, dblob.size());
-  ALLOC(h->ion_x, 3 * ion_tot);
-  ALLOC(h->ion_v, 3 * ion_tot);
-  ALLOC(h->ion_f, 3 * ion_tot);
-  ALLOC(h->mol_x, 3 * mol_tot);
-  ALLOC(h->mol_v, 3 * mol_tot);
-  ALLOC(h->region, mol_tot);
-  ALLOC(h->slot, mol_tot);
-  ALLOC(h->entries, mol_tot);
-  ALLOC(h->slab_x, 3 * slab_atoms);
-  ALLOC(h->slab_v, 3 * slab_atoms);
-  ALLOC(h->slab_f, 3 * slab_atoms);
-  ALLOC(h->slab_mol, slab_mols);
-  ALLOC(h->vslab_x, 3 * vslab_atoms);
-  ALLOC(h->vslab_v, 3 * vslab_atoms);
-  ALLOC(h->vslab_f, 3 * vslab_atoms);
-  ALLOC(h->vslab_w, vslab_atoms);
-  ALLOC(h->vslab_mol, vslab_mols);
-  ALLOC(h->near_rec, near_tot);
-  ALLOC(h->near_item, nit_tot);
-  ALLOC(h->near_cnt, 24 * (size_t)R);
-  ALLOC(h->far_list, near_tot);
-  ALLOC(h->near_s, ns_tot);
-  ALLOC(h->near_gi, slab_mols);
-  ALLOC(h->near_gv, slab_mols);
-  ALLOC(h->gil_n, slab_mols);
-  ALLOC(h->gvl_n, slab_mols);
-  ALLOC(h->gil, gil_tot);
-  ALLOC(h->gvl, gvl_tot);
+  /* one allocation for all pools: some forty cudaMalloc and cudaFree calls
+   * were most of the time to create and destroy a small handle */
+  struct Pool {
+    char** at;
+    size_t bytes;
+  };
+  std::vector<Pool> pools;
+  auto pool = [&](auto*& p, size_t count) {
+    pools.push_back({(char**)(void*)&p, (sizeof(*p) * std::max<size_t>(1, count) + 255) & ~(size_t)255});
+  };
+  pool(h->dP, R);
+  pool(h->dD, R);
+  pool(h->d_iblob, iblob.size());
+  pool(h->d_dblob, dblob.size());
+  pool(h->ion_x, 3 * ion_tot);
+  pool(h->ion_v, 3 * ion_tot);
+  pool(h->ion_f, 3 * ion_tot);
+  pool(h->mol_x, 3 * mol_tot);
+  pool(h->mol_v, 3 * mol_tot);
+  pool(h->region, mol_tot);
+  pool(h->slot, mol_tot);
+  pool(h->entries, mol_tot);
+  pool(h->slab_x, 3 * slab_atoms);
+  pool(h->slab_v, 3 * slab_atoms);
+  pool(h->slab_f, 3 * slab_atoms);
+  pool(h->slab_mol, slab_mols);
+  pool(h->vslab_x, 3 * vslab_atoms);
+  pool(h->vslab_v, 3 * vslab_atoms);
+  pool(h->vslab_f, 3 * vslab_atoms);
+  pool(h->vslab_w, vslab_atoms);
+  pool(h->vslab_mol, vslab_mols);
+  pool(h->near_rec, near_tot);
+  pool(h->near_item, nit_tot);
+  pool(h->near_cnt, 24 * (size_t)R);
+  pool(h->far_list, near_tot);
+  pool(h->near_s, ns_tot);
+  pool(h->near_gi, slab_mols);
+  pool(h->near_gv, slab_mols);
+  pool(h->gil_n, slab_mols);
+  pool(h->gvl_n, slab_mols);
+  pool(h->gil, gil_tot);
+  pool(h->gvl, gvl_tot);
   if (ggl_tot > 0) {
-    ALLOC(h->ggl_start, slab_mols);
-    ALLOC(h->ggl_n, slab_mols);
-    ALLOC(h->ggl, ggl_tot);
-    ALLOC(h->slab_fgg, 3 * slab_atoms);
-    ALLOC(h->slab_ins, slab_mols);
+    pool(h->ggl_start, slab_mols);
+    pool(h->ggl_n, slab_mols);
+    pool(h->ggl, ggl_tot);
+    pool(h->slab_fgg, 3 * slab_atoms);
+    pool(h->slab_ins, slab_mols);
   }
-  ALLOC(h->energy, 8 * (size_t)R);
-  ALLOC(h->events, (size_t)h->ev_cap);
-  ALLOC(h->n_events, 1);
-  ALLOC(h->status, R);
-  ALLOC(h->queue.d_order, R);
-  ALLOC(h->queue.d_counter, 1);
-  ALLOC(h->queue2.d_order, R);
-  ALLOC(h->queue2.d_counter, 1);
-  ALLOC(h->d_ctl_mode, R);
-  ALLOC(h->d_ctl_T, R);
-#undef ALLOC
+  pool(h->energy, 8 * (size_t)R);
+  pool(h->events, (size_t)h->ev_cap);
+  pool(h->n_events, 1);
+  pool(h->status, R);
+  pool(h->stage, kStage);
+  pool(h->queue.d_order, R);
+  pool(h->queue.d_counter, 1);
+  pool(h->queue2.d_order, R);
+  pool(h->queue2.d_counter, 1);
+  pool(h->d_ctl_mode, R);
+  pool(h->d_ctl_T, R);
+  {
+    size_t bytes = 0;
+    for (const Pool& q : pools) bytes += q.bytes;
+    cudaError_t e = cudaMalloc((void**)&h->arena, bytes);
+    if (e != cudaSuccess) {
+      h->arena = nullptr;
+      free_all(h);
+      delete h;
+      return fail(MDN_ERR_CUDA, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
+    }
+    char* at = h->arena;
+    for (const Pool& q : pools) {
+      *q.at = at;
+      at += q.bytes;
+    }
+  }
   int rc = MDN_OK;
   auto ck = [&](cudaError_t e, const char* what) {
     if (e != cudaSuccess && rc == MDN_OK) rc = fail(MDN_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
@@ -905,7 +952,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
   ck(cudaMemset(h->status, 0, sizeof(int) * R), "status");
   ck(cudaMemset(h->queue.d_counter, 0, sizeof(unsigned)), "queue");
   ck(cudaMemset(h->queue2.d_counter, 0, sizeof(unsigned)), "queue");
-  ck(cudaHostAlloc((void**)&h->h_status, sizeof(int) * R, cudaHostAllocDefault), "status");
+  h->h_status.assign(R, 0);
   ck(cudaMemset(h->near_cnt, 0, sizeof(int) * 24 * R), "near_cnt");
   ck(cudaMemset(h->near_gi, 0xff, sizeof(int) * slab_mols), "near_gi");
   if (h->slab_ins) ck(cudaMemset(h->slab_ins, 0xff, sizeof(int) * slab_mols), "slab_ins");
@@ -972,10 +1019,11 @@ void mdn_destroy(mdn_handle* h) {
   delete h;
 }
 
-/* Waits for the stream and looks at the replicas' status words, which come
- * with it: one wait instead of a wait and a blocking copy. */
+/* The replicas' status words, behind what the stream does: one blocking call
+ * instead of a wait and a blocking copy (page-locked memory for them would
+ * cost milliseconds at create). */
 static int check_status(mdn_handle* h) {
-  cudaError_t e = cudaMemcpyAsync(h->h_status, h->status, sizeof(int) * h->R, cudaMemcpyDeviceToHost, h->stream);
+  cudaError_t e = cudaMemcpyAsync(h->h_status.data(), h->status, sizeof(int) * h->R, cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return fail(MDN_ERR_CUDA, "kernel failed: %s", cudaGetErrorString(e));
   for (int r = 0; r < h->R; r++)
@@ -1149,26 +1197,41 @@ int mdn_download_state(mdn_handle* h, int r, mdn_state* s) {
   cudaSetDevice(h->dev);
   const RepParams& P = h->P[r];
   RepDyn D;
-  CK(cudaMemcpy(&D, h->dD + r, sizeof D, cudaMemcpyDeviceToHost));
+  Fetch get(h);
+  CK(get.add(&D, h->dD + r, sizeof D));
   const size_t ni = P.n_ion, nm = 1 + P.n_gas + P.n_vap;
-  if (s->ion_x) CK(cudaMemcpy(s->ion_x, h->ion_x + 3 * P.ion_off, 24 * ni, cudaMemcpyDeviceToHost));
-  if (s->ion_v) CK(cudaMemcpy(s->ion_v, h->ion_v + 3 * P.ion_off, 24 * ni, cudaMemcpyDeviceToHost));
-  if (s->ion_f) CK(cudaMemcpy(s->ion_f, h->ion_f + 3 * P.ion_off, 24 * ni, cudaMemcpyDeviceToHost));
-  if (s->mol_x) CK(cudaMemcpy(s->mol_x, h->mol_x + 3 * P.mol_off, 24 * nm, cudaMemcpyDeviceToHost));
-  if (s->mol_v) CK(cudaMemcpy(s->mol_v, h->mol_v + 3 * P.mol_off, 24 * nm, cudaMemcpyDeviceToHost));
-  if (s->region) CK(cudaMemcpy(s->region, h->region + P.mol_off, nm, cudaMemcpyDeviceToHost));
+  if (s->ion_x) CK(get.add(s->ion_x, h->ion_x + 3 * P.ion_off, 24 * ni));
+  if (s->ion_v) CK(get.add(s->ion_v, h->ion_v + 3 * P.ion_off, 24 * ni));
+  if (s->ion_f) CK(get.add(s->ion_f, h->ion_f + 3 * P.ion_off, 24 * ni));
+  if (s->mol_x) CK(get.add(s->mol_x, h->mol_x + 3 * P.mol_off, 24 * nm));
+  if (s->mol_v) CK(get.add(s->mol_v, h->mol_v + 3 * P.mol_off, 24 * nm));
+  if (s->region) CK(get.add(s->region, h->region + P.mol_off, nm));
+  CK(get.wait());
   /* gas slab -> rows of the in-domain molecules */
+  const int G = D.n_gas_in, ag = P.a_g, par = D.parity;
+  std::vector<int> mol(G);
+  std::vector<double> x(3 * (size_t)G * ag), v(x.size()), f(x.size());
+  const int V = P.n_vap > 0 ? D.n_vap_in : 0, av = P.a_v;
+  std::vector<int> vmol(V);
+  std::vector<double> vx(3 * (size_t)V * av), vv(vx.size()), vf(vx.size());
+  std::vector<float> vw((size_t)V * av);
+  if (G > 0) {
+    const size_t a0 = (size_t)P.slab_off + (size_t)par * P.slab_cap * ag;
+    CK(get.add(mol.data(), h->slab_mol + P.slab_moff + (size_t)par * P.slab_cap, sizeof(int) * G));
+    CK(get.add(x.data(), h->slab_x + 3 * a0, 8 * x.size()));
+    CK(get.add(v.data(), h->slab_v + 3 * a0, 8 * v.size()));
+    CK(get.add(f.data(), h->slab_f + 3 * a0, 8 * f.size()));
+  }
+  if (V > 0) {
+    const size_t a0 = (size_t)P.vslab_off + (size_t)par * P.vcap * av;
+    CK(get.add(vmol.data(), h->vslab_mol + P.vslab_moff + (size_t)par * P.vcap, sizeof(int) * V));
+    CK(get.add(vx.data(), h->vslab_x + 3 * a0, 8 * vx.size()));
+    CK(get.add(vv.data(), h->vslab_v + 3 * a0, 8 * vv.size()));
+    CK(get.add(vf.data(), h->vslab_f + 3 * a0, 8 * vf.size()));
+    CK(get.add(vw.data(), h->vslab_w + a0, 4 * vw.size()));
+  }
+  CK(get.wait());
   {
-    const int G = D.n_gas_in, ag = P.a_g, par = D.parity;
-    std::vector<int> mol(G);
-    std::vector<double> x(3 * (size_t)G * ag), v(x.size()), f(x.size());
-    if (G > 0) {
-      const size_t a0 = (size_t)P.slab_off + (size_t)par * P.slab_cap * ag;
-      CK(cudaMemcpy(mol.data(), h->slab_mol + P.slab_moff + (size_t)par * P.slab_cap, sizeof(int) * G, cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(x.data(), h->slab_x + 3 * a0, 8 * x.size(), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(v.data(), h->slab_v + 3 * a0, 8 * v.size(), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(f.data(), h->slab_f + 3 * a0, 8 * f.size(), cudaMemcpyDeviceToHost));
-    }
     for (int s_ = 0; s_ < G; s_++) {
       size_t dst = 3 * (size_t)mol[s_] * ag, src = 3 * (size_t)s_ * ag;
       for (int q = 0; q < 3 * ag; q++) {
@@ -1178,28 +1241,16 @@ int mdn_download_state(mdn_handle* h, int r, mdn_state* s) {
       }
     }
   }
-  if (P.n_vap > 0) {
-    const int V = D.n_vap_in, av = P.a_v, par = D.parity;
-    std::vector<int> mol(V);
-    std::vector<double> x(3 * (size_t)V * av), v(x.size()), f(x.size());
-    std::vector<float> w((size_t)V * av);
-    if (V > 0) {
-      const size_t a0 = (size_t)P.vslab_off + (size_t)par * P.vcap * av;
-      CK(cudaMemcpy(mol.data(), h->vslab_mol + P.vslab_moff + (size_t)par * P.vcap, sizeof(int) * V, cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(x.data(), h->vslab_x + 3 * a0, 8 * x.size(), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(v.data(), h->vslab_v + 3 * a0, 8 * v.size(), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(f.data(), h->vslab_f + 3 * a0, 8 * f.size(), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(w.data(), h->vslab_w + a0, 4 * w.size(), cudaMemcpyDeviceToHost));
-    }
+  {
     for (int s_ = 0; s_ < V; s_++) {
-      size_t dst = 3 * (size_t)mol[s_] * av, src = 3 * (size_t)s_ * av;
+      size_t dst = 3 * (size_t)vmol[s_] * av, src = 3 * (size_t)s_ * av;
       for (int q = 0; q < 3 * av; q++) {
-        if (s->vap_ax) s->vap_ax[dst + q] = x[src + q];
-        if (s->vap_av) s->vap_av[dst + q] = v[src + q];
-        if (s->vap_af) s->vap_af[dst + q] = f[src + q];
+        if (s->vap_ax) s->vap_ax[dst + q] = vx[src + q];
+        if (s->vap_av) s->vap_av[dst + q] = vv[src + q];
+        if (s->vap_af) s->vap_af[dst + q] = vf[src + q];
       }
       if (s->vap_w)
-        for (int at = 0; at < av; at++) s->vap_w[(size_t)mol[s_] * av + at] = w[(size_t)s_ * av + at];
+        for (int at = 0; at < av; at++) s->vap_w[(size_t)vmol[s_] * av + at] = vw[(size_t)s_ * av + at];
     }
   }
   s->loop_pair = D.loop_pair;

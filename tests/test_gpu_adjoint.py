@@ -193,3 +193,22 @@ def test_adjoint_matches_the_cpu_adjoint(eng, oracle_libs, shake):
     floor = 1e-4 * np.abs(gc).max()
     for k in range(len(gc)):
         assert abs(grad[k] - gc[k]) <= tol * max(abs(gc[k]), floor), f"parameter {k}: {grad[k]} vs {gc[k]}"
+
+
+def test_adjoint_with_large_constraint_groups(eng, oracle_libs):
+    """Every bond of the methanol a constraint: five that share atoms, which
+    go through the colour sweeps instead of the per-group solution.  Against
+    the FP64 CPU adjoint, the bar of the SHAKE case above."""
+    from md_nucleation_b200.gradients import parameters
+    spec = system(True)
+    v = spec.vapor
+    v.rigid = np.concatenate([v.rigid, v.bonds]).astype(np.int32)
+    v.bonds = np.zeros((0, 3), np.int32)
+    theta0, rows = parameters(spec)
+    e = eng.Engine([spec], force_mode=1)
+    J, grad, ms = e.adjoint(**WINDOW)
+    o = oracle_libs.OracleReplica(spec)
+    Jo, go = o.adjoint(WINDOW["n_steps"], theta0.numpy(), rows, WINDOW["count_radius"], WINDOW["count_width"],
+                       WINDOW["w_energy"], WINDOW["w_count"])
+    assert abs(J - Jo) <= 1e-8 * max(abs(Jo), 1.0)
+    check(grad, go, 1e-5)

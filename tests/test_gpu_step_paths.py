@@ -60,3 +60,51 @@ def test_near_records_do_not_depend_on_the_launch(eng, gas, chain, n_gas, force_
     a = _run(eng, spec, [(1, 512)] * 4, force_mode=force_mode)
     b = _run(eng, spec, [(8, 512), (1, 64), (3, 96), (2, 256)], force_mode=force_mode)
     assert np.array_equal(a, b)
+
+
+# energies of every step and the thermostats, whose kicks and factors each
+# thread applies to its own components: one CTA, two that exchange their sums,
+# more that take slices of them
+@pytest.mark.parametrize("mode", [abi.NVT_SCALE, abi.NVT_NH])
+def test_thermostats_and_energies_do_not_depend_on_the_launch(eng, mode):
+    spec = g.small_system(seed=33, gas="N2", vapor="water", ion="chain", chain_atoms=40, n_gas=2500, n_vap=30,
+                          box=245.0, shake_h=True)
+    out = []
+    for c, t in ((1, 512), (2, 512), (5, 128), (8, 256)):
+        e = eng.Engine([spec], quirks=CHECKED)
+        e.set_nvt(mode, 310.0)
+        e.set_launch(c, t)
+        for _ in range(3):
+            e.step(9, 2)
+        s = e.state(0)
+        out.append(np.concatenate([a.ravel() for a in (s.ion_x, s.ion_v, s.ion_f, s.gas_ax, s.gas_av, s.vap_ax,
+                                                       s.vap_av, e.energies())]))
+    assert all(np.array_equal(out[0], o) for o in out[1:])
+
+
+def all_rigid(spec):
+    """Every bond of the vapor a constraint: five that share atoms, more than
+    the kernels solve as a group."""
+    v = spec.vapor
+    v.rigid = np.concatenate([v.rigid, v.bonds]).astype(np.int32)
+    v.bonds = np.zeros((0, 3), np.int32)
+    return spec
+
+
+def test_large_constraint_groups_are_swept(eng, oracle_libs):
+    spec = all_rigid(g.small_system(seed=17, gas="He", vapor="methanol", ion="nacl", n_gas=800, n_vap=20, box=242.0,
+                                    shake_h=True))
+    o = oracle_libs.OracleReplica(spec)
+    out = []
+    for c, t in ((1, 512), (8, 128)):
+        e = eng.Engine([spec])
+        e.set_launch(c, t)
+        e.step(10)
+        out.append(e.state(0))
+        assert not e.status().any()
+    assert np.array_equal(out[0].vap_ax, out[1].vap_ax)
+    o.step(10)
+    inside = out[0].region[1 + spec.n_gas:].astype(bool)
+    assert inside.sum() >= 3
+    # the bar of the short trajectories in test_gpu_parity.py
+    assert np.abs(out[0].vap_ax[inside] - o.get_state().vap_ax[inside]).max() <= 1e-6
