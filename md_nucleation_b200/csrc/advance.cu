@@ -714,6 +714,42 @@ __device__ __forceinline__ float rsqrt_ftz(float r2) {
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(r2));
   return r;
 }
+
+/* Two FP32 values in one register pair, and the packed operations on them:
+ * one instruction for both, each rounded as the single operation is. */
+struct Pair2 {
+  unsigned long long b;
+};
+__device__ __forceinline__ Pair2 pack2(float lo, float hi) {
+  Pair2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.b) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(Pair2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.b));
+  return r;
+}
+__device__ __forceinline__ Pair2 mul2(Pair2 a, Pair2 b) {
+  Pair2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(a.b), "l"(b.b));
+  return r;
+}
+__device__ __forceinline__ Pair2 fma2(Pair2 a, Pair2 b, Pair2 c) {
+  Pair2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.b) : "l"(a.b), "l"(b.b), "l"(c.b));
+  return r;
+}
+/* a + b in single additions: a packed one of a product was made one operation
+ * with it, and rounded once, by the assembler */
+__device__ __forceinline__ Pair2 add2(Pair2 a, Pair2 b) {
+  const float2 u = unpack2(a), v = unpack2(b);
+  return pack2(__fadd_rn(u.x, v.x), __fadd_rn(u.y, v.y));
+}
+__device__ __forceinline__ Pair2 rsqrt2(Pair2 a) {
+  const float2 u = unpack2(a);
+  return pack2(rsqrt_ftz(u.x), rsqrt_ftz(u.y));
+}
 __device__ __forceinline__ float lj_coul(float r2, float A, float B, float qq, bool coul, float* e) {
   float rinv = rsqrt_ftz(r2);
   float r2inv = rinv * rinv;
@@ -943,7 +979,7 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
     constexpr bool kBorn = decltype(with_born)::value;
     const int j = min(j0 + ((lane + s) & 31), nc - 1);
     const AtomTag gj = x.c.tag[j];
-    double qj = 0.0, wj = 1.0;
+    [[maybe_unused]] double qj = 0.0, wj = 1.0;
     if constexpr (FP64 || E) qj = __shfl_sync(FULL, q_own, (lane + s) & 31);
     if constexpr (FP64) wj = __shfl_sync(FULL, w_own, (lane + s) & 31);
     const int tt = rowi + tag_type(gj.k);
@@ -1008,6 +1044,8 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
     const float2* const row = x.c.lj + rowi;
     for (int s0 = 0; s0 < s1; s0 += kSteps) {
       Acc fx[kSteps], fy[kSteps], fz[kSteps];
+      float A[kSteps], B[kSteps], qq[kSteps], w[kSteps];
+      bool tk[kSteps];
 #pragma unroll
       for (int u = 0; u < kSteps; u++) {
         const int jl = (lane + s0 + u) & 31, j = j0 + jl; /* past the core: type 0, not taken */
@@ -1033,14 +1071,23 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
         } else {
           const float4 pj = x.c.pos[j];
           const float2 AB = row[tag_type(gj.k)];
-          const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-          float ee;
-          const float f = lj_coul(r2, AB.x, AB.y, qi * pj.w, true, &ee) * (gi.w * gj.w);
-          const float fp = take ? f : 0.0f;
-          fx[u] = fp * dx;
-          fy[u] = fp * dy;
-          fz[u] = fp * dz;
+          fx[u] = pi.x - pj.x;
+          fy[u] = pi.y - pj.y;
+          fz[u] = pi.z - pj.z;
+          A[u] = AB.x;
+          B[u] = AB.y;
+          qq[u] = qi * pj.w;
+          w[u] = gi.w * gj.w;
+          tk[u] = take;
+          if constexpr (kGG) {
+            const float r2 = fmaf(fx[u], fx[u], fmaf(fy[u], fy[u], fz[u] * fz[u]));
+            float ee;
+            const float f = lj_coul(r2, A[u], B[u], qq[u], true, &ee) * w[u];
+            const float fp = take ? f : 0.0f;
+            fx[u] = fp * fx[u];
+            fy[u] = fp * fy[u];
+            fz[u] = fp * fz[u];
+          }
         }
         if constexpr (E) {
           const double ed = lj_coul_energy(R2d, x.db[P->d_ljA12 + tt], x.db[P->d_ljB6 + tt], qj);
@@ -1051,6 +1098,26 @@ __device__ __forceinline__ void core_tile(Ctx& x, int t, int nblk) {
           e_vv += !iion && !jion ? e : 0;
         }
       }
+      /* lj_coul, two steps in a register pair: fewer instructions per
+       * pair (100-atom chain 1418 -> 1371 us per 100 steps, 500-atom ion 2568
+       * -> 2533); not beside the gas-gas term, whose kernel has no registers
+       * left for it (1540 -> 1549 per 50 steps) */
+      if constexpr (!FP64 && !kGG)
+#pragma unroll
+        for (int u = 0; u < kSteps; u += 2) {
+          const Pair2 dx = pack2(fx[u], fx[u + 1]), dy = pack2(fy[u], fy[u + 1]), dz = pack2(fz[u], fz[u + 1]);
+          const Pair2 rinv = rsqrt2(fma2(dx, dx, fma2(dy, dy, mul2(dz, dz))));
+          const Pair2 r2inv = mul2(rinv, rinv), r6inv = mul2(mul2(r2inv, r2inv), r2inv);
+          const float2 r6 = unpack2(r6inv);
+          const Pair2 t = pack2(fmaf(A[u], r6.x, -B[u]), fmaf(A[u + 1], r6.y, -B[u + 1]));
+          const Pair2 fc = mul2(pack2(qq[u], qq[u + 1]), rinv);
+          const float2 f = unpack2(mul2(mul2(add2(mul2(r6inv, t), fc), r2inv), pack2(w[u], w[u + 1])));
+          const Pair2 fp = pack2(tk[u] ? f.x : 0.0f, tk[u + 1] ? f.y : 0.0f);
+          const float2 gx = unpack2(mul2(fp, dx)), gy = unpack2(mul2(fp, dy)), gz = unpack2(mul2(fp, dz));
+          fx[u] = gx.x; fx[u + 1] = gx.y;
+          fy[u] = gy.x; fy[u + 1] = gy.y;
+          fz[u] = gz.x; fz[u + 1] = gz.y;
+        }
       on >>= kSteps;
 #pragma unroll
       for (int u = 0; u < kSteps; u++) {
