@@ -449,10 +449,12 @@ int  mdn_get_split(mdn_handle* h, int* n_largest, int* cluster_size);
 /* Per-replica SM-cycle accounting of the step kernel: enable = 1 starts
  * accumulating (from zero), 0 stops.  out: [8*n_replicas] cycles per phase:
  * total, core integration, gas integration, rebuild, near gas molecules,
- * core bonded terms, core pair terms, core force sums and kick.  The gas
- * molecules are integrated beside the core's constraints, so their time is
- * counted under core integration; the gas slot holds the step's list
- * bookkeeping only. */
+ * core bonded terms, core pair terms, core force sums and kick.  The near
+ * gas molecules are integrated beside the core's constraints or in the force
+ * pass and counted there; the gas slot holds the far molecules' steps, made
+ * many at once.  While accounting is on, the near, bonded and pair items of a
+ * step run one kind after another (not as one queue), so that each can be
+ * timed; the results are the same. */
 int  mdn_profile(mdn_handle* h, int enable, long long* out);
 
 #ifdef __cplusplus

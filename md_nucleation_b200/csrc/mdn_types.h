@@ -44,7 +44,7 @@
 /* phases of the per-replica cycle accounting (mdn_profile) */
 #define MDN_PROF_TOTAL 0
 #define MDN_PROF_CORE_INT 1   /* kick, thermostat, drift, SHAKE, centre, weights */
-#define MDN_PROF_GAS_INT 2    /* gas kick/drift (+ far-molecule forces)          */
+#define MDN_PROF_GAS_INT 2    /* far gas molecules, many steps at once            */
 #define MDN_PROF_REBUILD 3    /* make_pair                                       */
 #define MDN_PROF_NEAR 4       /* near gas molecules: gas-ion, gas-vapor          */
 #define MDN_PROF_BONDED 5     /* core bonded terms                               */
