@@ -162,8 +162,9 @@ struct mdn_handle {
   std::vector<std::vector<int>> type_names;  /* unused placeholder */
   int nc_cap = 0, nt_cap = 0, excl_cap = 0;
   size_t smem = 0;
-  /* device pools, all cut from one allocation */
+  /* device pools, cut from two allocations: the large ones, the small ones */
   char* arena = nullptr;
+  char* arena_small = nullptr;
   RepParams* dP = nullptr;
   RepDyn* dD = nullptr;
   int* d_iblob = nullptr;
@@ -225,7 +226,7 @@ struct mdn_handle {
 namespace {
 
 void free_all(mdn_handle* h) {
-  void* ptrs[] = {h->arena, h->snap_off, h->snap_type, h->snap_x, h->snap_v, h->d_prof};
+  void* ptrs[] = {h->arena, h->arena_small, h->snap_off, h->snap_type, h->snap_x, h->snap_v, h->d_prof};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->ev0) cudaEventDestroy(h->ev0);
@@ -846,8 +847,11 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
     h->auto_cluster = c;
   }
 
-  /* one allocation for all pools: some forty cudaMalloc and cudaFree calls
-   * were most of the time to create and destroy a small handle */
+  /* two allocations for all pools: some forty cudaMalloc and cudaFree calls
+   * were most of the time to create and destroy a small handle.  The small
+   * pools have an allocation of their own: CUDA serves small allocations from
+   * a block that it keeps while one of them lives, and mdn_place, which makes
+   * and frees one, took 1.8 ms beside a handle without it, 1.2 with it */
   struct Pool {
     char** at;
     size_t bytes;
@@ -907,19 +911,25 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
   pool(h->d_ctl_mode, R);
   pool(h->d_ctl_T, R);
   {
-    size_t bytes = 0;
-    for (const Pool& q : pools) bytes += q.bytes;
-    cudaError_t e = cudaMalloc((void**)&h->arena, bytes);
-    if (e != cudaSuccess) {
-      h->arena = nullptr;
-      free_all(h);
-      delete h;
-      return fail(MDN_ERR_CUDA, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
-    }
-    char* at = h->arena;
-    for (const Pool& q : pools) {
-      *q.at = at;
-      at += q.bytes;
+    auto small = [](const Pool& q) { return q.bytes <= 16384; };
+    size_t bytes[2] = {0, 0};
+    for (const Pool& q : pools) bytes[small(q)] += q.bytes;
+    char** const to[2] = {&h->arena, &h->arena_small};
+    for (int k = 0; k < 2; k++) {
+      if (bytes[k] == 0) continue;
+      cudaError_t e = cudaMalloc((void**)to[k], bytes[k]);
+      if (e != cudaSuccess) {
+        *to[k] = nullptr;
+        free_all(h);
+        delete h;
+        return fail(MDN_ERR_CUDA, "cudaMalloc(%zu bytes): %s", bytes[k], cudaGetErrorString(e));
+      }
+      char* at = *to[k];
+      for (const Pool& q : pools)
+        if (small(q) == (k == 1)) {
+          *q.at = at;
+          at += q.bytes;
+        }
     }
   }
   int rc = MDN_OK;
