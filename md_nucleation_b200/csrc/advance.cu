@@ -169,8 +169,13 @@ __device__ __forceinline__ void load_vapor(Ctx& x) {
     x.c.tag[i].w = a->vslab_w[g];
     x.c.tag[i].k = (unsigned)x.ib[P->o_vap_type + at] | ((unsigned)(s + 1) << 8);
   }
-  /* core_tile reads whole blocks of 32 */
-  for (int i = x.n_core + threadIdx.x; i < ((x.n_core + 31) & ~31); i += blockDim.x) x.c.tag[i].k = 0;
+  /* core_tile reads whole blocks of 32 and multiplies what it does not count
+   * by 0: the places past the core hold finite positions, not what an earlier
+   * replica of this CTA left there */
+  for (int i = x.n_core + threadIdx.x; i < ((x.n_core + 31) & ~31); i += blockDim.x) {
+    x.c.tag[i].k = 0;
+    x.c.pos[i] = make_float4(0, 0, 0, 0);
+  }
 }
 
 __device__ __forceinline__ void store_core(Ctx& x) {
@@ -3068,7 +3073,6 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
   }
   /* the chunk sums start at zero and every core_reduce_kick leaves them so */
   for (int q = threadIdx.x; q < 9 * a.nc_cap; q += blockDim.x) x.c.chunk[q] = 0;
-  for (int q = threadIdx.x; q < ((a.nc_cap + 31) & ~31); q += blockDim.x) x.c.pos[q] = make_float4(0, 0, 0, 0);
   if (threadIdx.x == 0) iscr[62] = 0;
   __syncthreads();
   for (;;) {

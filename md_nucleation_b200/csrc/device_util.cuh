@@ -70,7 +70,8 @@ __device__ __forceinline__ void rotation(double& X, double& Y, double& Z, double
 }
 
 /* fixed-point conversion of one term, saturated at +-2^21 kcal/mol/A so that a
- * few saturated terms still sum inside int64 (NaN converts to 0) */
+ * few saturated terms still sum inside int64 (a NaN counts as -2^21: fmax
+ * returns its other argument) */
 __device__ __forceinline__ long long fixd(double f) {
   return __double2ll_rn(fmin(fmax(f, -2097152.0), 2097152.0) * MDN_FIX_SCALE);
 }

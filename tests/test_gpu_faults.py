@@ -14,6 +14,7 @@ import numpy as np
 import pytest
 
 from md_nucleation_b200 import abi
+from md_nucleation_b200 import generate as g
 from tests import systems
 from tests.gpu_helpers import need_gpu
 
@@ -139,3 +140,47 @@ def test_slab_overflow_is_fatal_and_recoverable(eng):
     assert ex.value.code == abi.ERR_REPLICA
     assert e.status()[0] & abi.ST_SLAB_OVERFLOW
     relaunch_clean(e, clean)
+
+
+@pytest.mark.parametrize("gg", [False, True])
+@pytest.mark.parametrize("force_mode", [0, 1])
+def test_a_nonfinite_replica_leaves_the_others_alone(eng, gg, force_mode):
+    """More replicas than clusters (18 of 8 CTAs on 148 SMs): the 20 large
+    ones are stepped first, the small ones after them on the same CTAs.  With
+    a NaN in every large replica the small ones, whose cores fill no whole
+    block of 32 atoms, keep their bits."""
+    terms = g.BASE_TERMS | abi.I_AMBER | (abi.I_GG if gg else 0)
+
+    def spec(chain, n_vap, n_gas, seed):
+        return g.small_system(seed=seed, gas="He", vapor="water", ion="chain", chain_atoms=chain, n_gas=n_gas,
+                              n_vap=n_vap, box=245.0, interactions=terms, gas_min_dist=4.0 if gg else 0.0)
+
+    large, small = spec(45, 40, 600, 3), [spec(17, 4, 150, 4), spec(26, 0, 150, 5)]
+    specs = [large] * 20 + small * 20
+
+    def run(bad):
+        e = eng.Engine(specs, force_mode=force_mode)
+        e.set_launch(8, 512)
+        if bad:
+            s = e.state(0)
+            s.ion_x[0, 0] = np.nan
+            for r in range(20):
+                e.upload(r, s)
+        out = []
+        for call in (lambda: e.step(3, 0), lambda: e.step(3, 2), lambda: e.compute_forces()):
+            if bad:
+                e.clear_status()
+                with pytest.raises(eng.MdnError):
+                    call()
+                assert not e.status()[20:].any()
+            else:
+                call()
+            U = e.energies()
+            for r in range(20, len(specs)):
+                s = e.state(r)
+                out.append(np.concatenate([a.ravel() for a in (s.ion_x, s.ion_v, s.ion_f, s.gas_ax, s.gas_av,
+                                                               s.gas_af, s.vap_ax, s.vap_av, s.vap_af, U[r])]))
+        return out
+
+    for a, b in zip(run(False), run(True)):
+        assert np.array_equal(a, b)
