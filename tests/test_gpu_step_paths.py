@@ -62,6 +62,22 @@ def test_near_records_do_not_depend_on_the_launch(eng, gas, chain, n_gas, force_
     assert np.array_equal(a, b)
 
 
+# CTAs of one warp: fewer threads than build_near has bins
+@pytest.mark.parametrize("gas,chain,n_gas", [("He", 0, 800), ("Ar", 20, 3000), ("N2", 90, 2500)])
+@pytest.mark.parametrize("force_mode", [0, 1])
+@pytest.mark.parametrize("gg", [False, True])
+def test_one_warp_per_block(eng, gas, chain, n_gas, force_mode, gg):
+    spec = g.small_system(seed=6 + chain, gas=gas, vapor="methanol", ion="chain" if chain else "nacl",
+                          chain_atoms=chain, n_gas=n_gas, n_vap=12, box=245.0, shake_h=True,
+                          gas_min_dist=4.0 if gg else 0.0)
+    if gg:
+        spec.interactions |= abi.I_GG
+    spec.margin = 2.0  # rebuilds among the steps
+    a = _run(eng, spec, [(1, 512)] * 3, steps=40, force_mode=force_mode)
+    for c in (1, 8):
+        assert np.array_equal(a, _run(eng, spec, [(c, 32)] * 3, steps=40, force_mode=force_mode))
+
+
 # energies of every step and the thermostats, whose kicks and factors each
 # thread applies to its own components: one CTA, two that exchange their sums,
 # more that take slices of them
