@@ -3096,7 +3096,9 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     const bool fatal = (a.status[r] & MDN_ST_FATAL) != 0;
     const bool fits = sP.n_types <= a.nt_cap && sP.n_ion * sP.excl_words <= a.excl_cap &&
                       sP.n_ion + sD.n_vap_in * sP.a_v <= a.nc_cap;
-    if (fatal || !fits) {
+    /* the lists of an uploaded state are made even before its status is
+     * cleared: the near records and their counts have to be of that state */
+    if ((fatal && a.mode != MDN_MODE_RELIST) || !fits) {
       if (!fits && x.rank == 0 && threadIdx.x == 0) atomicOr(&a.status[r], MDN_ST_CORE_OVERFLOW);
       __syncthreads();
       continue;

@@ -142,6 +142,43 @@ def test_slab_overflow_is_fatal_and_recoverable(eng):
     relaunch_clean(e, clean)
 
 
+@pytest.mark.parametrize("cluster", [1, 8])
+def test_upload_before_the_status_is_cleared(eng, cluster):
+    """A clean state uploaded to a frozen replica gets its own lists, whichever
+    comes first, the upload or mdn_clear_status."""
+    spec = systems.make("nacl_n2_meoh")
+    e = eng.Engine([spec], quirks=abi.Q_ALL)
+    later = e.state(0)
+    packed = _pack_gas_near_ion(spec, later, 60)   # enter at the next rebuild
+    before = int(later.region.sum())
+    e.upload(0, later)
+    e.step(3)
+    later = e.state(0)
+    assert int(later.region.sum()) > before + packed // 2
+
+    def frozen():
+        f = eng.Engine([spec], quirks=abi.Q_ALL)
+        f.set_launch(cluster, 512)
+        bad = f.state(0)
+        bad.ion_x[0, 0] = np.nan
+        f.upload(0, bad)
+        with pytest.raises(eng.MdnError):
+            f.step(1)
+        return f
+
+    a, b = frozen(), frozen()
+    a.upload(0, later)
+    a.clear_status()
+    b.clear_status()
+    b.upload(0, later)
+    for kind in (0, 1):
+        assert len(b.pair_list(0, 0)) and np.array_equal(a.pair_list(0, kind), b.pair_list(0, kind))
+    for f in (a, b):
+        f.step(4)
+    for x, y in zip(vars(a.state(0)).values(), vars(b.state(0)).values()):
+        assert np.array_equal(x, y)
+
+
 @pytest.mark.parametrize("gg", [False, True])
 @pytest.mark.parametrize("force_mode", [0, 1])
 def test_a_nonfinite_replica_leaves_the_others_alone(eng, gg, force_mode):
