@@ -839,17 +839,21 @@ __device__ void shake_adjoint(const Sys& S, const Buf& B, const double* x, const
  * warp: lane 3 a + q holds component q of the unit's atom a */
 __device__ __forceinline__ double comp(double v, int a, int q) { return __shfl_sync(0xffffffffu, v, 3 * a + q); }
 
-/* A d = b for up to three unknowns (identity rows past n), Cramer's rule */
-__device__ __forceinline__ void solve3(const double (*A)[3], const double* b, double* d) {
+/* A d = b for up to three unknowns (identity rows past n), Cramer's rule;
+ * false when A is singular (a constraint given twice) */
+__device__ __forceinline__ bool solve3(const double (*A)[3], const double* b, double* d) {
   const double c00 = A[1][1] * A[2][2] - A[1][2] * A[2][1];
   const double c01 = A[1][0] * A[2][2] - A[1][2] * A[2][0];
   const double c02 = A[1][0] * A[2][1] - A[1][1] * A[2][0];
-  const double inv = 1.0 / (A[0][0] * c00 - A[0][1] * c01 + A[0][2] * c02);
+  const double det = A[0][0] * c00 - A[0][1] * c01 + A[0][2] * c02;
+  if (!(fabs(det) > 1e-300)) return false;
+  const double inv = 1.0 / det;
   const double e12 = b[1] * A[2][2] - A[1][2] * b[2], e11 = b[1] * A[2][1] - A[1][1] * b[2],
                e10 = A[1][0] * b[2] - b[1] * A[2][0];
   d[0] = (b[0] * c00 - A[0][1] * e12 + A[0][2] * e11) * inv;
   d[1] = (A[0][0] * e12 - b[0] * c01 + A[0][2] * e10) * inv;
   d[2] = (-A[0][0] * e11 - A[0][1] * e10 + b[0] * c02) * inv;
+  return true;
 }
 
 /* a unit's constraints in registers */
@@ -871,7 +875,9 @@ __device__ __forceinline__ double pick(const double* v, int q) { return q == 0 ?
 /* Newton's method on a unit's constraints: y (this lane's component, im its
  * atom's inverse mass) moves along the reference bond vectors of xr; gam: the
  * multipliers.  One step past the sweeps' criterion, (|s|^2 - d^2)^2 <= 1e-20
- * A^4, which brings the residuals to rounding; false after 50 steps. */
+ * A^4, which brings the residuals to rounding.  After 50 steps, or with a
+ * singular system, the sweeps from the start, as for larger groups (shake);
+ * false when they reach their cap. */
 __device__ __forceinline__ bool unit_shake(const UnitCons& U, const double* d2, double im, double& y, double xr,
                                            double* gam) {
   const int lane = threadIdx.x & 31, a = lane / 3, q = lane - 3 * a;
@@ -883,6 +889,7 @@ __device__ __forceinline__ bool unit_shake(const UnitCons& U, const double* d2, 
 #pragma unroll
     for (int c = 0; c < 3; c++) r[k][c] = comp(xr, U.ci[k], c) - comp(xr, U.cj[k], c);
   }
+  const double y0 = y;
   bool done = false;
   for (int it = 0; it < 50; it++) {
     double A[3][3] = {{1, 0, 0}, {0, 1, 0}, {0, 0, 1}}, b[3] = {0, 0, 0}, d[3];
@@ -901,7 +908,7 @@ __device__ __forceinline__ bool unit_shake(const UnitCons& U, const double* d2, 
     }
     if (ok && done) return true;
     done = ok;
-    solve3(A, b, d);
+    if (!solve3(A, b, d)) break;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
       if (k >= U.nc) continue;
@@ -910,6 +917,35 @@ __device__ __forceinline__ bool unit_shake(const UnitCons& U, const double* d2, 
       if (a == U.ci[k]) y += rq;
       if (a == U.cj[k]) y -= rq;
     }
+  }
+  y = y0;
+  gam[0] = gam[1] = gam[2] = 0;
+  for (int sweep = 0; sweep < SHAKE_SWEEPS; sweep++) {
+    bool ok = true;
+    for (int pass = 0; pass < 2; pass++) /* the sweep, then the residuals */
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        if (k >= U.nc) continue;
+        double s2 = 0, dot = 0;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const double s = comp(y, U.ci[k], c) - comp(y, U.cj[k], c);
+          s2 += s * s;
+          dot += s * r[k][c];
+        }
+        const double res = d2[k] - s2;
+        if (pass == 1) {
+          if (!(res * res <= 1e-20)) ok = false;
+          continue;
+        }
+        if (dot < 1e-10) dot = 1e-10;
+        const double g = res / (2 * U.cf[k][k] * dot);
+        gam[k] += g;
+        const double rq = g * pick(r[k], q) * im;
+        if (a == U.ci[k]) y += rq;
+        if (a == U.cj[k]) y -= rq;
+      }
+    if (ok) return true;
   }
   return false;
 }
@@ -941,7 +977,25 @@ __device__ __forceinline__ double unit_shake_adjoint(const UnitCons& U, double i
     for (int k = 0; k < 3; k++)
       if (k < U.nc) A[l][k] = (sk[k][0] * r[0] + sk[k][1] * r[1] + sk[k][2] * r[2]) * U.cf[k][l];
   }
-  solve3(A, rho, mu);
+  if (!solve3(A, rho, mu)) {
+    /* the sweeps of shake_adjoint */
+    mu[0] = mu[1] = mu[2] = 0;
+    bool ok = false;
+    for (int sweep = 0; sweep < SHAKE_SWEEPS && !ok; sweep++) {
+      ok = true;
+#pragma unroll
+      for (int l = 0; l < 3; l++) {
+        if (l >= U.nc) continue;
+        double acc = rho[l];
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+          if (k != l && k < U.nc) acc -= A[l][k] * mu[k];
+        const double nm = acc / A[l][l];
+        if (fabs(nm - mu[l]) > 1e-13 * (fabs(nm) + 1e-300)) ok = false;
+        mu[l] = nm;
+      }
+    }
+  }
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     if (k >= U.nc) continue;

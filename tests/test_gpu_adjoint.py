@@ -212,3 +212,34 @@ def test_adjoint_with_large_constraint_groups(eng, oracle_libs):
                        WINDOW["w_energy"], WINDOW["w_count"])
     assert abs(J - Jo) <= 1e-8 * max(abs(Jo), 1.0)
     check(grad, go, 1e-5)
+
+
+@pytest.mark.parametrize("place", [0, 1])
+def test_adjoint_with_a_constraint_given_twice(eng, oracle_libs, place):
+    """The O-H constraint of the methanol, or one C-H constraint beside
+    another, stands twice in the descriptor, once in the other direction: the
+    group's system is singular, the sweeps solve it, in the step and in both
+    directions of the harness.  Against the FP64 CPU adjoint, the bar of the
+    SHAKE case above."""
+    from md_nucleation_b200.gradients import parameters
+    spec = system(True)
+    v = spec.vapor
+    if place:
+        keep, twice = [r for r in v.rigid.tolist() if 0 in r[:2]][:2], 1
+    else:
+        keep, twice = [r for r in v.rigid.tolist() if 0 not in r[:2]], 0
+    moved = [r for r in v.rigid.tolist() if r not in keep]
+    v.bonds = np.array(v.bonds.tolist() + moved, np.int32).reshape(-1, 3)
+    i, j, t = keep[twice]
+    v.rigid = np.array(keep + [[j, i, t]], np.int32)
+    assert len(keep) == 1 + place
+    theta0, rows = parameters(spec)
+    e = eng.Engine([spec], force_mode=1)
+    assert e.info(0).n_vapor_in >= 3
+    J, grad, ms = e.adjoint(**WINDOW)
+    assert not e.status().any()
+    o = oracle_libs.OracleReplica(spec)
+    Jo, go = o.adjoint(WINDOW["n_steps"], theta0.numpy(), rows, WINDOW["count_radius"], WINDOW["count_width"],
+                       WINDOW["w_energy"], WINDOW["w_count"])
+    assert abs(J - Jo) <= 1e-8 * max(abs(Jo), 1.0)
+    check(grad, go, 1e-5)
