@@ -1252,21 +1252,29 @@ std::vector<ParamRow> param_rows(const mdn_replica_desc* d) {
   return rows;
 }
 
+/* device memory of the call, listed in owned; a failed allocation is a null
+ * there, and its error is not left for a later call to read */
+void* dalloc(size_t bytes, std::vector<void*>& owned) {
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    p = nullptr;
+  }
+  owned.push_back(p);
+  return p;
+}
+
 template <class T>
 T* dput(const std::vector<T>& v, std::vector<void*>& owned) {
-  T* p = nullptr;
-  if (cudaMalloc((void**)&p, sizeof(T) * std::max<size_t>(v.size(), 1)) != cudaSuccess) return nullptr;
-  owned.push_back(p);
-  if (!v.empty()) cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
+  T* const p = (T*)dalloc(sizeof(T) * std::max<size_t>(v.size(), 1), owned);
+  if (p && !v.empty()) cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
   return p;
 }
 
 template <class T>
 T* dzero(size_t n, std::vector<void*>& owned) {
-  T* p = nullptr;
-  if (cudaMalloc((void**)&p, sizeof(T) * std::max<size_t>(n, 1)) != cudaSuccess) return nullptr;
-  owned.push_back(p);
-  cudaMemset(p, 0, sizeof(T) * std::max<size_t>(n, 1));
+  T* const p = (T*)dalloc(sizeof(T) * std::max<size_t>(n, 1), owned);
+  if (p) cudaMemset(p, 0, sizeof(T) * std::max<size_t>(n, 1));
   return p;
 }
 
@@ -1717,10 +1725,6 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
       cleanup();
       return err(MDN_ERR_CUDA, "mdn_adjoint: device allocation failed");
     }
-  if (!Bf.X || !cpx) {
-    cleanup();
-    return err(MDN_ERR_CUDA, "mdn_adjoint: device allocation failed");
-  }
   /* ---- forward window on the engine, checkpoint at each segment start ---- */
   cudaStream_t stream = (cudaStream_t)sa.stream;
   float fwd_ms = 0;

@@ -243,3 +243,24 @@ def test_adjoint_with_a_constraint_given_twice(eng, oracle_libs, place):
                        WINDOW["w_energy"], WINDOW["w_count"])
     assert abs(J - Jo) <= 1e-8 * max(abs(Jo), 1.0)
     check(grad, go, 1e-5)
+
+
+def test_adjoint_that_does_not_fit_the_memory(eng):
+    """A segment length whose trajectory takes 45 % of the free memory and
+    whose weights' gradients, as large again, do not fit beside it: an error
+    before any launch, nothing left allocated, and the next calls work."""
+    import torch
+    spec = system(False)
+    e = eng.Engine([spec], force_mode=1)
+    n = len(e.in_domain(0)[0])
+    free = torch.cuda.mem_get_info()[0]
+    with pytest.raises(eng.MdnError, match="allocation"):
+        e.adjoint(n_steps=10, checkpoint_every=int(0.45 * free / (24 * n)))
+    assert torch.cuda.mem_get_info()[0] >= free - (64 << 20)
+    buf = eng.SnapshotBuffer(1, 2 * n)
+    assert e.snapshot(buf)[1] == n
+    J, grad, _ = e.adjoint(n_steps=10, checkpoint_every=5)
+    Jf, gf, _ = eng.Engine([spec], force_mode=1).adjoint(n_steps=10, checkpoint_every=5)
+    # the same window: apart by the order of FP64 sums
+    assert abs(J - Jf) <= 1e-12 * max(abs(Jf), 1.0)
+    assert np.abs(grad - gf).max() <= 1e-9 * np.abs(gf).max()
