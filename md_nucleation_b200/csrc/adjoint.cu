@@ -1725,6 +1725,12 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
       cleanup();
       return err(MDN_ERR_CUDA, "mdn_adjoint: device allocation failed");
     }
+  /* the uploads and clears above were queued on the default stream, which the
+   * handle's stream does not wait for */
+  if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) {
+    cleanup();
+    return err(MDN_ERR_CUDA, "mdn_adjoint: %s", cudaGetErrorString(cudaGetLastError()));
+  }
   /* ---- forward window on the engine, checkpoint at each segment start ---- */
   cudaStream_t stream = (cudaStream_t)sa.stream;
   float fwd_ms = 0;

@@ -414,6 +414,12 @@ struct Fetch {
   }
 };
 
+/* Waits for the default stream: a handle's stream does not wait for it by
+ * itself, and a memset, or a copy from pageable memory, may return before the
+ * device has done it.  After such a change to what the kernels read, before
+ * the next launch. */
+cudaError_t wait_default() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 int sync_check(mdn_handle* h) {
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return fail(MDN_ERR_CUDA, "kernel failed: %s", cudaGetErrorString(e));
@@ -1001,6 +1007,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
     ck(cudaMemcpy(h->mol_x, mx.data(), sizeof(double) * mx.size(), cudaMemcpyHostToDevice), "mol_x");
     ck(cudaMemcpy(h->mol_v, mv.data(), sizeof(double) * mv.size(), cudaMemcpyHostToDevice), "mol_v");
   }
+  ck(wait_default(), "uploads");
   if (rc != MDN_OK) {
     free_all(h);
     delete h;
@@ -1122,6 +1129,7 @@ int mdn_recenter(mdn_handle* h, int compat) {
       CK(cudaMemcpy(h->dD + r, &D, sizeof D, cudaMemcpyHostToDevice));
     }
   }
+  CK(wait_default());
   /* MD::run calls make_pair right after the shift, with the ion centre entry
    * as the shift left it */
   int rc;
@@ -1140,6 +1148,7 @@ int mdn_set_nvt(mdn_handle* h, int replica, int mode, double T) {
   }
   CK(cudaMemcpy(h->d_ctl_mode, h->ctl_mode.data(), sizeof(int) * h->R, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(h->d_ctl_T, h->ctl_T.data(), sizeof(double) * h->R, cudaMemcpyHostToDevice));
+  CK(wait_default());
   return MDN_OK;
 }
 
@@ -1173,6 +1182,7 @@ int mdn_get_status(mdn_handle* h, int* status) {
 int mdn_clear_status(mdn_handle* h) {
   if (!h) return fail(MDN_ERR_ARG, "bad arguments");
   CK(cudaMemset(h->status, 0, sizeof(int) * h->R));
+  CK(wait_default());
   return MDN_OK;
 }
 
@@ -1361,6 +1371,7 @@ int mdn_upload_state(mdn_handle* h, int r, const mdn_state* s) {
     D.ion_com[3 + k] = s->mol_v[k];
   }
   CK(cudaMemcpy(h->dD + r, &D, sizeof D, cudaMemcpyHostToDevice));
+  CK(wait_default());
   /* lists from the given centres (no classification) */
   std::vector<int> one(1, r);
   int rc;
@@ -1544,6 +1555,7 @@ int mdn_events(mdn_handle* h, mdn_event* ev, int capacity, int* count) {
   }
   *count = n;
   CK(cudaMemset(h->n_events, 0, sizeof(int)));
+  CK(wait_default());
   return MDN_OK;
 }
 
@@ -1609,6 +1621,7 @@ int mdn_profile(mdn_handle* h, int enable, long long* out) {
     CK(cudaMemcpy(out, h->d_prof, sizeof(long long) * MDN_PROF_N * h->R, cudaMemcpyDeviceToHost));
   }
   if (enable && !h->prof_on) CK(cudaMemset(h->d_prof, 0, sizeof(long long) * MDN_PROF_N * h->R));
+  CK(wait_default());
   h->prof_on = enable != 0;
   return MDN_OK;
 }
@@ -1635,6 +1648,7 @@ static int order_by_measured(mdn_handle* h, long long n_steps, int* status) {
     if ((rc = mdn_profile(h, 1, keep.data()))) return rc;
   }
   CK(cudaMemset(h->d_prof, 0, sizeof(long long) * MDN_PROF_N * h->R));
+  CK(wait_default());
   h->prof_on = true;
   rc = mdn_step(h, n_steps, 0);
   if (rc == MDN_ERR_REPLICA) *status = rc;
@@ -1648,6 +1662,7 @@ static int order_by_measured(mdn_handle* h, long long n_steps, int* status) {
   /* the accounting as it was */
   if (was_on) CK(cudaMemcpy(h->d_prof, keep.data(), sizeof(long long) * keep.size(), cudaMemcpyHostToDevice));
   else CK(cudaMemset(h->d_prof, 0, sizeof(long long) * MDN_PROF_N * h->R));
+  CK(wait_default());
   h->prof_on = was_on;
   return MDN_OK;
 }
