@@ -3094,6 +3094,11 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     x.ib = a.iblob + sP.iblob_off;
     x.db = a.dblob + sP.dblob_off;
     const bool fatal = (a.status[r] & MDN_ST_FATAL) != 0;
+    /* the CTAs of the cluster have to agree on it, or some would wait for ones
+     * that skipped the replica: no CTA goes on to where it could set the status
+     * before all have read it (the wait stands behind the loads) */
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     const bool fits = sP.n_types <= a.nt_cap && sP.n_ion * sP.excl_words <= a.excl_cap &&
                       sP.n_ion + sD.n_vap_in * sP.a_v <= a.nc_cap;
     /* the lists of an uploaded state are made even before its status is
@@ -3101,6 +3106,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
     if ((fatal && a.mode != MDN_MODE_RELIST) || !fits) {
       if (!fits && x.rank == 0 && threadIdx.x == 0) atomicOr(&a.status[r], MDN_ST_CORE_OVERFLOW);
       __syncthreads();
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
       continue;
     }
     /* tables */
@@ -3119,6 +3125,7 @@ extern "C" __global__ void __launch_bounds__(512, 1) MDN_ADVANCE_KERNEL(KArgs a)
       iscr[threadIdx.x < 2 ? 56 + threadIdx.x : 61] = a.near_cnt[3 * ((size_t)r * 8 + x.rank) + threadIdx.x];
     if (threadIdx.x < MDN_PROF_N) s_prof[threadIdx.x] = 0;
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const long long job_t0 = clock64();
     if ((a.mode == MDN_MODE_STEP || a.mode == MDN_MODE_FORCES) && sD.near_C != x.C) build_near(x, cl);
     {

@@ -179,6 +179,31 @@ def test_upload_before_the_status_is_cleared(eng, cluster):
         assert np.array_equal(x, y)
 
 
+@pytest.mark.parametrize("cluster", [2, 8])
+def test_nonfinite_gas_is_noticed_by_one_cta(eng, cluster):
+    """A NaN in one gas molecule: the CTA that steps it sets the status in its
+    first drift, while the others of the cluster start on the replica.  All
+    of them step it, as the step count shows, and all skip it from then on."""
+    spec = systems.make("nacl_n2_meoh")
+    e = eng.Engine([spec] * 12)
+    e.set_launch(cluster, 512)
+    clean = e.state(0)
+    bad = clean.copy()
+    gin = np.nonzero(bad.region[1:1 + spec.n_gas])[0]
+    bad.gas_ax[gin[0], 0, 0] = np.nan
+    for _ in range(10):
+        for r in range(12):
+            e.upload(r, bad if r % 2 else clean)
+        before = [e.info(r).step for r in range(12)]
+        for _ in range(2):
+            with pytest.raises(eng.MdnError):
+                e.step(1)
+        st = e.status()
+        assert all(st[1::2] & abi.ST_NONFINITE) and not st[::2].any()
+        assert [e.info(r).step - before[r] for r in range(12)] == [2, 1] * 6
+        e.clear_status()
+
+
 @pytest.mark.parametrize("gg", [False, True])
 @pytest.mark.parametrize("force_mode", [0, 1])
 def test_a_nonfinite_replica_leaves_the_others_alone(eng, gg, force_mode):
