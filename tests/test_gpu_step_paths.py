@@ -6,6 +6,7 @@ import pytest
 
 from md_nucleation_b200 import abi
 from md_nucleation_b200 import generate as g
+from md_nucleation_b200.system import QQRD2E
 from tests.gpu_helpers import FORCE_ATOL, forces_of, need_gpu, rel_rms
 
 pytestmark = pytest.mark.gpu
@@ -36,6 +37,78 @@ def test_core_tile_edges(eng, oracle_libs, chain, n_vap):
         a, b = forces_of(e.state(0), spec), forces_of(o.get_state(), spec)
         assert rel_rms(a, b) <= 1e-9 or np.sqrt(np.mean((a - b) ** 2)) <= FORCE_ATOL, term
         assert np.abs(e.energies()[0] - Uo).max() <= 1e-4 * max(np.abs(Uo).max(), 1e-6)
+
+
+def _pair_bound(spec, st, term):
+    """What FP32 pair terms may be off by, per atom and component, on top of a
+    sum of FP64 pairs: u = 2^-24.  A pair's factor is a product of some 20
+    operations and a reciprocal root of 3 u that enters 14 times, summed over
+    at most 32 steps: 100 u of its terms.  Coordinates relative to the ion
+    centre are rounded to u of their size, which changes the force by the
+    displacement times (15, 9, 4) of the repulsive, dispersion and Coulomb
+    factor (their derivatives, and the factor itself)."""
+    vin = st.region[1 + spec.n_gas:].astype(bool)
+    ni, av, nv = spec.ion.n, spec.vapor.n, int(vin.sum())
+    x = np.concatenate([st.ion_x.reshape(-1, 3), st.vap_ax[vin].reshape(-1, 3)])
+    t = np.concatenate([spec.ion.type, np.tile(spec.vapor.type, nv)])
+    q = np.concatenate([spec.ion.charge, np.tile(spec.vapor.charge, nv)])
+    w = np.concatenate([np.ones(ni), st.vap_w[vin].reshape(-1)])
+    mol = np.concatenate([np.full(ni, -1), np.repeat(np.arange(nv), av)])
+    ion = mol < 0
+    if term == abi.I_AMBER:
+        on = ion[:, None] & ion[None]
+        np.fill_diagonal(on, False)
+        for rows, k in ((spec.ion.bonds, 1), (spec.ion.rigid, 1), (spec.ion.angles, 2), (spec.ion.dihedrals, 3)):
+            on[rows[:, 0], rows[:, k]] = on[rows[:, k], rows[:, 0]] = False
+    elif term == abi.I_VI:
+        on = ion[:, None] != ion[None]
+    else:
+        on = ~ion[:, None] & ~ion[None] & (mol[:, None] != mol[None])
+    r = np.linalg.norm(x[:, None] - x[None], axis=2)
+    r[~on] = 1.0
+    eps = np.sqrt(spec.atom_eps[t][:, None] * spec.atom_eps[t][None])
+    sig = 0.5 * (spec.atom_sigma[t][:, None] + spec.atom_sigma[t][None])
+    ww = np.where(on, w[:, None] * w[None], 0.0)
+    a, b = 48 * eps * sig ** 12 * r ** -14 * ww, 24 * eps * sig ** 6 * r ** -8 * ww
+    c = np.abs(QQRD2E * q[:, None] * q[None]) * r ** -3 * ww
+    com = np.average(x[:ni], axis=0, weights=spec.atom_mass[t[:ni]])
+    far = np.linalg.norm(x - com, axis=1)
+    u = 2.0 ** -24
+    return u * (100 * (a + b + c) * r + (15 * a + 9 * b + 4 * c) * (far[:, None] + far[None])).sum(axis=1)
+
+
+# The FP32 tile has loads, masks and packed arithmetic of its own: the same
+# edges term by term, in the kernels with and without gas-gas terms, and the
+# steps without energies (four pairs at once) against those with (two)
+@pytest.mark.parametrize("gg", [False, True])
+@pytest.mark.parametrize("n_vap", [0, 25])
+@pytest.mark.parametrize("chain", [31, 32, 33, 64, 65])
+def test_core_tile_edges_fp32(eng, oracle_libs, chain, n_vap, gg):
+    spec = g.small_system(seed=chain, gas="He", vapor="water", ion="chain", chain_atoms=chain, n_gas=300,
+                          n_vap=n_vap, box=242.0, gas_min_dist=4.0 if gg else 0.0)
+    if gg:
+        spec.interactions |= abi.I_GG
+    o = oracle_libs.OracleReplica(spec)
+    o.step(3)
+    start = o.get_state()
+    e = eng.Engine([spec])
+    e.upload(0, start)
+    gas = int(start.region[1:1 + spec.n_gas].sum()) * spec.gas.n
+    for term in (abi.I_AMBER, abi.I_VI, abi.I_VV):
+        e.compute_forces(term)
+        o.compute_forces(term)
+        a, b = forces_of(e.state(0), spec), forces_of(o.get_state(), spec)
+        bound = np.insert(_pair_bound(spec, start, term), [spec.ion.n] * gas, 0.0)
+        # and the fixed-point terms' rounding, the bonded terms' FP64
+        err = np.abs(a - b).max(axis=1)
+        assert (err <= bound + 1e-9 + 1e-11 * np.abs(b).max()).all(), (term, np.max(err - bound))
+    out = []
+    for mode in (0, 2):
+        e.upload(0, start)
+        e.step(3, mode)
+        out.append(e.state(0))
+    for x, y in zip(vars(out[0]).values(), vars(out[1]).values()):
+        assert np.array_equal(x, y)
 
 
 def _run(eng, spec, shapes, steps=12, **kw):
