@@ -264,3 +264,26 @@ def test_adjoint_that_does_not_fit_the_memory(eng):
     # the same window: apart by the order of FP64 sums
     assert abs(J - Jf) <= 1e-12 * max(abs(Jf), 1.0)
     assert np.abs(grad - gf).max() <= 1e-9 * np.abs(gf).max()
+
+
+# more atoms than the reverse sweep stages in shared memory (4,266), and more
+# than the recompute's weights have room for there (25,600)
+@pytest.mark.parametrize("n_gas,shake,n_atoms", [(5000, False, 4267), (5000, True, 4267), (27000, False, 25601)])
+def test_adjoint_of_a_large_domain(eng, oracle_libs, n_gas, shake, n_atoms):
+    """A few steps from a stepped state, in segments of two, against the FP64
+    CPU adjoint: the bars of test_adjoint_matches_the_cpu_adjoint."""
+    from md_nucleation_b200.gradients import parameters
+    spec = g.small_system(seed=37, gas="N2", vapor="methanol", ion="nacl", n_gas=n_gas, n_vap=40, box=220.0,
+                          shake_h=shake, rigid_gas=shake)
+    theta0, rows = parameters(spec)
+    e = eng.Engine([spec], force_mode=1)
+    e.step(2)
+    assert len(e.in_domain(0)[0]) >= n_atoms
+    o = oracle_libs.OracleReplica(spec)
+    o.step(2)  # and not set_state, which leaves the oracle at step 0, where the start forces have no parameters
+    w = dict(WINDOW, n_steps=5, checkpoint_every=2)
+    J, grad, _ = e.adjoint(**w)
+    Jc, gc = o.adjoint(w["n_steps"], theta0.numpy(), rows, w["count_radius"], w["count_width"], w["w_energy"],
+                       w["w_count"])
+    assert abs(J - Jc) <= 1e-9 * max(abs(Jc), 1.0)
+    check(grad, gc, 1e-5 if shake else 1e-6, floor=1e-4)
