@@ -859,12 +859,12 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
    * a block that it keeps while one of them lives, and mdn_place, which makes
    * and frees one, took 1.8 ms beside a handle without it, 1.2 with it */
   struct Pool {
-    char** at;
+    void* at; /* the pool's pointer, of any type */
     size_t bytes;
   };
   std::vector<Pool> pools;
   auto pool = [&](auto*& p, size_t count) {
-    pools.push_back({(char**)(void*)&p, (sizeof(*p) * std::max<size_t>(1, count) + 255) & ~(size_t)255});
+    pools.push_back({&p, (sizeof(*p) * std::max<size_t>(1, count) + 255) & ~(size_t)255});
   };
   pool(h->dP, R);
   pool(h->dD, R);
@@ -923,7 +923,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
     char** const to[2] = {&h->arena, &h->arena_small};
     for (int k = 0; k < 2; k++) {
       if (bytes[k] == 0) continue;
-      cudaError_t e = cudaMalloc((void**)to[k], bytes[k]);
+      cudaError_t e = cudaMalloc(to[k], bytes[k]);
       if (e != cudaSuccess) {
         *to[k] = nullptr;
         free_all(h);
@@ -933,7 +933,7 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
       char* at = *to[k];
       for (const Pool& q : pools)
         if (small(q) == (k == 1)) {
-          *q.at = at;
+          memcpy(q.at, &at, sizeof at);
           at += q.bytes;
         }
     }
