@@ -222,7 +222,6 @@ struct Sys {
   const double* mass;    /* [N] */
   const double* c;       /* [N] kick coefficient 0.5 dt 4.184e-4 / m */
   const unsigned char* vapor; /* [N] 1 for vapor atoms (taper weights) */
-  int n_pairs;
   const double* A;       /* [nt*nt] */
   const double* B;
   const double* ieps;    /* [nt*nt] 1 / pair eps, 1 / pair sigma (for the derivatives) */
@@ -269,8 +268,8 @@ struct Sys {
 
 struct Buf {
   double* X;     /* [(K+1)*3N] positions of the segment */
-  double* V;     /* [(K+1)*3N] */
-  double* F;     /* [(K+1)*3N] */
+  double* V;     /* [3N] velocities and forces of the segment's current step */
+  double* F;     /* [3N] (the recompute alone uses them) */
   double* gam;   /* [K*n_cons] converged SHAKE multipliers of each step */
   double* lx;    /* [3N] adjoint of x, carried across segments */
   double* lv;    /* [3N] adjoint of v */
@@ -342,7 +341,6 @@ __device__ void block_sum3(double* v, double* red) {
   __syncthreads();
 }
 
-/* x, v, f, ... that other CTAs write are read from L2 */
 /* this warp among the cluster's, the CTAs in turn */
 __device__ __forceinline__ int cwarp() {
   return (int)((threadIdx.x >> 5) * cg::this_cluster().num_blocks() + cg::this_cluster().block_rank());
@@ -427,7 +425,7 @@ __device__ double place_terms(const Sys& S, const Buf& B, const double* x, int t
  * of f (d eps, d sigma, d s at s = 1) */
 struct PairEval {
   double f, fp, fe, fs_sig, fq;
-  double ui, a7, b4; /* 1 / u, the two LJ terms of f */
+  double a7, b4; /* the two LJ terms of f */
   int p;  /* parameter base, -1 */
 };
 
@@ -474,7 +472,6 @@ __device__ __forceinline__ PairEval eval_pair(const Sys& S, int i, int j, int ki
   }
   o.f = f;
   o.fp = fp;
-  o.ui = ui;
   return o;
 }
 
@@ -1511,8 +1508,9 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
   S.mass = dput(mass, owned);
   S.c = dput(cc, owned);
   S.vapor = dput(isvap, owned);
-  /* pairs grouped by kind and type pair, so that a thread's strided run of
-   * pairs stays on one parameter row (ParamSums) */
+  /* pairs grouped by kind and type pair: an atom's row takes them in this
+   * order, so that the 32 pairs a warp has at a time are of few parameter rows
+   * (vjp_rows adds a row's 32 terms up at once) */
   {
     std::vector<size_t> ord(pi.size());
     for (size_t k = 0; k < ord.size(); k++) ord[k] = k;
@@ -1529,7 +1527,6 @@ extern "C" int mdn_adjoint(mdn_handle* h, const mdn_replica_desc* d, const mdn_a
     pj.swap(pj2);
     pk.swap(pk2);
   }
-  S.n_pairs = (int)pi.size();
   /* the pairs by atom, from both sides, in the sorted order (so that a
    * warp's lanes stay on few parameter rows).  One side is primary, the ion
    * atom's where there is one, the lower index in an ion-ion pair. */

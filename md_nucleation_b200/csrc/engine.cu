@@ -159,7 +159,6 @@ struct mdn_handle {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<RepParams> P;
   std::vector<RepDyn> D0;
-  std::vector<std::vector<int>> type_names;  /* unused placeholder */
   int nc_cap = 0, nt_cap = 0, excl_cap = 0;
   size_t smem = 0;
   /* device pools, cut from two allocations: the large ones, the small ones */
@@ -846,9 +845,10 @@ int mdn_create(const mdn_replica_desc* descs, int R, const mdn_options* opt_in, 
     /* a small replica is a chain of latencies that more CTAs do not shorten,
      * and the cluster's barriers lengthen: lone replicas of 332 and 538 units
      * take 10.4 and 11.3 us per step on one CTA against 11.7 and 12.7 on
-     * eight.  Up to 3,000 units steps still gain (1,225: 13.4 against 15.1),
-     * but a force evaluation alone, with its FP64 energies, loses (1,019: 4 of
-     * 62 us), and both need the same near records. */
+     * eight.  The line lies below what a force evaluation alone, with its FP64
+     * energies, loses on one CTA (1,019 units: 4 of 62 us), since the near
+     * records are of one size for both; steps alone would gain up to 3,000
+     * units (1,225: 13.4 us against 15.1), which mdn_tune_launch finds. */
     if (wmax < 700) c = 1;
     h->auto_cluster = c;
   }

@@ -166,7 +166,6 @@ typedef struct KArgs {
   int nc_cap;              /* core atoms the shared memory holds               */
   int nt_cap;              /* atom types the shared memory holds               */
   int excl_cap;            /* exclusion words the shared memory holds          */
-  int colors_cap;
 } KArgs;
 
 /* A handle's device arrays that the snapshot kernels read (filled by
