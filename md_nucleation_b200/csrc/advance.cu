@@ -1828,7 +1828,7 @@ __device__ __forceinline__ void build_near(Ctx& x, cg::cluster_group& cl) {
   int* const cur = x.cand + 64;    /* [kNearBins] next record                              */
   int* const heavy = x.cand + 128; /* partners of all heavy molecules, and the next one    */
   __syncthreads();
-  for (int b = threadIdx.x; b < kNearBins; b += blockDim.x) hist[b] = 0;
+  if (threadIdx.x < kNearBins / 2) hist[threadIdx.x] = hist[kNearBins / 2 + threadIdx.x] = 0; /* a block may be one warp */
   if (threadIdx.x < 2) heavy[threadIdx.x] = 0;
   __syncthreads();
   auto items_of = [&](size_t ms) {
