@@ -6,8 +6,9 @@
  * Forward: the engine advances the window (FP32 pair terms, FP64
  * integration) and the replica's in-domain atoms are gathered every K steps
  * (checkpoints).  Backward: every segment is recomputed in FP64 from its
- * checkpoint at once, one cluster each, keeping x_t, v_t, F_t, the taper
- * weights and the SHAKE multipliers of each step; then one cluster runs, last
+ * checkpoint at once, one cluster each, keeping x_t, the taper weights with
+ * their gradients, the count term's derivatives and the SHAKE multipliers of
+ * each step; then one cluster runs, last
  * segment first, the adjoint of
  *   (1) v_a = v + c F          (2) y = x + dt v_a          (3) x' = SHAKE(y; x)
  *   (4) v_b = v_a + (x' - y)/dt (5) F' = F(x'; theta)      (6) v' = v_b + c F'

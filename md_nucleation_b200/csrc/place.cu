@@ -88,8 +88,9 @@ struct IonSphere {
 /* candidates k0 .. k0+K-1: bits bit 0 = clear of every ion atom, bit 1 =
  * clear of the origin; *first = the smallest local index with bit 0 set.
  * Only candidates inside the ion's sphere are tested against its atoms:
- * 1,254,096 candidates against 500 atoms take 1.01 ms (the FP64 pipe 74 %
- * busy), while in a dilute box all but a few hundred lie outside. */
+ * 1,254,096 candidates against 500 atoms took 1.01 ms (the FP64 pipe 74 %
+ * busy), and take 80 us where, in a dilute box, all but a few hundred lie
+ * outside: mostly the random draws. */
 __global__ void __launch_bounds__(kTestThreads) place_test(const double* ion_x, int n_ion, IonSphere S, double L,
                                                             double dis, unsigned long long seed, uint32_t purpose,
                                                             long long k0, int K, unsigned char* bits, int* first) {
